@@ -26,6 +26,8 @@
 
 #include "common.cuh"
 #include "prims.cuh"
+#include "sweep.cuh"
+#include "team.cuh"
 
 namespace kb {
 
@@ -77,77 +79,92 @@ __device__ __forceinline__ void candidate(const JetArgs& A, int v, int own, long
     }
 }
 
-__global__ void __launch_bounds__(kThreads) jet_choose(JetArgs A) {
-    unsigned long long cut = 0;
-    for (long long v0 = (long long)blockIdx.x * kThreads + threadIdx.x; v0 < A.n; v0 += (long long)gridDim.x * kThreads) {
-        const int v = (int)v0;
-        A.dest[v] = -1;
-        const bool locked = A.moved_at[v] == A.it - 1;
-        const int beg = A.xadj[v], end = A.xadj[v + 1];
-        if (end - beg > kLaneRow) {
-            A.wide[atomicAdd(A.nwide, 1u)] = locked ? (v | kLocked) : v;
-            continue;
-        }
-        const int own = A.part[v];
-        if (locked) {
-            for (int e = beg; e < end; ++e)
-                if (A.part[A.adjncy[e]] != own) cut += (uint32_t)A.adjwgt[e];
-            continue;
-        }
-        uint32_t sl[kSlots], sc[kSlots];
+// The most connected other block of v and the cut of its row: candidate set
+// or row deferred to choose_wide (whose scan then sums its cut).  Four
+// entries are loaded together.  UNIT: every edge weight is 1 (adjwgt is not
+// read).
+template <bool UNIT>
+__device__ __forceinline__ void choose_one(const JetArgs& A, int v, unsigned long long& cut) {
+    A.dest[v] = -1;
+    const bool locked = A.moved_at[v] == A.it - 1;
+    const int beg = A.xadj[v], end = A.xadj[v + 1];
+    if (end - beg > kLaneRow) {
+        A.wide[atomicAdd(A.nwide, 1u)] = locked ? (v | kLocked) : v;
+        return;
+    }
+    const int own = A.part[v];
+    uint32_t sl[kSlots], sc[kSlots];
 #pragma unroll
-        for (int i = 0; i < kSlots; ++i) { sl[i] = kNone; sc[i] = 0; }
-        long long co = 0;
-        unsigned long long other = 0;
-        bool overflow = false;
-        for (int e = beg; e < end && !overflow; ++e) {
-            const uint32_t b = (uint32_t)A.part[A.adjncy[e]];
-            const uint32_t w = (uint32_t)A.adjwgt[e];
-            if ((int)b == own) { co += w; continue; }
-            other += w;
+    for (int i = 0; i < kSlots; ++i) { sl[i] = kNone; sc[i] = 0; }
+    long long co = 0;
+    unsigned long long other = 0;
+    bool overflow = false;
+    for (int e = beg; e < end && !overflow; e += 4) {
+        uint32_t b[4], w[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const bool in = e + t < end;
+            b[t] = in ? (uint32_t)A.adjncy[e + t] : kNone;
+            w[t] = in ? (UNIT ? 1u : (uint32_t)A.adjwgt[e + t]) : 0u;
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            if (b[t] != kNone) b[t] = (uint32_t)A.part[b[t]];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            if (b[t] == kNone) continue;
+            if ((int)b[t] == own) { co += w[t]; continue; }
+            other += w[t];
+            if (locked) continue;
             bool hit = false;
 #pragma unroll
             for (int i = 0; i < kSlots; ++i) {
-                const bool m = sl[i] == b;
-                sc[i] += m ? w : 0u;
+                const bool m = sl[i] == b[t];
+                sc[i] += m ? w[t] : 0u;
                 hit |= m;
             }
             if (!hit) {
                 overflow |= sl[kSlots - 1] != kNone;
 #pragma unroll
                 for (int i = kSlots - 1; i > 0; --i) { sl[i] = sl[i - 1]; sc[i] = sc[i - 1]; }
-                sl[0] = b;
-                sc[0] = w;
+                sl[0] = b[t];
+                sc[0] = w[t];
             }
         }
-        if (overflow) {
-            // the row is scanned again, and its cut summed, by jet_choose_wide
-            A.wide[atomicAdd(A.nwide, 1u)] = v;
-            continue;
-        }
-        cut += other;
-        uint32_t d = kNone, dc = 0;
-#pragma unroll
-        for (int i = 0; i < kSlots; ++i)
-            if (sl[i] != kNone && sc[i] > 0 && (d == kNone || beats(sc[i], sl[i], dc, d, A.ks_tie))) {
-                d = sl[i];
-                dc = sc[i];
-            }
-        candidate(A, v, own, co, d, dc);
     }
+    if (overflow) {
+        A.wide[atomicAdd(A.nwide, 1u)] = v;
+        return;
+    }
+    cut += other;
+    if (locked) return;
+    uint32_t d = kNone, dc = 0;
+#pragma unroll
+    for (int i = 0; i < kSlots; ++i)
+        if (sl[i] != kNone && sc[i] > 0 && (d == kNone || beats(sc[i], sl[i], dc, d, A.ks_tie))) {
+            d = sl[i];
+            dc = sc[i];
+        }
+    candidate(A, v, own, co, d, dc);
+}
+
+template <bool UNIT>
+__global__ void __launch_bounds__(kThreads) jet_choose(JetArgs A) {
+    unsigned long long cut = 0;
+    for (long long v = (long long)blockIdx.x * kThreads + threadIdx.x; v < A.n; v += (long long)gridDim.x * kThreads)
+        choose_one<UNIT>(A, (int)v, cut);
     add_cut(A, cut);
 }
 
 // Block per listed vertex; cnt = this block's k counters (zero between
 // vertices: every touched counter is read and cleared).
-__global__ void __launch_bounds__(kThreads) jet_choose_wide(JetArgs A, uint32_t* counters) {
+__device__ __forceinline__ void choose_wide(const JetArgs& A, uint32_t* cnt, unsigned blocks) {
     __shared__ uint64_t sk[kThreads / 32];
     __shared__ uint32_t sb[kThreads / 32];
-    uint32_t* cnt = counters + (size_t)blockIdx.x * A.k;
     const unsigned count = *A.nwide;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     unsigned long long cut = 0;
-    for (unsigned i = blockIdx.x; i < count; i += gridDim.x) {
+    for (unsigned i = blockIdx.x; i < count; i += blocks) {
         const int raw = A.wide[i];
         const int v = raw & ~kLocked;
         const int beg = A.xadj[v], end = A.xadj[v + 1];
@@ -201,6 +218,11 @@ __global__ void __launch_bounds__(kThreads) jet_choose_wide(JetArgs A, uint32_t*
     add_cut(A, cut);
 }
 
+__global__ void __launch_bounds__(kThreads) jet_choose_wide(JetArgs A, uint32_t* counters) {
+    choose_wide(A, counters + (size_t)blockIdx.x * A.k, gridDim.x);
+}
+
+template <bool UNIT>
 __device__ __forceinline__ long long afterburn_sum(const JetArgs& A, int v, int beg, int end, int step, int first) {
     const int dv = A.dest[v], pv = A.part[v];
     const long long gv = A.gain[v];
@@ -213,12 +235,13 @@ __device__ __forceinline__ long long afterburn_sum(const JetArgs& A, int v, int 
             const long long gu = A.gain[u];
             if (gu > gv || (gu == gv && u < v)) bu = du;
         }
-        if (bu == dv) adj += A.adjwgt[e];
-        else if (bu == pv) adj -= A.adjwgt[e];
+        if (bu == dv) adj += UNIT ? 1 : A.adjwgt[e];
+        else if (bu == pv) adj -= UNIT ? 1 : A.adjwgt[e];
     }
     return adj;
 }
 
+template <bool UNIT>
 __global__ void __launch_bounds__(kThreads) jet_afterburn(JetArgs A, uint8_t* keep, const int* stop) {
     if (*stop) return;  // the loop ended at this iteration's evaluation
     const int lane = threadIdx.x & 31;
@@ -235,12 +258,12 @@ __global__ void __launch_bounds__(kThreads) jet_afterburn(JetArgs A, uint8_t* ke
             wm &= wm - 1;
             const int hv = __shfl_sync(0xffffffffu, v, s);
             const int hb = __shfl_sync(0xffffffffu, beg, s), he = __shfl_sync(0xffffffffu, end, s);
-            long long adj = afterburn_sum(A, hv, hb, he, 32, lane);
+            long long adj = afterburn_sum<UNIT>(A, hv, hb, he, 32, lane);
 #pragma unroll
             for (int off = 16; off; off >>= 1) adj += __shfl_xor_sync(0xffffffffu, adj, off);
             if (lane == s) keep[hv] = adj >= 0 ? 1 : 0;
         }
-        if (cand && !wide) keep[v] = afterburn_sum(A, v, beg, end, 1, 0) >= 0 ? 1 : 0;
+        if (cand && !wide) keep[v] = afterburn_sum<UNIT>(A, v, beg, end, 1, 0) >= 0 ? 1 : 0;
     }
 }
 
@@ -320,6 +343,161 @@ __global__ void jet_restore(const JetCtl* c, int n, int k, int* part, uint32_t* 
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < k; b += gridDim.x * blockDim.x) bw[b] = best_bw[b];
 }
 
+// All iterations of one level in one kernel (team.cuh): a host-driven
+// iteration is ten launches and a synchronisation, 80-90 us however small
+// the level, of which its steps need a few.  Two partition buffers alternate,
+// so that the afterburner writes the moved state beside the one it reads and
+// an iteration without balance repair is two steps; block weights are judged
+// on a copy taken while they are at rest.
+struct JetLoop {
+    JetArgs A;
+    int* part;        // in/out
+    int* part2;       // n
+    int* best;        // n
+    uint32_t *bw, *bw2, *best_bw;
+    const int* vwgt;
+    int* moved_at;
+    uint32_t* counters;       // [blocks][k], zero
+    int wblocks;              // blocks with a row of counters
+    unsigned* ring;           // [0..1] wide rows, [2..3] moves, by the iteration's parity
+    unsigned long long* cut;  // [0..1] twice the cut
+    int iters, patience, seed, level;
+    uint32_t bound;
+};
+
+template <bool UNIT>
+__global__ void __launch_bounds__(kThreads, 4) jet_loop(JetLoop J, sweep::SweepArgs a, sweep::BalanceArgs B,
+                                                        TeamArgs T) {
+    __shared__ sweep::SweepSmem sm;
+    __shared__ sweep::WeighSmem ws;
+    Team team(T);
+    const int n = J.A.n, k = J.A.k;
+    const int lane = threadIdx.x & 31;
+    sweep::balance_clear(team, a, B);
+    for (long long v = team.rank(); v < n; v += team.size()) J.moved_at[v] = -2;
+    if (blockIdx.x == 0) {
+        for (int i = threadIdx.x; i < 2 * sweep::kTeamSet; i += kThreads) B.counters[i] = 0;
+        if (threadIdx.x < 4) J.ring[threadIdx.x] = 0;
+        if (threadIdx.x < 2) J.cut[threadIdx.x] = 0;
+    }
+    if ((int)blockIdx.x < J.wblocks)
+        for (int b = threadIdx.x; b < k; b += kThreads) J.counters[(size_t)blockIdx.x * k + b] = 0;
+    bool alive = team.sync();
+    int* cur = J.part;
+    int* nxt = J.part2;
+    unsigned long long best_ov = 0;
+    long long best_cut = 0;
+    int since = 0, p = 0;
+    bool part_is_best = false;
+    for (int it = 0; alive; ++it) {
+        JetArgs A = J.A;
+        A.it = it;
+        A.part = cur;
+        A.ks_tie = stream_key(J.seed, TAG_JTIE, J.level, it);
+        A.nwide = J.ring + (it & 1);
+        A.cut2 = J.cut + (it & 1);
+        // candidates, the cut of the current state and a copy of its weights
+        if (blockIdx.x == 0) {
+            if (threadIdx.x == 0) J.ring[2 + (it & 1)] = 0;
+            for (int b = threadIdx.x; b < k; b += kThreads) J.bw2[b] = J.bw[b];
+        }
+        unsigned long long cut = 0;
+        if (it < J.iters) {
+            for (long long v = team.rank(); v < n; v += team.size()) choose_one<UNIT>(A, (int)v, cut);
+        } else {
+            for (long long v = team.rank(); v < n; v += team.size()) {
+                const int own = cur[v];
+                for (int e = A.xadj[v]; e < A.xadj[v + 1]; ++e)
+                    if (cur[A.adjncy[e]] != own) cut += UNIT ? 1u : (uint32_t)A.adjwgt[e];
+            }
+        }
+        __syncwarp();
+        add_cut(A, cut);
+        if (!(alive = team.sync())) break;
+        if (*A.nwide) {
+            if ((int)blockIdx.x < J.wblocks) choose_wide(A, J.counters + (size_t)blockIdx.x * k, J.wblocks);
+            if (!(alive = team.sync())) break;
+        }
+        // best tracking and the stopping rule (jet_track), by every block
+        {
+            const unsigned long long ov = sweep::weigh(J.bw2, k, J.bound, ws).overload;
+            const long long c = (long long)(*A.cut2 / 2);
+            if (it == 0 || ov < best_ov || (ov == best_ov && c < best_cut)) {
+                best_ov = ov;
+                best_cut = c;
+                part_is_best = true;
+                since = 0;
+            } else {
+                part_is_best = false;
+                ++since;
+            }
+        }
+        if ((it > 0 && (J.ring[2 + ((it - 1) & 1)] == 0 || since >= J.patience)) || it == J.iters) break;
+        // the best state is saved, then the afterburner and its moves into
+        // the other buffer
+        if (blockIdx.x == 0) {
+            if (threadIdx.x == 0) {
+                J.ring[(it + 1) & 1] = 0;
+                J.cut[(it + 1) & 1] = 0;
+            }
+            if (part_is_best)
+                for (int b = threadIdx.x; b < k; b += kThreads) J.best_bw[b] = J.bw2[b];
+        }
+        unsigned moves = 0;
+        for (long long base = (long long)blockIdx.x * kThreads; base < n; base += team.size()) {
+            const int v = (int)(base + threadIdx.x);
+            const bool in = v < n;
+            const int own = in ? cur[v] : 0;
+            const int d = in ? A.dest[v] : -1;
+            int beg = 0, end = 0;
+            if (d >= 0) { beg = A.xadj[v]; end = A.xadj[v + 1]; }
+            const bool wide = end - beg > kLaneRow;
+            bool keep = false;
+            unsigned wm = __ballot_sync(0xffffffffu, wide);
+            while (wm) {
+                const int s = __ffs(wm) - 1;
+                wm &= wm - 1;
+                const int hv = __shfl_sync(0xffffffffu, v, s);
+                const int hb = __shfl_sync(0xffffffffu, beg, s), he = __shfl_sync(0xffffffffu, end, s);
+                long long adj = afterburn_sum<UNIT>(A, hv, hb, he, 32, lane);
+#pragma unroll
+                for (int off = 16; off; off >>= 1) adj += __shfl_xor_sync(0xffffffffu, adj, off);
+                if (lane == s) keep = adj >= 0;
+            }
+            if (d >= 0 && !wide) keep = afterburn_sum<UNIT>(A, v, beg, end, 1, 0) >= 0;
+            if (!in) continue;
+            if (part_is_best) J.best[v] = own;
+            nxt[v] = keep ? d : own;
+            if (keep) {
+                const uint32_t w = (uint32_t)J.vwgt[v];
+                atomicSub(&J.bw[own], w);
+                atomicAdd(&J.bw[d], w);
+                J.moved_at[v] = it;
+                ++moves;
+            }
+        }
+        __syncwarp();
+        moves = __reduce_add_sync(0xffffffffu, moves);
+        if (lane == 0 && moves) atomicAdd(J.ring + 2 + (it & 1), moves);
+        if (!(alive = team.sync())) break;
+        {
+            int* t = cur;
+            cur = nxt;
+            nxt = t;
+        }
+        B.part = cur;
+        alive = sweep::balance_steps<UNIT>(team, a, B, p, sm, ws);
+    }
+    if (alive) {
+        const int* src = part_is_best ? cur : J.best;
+        if (src != J.part)
+            for (long long v = team.rank(); v < n; v += team.size()) J.part[v] = src[v];
+        if (!part_is_best && blockIdx.x == 0)
+            for (int b = threadIdx.x; b < k; b += kThreads) J.bw[b] = J.best_bw[b];
+    }
+    team.leave();
+}
+
 __global__ void fill_i32_kernel(int n, int v, int* p) {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         p[i] = v;
@@ -329,10 +507,78 @@ int grid_for(long long items) {
     return (int)std::max<long long>(1, std::min<long long>(div_up(items, kThreads), (long long)kNumSMs * 16));
 }
 
+// The loop as one team kernel; false when the level is not one for it:
+// thresholds of more than kTeamMaxBlocks blocks or rows of more than
+// kSmemTab / 2 entries do not fit the blocks' shared memory.  There is no
+// line by size: at 4.0M nodes / 58M entries (33 iterations, eco) the level
+// loop took 9 ms in one kernel against 13 ms as launches, at 1k nodes (61
+// iterations over three levels) 0.57 ms against 5.0 ms.
+bool jet_refine_team(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, uint32_t bound, int* part,
+                     uint32_t* bw) {
+    const int n = g.n, k = kn.k;
+    if (k > sweep::kTeamMaxBlocks || !sweep::team_rows(g)) return false;
+    const size_t mk = ctx.scratch.mark();
+    auto kernel = g.unit_weights ? jet_loop<true> : jet_loop<false>;
+    const int blocks = team_blocks(sweep::team_want(n), team_most(ctx, kernel, 0));
+    JetLoop J{};
+    J.part = part;
+    J.part2 = ctx.scratch.alloc<int>((size_t)n);
+    J.best = ctx.scratch.alloc<int>((size_t)n);
+    J.bw = bw;
+    J.bw2 = ctx.scratch.alloc<uint32_t>((size_t)k);
+    J.best_bw = ctx.scratch.alloc<uint32_t>((size_t)k);
+    J.vwgt = g.vwgt;
+    J.moved_at = ctx.scratch.alloc<int>((size_t)n);
+    J.wblocks = std::min(blocks, 2 * kNumSMs);
+    J.counters = ctx.scratch.alloc<uint32_t>((size_t)J.wblocks * k);
+    J.cut = ctx.scratch.alloc<unsigned long long>(2);
+    J.ring = ctx.scratch.alloc<unsigned>(4);
+    J.iters = kn.jet_iters;
+    J.patience = kn.jet_patience;
+    J.seed = kn.seed;
+    J.level = level;
+    J.bound = bound;
+    J.A.n = n;
+    J.A.k = k;
+    J.A.xadj = g.xadj;
+    J.A.adjncy = g.adjncy;
+    J.A.adjwgt = g.adjwgt;
+    J.A.moved_at = J.moved_at;
+    J.A.c4 = level == 0 ? kn.jet_c0 : kn.jet_c;
+    J.A.gain = ctx.scratch.alloc<long long>((size_t)n);
+    const sweep::SweepBuffers b = sweep::make_buffers(ctx, g, blocks);
+    // the destinations and the wide rows are dead while the balance repair
+    // uses its proposal targets and high-degree list
+    J.A.dest = b.pt;
+    J.A.wide = b.heavy;
+    sweep::SweepArgs a = sweep::base_args(g, b);
+    a.bound = bound;
+    a.P = kn.ref_classes;
+    a.H = ctx.scratch.alloc<uint32_t>((size_t)k * a.P);
+    a.minvP = ctx.scratch.alloc<int>((size_t)k * a.P);
+    sweep::BalanceArgs B{};
+    B.k = k;
+    B.iters = kn.bal_iters;
+    B.seed = kn.seed;
+    B.level = level;
+    B.gcap = b.gcap;
+    B.bw = bw;
+    B.HS = ctx.scratch.alloc<uint32_t>((size_t)k * sweep::kBalClasses);
+    B.counters = b.counters;
+    bool done;
+    {
+        PhaseScope ps(ctx, "jet_loop", 0);
+        done = launch_team(ctx, kernel, blocks, 0, J, a, B);
+    }
+    ctx.scratch.release(mk);
+    return done;
+}
+
 }  // namespace
 
 void jet_refine(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, uint32_t bound, int* part, uint32_t* bw) {
     if (g.n == 0 || kn.jet_iters <= 0) return;
+    if (jet_refine_team(ctx, g, kn, level, bound, part, bw)) return;
     cudaStream_t s = ctx.stream;
     const size_t mk = ctx.scratch.mark();
     const int n = g.n, k = kn.k;
@@ -380,7 +626,8 @@ void jet_refine(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, uint32_
             A.ks_tie = stream_key(kn.seed, TAG_JTIE, level, it);
             PhaseScope ps(ctx, "jet_choose", 12.0 * (double)g.m + 16.0 * n);
             KB_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned), s));
-            jet_choose<<<grid_for(n), kThreads, 0, s>>>(A);
+            if (g.unit_weights) jet_choose<true><<<grid_for(n), kThreads, 0, s>>>(A);
+            else jet_choose<false><<<grid_for(n), kThreads, 0, s>>>(A);
             KB_LAUNCH();
             jet_choose_wide<<<wblocks, kThreads, 0, s>>>(A, counters);
             KB_LAUNCH();
@@ -393,7 +640,8 @@ void jet_refine(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, uint32_
             KB_LAUNCH();
             jet_save<<<grid_for(n), kThreads, 0, s>>>(ctl, n, k, part, bw, best, best_bw);
             KB_LAUNCH();
-            jet_afterburn<<<grid_for(n), kThreads, 0, s>>>(A, keep, stop);
+            if (g.unit_weights) jet_afterburn<true><<<grid_for(n), kThreads, 0, s>>>(A, keep, stop);
+            else jet_afterburn<false><<<grid_for(n), kThreads, 0, s>>>(A, keep, stop);
             KB_LAUNCH();
             KB_CUDA(cudaMemsetAsync(ctr + 1, 0, sizeof(unsigned), s));
             jet_apply<<<grid_for(n), kThreads, 0, s>>>(n, it, keep, dest, g.vwgt, part, moved_at, bw, ctr + 1, stop);

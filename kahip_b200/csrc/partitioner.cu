@@ -46,8 +46,11 @@ void Ctx::init(int dev, cudaStream_t s) {
     }
     if (!pinned) KB_CUDA(cudaMallocHost(&pinned, 64 * sizeof(uint32_t)));
     if (!dscalars) {
-        KB_CUDA(cudaMalloc(&dscalars, 64 * sizeof(int) + 4 * sizeof(unsigned long long)));
+        KB_CUDA(cudaMalloc(&dscalars, 64 * sizeof(int) + 4 * sizeof(unsigned long long) + 4 * sizeof(unsigned)));
         work = reinterpret_cast<unsigned long long*>(dscalars + 64);
+        team_bar = reinterpret_cast<unsigned*>(work + 4);
+        KB_CUDA(cudaMemsetAsync(team_bar, 0, 4 * sizeof(unsigned), stream));
+        KB_CUDA(cudaStreamSynchronize(stream));  // later calls may run on a caller's stream
     }
     (void)s;
 }

@@ -1,0 +1,1073 @@
+// sweep.cuh -- the device side of the label-propagation sweeps (clustering,
+// refinement, balance repair): the sweep over a sub-round's members, the
+// high-degree rows, the admission of the proposals, and the forms in which a
+// team of blocks (team.cuh) runs whole phases.  lp.cu and jet.cu launch them;
+// the rules are stated there.
+#pragma once
+
+#include <cooperative_groups.h>
+
+#include <climits>
+
+#include "lp.cuh"
+#include "team.cuh"
+
+namespace kb {
+namespace sweep {
+
+namespace cg = cooperative_groups;
+
+constexpr uint32_t kEmpty = 0xFFFFFFFFu;
+constexpr int kThreads = 256;
+constexpr int kBalClasses = 256;
+
+enum Mode { CLUSTER = 0, REFINE = 1, BALANCE = 2 };
+
+// A list filled by many warps without contention: warp w appends to stripe
+// w % ns through that stripe's counter.  Every stripe has a capacity `cap`
+// computed on the host from the number of warps of the producing kernels and
+// the work each warp can be given.
+constexpr int kStripes = 128;
+struct SList {
+    int* data;        // ns * cap entries
+    unsigned* counts; // ns counters
+    long long cap;
+    int ns;           // stripes, a power of two (kStripes, or fewer for a small team)
+};
+
+// Everything a sweep reads or writes; passed by value.
+struct SweepArgs {
+    int n;
+    const int* __restrict__ xadj;
+    const int* __restrict__ adjncy;
+    const int* __restrict__ adjwgt;
+    const int* __restrict__ vwgt;
+    // (state that a team's steps write between sweeps: not __restrict__)
+    const int* lab;                     // cluster id or block id per vertex
+    const uint32_t* lw;                 // weight per label (cluster / block)
+    const uint8_t* active;              // REFINE: vertex may move this round (null: every vertex)
+    const int* vlist;                   // REFINE: sweep only these vertices (null: ids 0 .. n-1)
+    const unsigned* vcount;             // their number
+    uint32_t bound;
+    uint32_t S, s;                      // sub-rounds, this sub-round
+    uint64_t ks_sub, ks_tie, ks_prio;
+    int P;                              // admission classes
+    // outputs
+    int* pt; int* pc;                   // per vertex: proposed target / class (-1: none)
+    uint32_t* inc;                      // CLUSTER: incoming weight per target
+    int* minv;                          // CLUSTER: smallest proposer per target
+    uint32_t* H;                        // REFINE/BALANCE: weight per (target, class)
+    int* minvP;                         // smallest proposer per (target, class)
+    int* heavy; unsigned* hcount;       // deferred high-degree vertices
+    SList plist;                        // vertices that proposed a move this sub-round
+    int* hplist; unsigned* hpcount;     // proposals of high-degree vertices
+    int singletons;                     // every label is its own vertex id and rows have
+                                        // strictly increasing targets (clustering round 0)
+    const uint32_t* tie;                // singletons: hash32(ks_tie, u) per vertex
+    int all_fit;                        // singletons: every neighbour cluster fits (2 max c(v) < bound)
+    int admit_all;                      // CLUSTER: every target takes all its proposers
+                                        // (max c(v) (max degree + 1) < bound): no admission data
+    int fuse_apply;                     // singletons + all_fit + admit_all, no row above kWin:
+                                        // moves are applied in the sweep (nothing reads labels
+                                        // or cluster weights of others in that round)
+    int* label_w;                       // fuse_apply: labels, written by their own vertex
+    uint32_t* cw_w;                     // fuse_apply: cluster weights
+    int stash;                          // host: sweep with lane_vertex's label stash
+    unsigned long long* work;           // [0] vertices, [1] edges
+    int* err;                           // set when an invariant breaks
+    // BALANCE
+    const int* lightest;
+    uint32_t* HS;                       // release weight per (own block, class)
+};
+
+__device__ __forceinline__ uint32_t table_slot(uint32_t key, int cap) {
+    return (key * 0x9E3779B1u) >> (32 - __ffs(cap) + 1);
+}
+
+// Linear probing; the caller guarantees fewer distinct keys than cap/2, so
+// the probe ends within cap steps.  The bound only guards against a broken
+// invariant: the key is then dropped and *err is set.
+__device__ __forceinline__ void table_insert(uint32_t* tk, uint32_t* tv, int cap, uint32_t key,
+                                             uint32_t val, int* err) {
+    uint32_t s = table_slot(key, cap);
+    for (int probe = 0; probe < cap; ++probe) {
+        uint32_t prev = atomicCAS(&tk[s], kEmpty, key);
+        if (prev == kEmpty || prev == key) {
+            atomicAdd(&tv[s], val);
+            return;
+        }
+        s = (s + 1) & (uint32_t)(cap - 1);
+    }
+    atomicOr(err, 1);
+}
+
+// candidate key: larger connection first, then smaller tie hash; id breaks
+// the remaining ties (smaller wins)
+__device__ __forceinline__ uint64_t cand_key(uint32_t conn, uint64_t ks_tie, uint32_t label) {
+    return ((uint64_t)conn << 32) | (uint32_t)~hash32(ks_tie, label);
+}
+
+__device__ __forceinline__ void better(uint64_t& k, uint32_t& id, uint64_t k2, uint32_t id2) {
+    if (k2 > k || (k2 == k && id2 < id)) { k = k2; id = id2; }
+}
+
+template <int G>
+__device__ __forceinline__ void group_argmax(uint64_t& k, uint32_t& id, unsigned gmask) {
+#pragma unroll
+    for (int o = G / 2; o >= 1; o >>= 1) {
+        uint64_t k2 = __shfl_xor_sync(gmask, k, o);
+        uint32_t i2 = __shfl_xor_sync(gmask, id, o);
+        better(k, id, k2, i2);
+    }
+}
+
+// Is label b (connection c) a candidate for vertex of weight cv?
+template <int MODE>
+__device__ __forceinline__ bool cand_ok(const SweepArgs& a, uint32_t b, uint32_t c, uint32_t cv) {
+    if (MODE == BALANCE) return (uint64_t)a.lw[b] + cv <= a.bound;
+    return c > 0 && (uint64_t)a.lw[b] + cv < a.bound;
+}
+
+__device__ __forceinline__ int loss_bucket(long long loss) {
+    if (loss <= 0) return 0;
+    int b = 1;
+    while (b < 31 && (loss >> b) > 0) ++b;
+    return b;
+}
+
+// Final decision for vertex v (executed by one lane).
+// Returns true when v proposes a move (pt[v] = target; the caller lists v).
+template <int MODE>
+__device__ __forceinline__ bool decide_emit(const SweepArgs& a, int v, uint32_t own, uint32_t cv, uint32_t conn_own,
+                            uint64_t key, uint32_t id) {
+    if (MODE == CLUSTER) {
+        if (id == kEmpty || (uint32_t)(key >> 32) <= conn_own) return false;
+        a.pt[v] = (int)id;
+        if (!a.admit_all) {
+            atomicAdd(&a.inc[id], cv);
+            atomicMin(&a.minv[id], v);
+        }
+    } else if (MODE == REFINE) {
+        uint32_t base = a.lw[own] <= a.bound ? conn_own : 0u;
+        if (id == kEmpty || (uint32_t)(key >> 32) <= base) return false;
+        int cls = (int)hash_range(hash32(a.ks_prio, (uint32_t)v), (uint32_t)a.P);
+        a.pt[v] = (int)id;
+        a.pc[v] = cls;
+        size_t h = (size_t)id * a.P + cls;
+        atomicAdd(&a.H[h], cv);
+        atomicMin(&a.minvP[h], v);
+    } else {  // BALANCE
+        uint32_t t = id, tc = (uint32_t)(key >> 32);
+        if (t == kEmpty) {
+            int L = *a.lightest;
+            if ((uint32_t)L == own || (uint64_t)a.lw[L] + cv > a.bound) return false;
+            t = (uint32_t)L;
+            tc = 0;
+        }
+        long long loss = (long long)conn_own - (long long)tc;
+        int cls = loss_bucket(loss) * 8 + (int)hash_range(hash32(a.ks_sub, (uint32_t)v), 8u);
+        a.pt[v] = (int)t;
+        a.pc[v] = cls;
+        atomicAdd(&a.HS[(size_t)own * kBalClasses + cls], cv);
+    }
+    return true;
+}
+
+__device__ __forceinline__ int warp_global_id() {
+    return (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+}
+
+// warp-aggregated append to a plain list (one atomic per warp call)
+__device__ __forceinline__ void append_aggregated(bool pred, int v, int* list, unsigned* count) {
+    const unsigned m = __ballot_sync(0xffffffffu, pred);
+    if (!m) return;
+    const int lane = threadIdx.x & 31;
+    const int leader = __ffs(m) - 1;
+    unsigned base = 0;
+    if (lane == leader) base = atomicAdd(count, (unsigned)__popc(m));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (pred) list[base + __popc(m & lanemask_lt())] = v;
+}
+
+// warp-aggregated append to this warp's stripe of a striped list
+__device__ __forceinline__ void append_striped(bool pred, int v, const SList& L) {
+    const int stripe = warp_global_id() & (L.ns - 1);
+    append_aggregated(pred, v, L.data + (long long)stripe * L.cap, L.counts + stripe);
+}
+
+template <int MODE>
+__device__ __forceinline__ bool member(const SweepArgs& a, int v) {
+    if (MODE == BALANCE) return a.lw[a.lab[v]] > a.bound;
+    if (MODE == REFINE && a.active && !a.active[v]) return false;
+    return hash_range(hash32(a.ks_sub, (uint32_t)v), a.S) == a.s;
+}
+
+// ------------------------------------------------ chunk-cooperative path
+
+constexpr int kWin = 128;                 // edges per window (<= 4 batches)
+constexpr int kBatches = kWin / 32;
+constexpr int kTab = 2 * kWin;            // table slots per warp (load <= 1/2)
+constexpr unsigned long long kEmpty64 = ~0ull;
+constexpr int kWarpsPerBlock = kThreads / 32;
+
+// Labels (and weights) that lane_vertex stashes per lane: column `lane` of a
+// row-major [kStash][32] array, so that lanes never share a bank.  The stash
+// overlays the chunk table, which chunk_process clears before each use.
+constexpr int kStashUnit = 24;  // unit edge weights: labels only
+constexpr int kStashWgt = 12;   // labels, then weights
+
+struct WarpTable {
+    union {
+        struct {
+            unsigned long long key[kTab];  // (member lane << 32) | label
+            uint32_t val[kTab];
+        };
+        uint32_t stash[3 * kTab];
+    };
+    uint16_t used[kWin];           // slots filled in the current window
+    unsigned long long bkey[32];   // per member: best candidate key
+    uint32_t bid[32];              // per member: best candidate label
+    uint32_t cown[32];             // per member: connection to its own label
+    uint32_t own[32];
+    uint32_t cv[32];
+    uint32_t nused;
+};
+
+__device__ __forceinline__ uint32_t slot64(unsigned long long k) {
+    return (uint32_t)((k * 0x9E3779B97F4A7C15ull) >> (64 - 8)) & (kTab - 1);  // kTab == 256
+}
+
+// Decides up to 32 vertices (lane i: vertex v when mem) with the per-warp
+// shared table: the members' edges are laid back to back (warp prefix sum of
+// degrees) and processed in windows of at most kWin edges; every lane takes
+// one edge slot per 32-edge batch, all adjacency loads of a window are issued
+// before the label gathers, (member, label) pairs are merged with a 64-bit
+// match_any and summed into the table, and each member's best candidate is
+// found with shared-memory atomicMax / atomicMin.  Used for the vertices
+// whose neighbours carry more distinct labels than the lane path's slots.
+template <int MODE>
+__device__ __forceinline__ void chunk_process(const SweepArgs& a, WarpTable& T, bool mem, int v, unsigned& wv, unsigned& we,
+                              unsigned& wo) {
+    const int lane = threadIdx.x & 31;
+    int beg = 0, deg = 0;
+    bool heavy = false;
+    if (mem) {
+        beg = a.xadj[v];
+        deg = a.xadj[v + 1] - beg;
+        if (deg > kWin) {  // high degree: block-per-vertex kernel decides it
+            a.heavy[atomicAdd(a.hcount, 1u)] = v;
+            deg = 0;
+            heavy = true;
+        } else {
+            wv += 1;
+            we += (unsigned)deg;
+            wo += 1;
+        }
+        T.own[lane] = (uint32_t)a.lab[v];
+        T.cv[lane] = (uint32_t)a.vwgt[v];
+    }
+    const bool light = mem && !heavy;
+    // inclusive prefix sum of degrees over the chunk
+    int incl = deg;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    const int off = incl - deg;
+    const unsigned lightmask = __ballot_sync(0xffffffffu, light);
+    if (!lightmask) return;
+    // the table doubles as lane_vertex's stash: clear it before use
+    for (int i = lane; i < kTab; i += 32) {
+        T.key[i] = kEmpty64;
+        T.val[i] = 0;
+    }
+    __syncwarp();
+    int wstart = __ffs(lightmask) - 1;
+    while (wstart < 32) {
+        // window: lanes [wstart, wend) whose edges fit into kWin slots
+        const int base = __shfl_sync(0xffffffffu, off, wstart);
+        const bool inwin = lane >= wstart && incl - base <= kWin;
+        const unsigned wmask = __ballot_sync(0xffffffffu, inwin);
+        const int wend = 32 - __clz(wmask);
+        const int E = __shfl_sync(0xffffffffu, incl, wend - 1) - base;
+        const bool wmember = light && lane >= wstart && lane < wend;
+        if (wmember) {
+            T.bkey[lane] = 0;
+            T.bid[lane] = kEmpty;
+            T.cown[lane] = 0;
+        }
+        // gather the window's edges: all adjacency loads, then all labels
+        int own_lane[kBatches];
+        int tgt[kBatches];
+        uint32_t wgt[kBatches];
+#pragma unroll
+        for (int b = 0; b < kBatches; ++b) {
+            const int q = b * 32 + lane;
+            // largest window lane o with off[o] - base <= q (binary lifting)
+            int o = wstart;
+#pragma unroll
+            for (int step = 16; step >= 1; step >>= 1) {
+                const int c = o + step;
+                const int oc = __shfl_sync(0xffffffffu, off, c < 32 ? c : 31) - base;
+                if (c < wend && oc <= q) o = c;
+            }
+            const int ob = __shfl_sync(0xffffffffu, beg, o);
+            const int oo = __shfl_sync(0xffffffffu, off, o) - base;
+            own_lane[b] = o;
+            tgt[b] = -1;
+            wgt[b] = 0;
+            if (q < E) {
+                const int e = ob + (q - oo);
+                tgt[b] = a.adjncy[e];
+                wgt[b] = (uint32_t)a.adjwgt[e];
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < kBatches; ++b)
+            if (tgt[b] >= 0) tgt[b] = a.lab[tgt[b]];
+#pragma unroll
+        for (int b = 0; b < kBatches; ++b) {
+            if (b * 32 >= E) break;
+            const bool ok = tgt[b] >= 0;
+            const unsigned long long key =
+                ok ? (((unsigned long long)own_lane[b] << 32) | (uint32_t)tgt[b]) : kEmpty64;
+            const unsigned peers = __match_any_sync(0xffffffffu, key);
+            const uint32_t sum = __reduce_add_sync(peers, wgt[b]);
+            if (ok && (peers & lanemask_lt()) == 0) {
+                uint32_t sl = slot64(key);
+                for (int probe = 0; probe < kTab; ++probe) {
+                    const unsigned long long prev = atomicCAS(&T.key[sl], kEmpty64, key);
+                    if (prev == kEmpty64) {
+                        T.used[atomicAdd(&T.nused, 1u)] = (uint16_t)sl;
+                        atomicAdd(&T.val[sl], sum);
+                        break;
+                    }
+                    if (prev == key) {
+                        atomicAdd(&T.val[sl], sum);
+                        break;
+                    }
+                    sl = (sl + 1) & (kTab - 1);
+                    if (probe == kTab - 1) atomicOr(a.err, 1);
+                }
+            }
+            __syncwarp();
+        }
+        // per member: connection to its own label and the best candidate
+        const uint32_t nused = T.nused;
+        for (uint32_t i = lane; i < nused; i += 32) {
+            const uint32_t sl = T.used[i];
+            const unsigned long long k = T.key[sl];
+            const int o = (int)(k >> 32);
+            const uint32_t l = (uint32_t)k;
+            const uint32_t c = T.val[sl];
+            if (l == T.own[o]) T.cown[o] = c;
+            else if (cand_ok<MODE>(a, l, c, T.cv[o])) atomicMax(&T.bkey[o], cand_key(c, a.ks_tie, l));
+        }
+        __syncwarp();
+        for (uint32_t i = lane; i < nused; i += 32) {
+            const uint32_t sl = T.used[i];
+            const unsigned long long k = T.key[sl];
+            const int o = (int)(k >> 32);
+            const uint32_t l = (uint32_t)k;
+            const uint32_t c = T.val[sl];
+            if (l != T.own[o] && cand_ok<MODE>(a, l, c, T.cv[o]) && cand_key(c, a.ks_tie, l) == T.bkey[o])
+                atomicMin(&T.bid[o], l);
+            T.key[sl] = kEmpty64;
+            T.val[sl] = 0;
+        }
+        __syncwarp();
+        if (lane == 0) T.nused = 0;
+        bool prop = false;
+        if (wmember) prop = decide_emit<MODE>(a, v, T.own[lane], T.cv[lane], T.cown[lane], T.bkey[lane], T.bid[lane]);
+        append_striped(prop, v, a.plist);
+        __syncwarp();
+        // next window starts at the first light lane at or after wend
+        const unsigned rest = lightmask & (wend < 32 ? (~0u << wend) : 0u);
+        wstart = rest ? __ffs(rest) - 1 : 32;
+    }
+}
+
+// ------------------------------------------------------ lane-per-vertex sweep
+//
+// The main sweep: a warp takes 32 * kSpan consecutive vertex ids, compacts the
+// members of the sub-round onto its lanes, and every lane aggregates its own
+// vertex's neighbourhood in kSlots register slots (connection per label; the
+// own label is kept apart), four edges at a time with all loads issued
+// before use.  A vertex whose neighbours carry more distinct labels than
+// slots is queued per warp and decided by chunk_process in the same kernel;
+// one of degree > kWin goes to the high-degree list (heavy_kernel).
+
+constexpr int kSlots = 6;  // 4: ~5 % of RGG rows overflow; 6: 0.6 %, fastest measured
+constexpr int kSpan = 2;  // chunks of 32 ids per warp task (2 measured 3 % faster than 4)
+
+// r-th set bit (0-based) of mask
+__device__ __forceinline__ int nth_set_bit(unsigned mask, int r) {
+    int lo = 0, hi = 31;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        const unsigned below = mid == 31 ? mask : (mask & ((2u << mid) - 1u));
+        if (__popc(below) > r) hi = mid;
+        else lo = mid + 1;
+    }
+    return lo;
+}
+
+// 0: decided (stays), 3: decided (proposes a move), 1: too many distinct
+// labels for NS slots, 2: degree above kWin
+template <int MODE, int NS, bool UNIT, bool STASH>
+__device__ __forceinline__ int lane_vertex(const SweepArgs& a, int v, uint32_t* st, unsigned& wv, unsigned& we) {
+    const int beg = a.xadj[v], end = a.xadj[v + 1];
+    if (end - beg > kWin) return 2;
+    // clustering round 0 (singletons): every label is its own vertex id
+    const uint32_t own = (MODE == CLUSTER && a.singletons) ? (uint32_t)v : (uint32_t)a.lab[v];
+    const uint32_t cv = (uint32_t)a.vwgt[v];
+    uint32_t cown = 0;
+    if (MODE == CLUSTER && a.singletons && UNIT && a.all_fit) {
+        // unit weights: every neighbour cluster has connection 1, so the best
+        // is the neighbour of smallest (tie hash, id) -- one 64-bit minimum
+        // per entry
+        uint64_t bk = ~0ull;
+        for (int e = beg; e < end; e += 4) {
+            int u[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) u[t] = e + t < end ? a.adjncy[e + t] : -1;
+            uint32_t h[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) h[t] = u[t] >= 0 ? a.tie[u[t]] : 0u;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                if (u[t] < 0) continue;
+                if ((uint32_t)u[t] == own) { cown += 1; continue; }
+                const uint64_t k = ((uint64_t)h[t] << 32) | (uint32_t)u[t];
+                bk = k < bk ? k : bk;
+            }
+        }
+        wv += 1;
+        we += (unsigned)(end - beg);
+        const uint32_t id = bk == ~0ull ? kEmpty : (uint32_t)bk;
+        if (a.fuse_apply) {
+            if (id == kEmpty || 1u <= cown) return 0;
+            a.label_w[v] = (int)id;
+            atomicSub(&a.cw_w[own], cv);
+            atomicAdd(&a.cw_w[id], cv);
+            return 0;
+        }
+        const uint64_t key = id == kEmpty ? 0ull : (1ull << 32);
+        return decide_emit<MODE>(a, v, own, cv, cown, key, id) ? 3 : 0;
+    }
+    if (MODE == CLUSTER && a.singletons) {
+        // label[u] == u and no target repeats: the connection to cluster u is
+        // exactly w(v,u), so the best candidate is a running maximum; the
+        // tie hashes come precomputed per vertex, and the size test is
+        // skipped when every pair of node weights fits under the bound
+        uint64_t key = 0;
+        uint32_t id = kEmpty;
+        for (int e = beg; e < end; e += 4) {
+            int u[4];
+            uint32_t w[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                u[t] = -1;
+                w[t] = 0;
+                if (e + t < end) {
+                    u[t] = a.adjncy[e + t];
+                    w[t] = UNIT ? 1u : (uint32_t)a.adjwgt[e + t];
+                }
+            }
+            uint32_t h[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) h[t] = u[t] >= 0 ? a.tie[u[t]] : 0u;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                if (u[t] < 0) continue;
+                const uint32_t l = (uint32_t)u[t];
+                if (l == own) { cown += w[t]; continue; }
+                if (a.all_fit ? w[t] > 0 : cand_ok<MODE>(a, l, w[t], cv))
+                    better(key, id, ((uint64_t)w[t] << 32) | (uint32_t)~h[t], l);
+            }
+        }
+        wv += 1;
+        we += (unsigned)(end - beg);
+        return decide_emit<MODE>(a, v, own, cv, cown, key, id) ? 3 : 0;
+    }
+    // NS register slots (label, connection); a new label enters at slot 0 and
+    // shifts the others up, so slot NS-1 filled means the slots are full
+    uint32_t sl[NS], sc[NS];
+#pragma unroll
+    for (int i = 0; i < NS; ++i) { sl[i] = kEmpty; sc[i] = 0; }
+    bool overflow = false;
+    auto add_label = [&](uint32_t lt, uint32_t wt) {
+        bool hit = false;
+#pragma unroll
+        for (int j = 0; j < NS; ++j) {
+            const bool m = sl[j] == lt;
+            sc[j] += m ? wt : 0u;
+            hit |= m;
+        }
+        if (!hit) {
+            overflow |= sl[NS - 1] != kEmpty;
+#pragma unroll
+            for (int j = NS - 1; j > 0; --j) { sl[j] = sl[j - 1]; sc[j] = sc[j - 1]; }
+            sl[0] = lt;
+            sc[0] = wt;
+        }
+    };
+    // STASH: two passes -- the gather pass adds entries of the own label to
+    // cown and stashes the others in shared memory, the slot pass merges the
+    // stash into the slots.  Once most entries carry the own label the slot
+    // search then runs over far fewer entries than the row has (without the
+    // stash every lane's slot search runs whenever one lane of the warp needs
+    // it).
+    constexpr int kStash = UNIT ? kStashUnit : kStashWgt;
+    uint32_t* const stl = st;
+    uint32_t* const stw = st + kStashWgt * 32;  // weights (not UNIT)
+    int ns = 0;
+    auto slot_pass = [&]() {
+        for (int i = 0; i < ns && !overflow; ++i) add_label(stl[i * 32], UNIT ? 1u : stw[i * 32]);
+        ns = 0;
+    };
+    // software pipeline: the row entries of the next group of four are
+    // loaded while the labels of the current group are gathered
+    int un[4];
+    uint32_t wn[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        un[t] = -1;
+        wn[t] = 0;
+        if (beg + t < end) {
+            un[t] = a.adjncy[beg + t];
+            wn[t] = UNIT ? 1u : (uint32_t)a.adjwgt[beg + t];
+        }
+    }
+    for (int e = beg; e < end && !overflow; e += 4) {
+        int u[4];
+        uint32_t w[4], l[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            u[t] = un[t];
+            w[t] = wn[t];
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) l[t] = u[t] >= 0 ? (uint32_t)a.lab[u[t]] : kEmpty;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            un[t] = -1;
+            wn[t] = 0;
+            if (e + 4 + t < end) {
+                un[t] = a.adjncy[e + 4 + t];
+                wn[t] = UNIT ? 1u : (uint32_t)a.adjwgt[e + 4 + t];
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            if (l[t] == kEmpty) continue;  // past the row's end (labels are < n)
+            if (l[t] == own) {
+                cown += w[t];
+            } else if (STASH) {
+                stl[ns * 32] = l[t];
+                if (!UNIT) stw[ns * 32] = w[t];
+                ++ns;
+            } else {
+                add_label(l[t], w[t]);
+            }
+        }
+        if (STASH && ns > kStash - 4) slot_pass();  // room for the next group of four
+    }
+    if (STASH) slot_pass();
+    if (overflow) return 1;
+    wv += 1;
+    we += (unsigned)(end - beg);
+    // best candidate: largest connection, ties by smaller tie hash, then
+    // smaller label; hashes are computed only for ties
+    uint32_t ok[NS];
+#pragma unroll
+    for (int i = 0; i < NS; ++i) ok[i] = sl[i] != kEmpty && cand_ok<MODE>(a, sl[i], sc[i], cv);
+    uint32_t bc = 0, id = kEmpty;
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+        if (!ok[i]) continue;
+        if (id == kEmpty || sc[i] > bc) {
+            bc = sc[i];
+            id = sl[i];
+        } else if (sc[i] == bc) {
+            const uint32_t hi = hash32(a.ks_tie, sl[i]), hb = hash32(a.ks_tie, id);
+            if (hi < hb || (hi == hb && sl[i] < id)) id = sl[i];
+        }
+    }
+    // decide_emit reads the connection (upper half) of the key only
+    const uint64_t key = id == kEmpty ? 0ull : ((uint64_t)bc << 32);
+    return decide_emit<MODE>(a, v, own, cv, cown, key, id) ? 3 : 0;
+}
+
+// A block's shared memory in a sweep: per warp a queue of members still to
+// be processed (so that every pass over the lanes is full), a queue of
+// vertices that overflowed the slots, and the chunk table.
+struct SweepSmem {
+    int queue[kWarpsPerBlock][32 * kSpan + 32];
+    int oqueue[kWarpsPerBlock][64];
+    WarpTable tabs[kWarpsPerBlock];
+};
+
+// The whole grid sweeps the members of one sub-round (kThreads a block).
+template <int MODE, bool UNIT, bool STASH>
+__device__ __forceinline__ void lane_sweep(const SweepArgs& a, SweepSmem& sm) {
+    static_assert(kTab == 256, "slot64 assumes 256 slots");
+    const int lane = threadIdx.x & 31;
+    int* q = sm.queue[threadIdx.x >> 5];
+    int* oq = sm.oqueue[threadIdx.x >> 5];
+    WarpTable& T = sm.tabs[threadIdx.x >> 5];
+    if (lane == 0) T.nused = 0;
+    __syncwarp();
+    int qn = 0, oqn = 0;  // warp-uniform
+    // per-lane work counts (32 bits: a lane never sees more than m < 2^31 entries)
+    unsigned wv = 0, we = 0, wo = 0;
+    const long long span = 32LL * kSpan;
+    // the swept items: vertex ids 0 .. n-1, or the entries of vlist
+    const long long nitems = a.vlist ? (long long)*a.vcount : (long long)a.n;
+    const long long ntasks = (nitems + span - 1) / span;
+    const long long warp = ((long long)blockIdx.x * kThreads + threadIdx.x) / 32;
+    const long long nwarps = (long long)gridDim.x * kThreads / 32;
+    auto overflow_pass = [&]() {
+        const bool mem = lane < oqn && lane < 32;
+        const int v = mem ? oq[lane] : 0;
+        __syncwarp();
+        for (int i = lane; i + 32 < oqn; i += 32) oq[i] = oq[i + 32];
+        __syncwarp();
+        oqn = oqn > 32 ? oqn - 32 : 0;
+        chunk_process<MODE>(a, T, mem, v, wv, we, wo);
+    };
+    auto pass = [&](int v) {
+        int status = 0;
+        if (v >= 0) status = lane_vertex<MODE, kSlots, UNIT, STASH>(a, v, T.stash + lane, wv, we);
+        const unsigned om = __ballot_sync(0xffffffffu, status == 1);
+        if (status == 1) oq[oqn + __popc(om & lanemask_lt())] = v;
+        oqn += __popc(om);
+        __syncwarp();
+        append_aggregated(status == 2, v, a.heavy, a.hcount);
+        append_striped(status == 3, v, a.plist);
+        if (oqn >= 32) overflow_pass();
+    };
+    for (long long task = warp; task < ntasks; task += nwarps) {
+        const long long base = task * span;
+#pragma unroll
+        for (int c = 0; c < kSpan; ++c) {
+            const long long vv = base + c * 32 + lane;
+            const bool valid = vv < nitems;
+            const int v = valid ? (a.vlist ? a.vlist[vv] : (int)vv) : 0;
+            const bool mem = valid && member<MODE>(a, v);
+            const unsigned m = __ballot_sync(0xffffffffu, mem);
+            if (mem) q[qn + __popc(m & lanemask_lt())] = v;
+            qn += __popc(m);
+        }
+        __syncwarp();
+        while (qn >= 32) {
+            const int v = q[lane];
+            __syncwarp();
+            for (int i = lane; i + 32 < qn; i += 32) q[i] = q[i + 32];
+            __syncwarp();
+            qn -= 32;
+            pass(v);
+        }
+    }
+    if (qn > 0) pass(lane < qn ? q[lane] : -1);
+    while (oqn > 0) overflow_pass();
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+        wv += __shfl_xor_sync(0xffffffffu, wv, o);
+        we += __shfl_xor_sync(0xffffffffu, we, o);
+        wo += __shfl_xor_sync(0xffffffffu, wo, o);
+    }
+    if (lane == 0 && (wv | we)) {
+        atomicAdd(&a.work[0], (unsigned long long)wv);
+        atomicAdd(&a.work[1], (unsigned long long)we);
+        if (wo) atomicAdd(&a.work[2], (unsigned long long)wo);
+    }
+}
+
+// High-degree vertices: one block per vertex.  Its connections aggregate in
+// a hash table in shared memory (rows up to kSmemTab / 2 entries) or, for
+// longer rows, in the block's global-memory table of `gcap` slots
+// (gcap >= 2 * maxdeg, power of two; gtk may be null when every row fits
+// the shared table).
+constexpr int kSmemTab = 4096;
+
+// BT threads per block (more for the longest rows).
+// `which`: 0 = every listed vertex, 1 = only those whose table fits in
+// shared memory, 2 = only the others (the two kinds can run as separate
+// launches with different grids; the decisions do not depend on the order).
+// The shared-memory table htab (stab slots, a power of two, keys then values)
+// has kSmemTab slots in the many-block launches, more in the launch of the
+// longest rows, whose rows up to stab / 2 entries then stay out of the
+// global table.
+template <int MODE, int BT>
+__device__ __forceinline__ void heavy_sweep(const SweepArgs& a, uint32_t* gtk, uint32_t* gtv, int gcap, int which,
+                                            int stab, uint32_t* htab) {
+    __shared__ uint64_t sk[BT / 32];
+    __shared__ uint32_t sid[BT / 32];
+    __shared__ uint32_t sco;
+    uint32_t* stk = htab;
+    uint32_t* stv = htab + stab;
+    for (int s = threadIdx.x; s < stab; s += BT) {
+        stk[s] = kEmpty;
+        stv[s] = 0;
+    }
+    __syncthreads();
+    uint32_t* gk = gtk ? gtk + (size_t)blockIdx.x * gcap : nullptr;
+    uint32_t* gv = gtv ? gtv + (size_t)blockIdx.x * gcap : nullptr;
+    const unsigned count = *a.hcount;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (unsigned i = blockIdx.x; i < count; i += gridDim.x) {
+        const int v = a.heavy[i];
+        const int beg = a.xadj[v], end = a.xadj[v + 1];
+        const uint32_t own = (uint32_t)a.lab[v];
+        const uint32_t cv = (uint32_t)a.vwgt[v];
+        // this vertex uses the first cap entries of the block's table (a
+        // power of two >= 2 * degree, at most gcap), so inserting, scanning
+        // and clearing cost O(degree), not O(max degree)
+        int cap = 256;
+        while (cap < 2 * (end - beg) && cap < gcap) cap <<= 1;
+        if ((which == 1 && cap > kSmemTab) || (which == 2 && cap <= kSmemTab)) continue;
+        uint32_t* tk = cap <= stab ? stk : gk;
+        uint32_t* tv = cap <= stab ? stv : gv;
+        if (threadIdx.x == 0) {
+            sco = 0;
+            atomicAdd(&a.work[0], 1ull);
+            atomicAdd(&a.work[1], (unsigned long long)(end - beg));
+        }
+        for (int c = beg; c < end; c += BT) {
+            int e = c + threadIdx.x;
+            uint32_t l = kEmpty, wt = 0;
+            if (e < end) {
+                wt = (uint32_t)a.adjwgt[e];
+                l = (uint32_t)a.lab[a.adjncy[e]];
+            }
+            unsigned peers = __match_any_sync(0xffffffffu, l);
+            uint32_t sum = __reduce_add_sync(peers, wt);
+            if (e < end && (peers & lanemask_lt()) == 0) table_insert(tk, tv, cap, l, sum, a.err);
+        }
+        __syncthreads();
+        uint64_t key = 0;
+        uint32_t id = kEmpty;
+        for (int s = threadIdx.x; s < cap; s += BT) {
+            uint32_t l = tk[s];
+            if (l == kEmpty) continue;
+            uint32_t c = tv[s];
+            tk[s] = kEmpty;
+            tv[s] = 0;
+            if (l == own) sco = c;
+            else if (cand_ok<MODE>(a, l, c, cv)) better(key, id, cand_key(c, a.ks_tie, l), l);
+        }
+        group_argmax<32>(key, id, 0xffffffffu);
+        if (lane == 0) { sk[w] = key; sid[w] = id; }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int j = 1; j < BT / 32; ++j) better(key, id, sk[j], sid[j]);
+            if (decide_emit<MODE>(a, v, own, cv, sco, key, id)) a.hplist[atomicAdd(a.hpcount, 1u)] = v;
+        }
+        __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------- admission
+//
+// Proposal encoding per vertex: pt[v] = target (>= 0), -1 = no proposal,
+// -2 - target = rejected (its accumulators still need resetting).
+
+// Threshold admission: classes of target b are admitted in increasing order
+// while the cumulative weight stays <= cap(b); in the first class that does
+// not fit, only its smallest proposer is tried alone.
+__device__ __forceinline__ bool admit(const uint32_t* H, const int* minvP, int P, int b, int c, int v,
+                                      uint32_t cv, long long cap) {
+    const uint32_t* h = H + (size_t)b * P;
+    unsigned long long cum = 0;
+    int t = 0;
+    while (t < P && (long long)(cum + h[t]) <= cap) { cum += h[t]; ++t; }
+    if (c < t) return true;
+    return c == t && minvP[(size_t)b * P + t] == v && (long long)(cum + cv) <= cap;
+}
+
+// The vertices a refinement round sweeps next: the neighbours of the ones it
+// moves, as flags (a round that moves many vertices) or as a list in which
+// each is listed once (the first thread to raise its stamp to this round's
+// tag appends it; appends are aggregated over the coalesced lanes).
+struct NextActive {
+    uint8_t* flags;   // non-null: flags[u] = 1
+    uint32_t* stamp;  // per vertex: the tag of the last round that listed it
+    uint32_t tag;     // this round's tag, larger than every earlier one
+    int* list;        // null (and no flags): nothing is kept
+    unsigned* count;
+    int* hubs;        // non-null: moved vertices of degree > kHubMark are listed
+    unsigned* nhubs;  // here instead, for mark_hubs (a warp per vertex)
+};
+
+// (a thread marks at most this many neighbours itself: in list mode every
+// mark waits for its atomic's result)
+constexpr int kHubMark = 32;
+
+// Marks (or lists) the neighbours of one moved vertex, row entries
+// [e0, e1), by the threads t, t + nt, ...
+__device__ __forceinline__ void mark_row(const NextActive& na, const int* adjncy, int e0, int e1, int t, int nt) {
+    if (na.flags) {
+        for (int e = e0 + t; e < e1; e += nt) na.flags[adjncy[e]] = 1;
+    } else if (na.list) {
+        for (int e = e0 + t; e < e1; e += nt) {
+            const int u = adjncy[e];
+            if (atomicMax(&na.stamp[u], na.tag) < na.tag) {
+                cg::coalesced_group g = cg::coalesced_threads();
+                unsigned at = 0;
+                if (g.thread_rank() == 0) at = atomicAdd(na.count, g.size());
+                at = g.shfl(at, 0);
+                na.list[at + g.thread_rank()] = u;
+            }
+        }
+    }
+}
+
+// -------------------------------------------------------------- team forms
+//
+// A team (team.cuh) runs all steps of a phase in one kernel: the sweep, the
+// high-degree rows, the admission and the moves of one sub-round after the
+// other, a barrier apart.  The counters of a sub-round's lists alternate
+// between two sets; a sub-round clears the set of the next one, which every
+// block stopped reading at the barrier that ended the sub-round before.
+
+constexpr int kTeamSet = kStripes + 8;  // counters of one set: stripes, heavy, heavy proposals
+constexpr int kTeamMaxBlocks = 8192;    // blocks of the partition (their thresholds sit in shared memory)
+
+__device__ __forceinline__ void use_set(SweepArgs& a, unsigned* counters, int p) {
+    a.plist.counts = counters + p * kTeamSet;
+    a.hcount = counters + p * kTeamSet + kStripes;
+    a.hpcount = counters + p * kTeamSet + kStripes + 1;
+    unsigned* other = counters + (p ^ 1) * kTeamSet;
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < kTeamSet; i += blockDim.x) other[i] = 0;
+}
+
+// f(v) for every proposal of the sub-round, warp by warp: all lanes of a warp
+// call f together, v = -1 for the lanes beyond the list's end.
+template <class F>
+__device__ __forceinline__ void each_proposal(const SweepArgs& a, F f) {
+    const unsigned lane = threadIdx.x & 31;
+    const unsigned W = gridDim.x * kWarpsPerBlock, w = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+    const unsigned ns = (unsigned)a.plist.ns + 1u;  // the stripes and the high-degree list
+    for (unsigned s = w % ns; s < ns; s += W) {
+        const bool stripe = s + 1 < ns;
+        const unsigned n = stripe ? a.plist.counts[s] : *a.hpcount;
+        const int* list = stripe ? a.plist.data + (long long)s * a.plist.cap : a.hplist;
+        const unsigned share = W > ns ? (W - s + ns - 1) / ns : 1u;  // warps on this stripe
+        for (unsigned i = (W > ns ? w / ns : 0u) * 32; i < n; i += share * 32) f(i + lane < n ? list[i + lane] : -1);
+    }
+}
+
+// The sub-round's members in a lane per vertex, then those of high degree;
+// every block has seen all proposals afterwards.  False: the team gave up.
+// (Rows of up to kSmemTab / 2 entries: gcap slots fit the block's table,
+// which takes the place of the chunk tables.)
+template <int MODE, bool UNIT, bool STASH>
+__device__ __forceinline__ bool team_sweep(Team& team, const SweepArgs& a, int gcap, SweepSmem& sm) {
+    static_assert(sizeof(sm.tabs) >= 8 * kSmemTab, "the high-degree table overlays the chunk tables");
+    lane_sweep<MODE, UNIT, STASH>(a, sm);
+    if (!team.sync()) return false;
+    if (gcap == 0 || *a.hcount == 0) return true;
+    heavy_sweep<MODE, kThreads>(a, nullptr, nullptr, gcap, 0, kSmemTab, reinterpret_cast<uint32_t*>(sm.tabs));
+    return team.sync();
+}
+
+// class_decide's and class_apply's rules for one proposal
+__device__ __forceinline__ void class_decide_one(const SweepArgs& a, const uint32_t* bw, int strict, int v) {
+    const int b = a.pt[v];
+    if (b < 0) return;
+    const int c = a.pc[v];
+    if (c < 0) return;
+    const long long cap = (long long)a.bound - (strict ? 1 : 0) - (long long)bw[b];
+    if (!admit(a.H, a.minvP, a.P, b, c, v, (uint32_t)a.vwgt[v], cap)) a.pt[v] = -2 - b;
+}
+
+// true when v moved
+__device__ __forceinline__ bool class_apply_one(const SweepArgs& a, int* part, uint32_t* bw, int v) {
+    const int t = a.pt[v];
+    if (t == -1) return false;
+    const int c = a.pc[v];
+    if (c < 0) return false;  // dropped before admission (balance)
+    const int b = t >= 0 ? t : -2 - t;
+    a.H[(size_t)b * a.P + c] = 0;
+    a.minvP[(size_t)b * a.P + c] = INT_MAX;
+    if (t < 0) return false;
+    const uint32_t cv = (uint32_t)a.vwgt[v];
+    atomicSub(&bw[part[v]], cv);
+    atomicAdd(&bw[t], cv);
+    part[v] = t;
+    return true;
+}
+
+// Block weights looked over by every block of the team for itself.
+struct Weighed {
+    unsigned long long overload;  // weight above the bound
+    int lightest;                 // lightest block, the smaller id on ties
+    bool over;                    // some block exceeds the bound
+};
+
+struct WeighSmem {
+    unsigned long long ov[kWarpsPerBlock], best[kWarpsPerBlock];
+    int lightest;  // for SweepArgs::lightest
+};
+
+__device__ __forceinline__ Weighed weigh(const uint32_t* bw, int k, uint32_t bound, WeighSmem& ws) {
+    __syncthreads();  // the last call's readers
+    unsigned long long ov = 0, best = ~0ull;
+    for (int b = threadIdx.x; b < k; b += blockDim.x) {
+        const uint32_t x = bw[b];
+        best = min(best, ((unsigned long long)x << 32) | (unsigned)b);
+        if (x > bound) ov += x - bound;
+    }
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+        ov += __shfl_xor_sync(0xffffffffu, ov, o);
+        best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        ws.ov[threadIdx.x >> 5] = ov;
+        ws.best[threadIdx.x >> 5] = best;
+    }
+    __syncthreads();
+    ov = 0;
+    best = ~0ull;
+#pragma unroll
+    for (int w = 0; w < kWarpsPerBlock; ++w) {
+        ov += ws.ov[w];
+        best = min(best, ws.best[w]);
+    }
+    if (threadIdx.x == 0) ws.lightest = (int)(best & 0xffffffffu);
+    __syncthreads();
+    return Weighed{ov, (int)(best & 0xffffffffu), ov > 0};
+}
+
+struct BalanceArgs {
+    int k, iters, seed, level, gcap;
+    int* part;
+    uint32_t* bw;
+    uint32_t* HS;        // k * kBalClasses, zero between calls
+    unsigned* counters;  // 2 kTeamSet, zero before the first call
+};
+
+// H, minvP and HS in the state the balance steps expect.
+__device__ __forceinline__ void balance_clear(Team& team, const SweepArgs& a, const BalanceArgs& B) {
+    for (long long i = team.rank(); i < (long long)B.k * kBalClasses; i += team.size()) B.HS[i] = 0;
+    for (long long i = team.rank(); i < (long long)B.k * a.P; i += team.size()) {
+        a.H[i] = 0;
+        a.minvP[i] = INT_MAX;
+    }
+}
+
+// The balance repair of lp.cu's balance(), all iterations; p: the counter
+// set in turn.  False: the team gave up.
+template <bool UNIT>
+__device__ __forceinline__ bool balance_steps(Team& team, SweepArgs a, const BalanceArgs& B, int& p, SweepSmem& sm,
+                                              WeighSmem& ws) {
+    a.lab = B.part;
+    a.lw = B.bw;
+    a.HS = B.HS;
+    a.lightest = &ws.lightest;
+    for (int it = 0; it < B.iters; ++it) {
+        if (!weigh(B.bw, B.k, a.bound, ws).over) return true;
+        a.ks_tie = stream_key(B.seed, TAG_BTIE, B.level, it);
+        a.ks_sub = stream_key(B.seed, TAG_BCLS, B.level, it);  // release class stream
+        const uint64_t ks_prio = stream_key(B.seed, TAG_BPRIO, B.level, it);
+        use_set(a, B.counters, p);
+        if (!team_sweep<BALANCE, UNIT, true>(team, a, B.gcap, sm)) return false;
+        // release thresholds, computed by every block for itself: the number
+        // of classes before which less than the excess is released
+        int* thr = reinterpret_cast<int*>(sm.tabs);
+        const int lane = threadIdx.x & 31;
+        for (int b = threadIdx.x >> 5; b < B.k; b += kWarpsPerBlock) {
+            const uint32_t x = B.bw[b];
+            if (x <= a.bound) {
+                if (lane == 0) thr[b] = 0;
+                continue;
+            }
+            const unsigned long long excess = x - a.bound;
+            unsigned long long h[kBalClasses / 32], sum = 0;
+#pragma unroll
+            for (int q = 0; q < kBalClasses / 32; ++q) {
+                h[q] = B.HS[(size_t)b * kBalClasses + lane * (kBalClasses / 32) + q];
+                sum += h[q];
+            }
+            unsigned long long run = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long y = __shfl_up_sync(0xffffffffu, run, o);
+                if (lane >= o) run += y;
+            }
+            run -= sum;
+            unsigned t = 0;
+#pragma unroll
+            for (int q = 0; q < kBalClasses / 32; ++q) {
+                t += run < excess ? 1u : 0u;
+                run += h[q];
+            }
+            t = __reduce_add_sync(0xffffffffu, t);
+            if (lane == 0) thr[b] = (int)t;
+        }
+        __syncthreads();
+        // released candidates get an admission class; others are dropped
+        each_proposal(a, [&](int v) {
+            if (v < 0) return;
+            const int t = a.pt[v];
+            if (t < 0) return;
+            if (a.pc[v] >= thr[B.part[v]]) {
+                a.pc[v] = -1;
+                return;
+            }
+            const int c = (int)hash_range(hash32(ks_prio, (uint32_t)v), (uint32_t)a.P);
+            a.pc[v] = c;
+            const size_t h = (size_t)t * a.P + c;
+            atomicAdd(&a.H[h], (uint32_t)a.vwgt[v]);
+            atomicMin(&a.minvP[h], v);
+        });
+        if (!team.sync()) return false;
+        each_proposal(a, [&](int v) {
+            if (v >= 0) class_decide_one(a, B.bw, 0, v);
+        });
+        if (!team.sync()) return false;
+        each_proposal(a, [&](int v) {
+            if (v >= 0) class_apply_one(a, B.part, B.bw, v);
+        });
+        for (int b = blockIdx.x; b < B.k; b += gridDim.x)
+            if (thr[b] > 0) B.HS[(size_t)b * kBalClasses + threadIdx.x] = 0;
+        static_assert(kBalClasses == kThreads, "a block clears one row of HS");
+        if (!team.sync()) return false;
+        p ^= 1;
+    }
+    return true;
+}
+
+// ------------------------------------------------------------ host helpers
+
+struct SweepBuffers {
+    int *pt, *pc;
+    unsigned* counters;  // [0, kStripes) unused, [kStripes, 2 kStripes) proposals,
+                         // [2 kStripes] heavy, [+1] heavy proposals, [+2] moved;
+                         // a team's two sets
+    int* heavy;
+    int* hplist;
+    SList plist;
+    int lblocks;
+    uint32_t *gtk, *gtv;
+    int gcap, hblocks;
+    unsigned long long* work;
+    int* err;
+};
+
+// Sweep buffers on the context's scratch, for the multi-launch sweeps
+// (team = 0) or for a team of that many blocks.
+SweepBuffers make_buffers(Ctx& ctx, const DevGraph& g, int team);
+SweepArgs base_args(const DevGraph& g, const SweepBuffers& b);
+
+// A team can sweep the level: its rows fit the blocks' shared-memory tables.
+inline bool team_rows(const DevGraph& g) { return g.maxdeg <= kSmemTab / 2; }
+// Blocks of a team that sweeps n vertices: a thread per vertex.
+inline long long team_want(long long n) { return (n + kThreads - 1) / kThreads; }
+
+}  // namespace sweep
+}  // namespace kb

@@ -1,0 +1,156 @@
+// team.cuh -- a kernel whose thread blocks work through the steps of one
+// phase together, with a barrier between steps, instead of one launch per
+// step.
+//
+// Why: on levels of up to a few hundred thousand nodes a step (a sweep, an
+// admission pass, a cut) takes 2-10 us of GPU time, and queueing it plus the
+// host's wait for its outcome takes longer than that; the same steps inside
+// one kernel are a barrier apart.  The barrier is __syncthreads for one
+// block, the cluster barrier for up to 8 blocks (hardware, co-scheduled by
+// definition), and for more blocks an arrival counter in global memory
+// under a cooperative launch, which guarantees that all blocks are resident.
+// The counter's wait is bounded: a team that gives up sets the error flag
+// and every block leaves the kernel at its next barrier.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <mutex>
+
+#include "common.cuh"
+#include "context.h"
+
+namespace kb {
+
+constexpr int kTeamThreads = 256;
+constexpr int kTeamCluster = 8;  // largest cluster every device accepts
+
+struct TeamArgs {
+    int kind;        // 0 one block, 1 one cluster, 2 cooperative grid
+    unsigned* bar;   // [0] arrivals, [1] given up, [2] exits; zero between launches
+    int* err;        // bit 1 is set when a wait runs out
+};
+
+class Team {
+public:
+    __device__ explicit Team(const TeamArgs& a) : a_(a), target_(0) {}
+    __device__ long long rank() const { return (long long)blockIdx.x * kTeamThreads + threadIdx.x; }
+    __device__ long long size() const { return (long long)gridDim.x * kTeamThreads; }
+    __device__ bool leader() const { return blockIdx.x == 0 && threadIdx.x == 0; }
+
+    // Every thread of the team calls it; what any of them wrote before is
+    // visible to all afterwards.  False: the team gave up, leave the kernel.
+    __device__ bool sync() {
+        if (a_.kind == 0) {
+            __syncthreads();
+            return true;
+        }
+        if (a_.kind == 1) {
+            asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+            return true;
+        }
+        __shared__ int dead;
+        target_ += gridDim.x;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicAdd(a_.bar, 1u);
+            int d = 0;
+            for (unsigned spin = 0;; ++spin) {
+                unsigned seen;
+                asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(a_.bar) : "memory");
+                if ((int)(seen - target_) >= 0) break;
+                if ((spin & 1023u) == 1023u) {
+                    // another block gave up, or this one has waited some seconds
+                    if (*(volatile unsigned*)(a_.bar + 1) || spin > (1u << 24)) {
+                        atomicExch(a_.bar + 1, 1u);
+                        atomicOr(a_.err, 2);
+                        d = 1;
+                        break;
+                    }
+                }
+            }
+            __threadfence();
+            dead = d;
+        }
+        __syncthreads();
+        return dead == 0;
+    }
+
+    // Last call of every thread (also after a failed sync): the last block
+    // to leave makes the counters ready for the next launch.
+    __device__ void leave() {
+        if (a_.kind != 2) return;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            if (atomicAdd(a_.bar + 2, 1u) == gridDim.x - 1) {
+                a_.bar[0] = 0;
+                a_.bar[1] = 0;
+                a_.bar[2] = 0;
+                __threadfence();
+            }
+        }
+    }
+
+private:
+    TeamArgs a_;
+    unsigned target_;
+};
+
+// Blocks of a team for `want` of them: as they are up to one cluster
+// (rounded up to a power of two), at most `most` above.
+inline int team_blocks(long long want, int most) {
+    if (want <= 1) return 1;
+    if (want <= kTeamCluster) {
+        int b = 2;
+        while (b < want) b <<= 1;
+        return b;
+    }
+    return (int)std::max<long long>(kTeamCluster, std::min<long long>(want, most));
+}
+
+// Blocks of `kernel` that are resident together on the context's device.
+template <class K>
+int team_most(Ctx& ctx, K kernel, size_t smem) {
+    int per = 0, sms = 0;
+    KB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kTeamThreads, smem));
+    KB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
+    return per * sms;
+}
+
+// Launches kernel(args..., TeamArgs) on `blocks` blocks (a team_blocks()
+// value).  False when the device cannot hold that many blocks at once (it is
+// shared with other work): nothing was launched.
+template <class K, class... Args>
+bool launch_team(Ctx& ctx, K kernel, int blocks, size_t smem, Args... args) {
+    TeamArgs t{blocks == 1 ? 0 : blocks <= kTeamCluster ? 1 : 2, ctx.team_bar, ctx.dscalars + 60};
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(kTeamThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx.stream;
+    cudaLaunchAttribute at{};
+    if (t.kind == 1) {
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)blocks;
+        at.val.clusterDim.y = 1;
+        at.val.clusterDim.z = 1;
+    } else if (t.kind == 2) {
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+    }
+    cfg.attrs = &at;
+    cfg.numAttrs = t.kind == 0 ? 0 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args..., t);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    KB_CUDA(e);
+    KB_LAUNCH();
+    return true;
+}
+
+}  // namespace kb

@@ -1,0 +1,87 @@
+"""Phases that a team of thread blocks runs in one kernel, against the CPU
+oracle, at the sizes where the team changes form (one block, a cluster, a
+cooperative grid; 256 vertices per block) and at the limits of its rule (rows
+of 2048 entries, 8192 blocks), just past which the per-step launches take
+over.  Integer outputs: equality.
+"""
+import numpy as np
+import pytest
+
+from conftest import csr_from_edges
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def N():
+    from kahip_b200 import native
+    assert native.device_count() > 0, "no CUDA device"
+    return native
+
+
+@pytest.fixture(scope="module")
+def O():
+    from oracle import oracle
+    return oracle
+
+
+def weighted(g, seed):
+    rng = np.random.default_rng(seed)
+    g["vwgt"] = rng.integers(0, 6, g["n"]).astype(np.int32)
+    src = np.repeat(np.arange(g["n"]), np.diff(g["xadj"]))
+    lo, hi = np.minimum(src, g["adjncy"]).astype(np.int64), np.maximum(src, g["adjncy"]).astype(np.int64)
+    g["adjwgt"] = ((lo * 31 + hi * 17 + seed) % 7).astype(np.int32)  # zero weights among them
+    return g
+
+
+def hub_graph(n, hub, seed):
+    """A ring, one vertex of `hub` neighbours and some of 100-400."""
+    rng = np.random.default_rng(seed)
+    edges = {(v, v + 1) for v in range(1, n - 1)}
+    edges |= {(0, v) for v in range(1, hub + 1)}
+    for c in (5, 900):
+        edges |= {(min(c, int(u)), max(c, int(u))) for u in rng.choice(np.arange(1000, n), 100 + 300 * (c > 5), False)}
+    return csr_from_edges(n, sorted(edges))
+
+
+def skewed(n, k, seed):
+    """Most vertices in the first blocks: the balance repair has work."""
+    rng = np.random.default_rng(seed)
+    p = np.minimum(rng.integers(0, k, n), rng.integers(0, k, n)).astype(np.int32)
+    return p
+
+
+SIZES = [1, 31, 255, 256, 257, 511, 513, 1024, 2047, 2048, 2049, 2305, 8192, 40001, 160000]
+
+
+@pytest.mark.parametrize("n", SIZES)
+@pytest.mark.parametrize("k", [2, 13])
+def test_jet_sizes(N, O, graphs, n, k):
+    g = graphs.rgg2d(n, seed=n) if n > 31 else csr_from_edges(n, [(i, i + 1) for i in range(n - 1)])
+    for unit in (True, False):
+        if not unit:
+            weighted(g, n)
+        kn_o, kn_p = O.knobs(g, k, 0.03, 5, 1), N.derive_knobs(n, g["vwgt"], k, 0.03, 5, 1)
+        part = skewed(n, k, n)
+        for level in (0, 1):
+            assert np.array_equal(O.jet_refine(g, kn_o, part, kn_o.upper_bound, level),
+                                  N.jet_refine(g, kn_p, part, kn_p.upper_bound, level))
+
+
+@pytest.mark.parametrize("hub", [128, 129, 256, 257, 2048, 2049])
+def test_jet_hubs(N, O, hub):
+    g = hub_graph(5000, hub, hub)
+    for k in (2, 40):
+        kn_o, kn_p = O.knobs(g, k, 0.03, 1, 1), N.derive_knobs(g["n"], g["vwgt"], k, 0.03, 1, 1)
+        part = skewed(g["n"], k, hub)
+        assert np.array_equal(O.jet_refine(g, kn_o, part, kn_o.upper_bound, 1),
+                              N.jet_refine(g, kn_p, part, kn_p.upper_bound, 1))
+
+
+@pytest.mark.parametrize("k", [8192, 8193])
+def test_jet_many_blocks(N, O, graphs, k):
+    g = graphs.rgg2d(20000, seed=2)
+    kn_o, kn_p = O.knobs(g, k, 0.10, 1, 1), N.derive_knobs(g["n"], g["vwgt"], k, 0.10, 1, 1)
+    part = skewed(g["n"], k, 3)
+    assert np.array_equal(O.jet_refine(g, kn_o, part, kn_o.upper_bound, 0),
+                          N.jet_refine(g, kn_p, part, kn_p.upper_bound, 0))
