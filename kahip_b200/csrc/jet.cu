@@ -83,12 +83,14 @@ __device__ __forceinline__ void candidate(const JetArgs& A, int v, int own, long
 // or row deferred to choose_wide (whose scan then sums its cut).  Four
 // entries are loaded together.  UNIT: every edge weight is 1 (adjwgt is not
 // read).
-template <bool UNIT>
+// DENSE: rows of more than kDeferRow entries are choose_row's.
+template <bool UNIT, bool DENSE>
 __device__ __forceinline__ void choose_one(const JetArgs& A, int v, unsigned long long& cut) {
+    const int beg = A.xadj[v], end = A.xadj[v + 1];
+    if (DENSE && end - beg > sweep::kDeferRow) return;
     A.dest[v] = -1;
     const bool locked = A.moved_at[v] == A.it - 1;
-    const int beg = A.xadj[v], end = A.xadj[v + 1];
-    if (end - beg > kLaneRow) {
+    if (!DENSE && end - beg > kLaneRow) {
         A.wide[atomicAdd(A.nwide, 1u)] = locked ? (v | kLocked) : v;
         return;
     }
@@ -152,7 +154,7 @@ template <bool UNIT>
 __global__ void __launch_bounds__(kThreads) jet_choose(JetArgs A) {
     unsigned long long cut = 0;
     for (long long v = (long long)blockIdx.x * kThreads + threadIdx.x; v < A.n; v += (long long)gridDim.x * kThreads)
-        choose_one<UNIT>(A, (int)v, cut);
+        choose_one<UNIT, false>(A, (int)v, cut);
     add_cut(A, cut);
 }
 
@@ -365,24 +367,111 @@ struct JetLoop {
     uint32_t bound;
 };
 
-template <bool UNIT>
-__global__ void __launch_bounds__(kThreads, 4) jet_loop(JetLoop J, sweep::SweepArgs a, sweep::BalanceArgs B,
+// One vertex by a warp (BLOCK: by the whole block), its connections in the
+// counters cnt (k, zero between uses).
+template <bool UNIT, bool BLOCK>
+__device__ __forceinline__ void choose_row(const JetArgs& A, int v, uint32_t* cnt, sweep::RowRed& red,
+                                           unsigned long long& cut) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int t = BLOCK ? (int)threadIdx.x : lane;
+    constexpr int NT = BLOCK ? kThreads : 32;
+    const int beg = A.xadj[v], end = A.xadj[v + 1];
+    const int own = A.part[v];
+    const bool locked = A.moved_at[v] == A.it - 1;
+    long long co = 0;
+    for (int e = beg + t; e < end; e += 4 * NT) {
+        int b[4];
+        uint32_t w[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const bool in = e + q * NT < end;
+            b[q] = in ? A.adjncy[e + q * NT] : -1;
+            w[q] = in ? (UNIT ? 1u : (uint32_t)A.adjwgt[e + q * NT]) : 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) b[q] = b[q] >= 0 ? A.part[b[q]] : own;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (b[q] == own) {
+                co += w[q];
+            } else {
+                cut += w[q];
+                if (!locked) atomicAdd(&cnt[b[q]], w[q]);
+            }
+        }
+    }
+    if (t == 0) A.dest[v] = -1;
+    if (locked) return;  // uniform over the group
+    if (BLOCK) __syncthreads();
+    else __syncwarp();
+    uint64_t key = 0;
+    uint32_t id = kNone;
+    for (int b = t; b < A.k; b += NT) {
+        const uint32_t c = cnt[b];
+        if (c == 0) continue;
+        cnt[b] = 0;
+        sweep::better(key, id, sweep::cand_key(c, A.ks_tie, (uint32_t)b), (uint32_t)b);
+    }
+    sweep::group_argmax<32>(key, id, 0xffffffffu);
+#pragma unroll
+    for (int off = 16; off; off >>= 1) co += __shfl_xor_sync(0xffffffffu, co, off);
+    if (BLOCK) {
+        if (lane == 0) {
+            red.key[wid] = key;
+            red.id[wid] = id;
+            red.own[wid] = co;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 1; w < kThreads / 32; ++w) {
+                sweep::better(key, id, red.key[w], red.id[w]);
+                co += red.own[w];
+            }
+    }
+    if (t == 0) candidate(A, v, own, co, id, (uint32_t)(key >> 32));
+    if (BLOCK) __syncthreads();
+    else __syncwarp();
+}
+
+// Rows of more than kDeferRow entries, listed once per level: a warp's from
+// the front of `list`, a block's from its end.
+struct JetRows {
+    int* list;
+    unsigned* count;  // [0] a warp's, [1] a block's
+};
+
+template <bool UNIT, bool DENSE>
+__global__ void __launch_bounds__(kThreads, 4) jet_loop(JetLoop J, JetRows R, sweep::SweepArgs a, sweep::BalanceArgs B,
                                                         TeamArgs T) {
-    __shared__ sweep::SweepSmem sm;
+    __shared__ sweep::SweepQueue queue;
     __shared__ sweep::WeighSmem ws;
+    __shared__ sweep::RowRed red;
+    extern __shared__ __align__(16) unsigned char dyn[];
     Team team(T);
     const int n = J.A.n, k = J.A.k;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned W = gridDim.x * (kThreads / 32), wg = blockIdx.x + wid * gridDim.x;
+    const sweep::TeamSpace S = sweep::team_space<DENSE>(dyn, k);
     sweep::balance_clear(team, a, B);
-    for (long long v = team.rank(); v < n; v += team.size()) J.moved_at[v] = -2;
     if (blockIdx.x == 0) {
         for (int i = threadIdx.x; i < 2 * sweep::kTeamSet; i += kThreads) B.counters[i] = 0;
         if (threadIdx.x < 4) J.ring[threadIdx.x] = 0;
         if (threadIdx.x < 2) J.cut[threadIdx.x] = 0;
     }
-    if ((int)blockIdx.x < J.wblocks)
-        for (int b = threadIdx.x; b < k; b += kThreads) J.counters[(size_t)blockIdx.x * k + b] = 0;
+    for (long long base = (long long)blockIdx.x * kThreads; base < n; base += team.size()) {
+        const int v = (int)(base + threadIdx.x);
+        if (v < n) J.moved_at[v] = -2;
+        if constexpr (DENSE) {
+            const int d = v < n ? J.A.xadj[v + 1] - J.A.xadj[v] : 0;
+            sweep::append_aggregated(d > sweep::kDeferRow && d <= sweep::kHugeDense, v, R.list, R.count);
+            if (d > sweep::kHugeDense) R.list[n - 1 - (int)atomicAdd(R.count + 1, 1u)] = v;
+        }
+    }
+    if constexpr (!DENSE)
+        if ((int)blockIdx.x < J.wblocks)
+            for (int b = threadIdx.x; b < k; b += kThreads) J.counters[(size_t)blockIdx.x * k + b] = 0;
     bool alive = team.sync();
+    const unsigned nrow = DENSE ? R.count[0] : 0, nhuge = DENSE ? R.count[1] : 0;
     int* cur = J.part;
     int* nxt = J.part2;
     unsigned long long best_ov = 0;
@@ -403,19 +492,34 @@ __global__ void __launch_bounds__(kThreads, 4) jet_loop(JetLoop J, sweep::SweepA
         }
         unsigned long long cut = 0;
         if (it < J.iters) {
-            for (long long v = team.rank(); v < n; v += team.size()) choose_one<UNIT>(A, (int)v, cut);
+            for (long long v = team.rank(); v < n; v += team.size()) choose_one<UNIT, DENSE>(A, (int)v, cut);
+            if constexpr (DENSE) {
+                __syncwarp();
+                for (unsigned i = wg; i < nrow; i += W)
+                    choose_row<UNIT, false>(A, R.list[i], S.tab + (size_t)wid * k, red, cut);
+                if (nhuge) __syncthreads();  // the first warp's counters serve the block
+                for (unsigned i = blockIdx.x; i < nhuge; i += gridDim.x)
+                    choose_row<UNIT, true>(A, R.list[n - 1 - (int)i], S.tab, red, cut);
+            }
         } else {
-            for (long long v = team.rank(); v < n; v += team.size()) {
+            for (long long v = team.rank() / 32; v < n; v += team.size() / 32) {
                 const int own = cur[v];
-                for (int e = A.xadj[v]; e < A.xadj[v + 1]; ++e)
+                for (int e = A.xadj[v] + lane; e < A.xadj[v + 1]; e += 32)
                     if (cur[A.adjncy[e]] != own) cut += UNIT ? 1u : (uint32_t)A.adjwgt[e];
             }
         }
         __syncwarp();
         add_cut(A, cut);
         if (!(alive = team.sync())) break;
-        if (*A.nwide) {
-            if ((int)blockIdx.x < J.wblocks) choose_wide(A, J.counters + (size_t)blockIdx.x * k, J.wblocks);
+        if (const unsigned nw = *A.nwide) {
+            if constexpr (DENSE) {  // short rows of too many blocks for the slots
+                cut = 0;
+                for (unsigned i = wg; i < nw; i += W)
+                    choose_row<UNIT, false>(A, A.wide[i], S.tab + (size_t)wid * k, red, cut);
+                add_cut(A, cut);
+            } else if ((int)blockIdx.x < J.wblocks) {
+                choose_wide(A, J.counters + (size_t)blockIdx.x * k, J.wblocks);
+            }
             if (!(alive = team.sync())) break;
         }
         // best tracking and the stopping rule (jet_track), by every block
@@ -444,28 +548,7 @@ __global__ void __launch_bounds__(kThreads, 4) jet_loop(JetLoop J, sweep::SweepA
                 for (int b = threadIdx.x; b < k; b += kThreads) J.best_bw[b] = J.bw2[b];
         }
         unsigned moves = 0;
-        for (long long base = (long long)blockIdx.x * kThreads; base < n; base += team.size()) {
-            const int v = (int)(base + threadIdx.x);
-            const bool in = v < n;
-            const int own = in ? cur[v] : 0;
-            const int d = in ? A.dest[v] : -1;
-            int beg = 0, end = 0;
-            if (d >= 0) { beg = A.xadj[v]; end = A.xadj[v + 1]; }
-            const bool wide = end - beg > kLaneRow;
-            bool keep = false;
-            unsigned wm = __ballot_sync(0xffffffffu, wide);
-            while (wm) {
-                const int s = __ffs(wm) - 1;
-                wm &= wm - 1;
-                const int hv = __shfl_sync(0xffffffffu, v, s);
-                const int hb = __shfl_sync(0xffffffffu, beg, s), he = __shfl_sync(0xffffffffu, end, s);
-                long long adj = afterburn_sum<UNIT>(A, hv, hb, he, 32, lane);
-#pragma unroll
-                for (int off = 16; off; off >>= 1) adj += __shfl_xor_sync(0xffffffffu, adj, off);
-                if (lane == s) keep = adj >= 0;
-            }
-            if (d >= 0 && !wide) keep = afterburn_sum<UNIT>(A, v, beg, end, 1, 0) >= 0;
-            if (!in) continue;
+        auto settle = [&](int v, int own, int d, bool keep) {
             if (part_is_best) J.best[v] = own;
             nxt[v] = keep ? d : own;
             if (keep) {
@@ -474,6 +557,47 @@ __global__ void __launch_bounds__(kThreads, 4) jet_loop(JetLoop J, sweep::SweepA
                 atomicAdd(&J.bw[d], w);
                 J.moved_at[v] = it;
                 ++moves;
+            }
+        };
+        constexpr int kRow = DENSE ? sweep::kDeferRow : kLaneRow;
+        for (long long base = (long long)blockIdx.x * kThreads; base < n; base += team.size()) {
+            const int v = (int)(base + threadIdx.x);
+            const bool in = v < n;
+            const int own = in ? cur[v] : 0;
+            int beg = 0, end = 0;
+            if (in) { beg = A.xadj[v]; end = A.xadj[v + 1]; }
+            const bool wide = end - beg > kRow;
+            // (a long row's destination is read where the row is)
+            const int d = in && !(DENSE && wide) ? A.dest[v] : -1;
+            bool keep = false;
+            if constexpr (!DENSE) {
+                unsigned wm = __ballot_sync(0xffffffffu, wide && d >= 0);
+                while (wm) {
+                    const int s = __ffs(wm) - 1;
+                    wm &= wm - 1;
+                    const int hv = __shfl_sync(0xffffffffu, v, s);
+                    const int hb = __shfl_sync(0xffffffffu, beg, s), he = __shfl_sync(0xffffffffu, end, s);
+                    long long adj = afterburn_sum<UNIT>(A, hv, hb, he, 32, lane);
+#pragma unroll
+                    for (int off = 16; off; off >>= 1) adj += __shfl_xor_sync(0xffffffffu, adj, off);
+                    if (lane == s) keep = adj >= 0;
+                }
+            }
+            if (d >= 0 && !wide) keep = afterburn_sum<UNIT>(A, v, beg, end, 1, 0) >= 0;
+            if (in && !(DENSE && wide)) settle(v, own, d, keep);
+        }
+        if constexpr (DENSE) {
+            __syncwarp();
+            for (unsigned i = wg; i < nrow + nhuge; i += W) {
+                const int v = i < nrow ? R.list[i] : R.list[n - 1 - (int)(i - nrow)];
+                const int d = A.dest[v];
+                long long adj = -1;
+                if (d >= 0) {
+                    adj = afterburn_sum<UNIT>(A, v, A.xadj[v], A.xadj[v + 1], 32, lane);
+#pragma unroll
+                    for (int off = 16; off; off >>= 1) adj += __shfl_xor_sync(0xffffffffu, adj, off);
+                }
+                if (lane == 0) settle(v, cur[v], d, d >= 0 && adj >= 0);
             }
         }
         __syncwarp();
@@ -486,7 +610,7 @@ __global__ void __launch_bounds__(kThreads, 4) jet_loop(JetLoop J, sweep::SweepA
             nxt = t;
         }
         B.part = cur;
-        alive = sweep::balance_steps<UNIT>(team, a, B, p, sm, ws);
+        alive = sweep::balance_steps<UNIT, DENSE>(team, a, B, p, queue, S, red, ws);
     }
     if (alive) {
         const int* src = part_is_best ? cur : J.best;
@@ -507,19 +631,22 @@ int grid_for(long long items) {
     return (int)std::max<long long>(1, std::min<long long>(div_up(items, kThreads), (long long)kNumSMs * 16));
 }
 
-// The loop as one team kernel; false when the level is not one for it:
-// thresholds of more than kTeamMaxBlocks blocks or rows of more than
-// kSmemTab / 2 entries do not fit the blocks' shared memory.  There is no
+// The loop as one team kernel; false when the level is not one for it
+// (sweep::team_fits).  There is no
 // line by size: at 4.0M nodes / 58M entries (33 iterations, eco) the level
 // loop took 9 ms in one kernel against 13 ms as launches, at 1k nodes (61
 // iterations over three levels) 0.57 ms against 5.0 ms.
 bool jet_refine_team(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, uint32_t bound, int* part,
                      uint32_t* bw) {
     const int n = g.n, k = kn.k;
-    if (k > sweep::kTeamMaxBlocks || !sweep::team_rows(g)) return false;
+    if (!sweep::team_fits(g, k)) return false;
     const size_t mk = ctx.scratch.mark();
-    auto kernel = g.unit_weights ? jet_loop<true> : jet_loop<false>;
-    const int blocks = team_blocks(sweep::team_want(n), team_most(ctx, kernel, 0));
+    const bool dense = sweep::team_dense(k);
+    auto kernel = dense ? (g.unit_weights ? jet_loop<true, true> : jet_loop<false, true>)
+                        : (g.unit_weights ? jet_loop<true, false> : jet_loop<false, false>);
+    const size_t smem = sweep::team_smem(k, dense);
+    const TeamRoom room = team_room(ctx, (const void*)kernel, smem);
+    const int blocks = team_blocks(room, sweep::team_want(g));
     JetLoop J{};
     J.part = part;
     J.part2 = ctx.scratch.alloc<int>((size_t)n);
@@ -530,7 +657,13 @@ bool jet_refine_team(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, ui
     J.vwgt = g.vwgt;
     J.moved_at = ctx.scratch.alloc<int>((size_t)n);
     J.wblocks = std::min(blocks, 2 * kNumSMs);
-    J.counters = ctx.scratch.alloc<uint32_t>((size_t)J.wblocks * k);
+    if (!dense) J.counters = ctx.scratch.alloc<uint32_t>((size_t)J.wblocks * k);
+    JetRows R{};
+    if (dense) {
+        R.list = ctx.scratch.alloc<int>((size_t)n);
+        R.count = ctx.scratch.alloc<unsigned>(2);
+        KB_CUDA(cudaMemsetAsync(R.count, 0, 2 * sizeof(unsigned), ctx.stream));
+    }
     J.cut = ctx.scratch.alloc<unsigned long long>(2);
     J.ring = ctx.scratch.alloc<unsigned>(4);
     J.iters = kn.jet_iters;
@@ -561,14 +694,13 @@ bool jet_refine_team(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, ui
     B.iters = kn.bal_iters;
     B.seed = kn.seed;
     B.level = level;
-    B.gcap = b.gcap;
     B.bw = bw;
     B.HS = ctx.scratch.alloc<uint32_t>((size_t)k * sweep::kBalClasses);
     B.counters = b.counters;
     bool done;
     {
         PhaseScope ps(ctx, "jet_loop", 0);
-        done = launch_team(ctx, kernel, blocks, 0, J, a, B);
+        done = launch_team(ctx, kernel, room, blocks, smem, J, R, a, B);
     }
     ctx.scratch.release(mk);
     return done;

@@ -33,7 +33,7 @@ namespace {
 template <int MODE, bool UNIT, bool STASH>
 __global__ void __launch_bounds__(kThreads, 4) lane_kernel(SweepArgs a) {
     __shared__ SweepSmem sm;
-    lane_sweep<MODE, UNIT, STASH>(a, sm);
+    lane_sweep<MODE, UNIT, STASH, 0>(a, sm.queue, sm.oqueue, sm.tabs);
 }
 
 template <int MODE, int BT>
@@ -245,7 +245,7 @@ SweepBuffers sweep::make_buffers(Ctx& ctx, const DevGraph& g, int team) {
     b.gcap = 0;
     b.hblocks = 0;
     b.gtk = b.gtv = nullptr;
-    if (g.maxdeg > kWin) {
+    if (g.maxdeg > kWin && !team) {
         int cap = 1;
         while (cap < 2 * g.maxdeg) cap <<= 1;
         b.gcap = cap;
@@ -358,6 +358,179 @@ double sweep_bytes(const DevGraph& g, double frac) {
 
 }  // namespace
 
+// ------------------------------------------------------------- team kernels
+
+namespace {
+
+struct RefineArgs {
+    int k, rounds, subrounds, seed, level;
+    int* part;
+    uint32_t* bw;
+    const uint8_t* active0;
+    uint8_t* flags[2];   // n, to a multiple of 4
+    uint32_t* stamp;     // n
+    int* list[2];        // n
+    unsigned* lcount;    // [2]
+    unsigned* moved;     // [2]
+    unsigned* counters;  // 2 kTeamSet
+};
+
+// All rounds of one level's refinement, ending after a round without moves.
+template <bool UNIT, bool DENSE>
+__global__ void __launch_bounds__(kThreads, 4) refine_team(SweepArgs a, RefineArgs R, TeamArgs T) {
+    __shared__ SweepQueue queue;
+    __shared__ RowRed red;
+    extern __shared__ __align__(16) unsigned char dyn[];
+    Team team(T);
+    const TeamSpace S = team_space<DENSE>(dyn, R.k);
+    const int lane = threadIdx.x & 31;
+    for (long long i = team.rank(); i < (long long)R.k * a.P; i += team.size()) {
+        a.H[i] = 0;
+        a.minvP[i] = INT_MAX;
+    }
+    for (long long v = team.rank(); v < a.n; v += team.size()) R.stamp[v] = 0;
+    if (blockIdx.x == 0) {
+        for (int i = threadIdx.x; i < 2 * kTeamSet; i += kThreads) R.counters[i] = 0;
+        if (threadIdx.x < 2) R.moved[threadIdx.x] = R.lcount[threadIdx.x] = 0;
+    }
+    bool alive = team.sync();
+    bool flags_in = false;
+    unsigned long long moved_prev = ~0ull;
+    int p = 0;
+    for (int r = 0; alive && r < R.rounds; ++r) {
+        const int in = r & 1, out = in ^ 1;
+        uint8_t* const flags_next = in ? R.flags[0] : R.flags[1];
+        a.active = r == 0 ? R.active0 : flags_in ? (in ? R.flags[1] : R.flags[0]) : nullptr;
+        a.vlist = r > 0 && !flags_in ? (in ? R.list[1] : R.list[0]) : nullptr;
+        a.vcount = R.lcount + in;
+        // the next round's set: flags when the last known round moved many,
+        // else a list (lp_refine)
+        const bool flags_out = moved_prev == ~0ull || moved_prev * 64 > (unsigned long long)a.n;
+        const NextActive na{flags_out ? flags_next : nullptr, R.stamp, (uint32_t)r + 1u, in ? R.list[0] : R.list[1],
+                            R.lcount + out, nullptr, nullptr};
+        a.ks_sub = stream_key(R.seed, TAG_RSUB, R.level, r);
+        a.ks_tie = stream_key(R.seed, TAG_RTIE, R.level, r);
+        a.ks_prio = stream_key(R.seed, TAG_RPRIO, R.level, r);
+        for (uint32_t s = 0; s < a.S; ++s, p ^= 1) {
+            a.s = s;
+            use_set(a, R.counters, p);
+            if (s == 0) {  // what round r - 1 swept from
+                if (flags_out)
+                    for (long long i = team.rank(); i < (a.n + 3LL) / 4; i += team.size())
+                        reinterpret_cast<uint32_t*>(flags_next)[i] = 0;
+                if (team.leader()) R.lcount[out] = 0;
+            }
+            if (!(alive = team_sweep<REFINE, UNIT, DENSE>(team, a, queue, S, red))) break;
+            if (s == 0 && team.leader()) R.moved[out] = 0;  // every block has read it by now
+            each_proposal(a, [&](int v) {
+                if (v >= 0) class_decide_one(a, R.bw, 1, v);
+            });
+            if (!(alive = team.sync())) break;
+            unsigned mv = 0;
+            each_proposal(a, [&](int v) {
+                const bool moved = v >= 0 && class_apply_one(a, R.part, R.bw, v);
+                int e0 = 0, e1 = 0;
+                if (moved) {
+                    ++mv;
+                    e0 = a.xadj[v];
+                    e1 = a.xadj[v + 1];
+                    if (e1 - e0 <= kHubMark) mark_row(na, a.adjncy, e0, e1, 0, 1);
+                }
+                __syncwarp();
+                // longer rows by the whole warp
+                unsigned wm = __ballot_sync(0xffffffffu, e1 - e0 > kHubMark);
+                while (wm) {
+                    const int src = __ffs(wm) - 1;
+                    wm &= wm - 1;
+                    const int b = __shfl_sync(0xffffffffu, e0, src), e = __shfl_sync(0xffffffffu, e1, src);
+                    mark_row(na, a.adjncy, b, e, lane, 32);
+                    __syncwarp();
+                }
+            });
+            __syncwarp();
+            mv = __reduce_add_sync(0xffffffffu, mv);
+            if (lane == 0 && mv) atomicAdd(R.moved + in, mv);
+            if (!(alive = team.sync())) break;
+        }
+        if (!alive) break;
+        const unsigned mv = R.moved[in];
+        if (mv == 0) break;
+        moved_prev = mv;
+        flags_in = flags_out;
+    }
+    team.leave();
+}
+
+// The balance repair; *ok = every block ended within the bound.
+template <bool UNIT, bool DENSE>
+__global__ void __launch_bounds__(kThreads, 4) balance_team(SweepArgs a, BalanceArgs B, int* ok, TeamArgs T) {
+    __shared__ SweepQueue queue;
+    __shared__ RowRed red;
+    __shared__ WeighSmem ws;
+    extern __shared__ __align__(16) unsigned char dyn[];
+    Team team(T);
+    const TeamSpace S = team_space<DENSE>(dyn, B.k);
+    balance_clear(team, a, B);
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < 2 * kTeamSet; i += kThreads) B.counters[i] = 0;
+    int p = 0;
+    const bool alive = team.sync() && balance_steps<UNIT, DENSE>(team, a, B, p, queue, S, red, ws);
+    if (alive && blockIdx.x == 0) {
+        const bool over = weigh(B.bw, B.k, a.bound, ws).over;
+        if (threadIdx.x == 0) *ok = over ? 0 : 1;
+    }
+    team.leave();
+}
+
+// The level's whole refinement in one kernel; false when it is not one for it.
+bool lp_refine_team(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, uint32_t bound, int* part, uint32_t* bw,
+                    const uint8_t* active0) {
+    if (!team_fits(g, kn.k)) return false;
+    const size_t mk = ctx.scratch.mark();
+    const size_t n = (size_t)g.n;
+    const bool dense = team_dense(kn.k);
+    auto kernel = dense ? (g.unit_weights ? refine_team<true, true> : refine_team<false, true>)
+                        : (g.unit_weights ? refine_team<true, false> : refine_team<false, false>);
+    const size_t smem = team_smem(kn.k, dense);
+    const TeamRoom room = team_room(ctx, (const void*)kernel, smem);
+    const int blocks = team_blocks(room, team_want(g));
+    const SweepBuffers b = make_buffers(ctx, g, blocks);
+    SweepArgs a = base_args(g, b);
+    RefineArgs R{};
+    R.k = kn.k;
+    R.rounds = kn.ref_rounds;
+    R.subrounds = kn.ref_subrounds;
+    R.seed = kn.seed;
+    R.level = level;
+    R.part = part;
+    R.bw = bw;
+    R.active0 = active0;
+    R.flags[0] = ctx.scratch.alloc<uint8_t>(n + 3);
+    R.flags[1] = ctx.scratch.alloc<uint8_t>(n + 3);
+    R.stamp = ctx.scratch.alloc<uint32_t>(n);
+    R.list[0] = ctx.scratch.alloc<int>(n);
+    R.list[1] = ctx.scratch.alloc<int>(n);
+    R.lcount = ctx.scratch.alloc<unsigned>(2);
+    R.moved = ctx.scratch.alloc<unsigned>(2);
+    R.counters = b.counters;
+    a.lab = part;
+    a.lw = bw;
+    a.bound = bound;
+    a.S = (uint32_t)kn.ref_subrounds;
+    a.P = kn.ref_classes;
+    a.H = ctx.scratch.alloc<uint32_t>((size_t)kn.k * a.P);
+    a.minvP = ctx.scratch.alloc<int>((size_t)kn.k * a.P);
+    bool done;
+    {
+        PhaseScope ps(ctx, "lp_refine_team", 0);
+        done = launch_team(ctx, kernel, room, blocks, smem, a, R);
+    }
+    ctx.scratch.release(mk);
+    return done;
+}
+
+}  // namespace
+
 // --------------------------------------------------------------- clustering
 
 __global__ void tie_hash_kernel(int n, uint64_t ks, uint32_t* tie) {
@@ -366,6 +539,7 @@ __global__ void tie_hash_kernel(int n, uint64_t ks, uint32_t* tie) {
 }
 
 void lp_cluster(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, int* label) {
+    const bool sorted_rows = g.rows_sorted >= 0 ? g.rows_sorted == 1 : rows_strictly_increasing(ctx, g);
     const size_t mk = ctx.scratch.mark();
     cudaStream_t st = ctx.stream;
     const size_t n = (size_t)std::max(g.n, 1);
@@ -383,7 +557,6 @@ void lp_cluster(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, int* la
     a.S = (uint32_t)kn.lpc_subrounds;
     a.inc = inc;
     a.minv = minv;
-    const bool sorted_rows = g.rows_sorted >= 0 ? g.rows_sorted == 1 : rows_strictly_increasing(ctx, g);
     for (int r = 0; r < kn.lpc_rounds; ++r) {
         a.ks_sub = stream_key(kn.seed, TAG_CSUB, level, r);
         a.ks_tie = stream_key(kn.seed, TAG_CTIE, level, r);
@@ -438,6 +611,7 @@ void lp_cluster(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, int* la
 void lp_refine(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, uint32_t bound, int* part,
                uint32_t* bw, const uint8_t* active0) {
     if (g.n == 0) return;
+    if (lp_refine_team(ctx, g, kn, level, bound, part, bw, active0)) return;
     const size_t mk = ctx.scratch.mark();
     cudaStream_t st = ctx.stream;
     const int k = kn.k, P = kn.ref_classes;
@@ -558,6 +732,33 @@ bool balance(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, uint32_t b
     uint32_t* H = ctx.scratch.alloc<uint32_t>((size_t)k * P);
     int* minvP = ctx.scratch.alloc<int>((size_t)k * P);
     uint32_t* HS = ctx.scratch.alloc<uint32_t>((size_t)k * kBalClasses);
+    if (team_fits(g, k)) {
+        const bool dense = team_dense(k);
+        auto kernel = dense ? (g.unit_weights ? balance_team<true, true> : balance_team<false, true>)
+                            : (g.unit_weights ? balance_team<true, false> : balance_team<false, false>);
+        const size_t smem = team_smem(k, dense), mk2 = ctx.scratch.mark();
+        const TeamRoom room = team_room(ctx, (const void*)kernel, smem);
+        const int blocks = team_blocks(room, team_want(g));
+        const SweepBuffers b = make_buffers(ctx, g, blocks);
+        SweepArgs a = base_args(g, b);
+        a.bound = bound;
+        a.P = P;
+        a.H = H;
+        a.minvP = minvP;
+        const BalanceArgs B{k, kn.bal_iters, kn.seed, level, part, bw, HS, b.counters};
+        bool done;
+        {
+            PhaseScope ps(ctx, "balance", 0);
+            done = launch_team(ctx, kernel, room, blocks, smem, a, B, flags);
+        }
+        ctx.scratch.release(mk2);
+        if (done) {
+            KB_CUDA(cudaMemcpyAsync(ctx.pinned, flags, sizeof(int), cudaMemcpyDeviceToHost, st));
+            KB_CUDA(cudaStreamSynchronize(st));
+            ctx.scratch.release(mk);
+            return ctx.pinned[0] != 0;
+        }
+    }
     int* thr = ctx.scratch.alloc<int>((size_t)k);
     SweepBuffers b = make_buffers(ctx, g, 0);
     fill_u32(H, (long long)k * P, 0u, st);

@@ -19,6 +19,7 @@
 #include "learned.cuh"
 #include "match.cuh"
 #include "prims.cuh"
+#include "team.cuh"
 
 namespace kb {
 
@@ -53,6 +54,43 @@ void Ctx::init(int dev, cudaStream_t s) {
         KB_CUDA(cudaStreamSynchronize(stream));  // later calls may run on a caller's stream
     }
     (void)s;
+}
+
+TeamRoom team_room(Ctx& ctx, const void* kernel, size_t smem) {
+    struct Known {
+        const void* kernel;
+        int device;
+        size_t smem;
+        TeamRoom room;
+    };
+    static std::mutex mu;
+    static std::vector<Known> known;
+    std::lock_guard<std::mutex> lk(mu);
+    for (const Known& k : known)
+        if (k.kernel == kernel && k.device == ctx.device && k.smem == smem) return k.room;
+    TeamRoom r{0, false};
+    int per = 0, sms = 0, clusters = 0;
+    if (smem > 40 * 1024)  // with the kernel's own shared memory above the default limit
+        KB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+    KB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kTeamThreads, smem));
+    KB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
+    r.most = per * sms;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = kTeamCluster;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kTeamCluster);
+    cfg.blockDim = dim3(kTeamThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    r.wide_cluster = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                     cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
+    if (!r.wide_cluster) (void)cudaGetLastError();
+    known.push_back(Known{kernel, ctx.device, smem, r});
+    return r;
 }
 
 int Ctx::phase_id(const char* name) {

@@ -59,6 +59,7 @@ struct SweepArgs {
     uint32_t* H;                        // REFINE/BALANCE: weight per (target, class)
     int* minvP;                         // smallest proposer per (target, class)
     int* heavy; unsigned* hcount;       // deferred high-degree vertices
+    unsigned* hugecount;                // a team: those listed from heavy's end
     SList plist;                        // vertices that proposed a move this sub-round
     int* hplist; unsigned* hpcount;     // proposals of high-degree vertices
     int singletons;                     // every label is its own vertex id and rows have
@@ -82,23 +83,6 @@ struct SweepArgs {
 
 __device__ __forceinline__ uint32_t table_slot(uint32_t key, int cap) {
     return (key * 0x9E3779B1u) >> (32 - __ffs(cap) + 1);
-}
-
-// Linear probing; the caller guarantees fewer distinct keys than cap/2, so
-// the probe ends within cap steps.  The bound only guards against a broken
-// invariant: the key is then dropped and *err is set.
-__device__ __forceinline__ void table_insert(uint32_t* tk, uint32_t* tv, int cap, uint32_t key,
-                                             uint32_t val, int* err) {
-    uint32_t s = table_slot(key, cap);
-    for (int probe = 0; probe < cap; ++probe) {
-        uint32_t prev = atomicCAS(&tk[s], kEmpty, key);
-        if (prev == kEmpty || prev == key) {
-            atomicAdd(&tv[s], val);
-            return;
-        }
-        s = (s + 1) & (uint32_t)(cap - 1);
-    }
-    atomicOr(err, 1);
 }
 
 // candidate key: larger connection first, then smaller tie hash; id breaks
@@ -130,9 +114,8 @@ __device__ __forceinline__ bool cand_ok(const SweepArgs& a, uint32_t b, uint32_t
 
 __device__ __forceinline__ int loss_bucket(long long loss) {
     if (loss <= 0) return 0;
-    int b = 1;
-    while (b < 31 && (loss >> b) > 0) ++b;
-    return b;
+    const int bits = 64 - __clzll(loss);
+    return bits < 31 ? bits : 31;
 }
 
 // Final decision for vertex v (executed by one lane).
@@ -414,11 +397,11 @@ __device__ __forceinline__ int nth_set_bit(unsigned mask, int r) {
 }
 
 // 0: decided (stays), 3: decided (proposes a move), 1: too many distinct
-// labels for NS slots, 2: degree above kWin
-template <int MODE, int NS, bool UNIT, bool STASH>
+// labels for NS slots, 2: degree above ROW
+template <int MODE, int NS, bool UNIT, bool STASH, int ROW>
 __device__ __forceinline__ int lane_vertex(const SweepArgs& a, int v, uint32_t* st, unsigned& wv, unsigned& we) {
     const int beg = a.xadj[v], end = a.xadj[v + 1];
-    if (end - beg > kWin) return 2;
+    if (end - beg > ROW) return 2;
     // clustering round 0 (singletons): every label is its own vertex id
     const uint32_t own = (MODE == CLUSTER && a.singletons) ? (uint32_t)v : (uint32_t)a.lab[v];
     const uint32_t cv = (uint32_t)a.vwgt[v];
@@ -609,15 +592,33 @@ struct SweepSmem {
     WarpTable tabs[kWarpsPerBlock];
 };
 
+using SweepQueue = int[kWarpsPerBlock][32 * kSpan + 32];
+
+// A team's lanes keep rows of up to kDeferRow entries; longer ones, and rows
+// of too many labels, are listed: those of up to HUGE entries from the front
+// of the list for a warp each, longer ones from its end for a block each.
+constexpr int kDeferRow = 32;
+
+template <int HUGE>
+__device__ __forceinline__ void defer_row(const SweepArgs& a, bool pred, int v) {
+    const bool huge = pred && a.xadj[v + 1] - a.xadj[v] > HUGE;
+    append_aggregated(pred && !huge, v, a.heavy, a.hcount);
+    if (huge) a.heavy[a.n - 1 - (int)atomicAdd(a.hugecount, 1u)] = v;
+}
+
 // The whole grid sweeps the members of one sub-round (kThreads a block).
-template <int MODE, bool UNIT, bool STASH>
-__device__ __forceinline__ void lane_sweep(const SweepArgs& a, SweepSmem& sm) {
+// HUGE > 0: the rows that defer_row<HUGE> takes are not decided here (oqueue
+// and tabs are not used).
+template <int MODE, bool UNIT, bool STASH, int HUGE>
+__device__ __forceinline__ void lane_sweep(const SweepArgs& a, SweepQueue& queue, int (*oqueue)[64], WarpTable* tabs) {
     static_assert(kTab == 256, "slot64 assumes 256 slots");
+    constexpr bool DEFER = HUGE > 0;
+    static_assert(!(DEFER && STASH), "the stash lies in the chunk tables");
     const int lane = threadIdx.x & 31;
-    int* q = sm.queue[threadIdx.x >> 5];
-    int* oq = sm.oqueue[threadIdx.x >> 5];
-    WarpTable& T = sm.tabs[threadIdx.x >> 5];
-    if (lane == 0) T.nused = 0;
+    int* q = queue[threadIdx.x >> 5];
+    int* oq = DEFER ? nullptr : oqueue[threadIdx.x >> 5];
+    WarpTable* T = DEFER ? nullptr : tabs + (threadIdx.x >> 5);
+    if (!DEFER && lane == 0) T->nused = 0;
     __syncwarp();
     int qn = 0, oqn = 0;  // warp-uniform
     // per-lane work counts (32 bits: a lane never sees more than m < 2^31 entries)
@@ -635,11 +636,18 @@ __device__ __forceinline__ void lane_sweep(const SweepArgs& a, SweepSmem& sm) {
         for (int i = lane; i + 32 < oqn; i += 32) oq[i] = oq[i + 32];
         __syncwarp();
         oqn = oqn > 32 ? oqn - 32 : 0;
-        chunk_process<MODE>(a, T, mem, v, wv, we, wo);
+        chunk_process<MODE>(a, *T, mem, v, wv, we, wo);
     };
     auto pass = [&](int v) {
         int status = 0;
-        if (v >= 0) status = lane_vertex<MODE, kSlots, UNIT, STASH>(a, v, T.stash + lane, wv, we);
+        if (v >= 0)
+            status = lane_vertex<MODE, kSlots, UNIT, STASH, DEFER ? kDeferRow : kWin>(
+                a, v, STASH ? T->stash + lane : nullptr, wv, we);
+        if constexpr (DEFER) {
+            defer_row<HUGE>(a, status == 1 || status == 2, v);
+            append_striped(status == 3, v, a.plist);
+            return;
+        }
         const unsigned om = __ballot_sync(0xffffffffu, status == 1);
         if (status == 1) oq[oqn + __popc(om & lanemask_lt())] = v;
         oqn += __popc(om);
@@ -671,7 +679,8 @@ __device__ __forceinline__ void lane_sweep(const SweepArgs& a, SweepSmem& sm) {
         }
     }
     if (qn > 0) pass(lane < qn ? q[lane] : -1);
-    while (oqn > 0) overflow_pass();
+    if constexpr (!DEFER)
+        while (oqn > 0) overflow_pass();
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) {
         wv += __shfl_xor_sync(0xffffffffu, wv, o);
@@ -692,81 +701,175 @@ __device__ __forceinline__ void lane_sweep(const SweepArgs& a, SweepSmem& sm) {
 // the shared table).
 constexpr int kSmemTab = 4096;
 
-// BT threads per block (more for the longest rows).
-// `which`: 0 = every listed vertex, 1 = only those whose table fits in
-// shared memory, 2 = only the others (the two kinds can run as separate
-// launches with different grids; the decisions do not depend on the order).
-// The shared-memory table htab (stab slots, a power of two, keys then values)
-// has kSmemTab slots in the many-block launches, more in the launch of the
-// longest rows, whose rows up to stab / 2 entries then stay out of the
-// global table.
+// Linear probing that looks before it swaps (most entries find their label
+// there).  The caller guarantees at most cap / 2 distinct keys, so the probe
+// ends within cap steps; the bound only guards against a broken invariant:
+// the key is then dropped and *err is set.
+__device__ __forceinline__ void table_add(uint32_t* tk, uint32_t* tv, int cap, uint32_t key, uint32_t val, int* err) {
+    uint32_t s = table_slot(key, cap);
+    for (int probe = 0; probe < cap; ++probe) {
+        uint32_t cur = *(volatile uint32_t*)(tk + s);
+        if (cur == kEmpty) {
+            cur = atomicCAS(&tk[s], kEmpty, key);
+            if (cur == kEmpty) cur = key;
+        }
+        if (cur == key) {
+            atomicAdd(&tv[s], val);
+            return;
+        }
+        s = (s + 1) & (uint32_t)(cap - 1);
+    }
+    atomicOr(err, 1);
+}
+
+template <int BT>
+struct HeavyRed {
+    uint64_t key[BT / 32];
+    uint32_t id[BT / 32], own[BT / 32];
+};
+
+// One vertex by a block of BT threads through the first cap slots (a power of
+// two >= 2 * degree) of a table that is empty between uses, so that
+// inserting, scanning and clearing cost O(degree).  Entries of the own label
+// are summed in registers.  Four entries a thread are in flight.
+template <int MODE, int BT>
+__device__ __forceinline__ void heavy_vertex(const SweepArgs& a, int v, uint32_t* tk, uint32_t* tv, int cap,
+                                             HeavyRed<BT>& red) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int beg = a.xadj[v], end = a.xadj[v + 1];
+    const uint32_t own = (uint32_t)a.lab[v], cv = (uint32_t)a.vwgt[v];
+    uint32_t co = 0;
+    for (int c = beg + (int)threadIdx.x; c < end; c += 4 * BT) {
+        uint32_t l[4], wt[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const bool in = c + q * BT < end;
+            l[q] = in ? (uint32_t)a.adjncy[c + q * BT] : kEmpty;
+            wt[q] = in ? (uint32_t)a.adjwgt[c + q * BT] : 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (l[q] != kEmpty) l[q] = (uint32_t)a.lab[l[q]];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (l[q] == own) co += wt[q];
+            else if (l[q] != kEmpty) table_add(tk, tv, cap, l[q], wt[q], a.err);
+        }
+    }
+    __syncthreads();
+    uint64_t key = 0;
+    uint32_t id = kEmpty;
+    for (int s = threadIdx.x; s < cap; s += BT) {
+        const uint32_t l = tk[s];
+        if (l == kEmpty) continue;
+        const uint32_t c = tv[s];
+        tk[s] = kEmpty;
+        tv[s] = 0;
+        if (cand_ok<MODE>(a, l, c, cv)) better(key, id, cand_key(c, a.ks_tie, l), l);
+    }
+    group_argmax<32>(key, id, 0xffffffffu);
+    co = __reduce_add_sync(0xffffffffu, co);
+    if (lane == 0) {
+        red.key[w] = key;
+        red.id[w] = id;
+        red.own[w] = co;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int j = 1; j < BT / 32; ++j) {
+            better(key, id, red.key[j], red.id[j]);
+            co += red.own[j];
+        }
+        atomicAdd(&a.work[0], 1ull);
+        atomicAdd(&a.work[1], (unsigned long long)(end - beg));
+        if (decide_emit<MODE>(a, v, own, cv, co, key, id)) a.hplist[atomicAdd(a.hpcount, 1u)] = v;
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ int heavy_cap(int deg, int most) {
+    int cap = 256;
+    while (cap < 2 * deg && cap < most) cap <<= 1;
+    return cap;
+}
+
+// The listed vertices, a block each.  `which`: 0 = every one, 1 = only those
+// whose table fits in shared memory, 2 = only the others (the two kinds can
+// run as separate launches with different grids; the decisions do not depend
+// on the order).  The shared-memory table htab (stab slots, a power of two,
+// keys then values) has kSmemTab slots in the many-block launches, more in
+// the launch of the longest rows, whose rows up to stab / 2 entries then
+// stay out of the global table.
 template <int MODE, int BT>
 __device__ __forceinline__ void heavy_sweep(const SweepArgs& a, uint32_t* gtk, uint32_t* gtv, int gcap, int which,
                                             int stab, uint32_t* htab) {
-    __shared__ uint64_t sk[BT / 32];
-    __shared__ uint32_t sid[BT / 32];
-    __shared__ uint32_t sco;
-    uint32_t* stk = htab;
-    uint32_t* stv = htab + stab;
+    __shared__ HeavyRed<BT> red;
     for (int s = threadIdx.x; s < stab; s += BT) {
-        stk[s] = kEmpty;
-        stv[s] = 0;
+        htab[s] = kEmpty;
+        htab[stab + s] = 0;
     }
     __syncthreads();
     uint32_t* gk = gtk ? gtk + (size_t)blockIdx.x * gcap : nullptr;
     uint32_t* gv = gtv ? gtv + (size_t)blockIdx.x * gcap : nullptr;
     const unsigned count = *a.hcount;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (unsigned i = blockIdx.x; i < count; i += gridDim.x) {
         const int v = a.heavy[i];
-        const int beg = a.xadj[v], end = a.xadj[v + 1];
-        const uint32_t own = (uint32_t)a.lab[v];
-        const uint32_t cv = (uint32_t)a.vwgt[v];
-        // this vertex uses the first cap entries of the block's table (a
-        // power of two >= 2 * degree, at most gcap), so inserting, scanning
-        // and clearing cost O(degree), not O(max degree)
-        int cap = 256;
-        while (cap < 2 * (end - beg) && cap < gcap) cap <<= 1;
+        const int cap = heavy_cap(a.xadj[v + 1] - a.xadj[v], gcap);
         if ((which == 1 && cap > kSmemTab) || (which == 2 && cap <= kSmemTab)) continue;
-        uint32_t* tk = cap <= stab ? stk : gk;
-        uint32_t* tv = cap <= stab ? stv : gv;
-        if (threadIdx.x == 0) {
-            sco = 0;
-            atomicAdd(&a.work[0], 1ull);
-            atomicAdd(&a.work[1], (unsigned long long)(end - beg));
-        }
-        for (int c = beg; c < end; c += BT) {
-            int e = c + threadIdx.x;
-            uint32_t l = kEmpty, wt = 0;
-            if (e < end) {
-                wt = (uint32_t)a.adjwgt[e];
-                l = (uint32_t)a.lab[a.adjncy[e]];
-            }
-            unsigned peers = __match_any_sync(0xffffffffu, l);
-            uint32_t sum = __reduce_add_sync(peers, wt);
-            if (e < end && (peers & lanemask_lt()) == 0) table_insert(tk, tv, cap, l, sum, a.err);
-        }
-        __syncthreads();
-        uint64_t key = 0;
-        uint32_t id = kEmpty;
-        for (int s = threadIdx.x; s < cap; s += BT) {
-            uint32_t l = tk[s];
-            if (l == kEmpty) continue;
-            uint32_t c = tv[s];
-            tk[s] = kEmpty;
-            tv[s] = 0;
-            if (l == own) sco = c;
-            else if (cand_ok<MODE>(a, l, c, cv)) better(key, id, cand_key(c, a.ks_tie, l), l);
-        }
-        group_argmax<32>(key, id, 0xffffffffu);
-        if (lane == 0) { sk[w] = key; sid[w] = id; }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int j = 1; j < BT / 32; ++j) better(key, id, sk[j], sid[j]);
-            if (decide_emit<MODE>(a, v, own, cv, sco, key, id)) a.hplist[atomicAdd(a.hpcount, 1u)] = v;
-        }
-        __syncthreads();
+        heavy_vertex<MODE, BT>(a, v, cap <= stab ? htab : gk, cap <= stab ? htab + stab : gv, cap, red);
     }
+}
+
+// One vertex by a warp, rows of up to kHashRow entries: the warp's table in
+// shared memory (kHashTab slots, empty between uses), the own label in
+// registers.
+constexpr int kHashRow = 256;
+constexpr int kHashTab = 2 * kHashRow;
+
+template <int MODE, bool UNIT>
+__device__ __forceinline__ void hash_vertex(const SweepArgs& a, int v, uint32_t* tk, uint32_t* tv) {
+    const int lane = threadIdx.x & 31;
+    const int beg = a.xadj[v], end = a.xadj[v + 1];
+    const uint32_t own = (uint32_t)a.lab[v], cv = (uint32_t)a.vwgt[v];
+    int cap = 64;
+    while (cap < 2 * (end - beg)) cap <<= 1;
+    uint32_t co = 0;
+    for (int c = beg + lane; c < end; c += 128) {
+        uint32_t l[4], wt[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const bool in = c + q * 32 < end;
+            l[q] = in ? (uint32_t)a.adjncy[c + q * 32] : kEmpty;
+            wt[q] = in ? (UNIT ? 1u : (uint32_t)a.adjwgt[c + q * 32]) : 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (l[q] != kEmpty) l[q] = (uint32_t)a.lab[l[q]];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (l[q] == own) co += wt[q];
+            else if (l[q] != kEmpty) table_add(tk, tv, cap, l[q], wt[q], a.err);
+        }
+    }
+    __syncwarp();
+    uint64_t key = 0;
+    uint32_t id = kEmpty;
+    for (int s = lane; s < cap; s += 32) {
+        const uint32_t l = tk[s];
+        if (l == kEmpty) continue;
+        const uint32_t c = tv[s];
+        tk[s] = kEmpty;
+        tv[s] = 0;
+        if (cand_ok<MODE>(a, l, c, cv)) better(key, id, cand_key(c, a.ks_tie, l), l);
+    }
+    group_argmax<32>(key, id, 0xffffffffu);
+    co = __reduce_add_sync(0xffffffffu, co);
+    if (lane == 0) {
+        atomicAdd(&a.work[0], 1ull);
+        atomicAdd(&a.work[1], (unsigned long long)(end - beg));
+        if (decide_emit<MODE>(a, v, own, cv, co, key, id)) a.hplist[atomicAdd(a.hpcount, 1u)] = v;
+    }
+    __syncwarp();
 }
 
 // ---------------------------------------------------------------- admission
@@ -782,7 +885,18 @@ __device__ __forceinline__ bool admit(const uint32_t* H, const int* minvP, int P
     const uint32_t* h = H + (size_t)b * P;
     unsigned long long cum = 0;
     int t = 0;
-    while (t < P && (long long)(cum + h[t]) <= cap) { cum += h[t]; ++t; }
+    // four classes are loaded together (one after the other, the loads' round
+    // trips are most of an admission pass)
+    for (bool fits = true; fits && t < P;) {
+        uint32_t x[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) x[q] = t + q < P ? h[t + q] : 0u;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            fits = fits && t < P && (long long)(cum + x[q]) <= cap;
+            if (fits) { cum += x[q]; ++t; }
+        }
+    }
     if (c < t) return true;
     return c == t && minvP[(size_t)b * P + t] == v && (long long)(cum + cv) <= cap;
 }
@@ -832,13 +946,15 @@ __device__ __forceinline__ void mark_row(const NextActive& na, const int* adjncy
 // between two sets; a sub-round clears the set of the next one, which every
 // block stopped reading at the barrier that ended the sub-round before.
 
-constexpr int kTeamSet = kStripes + 8;  // counters of one set: stripes, heavy, heavy proposals
+constexpr int kTeamSet = kStripes + 8;  // counters of one set: stripes, heavy, heavy proposals, huge
 constexpr int kTeamMaxBlocks = 8192;    // blocks of the partition (their thresholds sit in shared memory)
+constexpr int kDenseBlocks = 1024;      // ... up to which every warp has a counter per block in shared memory
 
 __device__ __forceinline__ void use_set(SweepArgs& a, unsigned* counters, int p) {
     a.plist.counts = counters + p * kTeamSet;
     a.hcount = counters + p * kTeamSet + kStripes;
     a.hpcount = counters + p * kTeamSet + kStripes + 1;
+    a.hugecount = counters + p * kTeamSet + kStripes + 2;
     unsigned* other = counters + (p ^ 1) * kTeamSet;
     if (blockIdx.x == 0)
         for (int i = threadIdx.x; i < kTeamSet; i += blockDim.x) other[i] = 0;
@@ -850,27 +966,162 @@ template <class F>
 __device__ __forceinline__ void each_proposal(const SweepArgs& a, F f) {
     const unsigned lane = threadIdx.x & 31;
     const unsigned W = gridDim.x * kWarpsPerBlock, w = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-    const unsigned ns = (unsigned)a.plist.ns + 1u;  // the stripes and the high-degree list
-    for (unsigned s = w % ns; s < ns; s += W) {
-        const bool stripe = s + 1 < ns;
-        const unsigned n = stripe ? a.plist.counts[s] : *a.hpcount;
-        const int* list = stripe ? a.plist.data + (long long)s * a.plist.cap : a.hplist;
+    const unsigned ns = (unsigned)a.plist.ns;
+    for (unsigned s = w & (ns - 1); s < ns; s += W) {
+        const unsigned n = a.plist.counts[s];
+        const int* list = a.plist.data + (long long)s * a.plist.cap;
         const unsigned share = W > ns ? (W - s + ns - 1) / ns : 1u;  // warps on this stripe
         for (unsigned i = (W > ns ? w / ns : 0u) * 32; i < n; i += share * 32) f(i + lane < n ? list[i + lane] : -1);
     }
+    const unsigned nh = *a.hpcount;
+    for (unsigned i = w * 32; i < nh; i += W * 32) f(i + lane < nh ? a.hplist[i + lane] : -1);
 }
 
-// The sub-round's members in a lane per vertex, then those of high degree;
+// A block's shared memory in a team, for the rows that a warp or the block
+// decides: DENSE, a counter per block of the partition for every warp (zero
+// between uses) and a bit per block for zero-weight contacts; else a hash
+// table per warp (kHashTab slots, all keys then all values), which are one
+// table of kSmemTab slots for the block.  The release thresholds lie behind.
+constexpr int kHugeDense = 1024;  // longest row of a warp with the counters
+
+struct TeamSpace {
+    uint32_t* tab;  // counters, or the keys
+    uint32_t* val;  // DENSE: the bits; else the values
+    int* thr;
+    int k;
+    __device__ int words() const { return (k + 31) / 32; }
+};
+
+struct RowRed {  // of a row counted by a whole block
+    uint64_t key[kWarpsPerBlock];
+    uint32_t id[kWarpsPerBlock];
+    long long own[kWarpsPerBlock];
+};
+
+static_assert(kWarpsPerBlock * kHashTab == kSmemTab, "the warps' tables make up the block's");
+
+inline size_t team_smem(int k, bool dense) {
+    if (!dense) return sizeof(uint32_t) * (2 * (size_t)kSmemTab + k);
+    return sizeof(uint32_t) * ((size_t)kWarpsPerBlock * (k + (k + 31) / 32) + k);
+}
+
+template <bool DENSE>
+__device__ __forceinline__ TeamSpace team_space(unsigned char* dyn, int k) {
+    TeamSpace S{};
+    S.k = k;
+    S.tab = reinterpret_cast<uint32_t*>(dyn);
+    const int keys = DENSE ? kWarpsPerBlock * k : kSmemTab;
+    const int vals = DENSE ? kWarpsPerBlock * S.words() : kSmemTab;
+    S.val = S.tab + keys;
+    S.thr = reinterpret_cast<int*>(S.val + vals);
+    for (int i = threadIdx.x; i < keys; i += kThreads) S.tab[i] = DENSE ? 0u : kEmpty;
+    for (int i = threadIdx.x; i < vals; i += kThreads) S.val[i] = 0;
+    __syncthreads();
+    return S;
+}
+
+// One vertex by a warp (BLOCK: by the whole block): its connection to every
+// block of the partition in the counters cnt, then the decision.  A row of
+// many entries or many labels costs its entries divided by the lanes plus
+// k / 32 counter reads, where the lane's slots or the hash tables walk it
+// entry by entry.
+template <int MODE, bool UNIT, bool BLOCK>
+__device__ __forceinline__ void dense_vertex(const SweepArgs& a, int v, int k, uint32_t* cnt, uint32_t* mask,
+                                             RowRed& red) {
+    static_assert(MODE != CLUSTER, "labels are blocks of the partition");
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int t = BLOCK ? (int)threadIdx.x : lane;
+    constexpr int NT = BLOCK ? kThreads : 32;
+    const int beg = a.xadj[v], end = a.xadj[v + 1];
+    const uint32_t own = (uint32_t)a.lab[v], cv = (uint32_t)a.vwgt[v];
+    for (int e = beg + t; e < end; e += 4 * NT) {
+        int u[4];
+        uint32_t w[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const bool in = e + q * NT < end;
+            u[q] = in ? a.adjncy[e + q * NT] : -1;
+            w[q] = in ? (UNIT ? 1u : (uint32_t)a.adjwgt[e + q * NT]) : 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (u[q] >= 0) u[q] = a.lab[u[q]];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (u[q] < 0) continue;
+            atomicAdd(&cnt[u[q]], w[q]);
+            // a zero-weight contact is a candidate of the balance repair too
+            if (MODE == BALANCE && !UNIT && w[q] == 0) atomicOr(&mask[u[q] >> 5], 1u << (u[q] & 31));
+        }
+    }
+    if (BLOCK) __syncthreads();
+    else __syncwarp();
+    const uint32_t cown = cnt[own];
+    uint64_t key = 0;
+    uint32_t id = kEmpty;
+    for (int b = t; b < k; b += NT) {
+        const uint32_t c = cnt[b];
+        const bool touched = c > 0 || (MODE == BALANCE && !UNIT && ((mask[b >> 5] >> (b & 31)) & 1u));
+        if (touched && (uint32_t)b != own && cand_ok<MODE>(a, (uint32_t)b, c, cv))
+            better(key, id, cand_key(c, a.ks_tie, (uint32_t)b), (uint32_t)b);
+    }
+    group_argmax<32>(key, id, 0xffffffffu);
+    if (BLOCK) {
+        if (lane == 0) {
+            red.key[wid] = key;
+            red.id[wid] = id;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 1; w < kWarpsPerBlock; ++w) better(key, id, red.key[w], red.id[w]);
+    }
+    if (t == 0) {
+        atomicAdd(&a.work[0], 1ull);
+        atomicAdd(&a.work[1], (unsigned long long)(end - beg));
+        if (decide_emit<MODE>(a, v, own, cv, cown, key, id)) a.hplist[atomicAdd(a.hpcount, 1u)] = v;
+    }
+    if (BLOCK) __syncthreads();
+    else __syncwarp();
+    for (int b = t; b < k; b += NT) cnt[b] = 0;
+    if (MODE == BALANCE && !UNIT)
+        for (int b = t; b < (k + 31) / 32; b += NT) mask[b] = 0;
+    if (BLOCK) __syncthreads();
+    else __syncwarp();
+}
+
+// The deferred rows of a sub-round.
+template <int MODE, bool UNIT, bool DENSE>
+__device__ __forceinline__ void deferred_rows(const SweepArgs& a, const TeamSpace& S, RowRed& red) {
+    const unsigned W = gridDim.x * kWarpsPerBlock, wid = threadIdx.x >> 5;
+    const unsigned n = *a.hcount, nh = *a.hugecount;
+    for (unsigned i = blockIdx.x + wid * gridDim.x; i < n; i += W) {
+        if constexpr (DENSE)
+            dense_vertex<MODE, UNIT, false>(a, a.heavy[i], S.k, S.tab + (size_t)wid * S.k, S.val + wid * S.words(),
+                                            red);
+        else
+            hash_vertex<MODE, UNIT>(a, a.heavy[i], S.tab + wid * kHashTab, S.val + wid * kHashTab);
+    }
+    __syncthreads();
+    for (unsigned i = blockIdx.x; i < nh; i += gridDim.x) {
+        const int v = a.heavy[a.n - 1 - (int)i];
+        if constexpr (DENSE) {
+            dense_vertex<MODE, UNIT, true>(a, v, S.k, S.tab, S.val, red);
+        } else {
+            __shared__ HeavyRed<kThreads> hred;
+            heavy_vertex<MODE, kThreads>(a, v, S.tab, S.val, heavy_cap(a.xadj[v + 1] - a.xadj[v], kSmemTab), hred);
+        }
+    }
+}
+
+// The sub-round's members in a lane per vertex, then the rows that need more;
 // every block has seen all proposals afterwards.  False: the team gave up.
-// (Rows of up to kSmemTab / 2 entries: gcap slots fit the block's table,
-// which takes the place of the chunk tables.)
-template <int MODE, bool UNIT, bool STASH>
-__device__ __forceinline__ bool team_sweep(Team& team, const SweepArgs& a, int gcap, SweepSmem& sm) {
-    static_assert(sizeof(sm.tabs) >= 8 * kSmemTab, "the high-degree table overlays the chunk tables");
-    lane_sweep<MODE, UNIT, STASH>(a, sm);
+template <int MODE, bool UNIT, bool DENSE>
+__device__ __forceinline__ bool team_sweep(Team& team, const SweepArgs& a, SweepQueue& queue, const TeamSpace& S,
+                                           RowRed& red) {
+    lane_sweep<MODE, UNIT, false, DENSE ? kHugeDense : kHashRow>(a, queue, nullptr, nullptr);
     if (!team.sync()) return false;
-    if (gcap == 0 || *a.hcount == 0) return true;
-    heavy_sweep<MODE, kThreads>(a, nullptr, nullptr, gcap, 0, kSmemTab, reinterpret_cast<uint32_t*>(sm.tabs));
+    if (*a.hcount == 0 && *a.hugecount == 0) return true;
+    deferred_rows<MODE, UNIT, DENSE>(a, S, red);
     return team.sync();
 }
 
@@ -944,7 +1195,7 @@ __device__ __forceinline__ Weighed weigh(const uint32_t* bw, int k, uint32_t bou
 }
 
 struct BalanceArgs {
-    int k, iters, seed, level, gcap;
+    int k, iters, seed, level;
     int* part;
     uint32_t* bw;
     uint32_t* HS;        // k * kBalClasses, zero between calls
@@ -962,9 +1213,9 @@ __device__ __forceinline__ void balance_clear(Team& team, const SweepArgs& a, co
 
 // The balance repair of lp.cu's balance(), all iterations; p: the counter
 // set in turn.  False: the team gave up.
-template <bool UNIT>
-__device__ __forceinline__ bool balance_steps(Team& team, SweepArgs a, const BalanceArgs& B, int& p, SweepSmem& sm,
-                                              WeighSmem& ws) {
+template <bool UNIT, bool DENSE>
+__device__ __forceinline__ bool balance_steps(Team& team, SweepArgs a, const BalanceArgs& B, int& p, SweepQueue& queue,
+                                              const TeamSpace& S, RowRed& red, WeighSmem& ws) {
     a.lab = B.part;
     a.lw = B.bw;
     a.HS = B.HS;
@@ -975,10 +1226,10 @@ __device__ __forceinline__ bool balance_steps(Team& team, SweepArgs a, const Bal
         a.ks_sub = stream_key(B.seed, TAG_BCLS, B.level, it);  // release class stream
         const uint64_t ks_prio = stream_key(B.seed, TAG_BPRIO, B.level, it);
         use_set(a, B.counters, p);
-        if (!team_sweep<BALANCE, UNIT, true>(team, a, B.gcap, sm)) return false;
+        if (!team_sweep<BALANCE, UNIT, DENSE>(team, a, queue, S, red)) return false;
         // release thresholds, computed by every block for itself: the number
         // of classes before which less than the excess is released
-        int* thr = reinterpret_cast<int*>(sm.tabs);
+        int* thr = S.thr;
         const int lane = threadIdx.x & 31;
         for (int b = threadIdx.x >> 5; b < B.k; b += kWarpsPerBlock) {
             const uint32_t x = B.bw[b];
@@ -1064,10 +1315,22 @@ struct SweepBuffers {
 SweepBuffers make_buffers(Ctx& ctx, const DevGraph& g, int team);
 SweepArgs base_args(const DevGraph& g, const SweepBuffers& b);
 
-// A team can sweep the level: its rows fit the blocks' shared-memory tables.
-inline bool team_rows(const DevGraph& g) { return g.maxdeg <= kSmemTab / 2; }
-// Blocks of a team that sweeps n vertices: a thread per vertex.
-inline long long team_want(long long n) { return (n + kThreads - 1) / kThreads; }
+// Every warp of a team has a counter per block of the partition in shared
+// memory (37 KB a block at the limit); with more blocks the team aggregates
+// in the hash tables of the clustering sweep.
+inline bool team_dense(int k) { return k <= kDenseBlocks; }
+// A team can sweep the level by blocks of the partition: with the dense
+// counters always, else when the rows and the release thresholds fit the
+// blocks' shared memory.
+inline bool team_fits(const DevGraph& g, int k) {
+    return team_dense(k) || (k <= kTeamMaxBlocks && g.maxdeg <= kSmemTab / 2);
+}
+// Blocks of a team that sweeps a level: a thread per vertex; on dense levels
+// (rows mostly a warp's) a thread per entry.
+inline long long team_want(const DevGraph& g) {
+    const long long work = g.m > 16LL * g.n ? g.m : g.n;
+    return (work + kThreads - 1) / kThreads;
+}
 
 }  // namespace sweep
 }  // namespace kb

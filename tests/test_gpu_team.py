@@ -1,8 +1,10 @@
 """Phases that a team of thread blocks runs in one kernel, against the CPU
 oracle, at the sizes where the team changes form (one block, a cluster, a
-cooperative grid; 256 vertices per block) and at the limits of its rule (rows
-of 2048 entries, 8192 blocks), just past which the per-step launches take
-over.  Integer outputs: equality.
+cooperative grid; 256 vertices per block), at the row lengths where a lane, a
+warp or a block takes over (32, 256, 1024) and at the limits of its rule (1024
+blocks for the dense counters; 8192 blocks and rows of 2048 entries for the
+hash tables), just past which the per-step launches take over.  Integer
+outputs: equality.
 """
 import numpy as np
 import pytest
@@ -51,7 +53,8 @@ def skewed(n, k, seed):
     return p
 
 
-SIZES = [1, 31, 255, 256, 257, 511, 513, 1024, 2047, 2048, 2049, 2305, 8192, 40001, 160000]
+SIZES = [1, 31, 255, 256, 257, 511, 513, 1024, 2047, 2048, 2049, 4096, 4097, 8192, 40001, 160000]
+HUBS = [32, 33, 128, 129, 256, 257, 1024, 1025, 2048, 2049]
 
 
 @pytest.mark.parametrize("n", SIZES)
@@ -68,17 +71,49 @@ def test_jet_sizes(N, O, graphs, n, k):
                                   N.jet_refine(g, kn_p, part, kn_p.upper_bound, level))
 
 
-@pytest.mark.parametrize("hub", [128, 129, 256, 257, 2048, 2049])
+@pytest.mark.parametrize("n", SIZES)
+@pytest.mark.parametrize("k", [9, 64])
+def test_refine_sizes(N, O, graphs, n, k):
+    g = graphs.rgg3d(n, seed=n) if n > 31 else csr_from_edges(n, [(i, i + 1) for i in range(n - 1)])
+    for unit in (True, False):
+        if not unit:
+            weighted(g, n)
+        kn_o, kn_p = O.knobs(g, k, 0.03, 5, 0), N.derive_knobs(n, g["vwgt"], k, 0.03, 5, 0)
+        part = skewed(n, k, n)
+        bal_o, ok_o = O.balance(g, kn_o, part, kn_o.upper_bound, 1)
+        bal_p, ok_p = N.balance(g, kn_p, part, kn_p.upper_bound, 1)
+        assert ok_o == ok_p and np.array_equal(bal_o, bal_p)
+        assert np.array_equal(O.lp_refine(g, kn_o, bal_o, kn_o.upper_bound, 1),
+                              N.lp_refine(g, kn_p, bal_o, kn_p.upper_bound, 1))
+
+
+@pytest.mark.parametrize("hub", HUBS)
+@pytest.mark.parametrize("k", [40, 1025])
+def test_refine_hubs(N, O, hub, k):
+    g = hub_graph(5000, hub, hub)
+    for unit in (True, False):
+        if not unit:
+            weighted(g, hub)
+        kn_o, kn_p = O.knobs(g, k, 0.10, 1, 0), N.derive_knobs(g["n"], g["vwgt"], k, 0.10, 1, 0)
+        part = skewed(g["n"], k, hub)
+        bal_o, ok_o = O.balance(g, kn_o, part, kn_o.upper_bound, 1)
+        bal_p, ok_p = N.balance(g, kn_p, part, kn_p.upper_bound, 1)
+        assert ok_o == ok_p and np.array_equal(bal_o, bal_p)
+        assert np.array_equal(O.lp_refine(g, kn_o, bal_o, kn_o.upper_bound, 1),
+                              N.lp_refine(g, kn_p, bal_o, kn_p.upper_bound, 1))
+
+
+@pytest.mark.parametrize("hub", HUBS)
 def test_jet_hubs(N, O, hub):
     g = hub_graph(5000, hub, hub)
-    for k in (2, 40):
+    for k in (2, 40, 1025):
         kn_o, kn_p = O.knobs(g, k, 0.03, 1, 1), N.derive_knobs(g["n"], g["vwgt"], k, 0.03, 1, 1)
         part = skewed(g["n"], k, hub)
         assert np.array_equal(O.jet_refine(g, kn_o, part, kn_o.upper_bound, 1),
                               N.jet_refine(g, kn_p, part, kn_p.upper_bound, 1))
 
 
-@pytest.mark.parametrize("k", [8192, 8193])
+@pytest.mark.parametrize("k", [1024, 1025, 8192, 8193])
 def test_jet_many_blocks(N, O, graphs, k):
     g = graphs.rgg2d(20000, seed=2)
     kn_o, kn_p = O.knobs(g, k, 0.10, 1, 1), N.derive_knobs(g["n"], g["vwgt"], k, 0.10, 1, 1)
