@@ -59,6 +59,7 @@ struct Lease {
         }
         if (!ctx) ctx.reset(new Ctx());
         ctx->init(d, nullptr);
+        ctx->team_share = 1;
     }
     ~Lease() {
         if (!ctx) return;
@@ -493,6 +494,7 @@ int kb200_kaffpae(int n, const int* vwgt, const int* xadj, const int* adjcwgt, c
         for (int w = 0; w < Wk; ++w) {
             leases.emplace_back(new Lease(dev));
             wctx.push_back(leases.back()->ctx.get());
+            wctx.back()->team_share = Wk;
         }
         const long long m = xadj[n];
         for (int attempt = 0;; ++attempt) {
@@ -967,6 +969,7 @@ int kb200_kaffpa_batch(kb200_batch_item* items, int count, int workers, kb200_ba
                     Knobs kn;
                     derive_knobs(it.n, it.vwgt, it.nparts, it.imbalance, it.seed, it.mode, kn);
                     if (!lease) lease.reset(new Lease(dev));
+                    lease->ctx->team_share = W;
                     return run_host_in(*lease->ctx, it.n, it.vwgt, it.xadj, it.adjwgt, it.adjncy, kn, &it.edgecut,
                                        it.part, nullptr, clk::now());
                 });
@@ -1033,6 +1036,7 @@ int kb200_kaffpa_population(int n, const int* d_vwgt, const int* d_xadj, const i
                 status[(size_t)i] = guarded([&]() -> int {
                     if (!lease) lease.reset(new Lease(dev));
                     Ctx& ctx = *lease->ctx;
+                    ctx.team_share = Wk;
                     Knobs kn;
                     derive_knobs_total(n, W, nparts, imbalance, seeds[i], mode, kn);
                     for (int attempt = 0;; ++attempt) {

@@ -81,6 +81,7 @@ struct Ctx {
     int* dscalars = nullptr;               // 64 ints
     unsigned long long* work = nullptr;    // [0] swept vertices, [1] swept edges
     unsigned* team_bar = nullptr;          // barrier counters of a team of blocks (team.cuh)
+    int team_share = 1;                    // calls that share the device with this one (team.cuh)
     uint32_t* pinned = nullptr;            // 64 words, page-locked
     // timing: 0 off, 1 every kernel family, 2 only the LP clustering sweep
     int timing = 0;

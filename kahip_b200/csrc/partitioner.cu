@@ -67,7 +67,8 @@ TeamRoom team_room(Ctx& ctx, const void* kernel, size_t smem) {
     static std::vector<Known> known;
     std::lock_guard<std::mutex> lk(mu);
     for (const Known& k : known)
-        if (k.kernel == kernel && k.device == ctx.device && k.smem == smem) return k.room;
+        if (k.kernel == kernel && k.device == ctx.device && k.smem == smem)
+            return TeamRoom{k.room.most / std::max(ctx.team_share, 1), k.room.wide_cluster};
     TeamRoom r{0, false};
     int per = 0, sms = 0, clusters = 0;
     if (smem > 40 * 1024)  // with the kernel's own shared memory above the default limit
@@ -90,7 +91,7 @@ TeamRoom team_room(Ctx& ctx, const void* kernel, size_t smem) {
                      cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
     if (!r.wide_cluster) (void)cudaGetLastError();
     known.push_back(Known{kernel, ctx.device, smem, r});
-    return r;
+    return TeamRoom{r.most / std::max(ctx.team_share, 1), r.wide_cluster};
 }
 
 int Ctx::phase_id(const char* name) {

@@ -120,3 +120,47 @@ def test_jet_many_blocks(N, O, graphs, k):
     part = skewed(g["n"], k, 3)
     assert np.array_equal(O.jet_refine(g, kn_o, part, kn_o.upper_bound, 0),
                           N.jet_refine(g, kn_p, part, kn_p.upper_bound, 0))
+
+
+@pytest.mark.parametrize("n", SIZES)
+def test_cluster_sizes(N, O, graphs, n):
+    g = graphs.rgg2d(n, seed=n) if n > 31 else csr_from_edges(n, [(i, i + 1) for i in range(n - 1)])
+    for unit in (True, False):
+        if not unit:
+            weighted(g, n)
+        for k in (2, 64):
+            kn_o, kn_p = O.knobs(g, k, 0.03, 5, 0), N.derive_knobs(n, g["vwgt"], k, 0.03, 5, 0)
+            for level in (0, 1):
+                assert np.array_equal(O.lp_cluster(g, kn_o, level), N.lp_cluster(g, kn_p, level))
+
+
+@pytest.mark.parametrize("hub", HUBS)
+def test_cluster_hubs(N, O, hub):
+    g = hub_graph(5000, hub, hub)
+    for unit in (True, False):
+        if not unit:
+            weighted(g, hub)
+        kn_o, kn_p = O.knobs(g, 2, 0.03, 1, 1), N.derive_knobs(g["n"], g["vwgt"], 2, 0.03, 1, 1)
+        assert np.array_equal(O.lp_cluster(g, kn_o, 0), N.lp_cluster(g, kn_p, 0))
+
+
+def test_cluster_unsorted_rows(N, O, graphs):
+    """Rows in no order and a target listed twice: no singleton shortcut."""
+    g = graphs.rgg2d(3000, seed=4)
+    rng = np.random.default_rng(0)
+    adj = g["adjncy"].copy()
+    for v in range(g["n"]):
+        rng.shuffle(adj[g["xadj"][v]:g["xadj"][v + 1]])
+    h = dict(g, adjncy=adj)
+    kn_o, kn_p = O.knobs(h, 8, 0.03, 1, 0), N.derive_knobs(h["n"], h["vwgt"], 8, 0.03, 1, 0)
+    assert np.array_equal(O.lp_cluster(h, kn_o, 0), N.lp_cluster(h, kn_p, 0))
+
+
+def test_teams_side_by_side(N, graphs):
+    """Workers share the device: every result is the single call's."""
+    gs = [graphs.rgg2d(20000 + 977 * i, seed=i) for i in range(6)] + [graphs.rmat(13, samples=4 << 13, seed=1)]
+    cuts, parts, status, _ = N.kaffpa_batch(gs, [2, 8, 16, 64, 5, 3, 8], 0.03, 7, N.FAST, workers=7)
+    assert (status >= 0).all()
+    for g, k, cut, part in zip(gs, [2, 8, 16, 64, 5, 3, 8], cuts, parts):
+        _, c, p = N.kaffpa_ex(g["xadj"], g["adjncy"], k, 0.03, 7, N.FAST, vwgt=g["vwgt"], adjwgt=g["adjwgt"])
+        assert c == cut and np.array_equal(p, part)
