@@ -164,3 +164,24 @@ def test_teams_side_by_side(N, graphs):
     for g, k, cut, part in zip(gs, [2, 8, 16, 64, 5, 3, 8], cuts, parts):
         _, c, p = N.kaffpa_ex(g["xadj"], g["adjncy"], k, 0.03, 7, N.FAST, vwgt=g["vwgt"], adjwgt=g["adjwgt"])
         assert c == cut and np.array_equal(p, part)
+
+
+@pytest.mark.parametrize("n,k", [(900, 2), (1200, 64), (1700, 3), (2600, 8), (6000, 64), (20000, 5)])
+def test_initial_partition_gangs(N, O, graphs, n, k):
+    """Tries by a block and by clusters of 2 to 16 blocks (from 16384 entries
+    on), thread rows and warp rows, several components, unreached nodes."""
+    rng = np.random.default_rng(n)
+    perm = rng.permutation(2 * n)[:n]  # half a graph: some nodes isolated
+    half = graphs.rgg2d(2 * n, seed=n, r_factor=0.9)
+    keep = np.zeros(2 * n, bool)
+    keep[perm] = True
+    src = np.repeat(np.arange(2 * n), np.diff(half["xadj"]))
+    sel = keep[src] & keep[half["adjncy"]] & (src < half["adjncy"])
+    new = np.cumsum(keep) - 1
+    sparse = csr_from_edges(n, list(zip(new[src[sel]].tolist(), new[half["adjncy"][sel]].tolist())))
+    dense = graphs.rmat(max(8, int(np.log2(n)) - 2), samples=24 * n, seed=n)
+    for g in (graphs.rgg3d(n, seed=n, r_factor=0.8), sparse, dense):
+        g["vwgt"] = rng.integers(1, 9, g["n"]).astype(np.int32)
+        for mode in (0, 1):
+            kn_o, kn_p = O.knobs(g, k, 0.03, 5, mode), N.derive_knobs(g["n"], g["vwgt"], k, 0.03, 5, mode)
+            assert np.array_equal(O.initial_partition_batched(g, kn_o), N.initial_partition_device(g, kn_p))
