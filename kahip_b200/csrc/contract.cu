@@ -12,16 +12,16 @@
 //   1. leader[c] = min member (atomicMin); prefix sum over leader flags
 //      gives coarse ids; cmap gather; coarse node weights (atomicAdd).
 //   2. every coarse row gets a bucket as large as its members' degrees
-//      together (prefix sum); every fine node merges its neighbours by
-//      coarse target in register slots and appends (cv << 32 | w) entries
-//      to its coarse row's bucket, one atomic reservation per slot flush
-//      (long rows: the whole warp).
-//   3. (no separate pass: the buckets are filled by the emission)
-//   4. a warp per coarse row sorts its bucket in shared memory (bitonic),
-//      sums the weights of equal targets and keeps the distinct entries;
-//      rows longer than kSegMax go through a stable LSD radix sort on the
-//      2*tb key bits and a reduce-by-key instead.
-//   5. distinct counts -> prefix sum -> xadj; rows copied into place.
+//      together (prefix sum).  Clusterings: a warp per coarse node walks its
+//      members' rows, merges the targets in a shared-memory table and writes
+//      the row sorted.  Matchings: every fine node merges its neighbours by
+//      coarse target in register slots and appends (cv << 32 | w) entries to
+//      its coarse row's bucket, one atomic reservation per slot flush (long
+//      rows: the whole warp); a warp per coarse row then sorts its bucket in
+//      shared memory (bitonic) and sums the weights of equal targets.
+//   3. rows of too many targets or entries for that: a block each, with a
+//      counter per coarse node.
+//   4. distinct counts -> prefix sum -> xadj; rows copied into place.
 #include "contract.cuh"
 #include "prims.cuh"
 
@@ -116,8 +116,7 @@ __global__ void scatter_members(int n, const int* __restrict__ cmap, const int* 
 // warp's shared-memory table (shared-memory atomics; a key is inserted by
 // compare-and-swap once), then sorts the distinct targets and writes them to
 // the node's bucket.  Nodes with more than kGatherMaxDistinct distinct targets, or more
-// than kGatherMaxEntries member entries, are flagged (sel) for the emission
-// path below.
+// than kGatherMaxEntries member entries, are listed for big_rows below.
 constexpr int kGatherWarps = 8;
 constexpr int kGatherTab = 256;                  // table slots per warp
 constexpr int kGatherMaxDistinct = kGatherTab / 2;
@@ -135,7 +134,7 @@ template <bool UNIT>
 __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) gather_rows(
     int nc, const uint32_t* __restrict__ mbeg, const int2* __restrict__ mrow, const int* __restrict__ adjncy,
     const int* __restrict__ adjwgt, const int* __restrict__ cmap, const uint32_t* __restrict__ rowoff,
-    uint64_t* bucket, uint32_t* ucnt, uint8_t* sel, unsigned* nsel) {
+    uint64_t* bucket, uint32_t* ucnt, int* big, unsigned* nbig) {
     static_assert(kGatherTab == 256 && kGatherSort >= kGatherList, "table layout");
     __shared__ uint32_t tk[kGatherWarps][kGatherTab];
     __shared__ uint32_t tv[kGatherWarps][kGatherTab];
@@ -171,10 +170,7 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) gather_
             nr1 = rowoff[cc + nwarps + 1];
         }
         if ((long long)r1 - r0 > kGatherMaxEntries) {
-            if (lane == 0) {
-                sel[c] = 1;
-                atomicAdd(nsel, 1u);
-            }
+            if (lane == 0) big[atomicAdd(nbig, 1u)] = c;
             continue;
         }
         bool over = false;
@@ -265,8 +261,7 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) gather_
                 V[sl] = 0;
             }
             if (lane == 0) {
-                sel[c] = 1;
-                atomicAdd(nsel, 1u);
+                big[atomicAdd(nbig, 1u)] = c;
                 tcount[wp] = 0;
             }
             __syncwarp();
@@ -370,22 +365,17 @@ __device__ __forceinline__ void emit_range(int e0, int e1, int step, uint32_t ow
 // Rows longer than kEmitLaneDeg are left to emit_wide.  UNIT: every edge
 // weight is 1 (adjwgt is not read).  The row entries of the next group of
 // four are loaded while the coarse ids of the current group are gathered.
-// With sel, only the fine nodes of flagged coarse nodes are emitted, and
-// nothing at all when *nsel is 0.
 template <bool UNIT>
 __global__ void __launch_bounds__(kThreads) emit_kernel(int n, const int* __restrict__ xadj,
                                                         const int* __restrict__ adjncy,
                                                         const int* __restrict__ adjwgt,
                                                         const int* __restrict__ cmap,
                                                         const uint32_t* __restrict__ rowoff, uint32_t* fill,
-                                                        uint64_t* bucket, const uint8_t* __restrict__ sel,
-                                                        const unsigned* __restrict__ nsel) {
-    if (nsel && *nsel == 0u) return;
+                                                        uint64_t* bucket) {
     for (long long base = (long long)blockIdx.x * blockDim.x; base < n; base += (long long)gridDim.x * blockDim.x) {
         const int v = (int)(base + threadIdx.x);
         if (v >= n) continue;
         const uint32_t own = (uint32_t)cmap[v];
-        if (sel && !sel[own]) continue;
         const int beg = xadj[v], end = xadj[v + 1];
         if (end - beg > kEmitLaneDeg) continue;
         uint32_t st[kEmitSlots], sw[kEmitSlots];
@@ -453,9 +443,7 @@ constexpr int kEmitChunk = 2048;
 __global__ void __launch_bounds__(kThreads) emit_wide(int n, long long m, const int* __restrict__ xadj,
                                                       const int* __restrict__ adjncy, const int* __restrict__ adjwgt,
                                                       const int* __restrict__ cmap, const uint32_t* __restrict__ rowoff,
-                                                      uint32_t* fill, uint64_t* bucket, const uint8_t* __restrict__ sel,
-                                                      const unsigned* __restrict__ nsel) {
-    if (nsel && *nsel == 0u) return;
+                                                      uint32_t* fill, uint64_t* bucket) {
     const int lane = threadIdx.x & 31;
     const long long chunks = (m + kEmitChunk - 1) / kEmitChunk;
     for (long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32; c < chunks;
@@ -472,19 +460,12 @@ __global__ void __launch_bounds__(kThreads) emit_wide(int n, long long m, const 
             const int beg = xadj[v], end = xadj[v + 1];
             if (end - beg <= kEmitLaneDeg) continue;
             const uint32_t own = (uint32_t)cmap[v];
-            if (sel && !sel[own]) continue;
             const int s = (int)std::max<long long>(lo, beg), e = (int)std::min<long long>(hi, end);
             emit_range(s + lane, e, 32, own, adjncy, adjwgt, cmap, rowoff, fill, bucket);
         }
     }
 }
 
-
-__global__ void head_flags(long long E, const uint64_t* __restrict__ K, uint32_t* h) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < E;
-         i += (long long)gridDim.x * blockDim.x)
-        h[i] = (i == 0 || K[i] != K[i - 1]) ? 1u : 0u;
-}
 
 // ---- segmented merge: entries bucketed by coarse source row, each row
 // sorted and merged on its own
@@ -499,25 +480,22 @@ constexpr int kMergeWarpsSmall = 8; // warps per block of the register merge
 // bucket; ucnt[row] = their number.  LARGE = false takes the rows of at
 // most kSegSmall entries (sorted in registers, a 512-byte staging buffer
 // per warp, so many warps fit on an SM); LARGE = true the rows of up to
-// kSegMax entries (sorted in an 8 KiB shared buffer per warp) and marks the
-// longer ones for the global path (bigsz[row] = their size).  With sel, only
-// the flagged rows (none when *nsel is 0).
+// kSegMax entries (sorted in an 8 KiB shared buffer per warp) and lists the
+// longer ones for big_rows.
 template <bool LARGE>
 __global__ void __launch_bounds__((LARGE ? kMergeWarps : kMergeWarpsSmall) * 32)
     merge_rows(int nc, const uint32_t* __restrict__ rowoff, const uint32_t* __restrict__ fill, uint64_t* bucket,
-               uint32_t* ucnt, uint32_t* bigsz, const uint8_t* __restrict__ sel, const unsigned* __restrict__ nsel) {
+               uint32_t* ucnt, int* big, unsigned* nbig) {
     constexpr int W = LARGE ? kMergeWarps : kMergeWarpsSmall;
     constexpr int CAP = LARGE ? kSegMax : kSegSmall;
     __shared__ uint64_t buf[W][CAP];
-    if (nsel && *nsel == 0u) return;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     uint64_t* b = buf[wp];
     for (long long r = (long long)blockIdx.x * W + wp; r < nc; r += (long long)gridDim.x * W) {
-        if (sel && !sel[r]) continue;  // a row of the gather path
         const long long beg = rowoff[r];
         const int s = (int)fill[r];
         if (LARGE && s > kSegMax) {
-            if (lane == 0) { bigsz[r] = (uint32_t)s; ucnt[r] = 0; }
+            if (lane == 0) big[atomicAdd(nbig, 1u)] = (int)r;
             continue;
         }
         if ((s <= kSegSmall) == LARGE) continue;  // the other kernel's row
@@ -596,43 +574,137 @@ __global__ void __launch_bounds__((LARGE ? kMergeWarps : kMergeWarpsSmall) * 32)
     }
 }
 
-// Entries of the long rows, gathered for the global sort: key cu << tb | cv.
-__global__ void gather_big(int nc, const uint32_t* __restrict__ rowoff, const uint32_t* __restrict__ bigsz,
-                           const uint32_t* __restrict__ bigoff, const uint64_t* __restrict__ bucket, int tb,
-                           uint64_t* K, uint32_t* V) {
-    for (int r = blockIdx.x; r < nc; r += gridDim.x) {
-        const uint32_t s = bigsz[r];
-        if (!s) continue;
-        const long long src = rowoff[r], dst = bigoff[r];
-        for (uint32_t i = threadIdx.x; i < s; i += blockDim.x) {
-            const uint64_t x = bucket[src + i];
-            K[dst + i] = ((uint64_t)r << tb) | (x >> 32);
-            V[dst + i] = (uint32_t)x;
+// ---- long coarse rows, a block each, by a counter per coarse node: the
+// weights add up in the block's counters in global memory (the touched ones
+// stay in L2 and are cleared behind the row), a bit per coarse node in shared
+// memory marks the targets, and walking the bits in order writes the row
+// sorted.  What a row costs is its entries plus nc / 32 words over the block;
+// sorting the same entries by (row, target) moved each of them six times
+// through memory (R-MAT 2^20, five levels: 12.6 ms of sorting, emission and
+// merge 4.5 ms -> this kernel 3.7 ms).  Targets beyond the mask's range are
+// taken in further passes over the row.
+constexpr int kBigThreads = 512;
+constexpr int kBigRange = 1 << 20;  // targets per pass: 128 KiB of mask
+constexpr int kBigBlocks = 2 * kNumSMs;
+constexpr int kBigMember = 256;     // longer member rows are walked by the whole block
+
+// bits of one pass in order -> the row's entries from `at` on; returns their number
+__device__ __forceinline__ uint32_t big_flush(uint32_t* mask, int words, int base, uint32_t* cnt, uint64_t* out) {
+    __shared__ uint32_t wsum[kBigThreads / 32 + 1];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int per = (words + kBigThreads - 1) / kBigThreads;
+    const int w0 = min(words, (int)threadIdx.x * per), w1 = min(words, w0 + per);
+    uint32_t mine = 0;
+    for (int w = w0; w < w1; ++w) mine += __popc(mask[w]);
+    uint32_t incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) wsum[wp] = incl;
+    __syncthreads();
+    if (wp == 0) {
+        const uint32_t x = lane < kBigThreads / 32 ? wsum[lane] : 0u;
+        uint32_t t = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
+            if (lane >= o) t += y;
+        }
+        if (lane < kBigThreads / 32) wsum[lane] = t - x;
+        if (lane == 31) wsum[kBigThreads / 32] = t;
+    }
+    __syncthreads();
+    uint64_t* o = out + wsum[wp] + (incl - mine);
+    for (int w = w0; w < w1; ++w) {
+        uint32_t m = mask[w];
+        if (!m) continue;
+        mask[w] = 0;
+        while (m) {
+            const int t = w * 32 + __ffs(m) - 1;
+            m &= m - 1;
+            *o++ = ((uint64_t)(uint32_t)(base + t) << 32) | __ldcg(cnt + t);
+            __stcg(cnt + t, 0u);
         }
     }
+    const uint32_t total = wsum[kBigThreads / 32];
+    __syncthreads();
+    return total;
 }
 
-// The distinct keys of the sorted long-row entries go back to the start of
-// their row's bucket, in order: position = global distinct index minus the
-// row's first distinct index (ufirst, an atomicMin).
-__global__ void first_unique(long long E, const uint64_t* __restrict__ K, const uint32_t* __restrict__ uidx, int tb,
-                             uint32_t* ufirst) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < E; i += (long long)gridDim.x * blockDim.x)
-        if (i == 0 || (K[i - 1] >> tb) != (K[i] >> tb)) ufirst[K[i] >> tb] = uidx[i];
-}
-
-__global__ void reduce_big(long long E, const uint64_t* __restrict__ K, const uint32_t* __restrict__ V,
-                           const uint32_t* __restrict__ uidx, const uint32_t* __restrict__ ufirst,
-                           const uint32_t* __restrict__ rowoff, int tb, uint64_t* bucket, uint32_t* ucnt) {
-    const uint64_t mask = (1ull << tb) - 1ull;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < E; i += (long long)gridDim.x * blockDim.x) {
-        const uint64_t k = K[i];
-        if (i > 0 && K[i - 1] == k) continue;
-        uint32_t s = V[i];
-        for (long long j = i + 1; j < E && K[j] == k; ++j) s += V[j];
-        const uint32_t r = (uint32_t)(k >> tb);
-        bucket[(long long)rowoff[r] + (uidx[i] - ufirst[r])] = ((k & mask) << 32) | s;
-        atomicAdd(&ucnt[r], 1u);
+// The rows of `list` (count of them).  MEMBERS: from the member rows of the
+// coarse node (member lists as in gather_rows); else from the fill[c] entries
+// that the emission left in the row's bucket, which the result replaces.
+template <bool UNIT, bool MEMBERS>
+__global__ void __launch_bounds__(kBigThreads) big_rows(
+    int nc, const int* __restrict__ list, const unsigned* __restrict__ count, const uint32_t* __restrict__ mbeg,
+    const int2* __restrict__ mrow, const int* __restrict__ adjncy, const int* __restrict__ adjwgt,
+    const int* __restrict__ cmap, const uint32_t* __restrict__ rowoff, const uint32_t* __restrict__ fill,
+    uint64_t* bucket, uint64_t* spare, uint32_t* counters, int range, uint32_t* ucnt) {
+    extern __shared__ uint32_t mask[];
+    const unsigned n = *count;
+    if (blockIdx.x >= n) return;
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    uint32_t* cnt = counters + (size_t)blockIdx.x * range;
+    for (int i = threadIdx.x; i < range; i += kBigThreads) __stcg(cnt + i, 0u);
+    for (int i = threadIdx.x; i < (range + 31) / 32; i += kBigThreads) mask[i] = 0;
+    __syncthreads();
+    for (unsigned i = blockIdx.x; i < n; i += gridDim.x) {
+        const int c = list[i];
+        uint64_t* row = bucket + rowoff[c];
+        uint32_t written = 0;
+        for (int base = 0; base < nc; base += range) {
+            const int R = min(range, nc - base);
+            auto add = [&](int t, uint32_t w) {
+                t -= base;
+                if ((unsigned)t >= (unsigned)R) return;
+                atomicAdd(cnt + t, w);
+                const uint32_t bit = 1u << (t & 31);
+                if (!(*(volatile uint32_t*)(mask + (t >> 5)) & bit)) atomicOr(mask + (t >> 5), bit);
+            };
+            if (MEMBERS) {
+                auto walk = [&](int b, int d, int t0, int nt) {
+                    for (int e = t0; e < d; e += 4 * nt) {
+                        int t[4];
+                        uint32_t w[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const bool in = e + q * nt < d;
+                            t[q] = in ? adjncy[b + e + q * nt] : -1;
+                            w[q] = in ? (UNIT ? 1u : (uint32_t)adjwgt[b + e + q * nt]) : 0u;
+                        }
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            if (t[q] >= 0) t[q] = cmap[t[q]];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            if (t[q] >= 0 && t[q] != c) add(t[q], w[q]);
+                    }
+                };
+                const uint32_t m0 = mbeg[c], m1 = mbeg[c + 1];
+                for (uint32_t m = m0 + wp; m < m1; m += kBigThreads / 32) {
+                    const int2 r = mrow[m];
+                    if (r.y <= kBigMember) walk(r.x, r.y, lane, 32);
+                }
+                for (uint32_t m = m0; m < m1; ++m) {
+                    const int2 r = mrow[m];
+                    if (r.y > kBigMember) walk(r.x, r.y, (int)threadIdx.x, kBigThreads);
+                }
+            } else {
+                const uint32_t s = fill[c];
+                const uint64_t* src = base == 0 ? row : spare + rowoff[c];
+                for (uint32_t e = threadIdx.x; e < s; e += kBigThreads) {
+                    const uint64_t x = src[e];
+                    // (further passes read a copy: the row is overwritten)
+                    if (base == 0 && range < nc) spare[rowoff[c] + e] = x;
+                    add((int)(x >> 32), (uint32_t)x);
+                }
+            }
+            __syncthreads();
+            written += big_flush(mask, (R + 31) / 32, base, cnt, row + written);
+        }
+        if (threadIdx.x == 0) ucnt[c] = written;
     }
 }
 
@@ -697,10 +769,16 @@ void contract(Ctx& ctx, const DevGraph& g, const int* label, int* cmap, DevGraph
         *out_adjncy = *out_adjwgt = *out_vwgt = nullptr;
         return;
     }
+    // device scalars: [0] coarse nodes, [38] long rows, [39] coarse entries,
+    // [40..43] the coarse graph's degree statistics
+    uint32_t* tot = reinterpret_cast<uint32_t*>(ctx.dscalars);
+    unsigned* nbig = reinterpret_cast<unsigned*>(ctx.dscalars + 38);
+    uint32_t* mct = reinterpret_cast<uint32_t*>(ctx.dscalars + 39);
+    unsigned* stats = reinterpret_cast<unsigned*>(ctx.dscalars + 40);
+    KB_CUDA(cudaMemsetAsync(nbig, 0, 6 * sizeof(unsigned), st));
     // 1. coarse ids
     int* mm = ctx.scratch.alloc<int>((size_t)n);
     uint32_t* pos = ctx.scratch.alloc<uint32_t>((size_t)n + 1);
-    uint32_t* tot = reinterpret_cast<uint32_t*>(ctx.dscalars);
     {
         PhaseScope ps(ctx, "contract_ids", 20.0 * n);
         fill_i32(mm, n, INT_MAX, st);
@@ -716,20 +794,19 @@ void contract(Ctx& ctx, const DevGraph& g, const int* label, int* cmap, DevGraph
     int* cvw = ctx.hier.alloc<int>((size_t)nc);
     int* cxadj = ctx.hier.alloc<int>((size_t)nc + 1);
     const long long m = g.m;
-    uint32_t* rowcap = ctx.scratch.alloc<uint32_t>((size_t)nc + 1);
-    uint32_t* rowoff = ctx.scratch.alloc<uint32_t>((size_t)nc + 1);
-    uint32_t* fill = ctx.scratch.alloc<uint32_t>((size_t)nc + 1);
-    KB_CUDA(cudaMemsetAsync(cvw, 0, sizeof(int) * (size_t)nc, st));
-    KB_CUDA(cudaMemsetAsync(rowcap, 0, sizeof(uint32_t) * ((size_t)nc + 1), st));
-    KB_CUDA(cudaMemsetAsync(fill, 0, sizeof(uint32_t) * ((size_t)nc + 1), st));
     // clusterings (several members per coarse node on average) take the
     // gather path; matchings (at most two) the emission path
     const bool gather = (long long)n * 2 >= (long long)nc * 5;
-    uint32_t* msize = nullptr;
-    if (gather) {
-        msize = ctx.scratch.alloc<uint32_t>((size_t)nc + 1);
-        KB_CUDA(cudaMemsetAsync(msize, 0, sizeof(uint32_t) * ((size_t)nc + 1), st));
-    }
+    // zeroed together: row capacities, entries (emission), distinct entries
+    // (the scans read the last one) and, gather, member counts and cursors
+    const size_t nc1 = (size_t)nc + 1;
+    uint32_t* zeroed = ctx.scratch.alloc<uint32_t>((gather ? 5 : 3) * nc1);
+    uint32_t *rowcap = zeroed, *fill = zeroed + nc1, *ucnt = zeroed + 2 * nc1;
+    uint32_t* msize = gather ? zeroed + 3 * nc1 : nullptr;
+    uint32_t* mfill = gather ? zeroed + 4 * nc1 : nullptr;
+    uint32_t* rowoff = ctx.scratch.alloc<uint32_t>(nc1);
+    KB_CUDA(cudaMemsetAsync(cvw, 0, sizeof(int) * (size_t)nc, st));
+    KB_CUDA(cudaMemsetAsync(zeroed, 0, sizeof(uint32_t) * (gather ? 5 : 3) * nc1, st));
     {
         PhaseScope ps(ctx, "contract_ids", 16.0 * n);
         make_cmap<<<grid_for(n, 256), 256, 0, st>>>(n, label, mm, pos, g.vwgt, g.xadj, cmap,
@@ -738,29 +815,14 @@ void contract(Ctx& ctx, const DevGraph& g, const int* label, int* cmap, DevGraph
         // bucket of coarse row c: [rowoff[c], rowoff[c] + its members' degrees)
         exclusive_scan_u32(rowcap, rowoff, (long long)nc + 1, nullptr, st, ctx.scratch);
     }
-    int tb = 1;
-    while ((1LL << tb) < (long long)nc) ++tb;
     uint64_t* bucket = ctx.scratch.alloc<uint64_t>((size_t)std::max<long long>(m, 1));
-    uint32_t* ucnt = ctx.scratch.alloc<uint32_t>((size_t)nc + 1);
-    uint32_t* bigsz = ctx.scratch.alloc<uint32_t>((size_t)nc + 1);
-    uint32_t* bigoff = ctx.scratch.alloc<uint32_t>((size_t)nc + 1);
-    uint32_t* big = reinterpret_cast<uint32_t*>(ctx.dscalars + 16);  // [16] long-row entries
-    // ucnt / bigsz have nc + 1 entries (the scans read the last one)
-    KB_CUDA(cudaMemsetAsync(ucnt, 0, sizeof(uint32_t) * ((size_t)nc + 1), st));
-    KB_CUDA(cudaMemsetAsync(bigsz, 0, sizeof(uint32_t) * ((size_t)nc + 1), st));
-    // 2a. gather path: member lists, then a warp per coarse node; the nodes it
-    // flags go through the emission path, which then skips all others
-    uint8_t* sel = nullptr;
-    unsigned* nsel = nullptr;
+    int* big = ctx.scratch.alloc<int>((size_t)nc);
+    uint32_t* mbeg = nullptr;
+    int2* mrow = nullptr;
     if (gather) {
-        uint32_t* mbeg = ctx.scratch.alloc<uint32_t>((size_t)nc + 1);
-        uint32_t* mfill = ctx.scratch.alloc<uint32_t>((size_t)nc);
-        int2* mrow = ctx.scratch.alloc<int2>((size_t)n);
-        sel = ctx.scratch.alloc<uint8_t>((size_t)nc);
-        nsel = reinterpret_cast<unsigned*>(ctx.dscalars + 18);  // [18] flagged nodes
-        KB_CUDA(cudaMemsetAsync(mfill, 0, sizeof(uint32_t) * (size_t)nc, st));
-        KB_CUDA(cudaMemsetAsync(sel, 0, (size_t)nc, st));
-        KB_CUDA(cudaMemsetAsync(nsel, 0, sizeof(unsigned), st));
+        // 2a. member lists, then a warp per coarse node
+        mbeg = ctx.scratch.alloc<uint32_t>(nc1);
+        mrow = ctx.scratch.alloc<int2>((size_t)n);
         {
             PhaseScope ps(ctx, "contract_ids", 12.0 * n);
             exclusive_scan_u32(msize, mbeg, (long long)nc + 1, nullptr, st, ctx.scratch);
@@ -771,85 +833,64 @@ void contract(Ctx& ctx, const DevGraph& g, const int* label, int* cmap, DevGraph
         const int gg = (int)std::max<long long>(1, std::min<long long>(div_up(nc, kGatherWarps), (long long)kNumSMs * kGatherBlocksPerSM));
         if (g.unit_weights)
             gather_rows<true><<<gg, kGatherWarps * 32, 0, st>>>(nc, mbeg, mrow, g.adjncy, g.adjwgt, cmap, rowoff,
-                                                                bucket, ucnt, sel, nsel);
+                                                                bucket, ucnt, big, nbig);
         else
             gather_rows<false><<<gg, kGatherWarps * 32, 0, st>>>(nc, mbeg, mrow, g.adjncy, g.adjwgt, cmap, rowoff,
-                                                                 bucket, ucnt, sel, nsel);
+                                                                 bucket, ucnt, big, nbig);
         KB_LAUNCH();
-    }
-    // 2b. emission straight into the coarse rows' buckets (at most m entries)
-    {
-        PhaseScope ps(ctx, "contract_emit", gather ? 0.0 : (g.unit_weights ? 8.0 : 12.0) * m + 8.0 * n);
-        if (g.unit_weights)
-            emit_kernel<true><<<grid_for(n, kThreads), kThreads, 0, st>>>(n, g.xadj, g.adjncy, g.adjwgt, cmap, rowoff,
-                                                                          fill, bucket, sel, nsel);
-        else
-            emit_kernel<false><<<grid_for(n, kThreads), kThreads, 0, st>>>(n, g.xadj, g.adjncy, g.adjwgt, cmap, rowoff,
-                                                                           fill, bucket, sel, nsel);
-        KB_LAUNCH();
-        if (g.maxdeg > kEmitLaneDeg) {
-            const long long chunks = (m + kEmitChunk - 1) / kEmitChunk;
-            emit_wide<<<grid_for(32LL * chunks, kThreads), kThreads, 0, st>>>(n, m, g.xadj, g.adjncy, g.adjwgt, cmap,
-                                                                           rowoff, fill, bucket, sel, nsel);
+    } else {
+        // 2b. emission straight into the coarse rows' buckets (at most m
+        // entries), then each row merged
+        {
+            PhaseScope ps(ctx, "contract_emit", (g.unit_weights ? 8.0 : 12.0) * m + 8.0 * n);
+            if (g.unit_weights)
+                emit_kernel<true><<<grid_for(n, kThreads), kThreads, 0, st>>>(n, g.xadj, g.adjncy, g.adjwgt, cmap,
+                                                                              rowoff, fill, bucket);
+            else
+                emit_kernel<false><<<grid_for(n, kThreads), kThreads, 0, st>>>(n, g.xadj, g.adjncy, g.adjwgt, cmap,
+                                                                               rowoff, fill, bucket);
             KB_LAUNCH();
+            if (g.maxdeg > kEmitLaneDeg) {
+                const long long chunks = (m + kEmitChunk - 1) / kEmitChunk;
+                emit_wide<<<grid_for(32LL * chunks, kThreads), kThreads, 0, st>>>(n, m, g.xadj, g.adjncy, g.adjwgt,
+                                                                                  cmap, rowoff, fill, bucket);
+                KB_LAUNCH();
+            }
         }
-    }
-    // 4. merge each row: shared-memory sort for rows up to kSegMax entries
-    {
-        PhaseScope ps(ctx, "contract_merge", gather ? 0.0 : 16.0 * m);
+        PhaseScope ps(ctx, "contract_merge", 16.0 * m);
         const int gs = (int)std::max<long long>(1, std::min<long long>(div_up(nc, kMergeWarpsSmall), (long long)kNumSMs * 16));
-        merge_rows<false><<<gs, kMergeWarpsSmall * 32, 0, st>>>(nc, rowoff, fill, bucket, ucnt, bigsz, sel, nsel);
+        merge_rows<false><<<gs, kMergeWarpsSmall * 32, 0, st>>>(nc, rowoff, fill, bucket, ucnt, big, nbig);
         KB_LAUNCH();
-        if (g.maxdeg > 0) {
-            const int gb = (int)std::max<long long>(1, std::min<long long>(div_up(nc, kMergeWarps), (long long)kNumSMs * 7));
-            merge_rows<true><<<gb, kMergeWarps * 32, 0, st>>>(nc, rowoff, fill, bucket, ucnt, bigsz, sel, nsel);
-            KB_LAUNCH();
-        }
-        exclusive_scan_u32(bigsz, bigoff, (long long)nc + 1, big, st, ctx.scratch);
+        const int gb = (int)std::max<long long>(1, std::min<long long>(div_up(nc, kMergeWarps), (long long)kNumSMs * 7));
+        merge_rows<true><<<gb, kMergeWarps * 32, 0, st>>>(nc, rowoff, fill, bucket, ucnt, big, nbig);
+        KB_LAUNCH();
     }
-    // row lengths -> coarse xadj and the coarse degree statistics, read back
-    // with the long-row count in one synchronisation (redone below in the
-    // rare case of long rows, whose lengths the global path still has to add)
-    unsigned* stats = reinterpret_cast<unsigned*>(ctx.dscalars + 40);  // [40..43]
-    uint32_t* mct = reinterpret_cast<uint32_t*>(ctx.dscalars + 17);    // [17] coarse entries
-    auto rows_and_stats = [&]() {
+    // 3. the long rows: counters of up to 20 B per entry of the level
+    {
+        PhaseScope ps(ctx, "contract_big", 0);
+        const int range = std::min(nc, kBigRange);
+        const int blocks = (int)std::max<long long>(1, std::min<long long>({(long long)kBigBlocks, (long long)nc,
+                                                                            5 * m / range}));
+        uint32_t* counters = ctx.scratch.alloc<uint32_t>((size_t)blocks * range);
+        uint64_t* spare = !gather && range < nc ? ctx.scratch.alloc<uint64_t>((size_t)std::max<long long>(m, 1)) : nullptr;
+        const size_t smem = sizeof(uint32_t) * (size_t)((range + 31) / 32);
+        auto kernel = gather ? (g.unit_weights ? big_rows<true, true> : big_rows<false, true>) : big_rows<false, false>;
+        if (smem > 40 * 1024)
+            KB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<blocks, kBigThreads, smem, st>>>(nc, big, nbig, mbeg, mrow, g.adjncy, g.adjwgt, cmap, rowoff, fill,
+                                                  bucket, spare, counters, range, ucnt);
+        KB_LAUNCH();
+    }
+    // 4. row lengths -> coarse xadj and the coarse degree statistics, read
+    // back in one synchronisation
+    {
         PhaseScope ps(ctx, "contract_rows", 8.0 * nc);
         exclusive_scan_u32(ucnt, reinterpret_cast<uint32_t*>(cxadj), (long long)nc + 1, mct, st, ctx.scratch);
-        KB_CUDA(cudaMemsetAsync(stats, 0, 4 * sizeof(unsigned), st));
         coarse_stats<<<grid_for(nc, 256), 256, 0, st>>>(nc, ucnt, cvw, stats);
         KB_LAUNCH();
-        // pinned[0] long-row entries, [1] coarse entries, [2..5] statistics
-        KB_CUDA(cudaMemcpyAsync(ctx.pinned, big, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-        KB_CUDA(cudaMemcpyAsync(ctx.pinned + 1, mct, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-        KB_CUDA(cudaMemcpyAsync(ctx.pinned + 2, stats, 4 * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+        // pinned[1] coarse entries, [2..5] statistics
+        KB_CUDA(cudaMemcpyAsync(ctx.pinned + 1, mct, 5 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
         KB_CUDA(cudaStreamSynchronize(st));
-    };
-    rows_and_stats();
-    const long long EB = ctx.pinned[0];
-    if (EB > 0) {
-        // longer rows: global LSD radix sort of their entries, then reduce
-        const size_t mk2 = ctx.scratch.mark();
-        uint64_t* K0 = ctx.scratch.alloc<uint64_t>((size_t)EB);
-        uint32_t* V0 = ctx.scratch.alloc<uint32_t>((size_t)EB);
-        uint64_t* K1 = ctx.scratch.alloc<uint64_t>((size_t)EB);
-        uint32_t* V1 = ctx.scratch.alloc<uint32_t>((size_t)EB);
-        uint32_t* uidx = ctx.scratch.alloc<uint32_t>((size_t)EB);
-        uint32_t* ufirst = ctx.scratch.alloc<uint32_t>((size_t)nc + 1);
-        PhaseScope ps(ctx, "contract_sort", 32.0 * EB * ((2 * tb + 7) / 8));
-        gather_big<<<grid_for(nc, 256), 256, 0, st>>>(nc, rowoff, bigsz, bigoff, bucket, tb, K0, V0);
-        KB_LAUNCH();
-        const int which = radix_sort_pairs(K0, V0, K1, V1, EB, 2 * tb, st, ctx.scratch);
-        uint64_t* K = which ? K1 : K0;
-        uint32_t* V = which ? V1 : V0;
-        head_flags<<<grid_for(EB, 256), 256, 0, st>>>(EB, K, uidx);
-        KB_LAUNCH();
-        exclusive_scan_u32(uidx, uidx, EB, nullptr, st, ctx.scratch);
-        first_unique<<<grid_for(EB, 256), 256, 0, st>>>(EB, K, uidx, tb, ufirst);
-        KB_LAUNCH();
-        reduce_big<<<grid_for(EB, 256), 256, 0, st>>>(EB, K, V, uidx, ufirst, rowoff, tb, bucket, ucnt);
-        KB_LAUNCH();
-        ctx.scratch.release(mk2);
-        rows_and_stats();
     }
     // 5. the rows themselves
     const long long mc = (long long)ctx.pinned[1];
