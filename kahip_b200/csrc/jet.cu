@@ -433,15 +433,8 @@ __device__ __forceinline__ void choose_row(const JetArgs& A, int v, uint32_t* cn
     else __syncwarp();
 }
 
-// Rows of more than kDeferRow entries, listed once per level: a warp's from
-// the front of `list`, a block's from its end.
-struct JetRows {
-    int* list;
-    unsigned* count;  // [0] a warp's, [1] a block's
-};
-
 template <bool UNIT, bool DENSE>
-__global__ void __launch_bounds__(kThreads, 4) jet_loop(JetLoop J, JetRows R, sweep::SweepArgs a, sweep::BalanceArgs B,
+__global__ void __launch_bounds__(kThreads, 4) jet_loop(JetLoop J, sweep::SweepArgs a, sweep::BalanceArgs B,
                                                         TeamArgs T) {
     __shared__ sweep::SweepQueue queue;
     __shared__ sweep::WeighSmem ws;
@@ -458,15 +451,9 @@ __global__ void __launch_bounds__(kThreads, 4) jet_loop(JetLoop J, JetRows R, sw
         if (threadIdx.x < 4) J.ring[threadIdx.x] = 0;
         if (threadIdx.x < 2) J.cut[threadIdx.x] = 0;
     }
-    for (long long base = (long long)blockIdx.x * kThreads; base < n; base += team.size()) {
-        const int v = (int)(base + threadIdx.x);
-        if (v < n) J.moved_at[v] = -2;
-        if constexpr (DENSE) {
-            const int d = v < n ? J.A.xadj[v + 1] - J.A.xadj[v] : 0;
-            sweep::append_aggregated(d > sweep::kDeferRow && d <= sweep::kHugeDense, v, R.list, R.count);
-            if (d > sweep::kHugeDense) R.list[n - 1 - (int)atomicAdd(R.count + 1, 1u)] = v;
-        }
-    }
+    for (long long v = team.rank(); v < n; v += team.size()) J.moved_at[v] = -2;
+    const sweep::LongRows R = a.rows;
+    sweep::list_rows<DENSE>(team, J.A.xadj, n, R);
     if constexpr (!DENSE)
         if ((int)blockIdx.x < J.wblocks)
             for (int b = threadIdx.x; b < k; b += kThreads) J.counters[(size_t)blockIdx.x * k + b] = 0;
@@ -658,12 +645,6 @@ bool jet_refine_team(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, ui
     J.moved_at = ctx.scratch.alloc<int>((size_t)n);
     J.wblocks = std::min(blocks, 2 * kNumSMs);
     if (!dense) J.counters = ctx.scratch.alloc<uint32_t>((size_t)J.wblocks * k);
-    JetRows R{};
-    if (dense) {
-        R.list = ctx.scratch.alloc<int>((size_t)n);
-        R.count = ctx.scratch.alloc<unsigned>(2);
-        KB_CUDA(cudaMemsetAsync(R.count, 0, 2 * sizeof(unsigned), ctx.stream));
-    }
     J.cut = ctx.scratch.alloc<unsigned long long>(2);
     J.ring = ctx.scratch.alloc<unsigned>(4);
     J.iters = kn.jet_iters;
@@ -687,9 +668,9 @@ bool jet_refine_team(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, ui
     sweep::SweepArgs a = sweep::base_args(g, b);
     a.bound = bound;
     a.P = kn.ref_classes;
-    a.H = ctx.scratch.alloc<uint32_t>((size_t)k * a.P);
-    a.minvP = ctx.scratch.alloc<int>((size_t)k * a.P);
+    a.rows = sweep::alloc_rows(ctx, n);
     sweep::BalanceArgs B{};
+    B.adm = sweep::alloc_admission(ctx, k, a.P);
     B.k = k;
     B.iters = kn.bal_iters;
     B.seed = kn.seed;
@@ -700,7 +681,7 @@ bool jet_refine_team(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, ui
     bool done;
     {
         PhaseScope ps(ctx, "jet_loop", 0);
-        done = launch_team(ctx, kernel, room, blocks, smem, J, R, a, B);
+        done = launch_team(ctx, kernel, room, blocks, smem, J, a, B);
     }
     ctx.scratch.release(mk);
     return done;

@@ -220,6 +220,18 @@ int admit_blocks() { return (kStripes + 1) * 4; }
 
 }  // namespace
 
+// Memory of a team's admission data and of its list of long rows.
+Admission sweep::alloc_admission(Ctx& ctx, int k, int P) {
+    return Admission{ctx.scratch.alloc<uint32_t>(2 * (size_t)k * P), ctx.scratch.alloc<int>(2 * (size_t)k * P),
+                     ctx.scratch.alloc<uint32_t>((size_t)k)};
+}
+
+LongRows sweep::alloc_rows(Ctx& ctx, int n) {
+    LongRows r{ctx.scratch.alloc<int>((size_t)n), ctx.scratch.alloc<unsigned>(2)};
+    KB_CUDA(cudaMemsetAsync(r.count, 0, 2 * sizeof(unsigned), ctx.stream));
+    return r;
+}
+
 SweepBuffers sweep::make_buffers(Ctx& ctx, const DevGraph& g, int team) {
     SweepBuffers b;
     Arena& A = ctx.scratch;
@@ -446,6 +458,7 @@ struct RefineArgs {
     unsigned* lcount;    // [2]
     unsigned* moved;     // [2]
     unsigned* counters;  // 2 kTeamSet
+    Admission adm;
 };
 
 // All rounds of one level's refinement, ending after a round without moves.
@@ -457,10 +470,9 @@ __global__ void __launch_bounds__(kThreads, 4) refine_team(SweepArgs a, RefineAr
     Team team(T);
     const TeamSpace S = team_space<DENSE>(dyn, R.k);
     const int lane = threadIdx.x & 31;
-    for (long long i = team.rank(); i < (long long)R.k * a.P; i += team.size()) {
-        a.H[i] = 0;
-        a.minvP[i] = INT_MAX;
-    }
+    const LongRows rows = a.rows;
+    clear_admission(team, a, R.adm, R.k);
+    list_rows<DENSE>(team, a.xadj, a.n, rows);
     for (long long v = team.rank(); v < a.n; v += team.size()) R.stamp[v] = 0;
     if (blockIdx.x == 0) {
         for (int i = threadIdx.x; i < 2 * kTeamSet; i += kThreads) R.counters[i] = 0;
@@ -476,6 +488,7 @@ __global__ void __launch_bounds__(kThreads, 4) refine_team(SweepArgs a, RefineAr
         a.active = r == 0 ? R.active0 : flags_in ? (in ? R.flags[1] : R.flags[0]) : nullptr;
         a.vlist = r > 0 && !flags_in ? (in ? R.list[1] : R.list[0]) : nullptr;
         a.vcount = R.lcount + in;
+        a.rows.list = a.vlist ? nullptr : rows.list;  // (a list of vertices holds its long rows itself)
         // the next round's set: flags when the last known round moved many,
         // else a list (lp_refine)
         const bool flags_out = moved_prev == ~0ull || moved_prev * 64 > (unsigned long long)a.n;
@@ -487,6 +500,7 @@ __global__ void __launch_bounds__(kThreads, 4) refine_team(SweepArgs a, RefineAr
         for (uint32_t s = 0; s < a.S; ++s, p ^= 1) {
             a.s = s;
             use_set(a, R.counters, p);
+            use_admission(team, a, R.adm, R.k, p, R.bw);
             if (s == 0) {  // what round r - 1 swept from
                 if (flags_out)
                     for (long long i = team.rank(); i < (a.n + 3LL) / 4; i += team.size())
@@ -495,13 +509,9 @@ __global__ void __launch_bounds__(kThreads, 4) refine_team(SweepArgs a, RefineAr
             }
             if (!(alive = team_sweep<REFINE, UNIT, DENSE>(team, a, queue, S, red))) break;
             if (s == 0 && team.leader()) R.moved[out] = 0;  // every block has read it by now
-            each_proposal(a, [&](int v) {
-                if (v >= 0) class_decide_one(a, R.bw, 1, v);
-            });
-            if (!(alive = team.sync())) break;
             unsigned mv = 0;
             each_proposal(a, [&](int v) {
-                const bool moved = v >= 0 && class_apply_one(a, R.part, R.bw, v);
+                const bool moved = v >= 0 && class_settle(a, R.adm.snap, 1, R.part, R.bw, v);
                 int e0 = 0, e1 = 0;
                 if (moved) {
                     ++mv;
@@ -544,6 +554,7 @@ __global__ void __launch_bounds__(kThreads, 4) balance_team(SweepArgs a, Balance
     Team team(T);
     const TeamSpace S = team_space<DENSE>(dyn, B.k);
     balance_clear(team, a, B);
+    list_rows<DENSE>(team, a.xadj, a.n, a.rows);
     if (blockIdx.x == 0)
         for (int i = threadIdx.x; i < 2 * kTeamSet; i += kThreads) B.counters[i] = 0;
     int p = 0;
@@ -640,8 +651,8 @@ bool lp_refine_team(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, uin
     a.bound = bound;
     a.S = (uint32_t)kn.ref_subrounds;
     a.P = kn.ref_classes;
-    a.H = ctx.scratch.alloc<uint32_t>((size_t)kn.k * a.P);
-    a.minvP = ctx.scratch.alloc<int>((size_t)kn.k * a.P);
+    a.rows = alloc_rows(ctx, g.n);
+    R.adm = alloc_admission(ctx, kn.k, a.P);
     bool done;
     {
         PhaseScope ps(ctx, "lp_refine_team", 0);
@@ -866,9 +877,8 @@ bool balance(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, uint32_t b
         SweepArgs a = base_args(g, b);
         a.bound = bound;
         a.P = P;
-        a.H = H;
-        a.minvP = minvP;
-        const BalanceArgs B{k, kn.bal_iters, kn.seed, level, part, bw, HS, b.counters};
+        a.rows = alloc_rows(ctx, g.n);
+        const BalanceArgs B{k, kn.bal_iters, kn.seed, level, part, bw, HS, alloc_admission(ctx, k, P), b.counters};
         bool done;
         {
             PhaseScope ps(ctx, "balance", 0);

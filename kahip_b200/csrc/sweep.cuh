@@ -35,6 +35,13 @@ struct SList {
     int ns;           // stripes, a power of two (kStripes, or fewer for a small team)
 };
 
+// Rows of more than kDeferRow entries, listed once per level: a warp's from
+// the front of the list, a block's from its end.
+struct LongRows {
+    int* list;        // n; null: not listed
+    unsigned* count;  // [0] a warp's, [1] a block's
+};
+
 // Everything a sweep reads or writes; passed by value.
 struct SweepArgs {
     int n;
@@ -60,6 +67,7 @@ struct SweepArgs {
     int* minvP;                         // smallest proposer per (target, class)
     int* heavy; unsigned* hcount;       // deferred high-degree vertices
     unsigned* hugecount;                // a team: those listed from heavy's end
+    LongRows rows;                      // a team: the level's long rows, when they are listed
     SList plist;                        // vertices that proposed a move this sub-round
     int* hplist; unsigned* hpcount;     // proposals of high-degree vertices
     int singletons;                     // every label is its own vertex id and rows have
@@ -644,7 +652,7 @@ __device__ __forceinline__ void lane_sweep(const SweepArgs& a, SweepQueue& queue
             status = lane_vertex<MODE, kSlots, UNIT, STASH, DEFER ? kDeferRow : kWin>(
                 a, v, STASH ? T->stash + lane : nullptr, wv, we);
         if constexpr (DEFER) {
-            defer_row<HUGE>(a, status == 1 || status == 2, v);
+            defer_row<HUGE>(a, status == 1 || (status == 2 && !a.rows.list), v);
             append_striped(status == 3, v, a.plist);
             return;
         }
@@ -1089,21 +1097,24 @@ __device__ __forceinline__ void dense_vertex(const SweepArgs& a, int v, int k, u
     else __syncwarp();
 }
 
-// The deferred rows of a sub-round.
-template <int MODE, bool UNIT, bool DENSE>
-__device__ __forceinline__ void deferred_rows(const SweepArgs& a, const TeamSpace& S, RowRed& red) {
+// Listed rows: n a warp's, nh a block's.  MEMBERS: only those that take part
+// in the sub-round (the level's list holds all long rows).
+template <int MODE, bool UNIT, bool DENSE, bool MEMBERS>
+__device__ __forceinline__ void listed_rows(const SweepArgs& a, const int* list, unsigned n, unsigned nh,
+                                            const TeamSpace& S, RowRed& red) {
     const unsigned W = gridDim.x * kWarpsPerBlock, wid = threadIdx.x >> 5;
-    const unsigned n = *a.hcount, nh = *a.hugecount;
     for (unsigned i = blockIdx.x + wid * gridDim.x; i < n; i += W) {
+        const int v = list[i];
+        if (MEMBERS && !member<MODE>(a, v)) continue;
         if constexpr (DENSE)
-            dense_vertex<MODE, UNIT, false>(a, a.heavy[i], S.k, S.tab + (size_t)wid * S.k, S.val + wid * S.words(),
-                                            red);
+            dense_vertex<MODE, UNIT, false>(a, v, S.k, S.tab + (size_t)wid * S.k, S.val + wid * S.words(), red);
         else
-            hash_vertex<MODE, UNIT>(a, a.heavy[i], S.tab + wid * kHashTab, S.val + wid * kHashTab);
+            hash_vertex<MODE, UNIT>(a, v, S.tab + wid * kHashTab, S.val + wid * kHashTab);
     }
-    __syncthreads();
+    if (nh) __syncthreads();  // the warps' tables become the block's
     for (unsigned i = blockIdx.x; i < nh; i += gridDim.x) {
-        const int v = a.heavy[a.n - 1 - (int)i];
+        const int v = list[a.n - 1 - (int)i];
+        if (MEMBERS && !member<MODE>(a, v)) continue;
         if constexpr (DENSE) {
             dense_vertex<MODE, UNIT, true>(a, v, S.k, S.tab, S.val, red);
         } else {
@@ -1119,37 +1130,72 @@ template <int MODE, bool UNIT, bool DENSE>
 __device__ __forceinline__ bool team_sweep(Team& team, const SweepArgs& a, SweepQueue& queue, const TeamSpace& S,
                                            RowRed& red) {
     lane_sweep<MODE, UNIT, false, DENSE ? kHugeDense : kHashRow>(a, queue, nullptr, nullptr);
+    if (a.rows.list)
+        listed_rows<MODE, UNIT, DENSE, true>(a, a.rows.list, a.rows.count[0], a.rows.count[1], S, red);
     if (!team.sync()) return false;
-    if (*a.hcount == 0 && *a.hugecount == 0) return true;
-    deferred_rows<MODE, UNIT, DENSE>(a, S, red);
+    const unsigned n = *a.hcount, nh = *a.hugecount;
+    if (n == 0 && nh == 0) return true;
+    listed_rows<MODE, UNIT, DENSE, false>(a, a.heavy, n, nh, S, red);
     return team.sync();
 }
 
-// class_decide's and class_apply's rules for one proposal
-__device__ __forceinline__ void class_decide_one(const SweepArgs& a, const uint32_t* bw, int strict, int v) {
-    const int b = a.pt[v];
-    if (b < 0) return;
-    const int c = a.pc[v];
-    if (c < 0) return;
-    const long long cap = (long long)a.bound - (strict ? 1 : 0) - (long long)bw[b];
-    if (!admit(a.H, a.minvP, a.P, b, c, v, (uint32_t)a.vwgt[v], cap)) a.pt[v] = -2 - b;
+// Lists the level's long rows (count zero before; a barrier after).
+template <bool DENSE>
+__device__ __forceinline__ void list_rows(Team& team, const int* xadj, int n, const LongRows& R) {
+    constexpr int HUGE = DENSE ? kHugeDense : kHashRow;
+    for (long long base = (long long)blockIdx.x * kThreads; base < n; base += team.size()) {
+        const int v = (int)(base + threadIdx.x);
+        const int d = v < n ? xadj[v + 1] - xadj[v] : 0;
+        append_aggregated(d > kDeferRow && d <= HUGE, v, R.list, R.count);
+        if (d > HUGE) R.list[n - 1 - (int)atomicAdd(R.count + 1, 1u)] = v;
+    }
 }
 
-// true when v moved
-__device__ __forceinline__ bool class_apply_one(const SweepArgs& a, int* part, uint32_t* bw, int v) {
-    const int t = a.pt[v];
-    if (t == -1) return false;
-    const int c = a.pc[v];
-    if (c < 0) return false;  // dropped before admission (balance)
-    const int b = t >= 0 ? t : -2 - t;
-    a.H[(size_t)b * a.P + c] = 0;
-    a.minvP[(size_t)b * a.P + c] = INT_MAX;
-    if (t < 0) return false;
+// class_decide's and class_apply's rules for one proposal in one step: the
+// decision reads the block weights as they were at the sweep (snap) and the
+// admission data, which no one changes meanwhile.  True when v moved.
+__device__ __forceinline__ bool class_settle(const SweepArgs& a, const uint32_t* snap, int strict, int* part,
+                                             uint32_t* bw, int v) {
+    const int b = a.pt[v], c = a.pc[v];
+    if (b < 0 || c < 0) return false;  // (no class: dropped before admission, balance)
     const uint32_t cv = (uint32_t)a.vwgt[v];
+    const long long cap = (long long)a.bound - (strict ? 1 : 0) - (long long)snap[b];
+    if (!admit(a.H, a.minvP, a.P, b, c, v, cv, cap)) return false;
     atomicSub(&bw[part[v]], cv);
-    atomicAdd(&bw[t], cv);
-    part[v] = t;
+    atomicAdd(&bw[b], cv);
+    part[v] = b;
     return true;
+}
+
+// Admission data of a team, two sets in turn: a sub-round fills one and
+// clears the other, which every block stopped reading at the barrier that
+// ended the sub-round before.
+struct Admission {
+    uint32_t* H;     // 2 k P
+    int* minvP;      // 2 k P
+    uint32_t* snap;  // k: the block weights at the sweep
+};
+
+__device__ __forceinline__ void use_admission(Team& team, SweepArgs& a, const Admission& M, int k, int p,
+                                              const uint32_t* bw) {
+    const size_t kP = (size_t)k * a.P;
+    a.H = M.H + (p ? kP : 0);
+    a.minvP = M.minvP + (p ? kP : 0);
+    uint32_t* h = M.H + (p ? 0 : kP);
+    int* mv = M.minvP + (p ? 0 : kP);
+    for (long long i = team.rank(); i < (long long)kP; i += team.size()) {
+        h[i] = 0;
+        mv[i] = INT_MAX;
+    }
+    if (blockIdx.x == 0)
+        for (int b = threadIdx.x; b < k; b += kThreads) M.snap[b] = bw[b];
+}
+
+__device__ __forceinline__ void clear_admission(Team& team, const SweepArgs& a, const Admission& M, int k) {
+    for (long long i = team.rank(); i < 2LL * k * a.P; i += team.size()) {
+        M.H[i] = 0;
+        M.minvP[i] = INT_MAX;
+    }
 }
 
 // Block weights looked over by every block of the team for itself.
@@ -1199,16 +1245,14 @@ struct BalanceArgs {
     int* part;
     uint32_t* bw;
     uint32_t* HS;        // k * kBalClasses, zero between calls
+    Admission adm;
     unsigned* counters;  // 2 kTeamSet, zero before the first call
 };
 
-// H, minvP and HS in the state the balance steps expect.
+// The admission data and HS in the state the balance steps expect.
 __device__ __forceinline__ void balance_clear(Team& team, const SweepArgs& a, const BalanceArgs& B) {
     for (long long i = team.rank(); i < (long long)B.k * kBalClasses; i += team.size()) B.HS[i] = 0;
-    for (long long i = team.rank(); i < (long long)B.k * a.P; i += team.size()) {
-        a.H[i] = 0;
-        a.minvP[i] = INT_MAX;
-    }
+    clear_admission(team, a, B.adm, B.k);
 }
 
 // The balance repair of lp.cu's balance(), all iterations; p: the counter
@@ -1226,6 +1270,7 @@ __device__ __forceinline__ bool balance_steps(Team& team, SweepArgs a, const Bal
         a.ks_sub = stream_key(B.seed, TAG_BCLS, B.level, it);  // release class stream
         const uint64_t ks_prio = stream_key(B.seed, TAG_BPRIO, B.level, it);
         use_set(a, B.counters, p);
+        use_admission(team, a, B.adm, B.k, p, B.bw);
         if (!team_sweep<BALANCE, UNIT, DENSE>(team, a, queue, S, red)) return false;
         // release thresholds, computed by every block for itself: the number
         // of classes before which less than the excess is released
@@ -1278,11 +1323,7 @@ __device__ __forceinline__ bool balance_steps(Team& team, SweepArgs a, const Bal
         });
         if (!team.sync()) return false;
         each_proposal(a, [&](int v) {
-            if (v >= 0) class_decide_one(a, B.bw, 0, v);
-        });
-        if (!team.sync()) return false;
-        each_proposal(a, [&](int v) {
-            if (v >= 0) class_apply_one(a, B.part, B.bw, v);
+            if (v >= 0) class_settle(a, B.adm.snap, 0, B.part, B.bw, v);
         });
         for (int b = blockIdx.x; b < B.k; b += gridDim.x)
             if (thr[b] > 0) B.HS[(size_t)b * kBalClasses + threadIdx.x] = 0;
@@ -1314,6 +1355,8 @@ struct SweepBuffers {
 // (team = 0) or for a team of that many blocks.
 SweepBuffers make_buffers(Ctx& ctx, const DevGraph& g, int team);
 SweepArgs base_args(const DevGraph& g, const SweepBuffers& b);
+Admission alloc_admission(Ctx& ctx, int k, int P);
+LongRows alloc_rows(Ctx& ctx, int n);
 
 // Every warp of a team has a counter per block of the partition in shared
 // memory (37 KB a block at the limit); with more blocks the team aggregates
