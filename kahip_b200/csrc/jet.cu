@@ -224,21 +224,35 @@ __global__ void __launch_bounds__(kThreads) jet_choose_wide(JetArgs A, uint32_t*
     choose_wide(A, counters + (size_t)blockIdx.x * A.k, gridDim.x);
 }
 
+// Four entries are in flight: an entry is a chain of three loads (target, its
+// destination and block, a candidate's gain).
 template <bool UNIT>
 __device__ __forceinline__ long long afterburn_sum(const JetArgs& A, int v, int beg, int end, int step, int first) {
     const int dv = A.dest[v], pv = A.part[v];
     const long long gv = A.gain[v];
     long long adj = 0;
-    for (int e = beg + first; e < end; e += step) {
-        const int u = A.adjncy[e];
-        int bu = A.part[u];
-        const int du = A.dest[u];
-        if (du >= 0) {
-            const long long gu = A.gain[u];
-            if (gu > gv || (gu == gv && u < v)) bu = du;
+    for (int e = beg + first; e < end; e += 4 * step) {
+        int u[4], w[4], bu[4], du[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const bool in = e + q * step < end;
+            u[q] = in ? A.adjncy[e + q * step] : -1;
+            w[q] = in ? (UNIT ? 1 : A.adjwgt[e + q * step]) : 0;
         }
-        if (bu == dv) adj += UNIT ? 1 : A.adjwgt[e];
-        else if (bu == pv) adj -= UNIT ? 1 : A.adjwgt[e];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            bu[q] = u[q] >= 0 ? A.part[u[q]] : -1;
+            du[q] = u[q] >= 0 ? A.dest[u[q]] : -1;
+        }
+        long long gu[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) gu[q] = du[q] >= 0 ? A.gain[u[q]] : 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (du[q] >= 0 && (gu[q] > gv || (gu[q] == gv && u[q] < v))) bu[q] = du[q];
+            if (bu[q] == dv) adj += w[q];
+            else if (bu[q] == pv) adj -= w[q];
+        }
     }
     return adj;
 }
@@ -439,8 +453,10 @@ __global__ void __launch_bounds__(kThreads, 4) jet_loop(JetLoop J, sweep::SweepA
     __shared__ sweep::SweepQueue queue;
     __shared__ sweep::WeighSmem ws;
     __shared__ sweep::RowRed red;
+    __shared__ int tcount[sweep::kWarpsPerBlock];
     extern __shared__ __align__(16) unsigned char dyn[];
     Team team(T);
+    a.tcount = tcount;
     const int n = J.A.n, k = J.A.k;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned W = gridDim.x * (kThreads / 32), wg = blockIdx.x + wid * gridDim.x;
@@ -660,16 +676,14 @@ bool jet_refine_team(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, ui
     J.A.moved_at = J.moved_at;
     J.A.c4 = level == 0 ? kn.jet_c0 : kn.jet_c;
     J.A.gain = ctx.scratch.alloc<long long>((size_t)n);
-    const sweep::SweepBuffers b = sweep::make_buffers(ctx, g, blocks);
-    // the destinations and the wide rows are dead while the balance repair
-    // uses its proposal targets and high-degree list
-    J.A.dest = b.pt;
-    J.A.wide = b.heavy;
-    sweep::SweepArgs a = sweep::base_args(g, b);
+    J.A.dest = ctx.scratch.alloc<int>((size_t)n);
+    sweep::BalanceArgs B{};
+    sweep::SweepArgs a = sweep::team_args(ctx, g, blocks, &B.counters);
+    // the wide rows are dead while the balance repair uses its list
+    J.A.wide = a.heavy;
     a.bound = bound;
     a.P = kn.ref_classes;
     a.rows = sweep::alloc_rows(ctx, n);
-    sweep::BalanceArgs B{};
     B.adm = sweep::alloc_admission(ctx, k, a.P);
     B.k = k;
     B.iters = kn.bal_iters;
@@ -677,7 +691,6 @@ bool jet_refine_team(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, ui
     B.level = level;
     B.bw = bw;
     B.HS = ctx.scratch.alloc<uint32_t>((size_t)k * sweep::kBalClasses);
-    B.counters = b.counters;
     bool done;
     {
         PhaseScope ps(ctx, "jet_loop", 0);

@@ -222,8 +222,29 @@ int admit_blocks() { return (kStripes + 1) * 4; }
 
 // Memory of a team's admission data and of its list of long rows.
 Admission sweep::alloc_admission(Ctx& ctx, int k, int P) {
-    return Admission{ctx.scratch.alloc<uint32_t>(2 * (size_t)k * P), ctx.scratch.alloc<int>(2 * (size_t)k * P),
-                     ctx.scratch.alloc<uint32_t>((size_t)k)};
+    return Admission{ctx.scratch.alloc<uint32_t>(2 * (size_t)k * P), ctx.scratch.alloc<int>(2 * (size_t)k * P)};
+}
+
+SweepArgs sweep::team_args(Ctx& ctx, const DevGraph& g, int blocks, unsigned** counters) {
+    SweepArgs a{};
+    const long long n = std::max(g.n, 1), W = (long long)blocks * kWarpsPerBlock;
+    a.n = g.n;
+    a.xadj = g.xadj;
+    a.adjncy = g.adjncy;
+    a.adjwgt = g.adjwgt;
+    a.vwgt = g.vwgt;
+    a.heavy = ctx.scratch.alloc<int>((size_t)n);
+    a.work = ctx.work;
+    a.err = ctx.dscalars + 60;
+    // a warp's list: the vertices of its share of the sweep's tasks, of the
+    // two lists of rows (which have no vertex in common), and the block's
+    // rows, which its first warp lists
+    const long long tasks = (n + 32 * kSpan - 1) / (32 * kSpan), huge = std::min(n, g.m / (kHashRow + 1));
+    const long long cap = (tasks + W - 1) / W * 32 * kSpan + n / W + 2 + huge / blocks + 2;
+    a.tcap = (int)cap;
+    a.tlist = ctx.scratch.alloc<int2>((size_t)(W * cap));
+    *counters = ctx.scratch.alloc<unsigned>(2 * kTeamSet);
+    return a;
 }
 
 LongRows sweep::alloc_rows(Ctx& ctx, int n) {
@@ -232,7 +253,7 @@ LongRows sweep::alloc_rows(Ctx& ctx, int n) {
     return r;
 }
 
-SweepBuffers sweep::make_buffers(Ctx& ctx, const DevGraph& g, int team) {
+SweepBuffers sweep::make_buffers(Ctx& ctx, const DevGraph& g) {
     SweepBuffers b;
     Arena& A = ctx.scratch;
     const long long n = std::max(g.n, 1);
@@ -240,24 +261,21 @@ SweepBuffers sweep::make_buffers(Ctx& ctx, const DevGraph& g, int team) {
     b.pc = A.alloc<int>((size_t)n);
     b.heavy = A.alloc<int>((size_t)n);
     b.hplist = A.alloc<int>((size_t)n);
-    b.counters = A.alloc<unsigned>(2 * kTeamSet);
+    b.counters = A.alloc<unsigned>(2 * kStripes + 8);
     // stripe capacities from the producers' warp counts and per-warp work
     const long long tasks = (n + 32 * kSpan - 1) / (32 * kSpan);
     // one wave: 64 registers and 37 KB of shared memory per 256-thread
     // block leave room for 4 blocks per SM
     b.lblocks = (int)std::max<long long>(1, std::min<long long>(div_up(tasks, kWarpsPerBlock), kNumSMs * 4LL));
-    if (team) b.lblocks = team;
     const long long wl = (long long)b.lblocks * kWarpsPerBlock;
-    int ns = kStripes;  // a small team: at most a stripe per warp
-    while (team && ns > wl) ns >>= 1;
-    const long long cap_l = ((wl + ns - 1) / ns) * ((tasks + wl - 1) / wl) * 32 * kSpan;
-    b.plist = SList{A.alloc<int>((size_t)(ns * cap_l)), b.counters + kStripes, cap_l, ns};
+    const long long cap_l = ((wl + kStripes - 1) / kStripes) * ((tasks + wl - 1) / wl) * 32 * kSpan;
+    b.plist = SList{A.alloc<int>((size_t)(kStripes * cap_l)), b.counters + kStripes, cap_l};
     b.work = ctx.work;
     b.err = ctx.dscalars + 60;
     b.gcap = 0;
     b.hblocks = 0;
     b.gtk = b.gtv = nullptr;
-    if (g.maxdeg > kWin && !team) {
+    if (g.maxdeg > kWin) {
         int cap = 1;
         while (cap < 2 * g.maxdeg) cap <<= 1;
         b.gcap = cap;
@@ -389,8 +407,10 @@ template <bool UNIT>
 __global__ void __launch_bounds__(kThreads, 4) cluster_team(SweepArgs a, ClusterArgs C, TeamArgs T) {
     __shared__ SweepQueue queue;
     __shared__ RowRed red;
+    __shared__ int tcount[kWarpsPerBlock];
     extern __shared__ __align__(16) unsigned char dyn[];
     Team team(T);
+    a.tcount = tcount;
     const TeamSpace S = team_space<false>(dyn, 0);
     const uint64_t ks_tie0 = stream_key(C.seed, TAG_CTIE, C.level, 0);
     for (long long v = team.rank(); v < a.n; v += team.size()) {
@@ -418,18 +438,16 @@ __global__ void __launch_bounds__(kThreads, 4) cluster_team(SweepArgs a, Cluster
             if (!(alive = team_sweep<CLUSTER, UNIT, false>(team, a, queue, S, red))) break;
             if (a.fuse_apply) continue;
             if (!a.admit_all) {
-                each_proposal(a, [&](int v) {
+                each_proposal(a, [&](int2& entry, int v, int b) {
                     if (v < 0) return;
-                    const int b = a.pt[v];
-                    if (b < 0) return;
-                    if (!((uint64_t)C.cw[b] + a.inc[b] < a.bound || a.minv[b] == v)) a.pt[v] = -2 - b;
+                    const uint32_t w = C.cw[b], in = a.inc[b];
+                    const int first = a.minv[b];
+                    if (!((uint64_t)w + in < a.bound || first == v)) entry.y = -2 - b;
                 });
                 if (!(alive = team.sync())) break;
             }
-            each_proposal(a, [&](int v) {
+            each_proposal(a, [&](int2&, int v, int t) {
                 if (v < 0) return;
-                const int t = a.pt[v];
-                if (t == -1) return;
                 const int b = t >= 0 ? t : -2 - t;
                 if (!a.admit_all) {
                     a.inc[b] = 0;
@@ -466,11 +484,14 @@ template <bool UNIT, bool DENSE>
 __global__ void __launch_bounds__(kThreads, 4) refine_team(SweepArgs a, RefineArgs R, TeamArgs T) {
     __shared__ SweepQueue queue;
     __shared__ RowRed red;
+    __shared__ int tcount[kWarpsPerBlock];
     extern __shared__ __align__(16) unsigned char dyn[];
     Team team(T);
+    a.tcount = tcount;
     const TeamSpace S = team_space<DENSE>(dyn, R.k);
     const int lane = threadIdx.x & 31;
     const LongRows rows = a.rows;
+    a.lw = S.lw;
     clear_admission(team, a, R.adm, R.k);
     list_rows<DENSE>(team, a.xadj, a.n, rows);
     for (long long v = team.rank(); v < a.n; v += team.size()) R.stamp[v] = 0;
@@ -500,7 +521,9 @@ __global__ void __launch_bounds__(kThreads, 4) refine_team(SweepArgs a, RefineAr
         for (uint32_t s = 0; s < a.S; ++s, p ^= 1) {
             a.s = s;
             use_set(a, R.counters, p);
-            use_admission(team, a, R.adm, R.k, p, R.bw);
+            use_admission(team, a, R.adm, R.k, p);
+            for (int b = threadIdx.x; b < R.k; b += kThreads) S.lw[b] = R.bw[b];
+            __syncthreads();
             if (s == 0) {  // what round r - 1 swept from
                 if (flags_out)
                     for (long long i = team.rank(); i < (a.n + 3LL) / 4; i += team.size())
@@ -510,8 +533,8 @@ __global__ void __launch_bounds__(kThreads, 4) refine_team(SweepArgs a, RefineAr
             if (!(alive = team_sweep<REFINE, UNIT, DENSE>(team, a, queue, S, red))) break;
             if (s == 0 && team.leader()) R.moved[out] = 0;  // every block has read it by now
             unsigned mv = 0;
-            each_proposal(a, [&](int v) {
-                const bool moved = v >= 0 && class_settle(a, R.adm.snap, 1, R.part, R.bw, v);
+            each_proposal(a, [&](int2&, int v, int t) {
+                const bool moved = v >= 0 && class_settle(a, S.lw, 1, R.part, R.bw, v, t);
                 int e0 = 0, e1 = 0;
                 if (moved) {
                     ++mv;
@@ -550,8 +573,10 @@ __global__ void __launch_bounds__(kThreads, 4) balance_team(SweepArgs a, Balance
     __shared__ SweepQueue queue;
     __shared__ RowRed red;
     __shared__ WeighSmem ws;
+    __shared__ int tcount[kWarpsPerBlock];
     extern __shared__ __align__(16) unsigned char dyn[];
     Team team(T);
+    a.tcount = tcount;
     const TeamSpace S = team_space<DENSE>(dyn, B.k);
     balance_clear(team, a, B);
     list_rows<DENSE>(team, a.xadj, a.n, a.rows);
@@ -583,9 +608,8 @@ bool lp_cluster_team(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, in
     const size_t smem = team_smem(0, false);
     const TeamRoom room = team_room(ctx, (const void*)kernel, smem);
     const int blocks = team_blocks(room, team_want(g));
-    const SweepBuffers b = make_buffers(ctx, g, blocks);
-    SweepArgs a = base_args(g, b);
     ClusterArgs C{};
+    SweepArgs a = team_args(ctx, g, blocks, &C.counters);
     C.rounds = kn.lpc_rounds;
     C.subrounds = kn.lpc_subrounds;
     C.seed = kn.seed;
@@ -593,7 +617,6 @@ bool lp_cluster_team(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, in
     C.label = label;
     C.cw = ctx.scratch.alloc<uint32_t>(n);
     C.tie = ctx.scratch.alloc<uint32_t>(n);
-    C.counters = b.counters;
     a.lab = label;
     a.lw = C.cw;
     a.bound = kn.cluster_bound;
@@ -627,9 +650,8 @@ bool lp_refine_team(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, uin
     const size_t smem = team_smem(kn.k, dense);
     const TeamRoom room = team_room(ctx, (const void*)kernel, smem);
     const int blocks = team_blocks(room, team_want(g));
-    const SweepBuffers b = make_buffers(ctx, g, blocks);
-    SweepArgs a = base_args(g, b);
     RefineArgs R{};
+    SweepArgs a = team_args(ctx, g, blocks, &R.counters);
     R.k = kn.k;
     R.rounds = kn.ref_rounds;
     R.subrounds = kn.ref_subrounds;
@@ -645,9 +667,7 @@ bool lp_refine_team(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, uin
     R.list[1] = ctx.scratch.alloc<int>(n);
     R.lcount = ctx.scratch.alloc<unsigned>(2);
     R.moved = ctx.scratch.alloc<unsigned>(2);
-    R.counters = b.counters;
     a.lab = part;
-    a.lw = bw;
     a.bound = bound;
     a.S = (uint32_t)kn.ref_subrounds;
     a.P = kn.ref_classes;
@@ -680,7 +700,7 @@ void lp_cluster(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, int* la
     uint32_t* cw = ctx.scratch.alloc<uint32_t>(n);
     uint32_t* inc = ctx.scratch.alloc<uint32_t>(n);
     int* minv = ctx.scratch.alloc<int>(n);
-    SweepBuffers b = make_buffers(ctx, g, 0);
+    SweepBuffers b = make_buffers(ctx, g);
     init_labels(ctx, g, label, cw);
     fill_u32(inc, g.n, 0u, st);
     fill_i32(minv, g.n, INT_MAX, st);
@@ -764,7 +784,7 @@ void lp_refine(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, uint32_t
     // rows cost less than the extra launches)
     int* hubs = g.maxdeg > 128 ? ctx.scratch.alloc<int>((size_t)g.n) : nullptr;
     unsigned* nhubs = hubs ? ctx.scratch.alloc<unsigned>(1) : nullptr;
-    SweepBuffers b = make_buffers(ctx, g, 0);
+    SweepBuffers b = make_buffers(ctx, g);
     fill_u32(H, (long long)k * P, 0u, st);
     fill_i32(minvP, (long long)k * P, INT_MAX, st);
     fill_u32(stamp, g.n, 0u, st);
@@ -873,12 +893,12 @@ bool balance(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, uint32_t b
         const size_t smem = team_smem(k, dense), mk2 = ctx.scratch.mark();
         const TeamRoom room = team_room(ctx, (const void*)kernel, smem);
         const int blocks = team_blocks(room, team_want(g));
-        const SweepBuffers b = make_buffers(ctx, g, blocks);
-        SweepArgs a = base_args(g, b);
+        unsigned* counters;
+        SweepArgs a = team_args(ctx, g, blocks, &counters);
         a.bound = bound;
         a.P = P;
         a.rows = alloc_rows(ctx, g.n);
-        const BalanceArgs B{k, kn.bal_iters, kn.seed, level, part, bw, HS, alloc_admission(ctx, k, P), b.counters};
+        const BalanceArgs B{k, kn.bal_iters, kn.seed, level, part, bw, HS, alloc_admission(ctx, k, P), counters};
         bool done;
         {
             PhaseScope ps(ctx, "balance", 0);
@@ -893,7 +913,7 @@ bool balance(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, uint32_t b
         }
     }
     int* thr = ctx.scratch.alloc<int>((size_t)k);
-    SweepBuffers b = make_buffers(ctx, g, 0);
+    SweepBuffers b = make_buffers(ctx, g);
     fill_u32(H, (long long)k * P, 0u, st);
     fill_i32(minvP, (long long)k * P, INT_MAX, st);
     SweepArgs a = base_args(g, b);

@@ -24,15 +24,14 @@ constexpr int kBalClasses = 256;
 enum Mode { CLUSTER = 0, REFINE = 1, BALANCE = 2 };
 
 // A list filled by many warps without contention: warp w appends to stripe
-// w % ns through that stripe's counter.  Every stripe has a capacity `cap`
-// computed on the host from the number of warps of the producing kernels and
-// the work each warp can be given.
+// w % kStripes through that stripe's counter.  Every stripe has a capacity
+// `cap` computed on the host from the number of warps of the producing
+// kernels and the work each warp can be given.
 constexpr int kStripes = 128;
 struct SList {
-    int* data;        // ns * cap entries
-    unsigned* counts; // ns counters
+    int* data;        // kStripes * cap entries
+    unsigned* counts; // kStripes counters
     long long cap;
-    int ns;           // stripes, a power of two (kStripes, or fewer for a small team)
 };
 
 // Rows of more than kDeferRow entries, listed once per level: a warp's from
@@ -67,7 +66,13 @@ struct SweepArgs {
     int* minvP;                         // smallest proposer per (target, class)
     int* heavy; unsigned* hcount;       // deferred high-degree vertices
     unsigned* hugecount;                // a team: those listed from heavy's end
-    LongRows rows;                      // a team: the level's long rows, when they are listed
+    // a team: the level's long rows, when they are listed; the proposals, a
+    // list of (vertex, target) of capacity tcap per warp with its length in
+    // shared memory
+    LongRows rows;
+    int2* tlist;
+    int tcap;
+    int* tcount;
     SList plist;                        // vertices that proposed a move this sub-round
     int* hplist; unsigned* hpcount;     // proposals of high-degree vertices
     int singletons;                     // every label is its own vertex id and rows have
@@ -126,14 +131,15 @@ __device__ __forceinline__ int loss_bucket(long long loss) {
     return bits < 31 ? bits : 31;
 }
 
-// Final decision for vertex v (executed by one lane).
-// Returns true when v proposes a move (pt[v] = target; the caller lists v).
+// Final decision for vertex v (executed by one lane).  Returns true when v
+// proposes a move: to prop.x, with class prop.y (not CLUSTER); the caller
+// records it.
 template <int MODE>
 __device__ __forceinline__ bool decide_emit(const SweepArgs& a, int v, uint32_t own, uint32_t cv, uint32_t conn_own,
-                            uint64_t key, uint32_t id) {
+                                            uint64_t key, uint32_t id, int2& prop) {
     if (MODE == CLUSTER) {
         if (id == kEmpty || (uint32_t)(key >> 32) <= conn_own) return false;
-        a.pt[v] = (int)id;
+        prop = make_int2((int)id, 0);
         if (!a.admit_all) {
             atomicAdd(&a.inc[id], cv);
             atomicMin(&a.minv[id], v);
@@ -142,8 +148,7 @@ __device__ __forceinline__ bool decide_emit(const SweepArgs& a, int v, uint32_t 
         uint32_t base = a.lw[own] <= a.bound ? conn_own : 0u;
         if (id == kEmpty || (uint32_t)(key >> 32) <= base) return false;
         int cls = (int)hash_range(hash32(a.ks_prio, (uint32_t)v), (uint32_t)a.P);
-        a.pt[v] = (int)id;
-        a.pc[v] = cls;
+        prop = make_int2((int)id, cls);
         size_t h = (size_t)id * a.P + cls;
         atomicAdd(&a.H[h], cv);
         atomicMin(&a.minvP[h], v);
@@ -157,11 +162,44 @@ __device__ __forceinline__ bool decide_emit(const SweepArgs& a, int v, uint32_t 
         }
         long long loss = (long long)conn_own - (long long)tc;
         int cls = loss_bucket(loss) * 8 + (int)hash_range(hash32(a.ks_sub, (uint32_t)v), 8u);
-        a.pt[v] = (int)t;
-        a.pc[v] = cls;
+        prop = make_int2((int)t, cls);
         atomicAdd(&a.HS[(size_t)own * kBalClasses + cls], cv);
     }
     return true;
+}
+
+// Records a proposal by vertex (the multi-launch form; the caller lists v).
+template <int MODE>
+__device__ __forceinline__ void record(const SweepArgs& a, int v, int2 prop) {
+    a.pt[v] = prop.x;
+    if (MODE != CLUSTER) a.pc[v] = prop.y;
+}
+
+// A proposal's second word in a team's list: the target, and in the balance
+// repair its release class above it (at most 2^16 blocks).
+template <int MODE>
+__device__ __forceinline__ int packed(int2 prop) {
+    return MODE == BALANCE ? (prop.y << 16) | prop.x : prop.x;
+}
+
+// Appends to the calling warp's own list: no atomics, no other reader before
+// the sub-round's barrier.  All lanes call it.
+__device__ __forceinline__ void append_own(const SweepArgs& a, bool pred, int v, int y) {
+    const unsigned m = __ballot_sync(0xffffffffu, pred);
+    if (!m) return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int base = a.tcount[wid];
+    int2* list = a.tlist + ((long long)blockIdx.x * (blockDim.x >> 5) + wid) * a.tcap;
+    __syncwarp();
+    if (pred) list[base + __popc(m & lanemask_lt())] = make_int2(v, y);
+    if (lane == 0) a.tcount[wid] = base + __popc(m);
+    __syncwarp();
+}
+
+// ... by one lane of the warp (or thread 0 of the block) for its row.
+__device__ __forceinline__ void append_one(const SweepArgs& a, int v, int y) {
+    const int wid = threadIdx.x >> 5;
+    a.tlist[((long long)blockIdx.x * (blockDim.x >> 5) + wid) * a.tcap + a.tcount[wid]++] = make_int2(v, y);
 }
 
 __device__ __forceinline__ int warp_global_id() {
@@ -182,7 +220,7 @@ __device__ __forceinline__ void append_aggregated(bool pred, int v, int* list, u
 
 // warp-aggregated append to this warp's stripe of a striped list
 __device__ __forceinline__ void append_striped(bool pred, int v, const SList& L) {
-    const int stripe = warp_global_id() & (L.ns - 1);
+    const int stripe = warp_global_id() % kStripes;
     append_aggregated(pred, v, L.data + (long long)stripe * L.cap, L.counts + stripe);
 }
 
@@ -370,7 +408,10 @@ __device__ __forceinline__ void chunk_process(const SweepArgs& a, WarpTable& T, 
         __syncwarp();
         if (lane == 0) T.nused = 0;
         bool prop = false;
-        if (wmember) prop = decide_emit<MODE>(a, v, T.own[lane], T.cv[lane], T.cown[lane], T.bkey[lane], T.bid[lane]);
+        int2 pr;
+        if (wmember)
+            prop = decide_emit<MODE>(a, v, T.own[lane], T.cv[lane], T.cown[lane], T.bkey[lane], T.bid[lane], pr);
+        if (prop) record<MODE>(a, v, pr);
         append_striped(prop, v, a.plist);
         __syncwarp();
         // next window starts at the first light lane at or after wend
@@ -407,7 +448,8 @@ __device__ __forceinline__ int nth_set_bit(unsigned mask, int r) {
 // 0: decided (stays), 3: decided (proposes a move), 1: too many distinct
 // labels for NS slots, 2: degree above ROW
 template <int MODE, int NS, bool UNIT, bool STASH, int ROW>
-__device__ __forceinline__ int lane_vertex(const SweepArgs& a, int v, uint32_t* st, unsigned& wv, unsigned& we) {
+__device__ __forceinline__ int lane_vertex(const SweepArgs& a, int v, uint32_t* st, unsigned& wv, unsigned& we,
+                                           int2& prop) {
     const int beg = a.xadj[v], end = a.xadj[v + 1];
     if (end - beg > ROW) return 2;
     // clustering round 0 (singletons): every label is its own vertex id
@@ -445,7 +487,7 @@ __device__ __forceinline__ int lane_vertex(const SweepArgs& a, int v, uint32_t* 
             return 0;
         }
         const uint64_t key = id == kEmpty ? 0ull : (1ull << 32);
-        return decide_emit<MODE>(a, v, own, cv, cown, key, id) ? 3 : 0;
+        return decide_emit<MODE>(a, v, own, cv, cown, key, id, prop) ? 3 : 0;
     }
     if (MODE == CLUSTER && a.singletons) {
         // label[u] == u and no target repeats: the connection to cluster u is
@@ -480,7 +522,7 @@ __device__ __forceinline__ int lane_vertex(const SweepArgs& a, int v, uint32_t* 
         }
         wv += 1;
         we += (unsigned)(end - beg);
-        return decide_emit<MODE>(a, v, own, cv, cown, key, id) ? 3 : 0;
+        return decide_emit<MODE>(a, v, own, cv, cown, key, id, prop) ? 3 : 0;
     }
     // NS register slots (label, connection); a new label enters at slot 0 and
     // shifts the others up, so slot NS-1 filled means the slots are full
@@ -588,7 +630,7 @@ __device__ __forceinline__ int lane_vertex(const SweepArgs& a, int v, uint32_t* 
     }
     // decide_emit reads the connection (upper half) of the key only
     const uint64_t key = id == kEmpty ? 0ull : ((uint64_t)bc << 32);
-    return decide_emit<MODE>(a, v, own, cv, cown, key, id) ? 3 : 0;
+    return decide_emit<MODE>(a, v, own, cv, cown, key, id, prop) ? 3 : 0;
 }
 
 // A block's shared memory in a sweep: per warp a queue of members still to
@@ -628,6 +670,8 @@ __device__ __forceinline__ void lane_sweep(const SweepArgs& a, SweepQueue& queue
     WarpTable* T = DEFER ? nullptr : tabs + (threadIdx.x >> 5);
     if (!DEFER && lane == 0) T->nused = 0;
     __syncwarp();
+    if (DEFER && lane == 0) a.tcount[threadIdx.x >> 5] = 0;
+    __syncwarp();
     int qn = 0, oqn = 0;  // warp-uniform
     // per-lane work counts (32 bits: a lane never sees more than m < 2^31 entries)
     unsigned wv = 0, we = 0, wo = 0;
@@ -648,14 +692,16 @@ __device__ __forceinline__ void lane_sweep(const SweepArgs& a, SweepQueue& queue
     };
     auto pass = [&](int v) {
         int status = 0;
+        int2 pr = make_int2(-1, 0);
         if (v >= 0)
             status = lane_vertex<MODE, kSlots, UNIT, STASH, DEFER ? kDeferRow : kWin>(
-                a, v, STASH ? T->stash + lane : nullptr, wv, we);
+                a, v, STASH ? T->stash + lane : nullptr, wv, we, pr);
         if constexpr (DEFER) {
             defer_row<HUGE>(a, status == 1 || (status == 2 && !a.rows.list), v);
-            append_striped(status == 3, v, a.plist);
+            append_own(a, status == 3, v, packed<MODE>(pr));
             return;
         }
+        if (status == 3) record<MODE>(a, v, pr);
         const unsigned om = __ballot_sync(0xffffffffu, status == 1);
         if (status == 1) oq[oqn + __popc(om & lanemask_lt())] = v;
         oqn += __popc(om);
@@ -740,7 +786,7 @@ struct HeavyRed {
 // two >= 2 * degree) of a table that is empty between uses, so that
 // inserting, scanning and clearing cost O(degree).  Entries of the own label
 // are summed in registers.  Four entries a thread are in flight.
-template <int MODE, int BT>
+template <int MODE, int BT, bool TEAM>
 __device__ __forceinline__ void heavy_vertex(const SweepArgs& a, int v, uint32_t* tk, uint32_t* tv, int cap,
                                              HeavyRed<BT>& red) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -790,7 +836,15 @@ __device__ __forceinline__ void heavy_vertex(const SweepArgs& a, int v, uint32_t
         }
         atomicAdd(&a.work[0], 1ull);
         atomicAdd(&a.work[1], (unsigned long long)(end - beg));
-        if (decide_emit<MODE>(a, v, own, cv, co, key, id)) a.hplist[atomicAdd(a.hpcount, 1u)] = v;
+        int2 pr;
+        if (decide_emit<MODE>(a, v, own, cv, co, key, id, pr)) {
+            if (TEAM) {
+                append_one(a, v, packed<MODE>(pr));
+            } else {
+                record<MODE>(a, v, pr);
+                a.hplist[atomicAdd(a.hpcount, 1u)] = v;
+            }
+        }
     }
     __syncthreads();
 }
@@ -824,7 +878,7 @@ __device__ __forceinline__ void heavy_sweep(const SweepArgs& a, uint32_t* gtk, u
         const int v = a.heavy[i];
         const int cap = heavy_cap(a.xadj[v + 1] - a.xadj[v], gcap);
         if ((which == 1 && cap > kSmemTab) || (which == 2 && cap <= kSmemTab)) continue;
-        heavy_vertex<MODE, BT>(a, v, cap <= stab ? htab : gk, cap <= stab ? htab + stab : gv, cap, red);
+        heavy_vertex<MODE, BT, false>(a, v, cap <= stab ? htab : gk, cap <= stab ? htab + stab : gv, cap, red);
     }
 }
 
@@ -875,7 +929,8 @@ __device__ __forceinline__ void hash_vertex(const SweepArgs& a, int v, uint32_t*
     if (lane == 0) {
         atomicAdd(&a.work[0], 1ull);
         atomicAdd(&a.work[1], (unsigned long long)(end - beg));
-        if (decide_emit<MODE>(a, v, own, cv, co, key, id)) a.hplist[atomicAdd(a.hpcount, 1u)] = v;
+        int2 pr;
+        if (decide_emit<MODE>(a, v, own, cv, co, key, id, pr)) append_one(a, v, packed<MODE>(pr));
     }
     __syncwarp();
 }
@@ -893,14 +948,14 @@ __device__ __forceinline__ bool admit(const uint32_t* H, const int* minvP, int P
     const uint32_t* h = H + (size_t)b * P;
     unsigned long long cum = 0;
     int t = 0;
-    // four classes are loaded together (one after the other, the loads' round
+    // eight classes are loaded together (one after the other, the loads' round
     // trips are most of an admission pass)
     for (bool fits = true; fits && t < P;) {
-        uint32_t x[4];
+        uint32_t x[8];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) x[q] = t + q < P ? h[t + q] : 0u;
+        for (int q = 0; q < 8; ++q) x[q] = t + q < P ? h[t + q] : 0u;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < 8; ++q) {
             fits = fits && t < P && (long long)(cum + x[q]) <= cap;
             if (fits) { cum += x[q]; ++t; }
         }
@@ -954,35 +1009,29 @@ __device__ __forceinline__ void mark_row(const NextActive& na, const int* adjncy
 // between two sets; a sub-round clears the set of the next one, which every
 // block stopped reading at the barrier that ended the sub-round before.
 
-constexpr int kTeamSet = kStripes + 8;  // counters of one set: stripes, heavy, heavy proposals, huge
+constexpr int kTeamSet = 2;             // counters of one set: deferred rows of a warp, of a block
 constexpr int kTeamMaxBlocks = 8192;    // blocks of the partition (their thresholds sit in shared memory)
 constexpr int kDenseBlocks = 1024;      // ... up to which every warp has a counter per block in shared memory
 
 __device__ __forceinline__ void use_set(SweepArgs& a, unsigned* counters, int p) {
-    a.plist.counts = counters + p * kTeamSet;
-    a.hcount = counters + p * kTeamSet + kStripes;
-    a.hpcount = counters + p * kTeamSet + kStripes + 1;
-    a.hugecount = counters + p * kTeamSet + kStripes + 2;
-    unsigned* other = counters + (p ^ 1) * kTeamSet;
-    if (blockIdx.x == 0)
-        for (int i = threadIdx.x; i < kTeamSet; i += blockDim.x) other[i] = 0;
+    a.hcount = counters + p * kTeamSet;
+    a.hugecount = counters + p * kTeamSet + 1;
+    if (blockIdx.x == 0 && threadIdx.x < kTeamSet) counters[(p ^ 1) * kTeamSet + threadIdx.x] = 0;
 }
 
-// f(v) for every proposal of the sub-round, warp by warp: all lanes of a warp
-// call f together, v = -1 for the lanes beyond the list's end.
+// f(entry, v, y) for the proposals of the calling warp, 32 at a time: all
+// lanes call f together, v = -1 for the lanes beyond the list's end.  (A warp
+// handles the proposals that it made itself, so a list needs no counter in
+// global memory and no barrier of its own.)
 template <class F>
 __device__ __forceinline__ void each_proposal(const SweepArgs& a, F f) {
-    const unsigned lane = threadIdx.x & 31;
-    const unsigned W = gridDim.x * kWarpsPerBlock, w = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-    const unsigned ns = (unsigned)a.plist.ns;
-    for (unsigned s = w & (ns - 1); s < ns; s += W) {
-        const unsigned n = a.plist.counts[s];
-        const int* list = a.plist.data + (long long)s * a.plist.cap;
-        const unsigned share = W > ns ? (W - s + ns - 1) / ns : 1u;  // warps on this stripe
-        for (unsigned i = (W > ns ? w / ns : 0u) * 32; i < n; i += share * 32) f(i + lane < n ? list[i + lane] : -1);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int2* list = a.tlist + ((long long)blockIdx.x * (blockDim.x >> 5) + wid) * a.tcap;
+    const int n = a.tcount[wid];
+    for (int i = lane; i - lane < n; i += 32) {
+        const int2 e = i < n ? list[i] : make_int2(-1, -1);
+        f(list[i < n ? i : 0], e.x, e.y);
     }
-    const unsigned nh = *a.hpcount;
-    for (unsigned i = w * 32; i < nh; i += W * 32) f(i + lane < nh ? a.hplist[i + lane] : -1);
 }
 
 // A block's shared memory in a team, for the rows that a warp or the block
@@ -995,7 +1044,8 @@ constexpr int kHugeDense = 1024;  // longest row of a warp with the counters
 struct TeamSpace {
     uint32_t* tab;  // counters, or the keys
     uint32_t* val;  // DENSE: the bits; else the values
-    int* thr;
+    int* thr;       // k release thresholds
+    uint32_t* lw;   // k block weights at the sub-round's start
     int k;
     __device__ int words() const { return (k + 31) / 32; }
 };
@@ -1009,8 +1059,8 @@ struct RowRed {  // of a row counted by a whole block
 static_assert(kWarpsPerBlock * kHashTab == kSmemTab, "the warps' tables make up the block's");
 
 inline size_t team_smem(int k, bool dense) {
-    if (!dense) return sizeof(uint32_t) * (2 * (size_t)kSmemTab + k);
-    return sizeof(uint32_t) * ((size_t)kWarpsPerBlock * (k + (k + 31) / 32) + k);
+    if (!dense) return sizeof(uint32_t) * (2 * (size_t)kSmemTab + 2 * (size_t)k);
+    return sizeof(uint32_t) * ((size_t)kWarpsPerBlock * (k + (k + 31) / 32) + 2 * (size_t)k);
 }
 
 template <bool DENSE>
@@ -1022,6 +1072,7 @@ __device__ __forceinline__ TeamSpace team_space(unsigned char* dyn, int k) {
     const int vals = DENSE ? kWarpsPerBlock * S.words() : kSmemTab;
     S.val = S.tab + keys;
     S.thr = reinterpret_cast<int*>(S.val + vals);
+    S.lw = reinterpret_cast<uint32_t*>(S.thr + k);
     for (int i = threadIdx.x; i < keys; i += kThreads) S.tab[i] = DENSE ? 0u : kEmpty;
     for (int i = threadIdx.x; i < vals; i += kThreads) S.val[i] = 0;
     __syncthreads();
@@ -1086,7 +1137,8 @@ __device__ __forceinline__ void dense_vertex(const SweepArgs& a, int v, int k, u
     if (t == 0) {
         atomicAdd(&a.work[0], 1ull);
         atomicAdd(&a.work[1], (unsigned long long)(end - beg));
-        if (decide_emit<MODE>(a, v, own, cv, cown, key, id)) a.hplist[atomicAdd(a.hpcount, 1u)] = v;
+        int2 pr;
+        if (decide_emit<MODE>(a, v, own, cv, cown, key, id, pr)) append_one(a, v, packed<MODE>(pr));
     }
     if (BLOCK) __syncthreads();
     else __syncwarp();
@@ -1119,7 +1171,7 @@ __device__ __forceinline__ void listed_rows(const SweepArgs& a, const int* list,
             dense_vertex<MODE, UNIT, true>(a, v, S.k, S.tab, S.val, red);
         } else {
             __shared__ HeavyRed<kThreads> hred;
-            heavy_vertex<MODE, kThreads>(a, v, S.tab, S.val, heavy_cap(a.xadj[v + 1] - a.xadj[v], kSmemTab), hred);
+            heavy_vertex<MODE, kThreads, true>(a, v, S.tab, S.val, heavy_cap(a.xadj[v + 1] - a.xadj[v], kSmemTab), hred);
         }
     }
 }
@@ -1151,17 +1203,18 @@ __device__ __forceinline__ void list_rows(Team& team, const int* xadj, int n, co
     }
 }
 
-// class_decide's and class_apply's rules for one proposal in one step: the
-// decision reads the block weights as they were at the sweep (snap) and the
-// admission data, which no one changes meanwhile.  True when v moved.
-__device__ __forceinline__ bool class_settle(const SweepArgs& a, const uint32_t* snap, int strict, int* part,
-                                             uint32_t* bw, int v) {
-    const int b = a.pt[v], c = a.pc[v];
-    if (b < 0 || c < 0) return false;  // (no class: dropped before admission, balance)
+// class_decide's and class_apply's rules for one proposal (v to block b) in one
+// step: the decision reads the block weights as they were at the sweep (lw)
+// and the admission data, which no one changes meanwhile.  The class is the
+// proposal's hashed priority.  True when v moved.
+__device__ __forceinline__ bool class_settle(const SweepArgs& a, const uint32_t* lw, int strict, int* part,
+                                             uint32_t* bw, int v, int b) {
     const uint32_t cv = (uint32_t)a.vwgt[v];
-    const long long cap = (long long)a.bound - (strict ? 1 : 0) - (long long)snap[b];
+    const int own = part[v];
+    const int c = (int)hash_range(hash32(a.ks_prio, (uint32_t)v), (uint32_t)a.P);
+    const long long cap = (long long)a.bound - (strict ? 1 : 0) - (long long)lw[b];
     if (!admit(a.H, a.minvP, a.P, b, c, v, cv, cap)) return false;
-    atomicSub(&bw[part[v]], cv);
+    atomicSub(&bw[own], cv);
     atomicAdd(&bw[b], cv);
     part[v] = b;
     return true;
@@ -1173,11 +1226,9 @@ __device__ __forceinline__ bool class_settle(const SweepArgs& a, const uint32_t*
 struct Admission {
     uint32_t* H;     // 2 k P
     int* minvP;      // 2 k P
-    uint32_t* snap;  // k: the block weights at the sweep
 };
 
-__device__ __forceinline__ void use_admission(Team& team, SweepArgs& a, const Admission& M, int k, int p,
-                                              const uint32_t* bw) {
+__device__ __forceinline__ void use_admission(Team& team, SweepArgs& a, const Admission& M, int k, int p) {
     const size_t kP = (size_t)k * a.P;
     a.H = M.H + (p ? kP : 0);
     a.minvP = M.minvP + (p ? kP : 0);
@@ -1187,8 +1238,6 @@ __device__ __forceinline__ void use_admission(Team& team, SweepArgs& a, const Ad
         h[i] = 0;
         mv[i] = INT_MAX;
     }
-    if (blockIdx.x == 0)
-        for (int b = threadIdx.x; b < k; b += kThreads) M.snap[b] = bw[b];
 }
 
 __device__ __forceinline__ void clear_admission(Team& team, const SweepArgs& a, const Admission& M, int k) {
@@ -1210,11 +1259,14 @@ struct WeighSmem {
     int lightest;  // for SweepArgs::lightest
 };
 
-__device__ __forceinline__ Weighed weigh(const uint32_t* bw, int k, uint32_t bound, WeighSmem& ws) {
+// (keep: a copy of the weights, shared memory)
+__device__ __forceinline__ Weighed weigh(const uint32_t* bw, int k, uint32_t bound, WeighSmem& ws,
+                                         uint32_t* keep = nullptr) {
     __syncthreads();  // the last call's readers
     unsigned long long ov = 0, best = ~0ull;
     for (int b = threadIdx.x; b < k; b += blockDim.x) {
         const uint32_t x = bw[b];
+        if (keep) keep[b] = x;
         best = min(best, ((unsigned long long)x << 32) | (unsigned)b);
         if (x > bound) ov += x - bound;
     }
@@ -1261,69 +1313,77 @@ template <bool UNIT, bool DENSE>
 __device__ __forceinline__ bool balance_steps(Team& team, SweepArgs a, const BalanceArgs& B, int& p, SweepQueue& queue,
                                               const TeamSpace& S, RowRed& red, WeighSmem& ws) {
     a.lab = B.part;
-    a.lw = B.bw;
+    a.lw = S.lw;
     a.HS = B.HS;
     a.lightest = &ws.lightest;
     for (int it = 0; it < B.iters; ++it) {
-        if (!weigh(B.bw, B.k, a.bound, ws).over) return true;
+        if (!weigh(B.bw, B.k, a.bound, ws, S.lw).over) return true;
         a.ks_tie = stream_key(B.seed, TAG_BTIE, B.level, it);
         a.ks_sub = stream_key(B.seed, TAG_BCLS, B.level, it);  // release class stream
-        const uint64_t ks_prio = stream_key(B.seed, TAG_BPRIO, B.level, it);
+        a.ks_prio = stream_key(B.seed, TAG_BPRIO, B.level, it);
         use_set(a, B.counters, p);
-        use_admission(team, a, B.adm, B.k, p, B.bw);
+        use_admission(team, a, B.adm, B.k, p);
         if (!team_sweep<BALANCE, UNIT, DENSE>(team, a, queue, S, red)) return false;
         // release thresholds, computed by every block for itself: the number
         // of classes before which less than the excess is released
         int* thr = S.thr;
-        const int lane = threadIdx.x & 31;
-        for (int b = threadIdx.x >> 5; b < B.k; b += kWarpsPerBlock) {
-            const uint32_t x = B.bw[b];
-            if (x <= a.bound) {
-                if (lane == 0) thr[b] = 0;
-                continue;
-            }
-            const unsigned long long excess = x - a.bound;
-            unsigned long long h[kBalClasses / 32], sum = 0;
+        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+        for (int base = 0, turn = 0; base < B.k; base += 32) {
+            // 32 blocks at a time, the overloaded ones dealt to the warps
+            const int bb = base + lane;
+            const bool over = bb < B.k && S.lw[bb] > a.bound;
+            if (wid == 0 && bb < B.k && !over) thr[bb] = 0;
+            unsigned m = __ballot_sync(0xffffffffu, over);
+            for (; m; m &= m - 1, ++turn) {
+                if (turn % kWarpsPerBlock != wid) continue;
+                const int b = base + __ffs(m) - 1;
+                const unsigned long long excess = S.lw[b] - a.bound;
+                constexpr int Q = kBalClasses / 32;
+                uint32_t h[Q];
+                const uint4* hs = reinterpret_cast<const uint4*>(B.HS + (size_t)b * kBalClasses + lane * Q);
+                static_assert(Q == 8, "two 16-byte loads");
+                const uint4 h0 = hs[0], h1 = hs[1];
+                h[0] = h0.x; h[1] = h0.y; h[2] = h0.z; h[3] = h0.w;
+                h[4] = h1.x; h[5] = h1.y; h[6] = h1.z; h[7] = h1.w;
+                unsigned long long sum = 0;
 #pragma unroll
-            for (int q = 0; q < kBalClasses / 32; ++q) {
-                h[q] = B.HS[(size_t)b * kBalClasses + lane * (kBalClasses / 32) + q];
-                sum += h[q];
-            }
-            unsigned long long run = sum;
+                for (int q = 0; q < Q; ++q) sum += h[q];
+                unsigned long long run = sum;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned long long y = __shfl_up_sync(0xffffffffu, run, o);
-                if (lane >= o) run += y;
-            }
-            run -= sum;
-            unsigned t = 0;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned long long y = __shfl_up_sync(0xffffffffu, run, o);
+                    if (lane >= o) run += y;
+                }
+                run -= sum;
+                unsigned t = 0;
 #pragma unroll
-            for (int q = 0; q < kBalClasses / 32; ++q) {
-                t += run < excess ? 1u : 0u;
-                run += h[q];
+                for (int q = 0; q < Q; ++q) {
+                    t += run < excess ? 1u : 0u;
+                    run += h[q];
+                }
+                t = __reduce_add_sync(0xffffffffu, t);
+                if (lane == 0) thr[b] = (int)t;
             }
-            t = __reduce_add_sync(0xffffffffu, t);
-            if (lane == 0) thr[b] = (int)t;
         }
         __syncthreads();
         // released candidates get an admission class; others are dropped
-        each_proposal(a, [&](int v) {
+        each_proposal(a, [&](int2& entry, int v, int y) {
             if (v < 0) return;
-            const int t = a.pt[v];
-            if (t < 0) return;
-            if (a.pc[v] >= thr[B.part[v]]) {
-                a.pc[v] = -1;
+            const int t = y & 0xffff;
+            const uint32_t cv = (uint32_t)a.vwgt[v];
+            if ((y >> 16) >= thr[B.part[v]]) {
+                entry.y = -1;
                 return;
             }
-            const int c = (int)hash_range(hash32(ks_prio, (uint32_t)v), (uint32_t)a.P);
-            a.pc[v] = c;
+            entry.y = t;
+            const int c = (int)hash_range(hash32(a.ks_prio, (uint32_t)v), (uint32_t)a.P);
             const size_t h = (size_t)t * a.P + c;
-            atomicAdd(&a.H[h], (uint32_t)a.vwgt[v]);
+            atomicAdd(&a.H[h], cv);
             atomicMin(&a.minvP[h], v);
         });
         if (!team.sync()) return false;
-        each_proposal(a, [&](int v) {
-            if (v >= 0) class_settle(a, B.adm.snap, 0, B.part, B.bw, v);
+        each_proposal(a, [&](int2&, int v, int t) {
+            if (v >= 0 && t >= 0) class_settle(a, S.lw, 0, B.part, B.bw, v, t);
         });
         for (int b = blockIdx.x; b < B.k; b += gridDim.x)
             if (thr[b] > 0) B.HS[(size_t)b * kBalClasses + threadIdx.x] = 0;
@@ -1339,8 +1399,7 @@ __device__ __forceinline__ bool balance_steps(Team& team, SweepArgs a, const Bal
 struct SweepBuffers {
     int *pt, *pc;
     unsigned* counters;  // [0, kStripes) unused, [kStripes, 2 kStripes) proposals,
-                         // [2 kStripes] heavy, [+1] heavy proposals, [+2] moved;
-                         // a team's two sets
+                         // [2 kStripes] heavy, [+1] heavy proposals, [+2] moved
     int* heavy;
     int* hplist;
     SList plist;
@@ -1351,10 +1410,13 @@ struct SweepBuffers {
     int* err;
 };
 
-// Sweep buffers on the context's scratch, for the multi-launch sweeps
-// (team = 0) or for a team of that many blocks.
-SweepBuffers make_buffers(Ctx& ctx, const DevGraph& g, int team);
+// Sweep buffers on the context's scratch, for the multi-launch sweeps.
+SweepBuffers make_buffers(Ctx& ctx, const DevGraph& g);
 SweepArgs base_args(const DevGraph& g, const SweepBuffers& b);
+
+// The arguments of a team of that many blocks, its buffers on the context's
+// scratch, and the counters of its two sets (not yet zero).
+SweepArgs team_args(Ctx& ctx, const DevGraph& g, int blocks, unsigned** counters);
 Admission alloc_admission(Ctx& ctx, int k, int P);
 LongRows alloc_rows(Ctx& ctx, int n);
 
@@ -1369,9 +1431,9 @@ inline bool team_fits(const DevGraph& g, int k) {
     return team_dense(k) || (k <= kTeamMaxBlocks && g.maxdeg <= kSmemTab / 2);
 }
 // Blocks of a team that sweeps a level: a thread per vertex; on dense levels
-// (rows mostly a warp's) a thread per entry.
+// and those with hubs (rows mostly a warp's or a block's) a thread per entry.
 inline long long team_want(const DevGraph& g) {
-    const long long work = g.m > 16LL * g.n ? g.m : g.n;
+    const long long work = g.m > 16LL * g.n || g.maxdeg > kHugeDense ? g.m : g.n;
     return (work + kThreads - 1) / kThreads;
 }
 
