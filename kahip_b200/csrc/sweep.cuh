@@ -788,7 +788,7 @@ struct HeavyRed {
 // are summed in registers.  Four entries a thread are in flight.
 template <int MODE, int BT, bool TEAM>
 __device__ __forceinline__ void heavy_vertex(const SweepArgs& a, int v, uint32_t* tk, uint32_t* tv, int cap,
-                                             HeavyRed<BT>& red) {
+                                             HeavyRed<BT>& red, unsigned& wv, unsigned& we) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int beg = a.xadj[v], end = a.xadj[v + 1];
     const uint32_t own = (uint32_t)a.lab[v], cv = (uint32_t)a.vwgt[v];
@@ -834,8 +834,8 @@ __device__ __forceinline__ void heavy_vertex(const SweepArgs& a, int v, uint32_t
             better(key, id, red.key[j], red.id[j]);
             co += red.own[j];
         }
-        atomicAdd(&a.work[0], 1ull);
-        atomicAdd(&a.work[1], (unsigned long long)(end - beg));
+        wv += 1;
+        we += (unsigned)(end - beg);
         int2 pr;
         if (decide_emit<MODE>(a, v, own, cv, co, key, id, pr)) {
             if (TEAM) {
@@ -874,11 +874,16 @@ __device__ __forceinline__ void heavy_sweep(const SweepArgs& a, uint32_t* gtk, u
     uint32_t* gk = gtk ? gtk + (size_t)blockIdx.x * gcap : nullptr;
     uint32_t* gv = gtv ? gtv + (size_t)blockIdx.x * gcap : nullptr;
     const unsigned count = *a.hcount;
+    unsigned wv = 0, we = 0;  // thread 0's
     for (unsigned i = blockIdx.x; i < count; i += gridDim.x) {
         const int v = a.heavy[i];
         const int cap = heavy_cap(a.xadj[v + 1] - a.xadj[v], gcap);
         if ((which == 1 && cap > kSmemTab) || (which == 2 && cap <= kSmemTab)) continue;
-        heavy_vertex<MODE, BT, false>(a, v, cap <= stab ? htab : gk, cap <= stab ? htab + stab : gv, cap, red);
+        heavy_vertex<MODE, BT, false>(a, v, cap <= stab ? htab : gk, cap <= stab ? htab + stab : gv, cap, red, wv, we);
+    }
+    if (wv) {
+        atomicAdd(&a.work[0], (unsigned long long)wv);
+        atomicAdd(&a.work[1], (unsigned long long)we);
     }
 }
 
@@ -889,7 +894,8 @@ constexpr int kHashRow = 256;
 constexpr int kHashTab = 2 * kHashRow;
 
 template <int MODE, bool UNIT>
-__device__ __forceinline__ void hash_vertex(const SweepArgs& a, int v, uint32_t* tk, uint32_t* tv) {
+__device__ __forceinline__ void hash_vertex(const SweepArgs& a, int v, uint32_t* tk, uint32_t* tv, unsigned& wv,
+                                            unsigned& we) {
     const int lane = threadIdx.x & 31;
     const int beg = a.xadj[v], end = a.xadj[v + 1];
     const uint32_t own = (uint32_t)a.lab[v], cv = (uint32_t)a.vwgt[v];
@@ -927,8 +933,8 @@ __device__ __forceinline__ void hash_vertex(const SweepArgs& a, int v, uint32_t*
     group_argmax<32>(key, id, 0xffffffffu);
     co = __reduce_add_sync(0xffffffffu, co);
     if (lane == 0) {
-        atomicAdd(&a.work[0], 1ull);
-        atomicAdd(&a.work[1], (unsigned long long)(end - beg));
+        wv += 1;
+        we += (unsigned)(end - beg);
         int2 pr;
         if (decide_emit<MODE>(a, v, own, cv, co, key, id, pr)) append_one(a, v, packed<MODE>(pr));
     }
@@ -1086,7 +1092,7 @@ __device__ __forceinline__ TeamSpace team_space(unsigned char* dyn, int k) {
 // entry by entry.
 template <int MODE, bool UNIT, bool BLOCK>
 __device__ __forceinline__ void dense_vertex(const SweepArgs& a, int v, int k, uint32_t* cnt, uint32_t* mask,
-                                             RowRed& red) {
+                                             RowRed& red, unsigned& wv, unsigned& we) {
     static_assert(MODE != CLUSTER, "labels are blocks of the partition");
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int t = BLOCK ? (int)threadIdx.x : lane;
@@ -1135,8 +1141,8 @@ __device__ __forceinline__ void dense_vertex(const SweepArgs& a, int v, int k, u
             for (int w = 1; w < kWarpsPerBlock; ++w) better(key, id, red.key[w], red.id[w]);
     }
     if (t == 0) {
-        atomicAdd(&a.work[0], 1ull);
-        atomicAdd(&a.work[1], (unsigned long long)(end - beg));
+        wv += 1;
+        we += (unsigned)(end - beg);
         int2 pr;
         if (decide_emit<MODE>(a, v, own, cv, cown, key, id, pr)) append_one(a, v, packed<MODE>(pr));
     }
@@ -1155,24 +1161,31 @@ template <int MODE, bool UNIT, bool DENSE, bool MEMBERS>
 __device__ __forceinline__ void listed_rows(const SweepArgs& a, const int* list, unsigned n, unsigned nh,
                                             const TeamSpace& S, RowRed& red) {
     const unsigned W = gridDim.x * kWarpsPerBlock, wid = threadIdx.x >> 5;
+    unsigned wv = 0, we = 0;  // rows and entries of this lane
     for (unsigned i = blockIdx.x + wid * gridDim.x; i < n; i += W) {
         const int v = list[i];
         if (MEMBERS && !member<MODE>(a, v)) continue;
         if constexpr (DENSE)
-            dense_vertex<MODE, UNIT, false>(a, v, S.k, S.tab + (size_t)wid * S.k, S.val + wid * S.words(), red);
+            dense_vertex<MODE, UNIT, false>(a, v, S.k, S.tab + (size_t)wid * S.k, S.val + wid * S.words(), red,
+                                            wv, we);
         else
-            hash_vertex<MODE, UNIT>(a, v, S.tab + wid * kHashTab, S.val + wid * kHashTab);
+            hash_vertex<MODE, UNIT>(a, v, S.tab + wid * kHashTab, S.val + wid * kHashTab, wv, we);
     }
     if (nh) __syncthreads();  // the warps' tables become the block's
     for (unsigned i = blockIdx.x; i < nh; i += gridDim.x) {
         const int v = list[a.n - 1 - (int)i];
         if (MEMBERS && !member<MODE>(a, v)) continue;
         if constexpr (DENSE) {
-            dense_vertex<MODE, UNIT, true>(a, v, S.k, S.tab, S.val, red);
+            dense_vertex<MODE, UNIT, true>(a, v, S.k, S.tab, S.val, red, wv, we);
         } else {
             __shared__ HeavyRed<kThreads> hred;
-            heavy_vertex<MODE, kThreads, true>(a, v, S.tab, S.val, heavy_cap(a.xadj[v + 1] - a.xadj[v], kSmemTab), hred);
+            heavy_vertex<MODE, kThreads, true>(a, v, S.tab, S.val, heavy_cap(a.xadj[v + 1] - a.xadj[v], kSmemTab), hred,
+                                               wv, we);
         }
+    }
+    if (wv) {  // (an atomic per row on one address would cost more than the row)
+        atomicAdd(&a.work[0], (unsigned long long)wv);
+        atomicAdd(&a.work[1], (unsigned long long)we);
     }
 }
 
