@@ -26,6 +26,11 @@ __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__floa
 
 __device__ __forceinline__ float ld(const float* p) { return *p; }
 __device__ __forceinline__ float ld(const __nv_bfloat16* p) { return __bfloat162float(*p); }
+// two consecutive values, the first of even index
+__device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ float2 ld2(const __nv_bfloat16* p) {
+    return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+}
 __device__ __forceinline__ void st(float* p, float v) { *p = v; }
 __device__ __forceinline__ void st(__nv_bfloat16* p, float v) { *p = __float2bfloat16(v); }
 
@@ -79,11 +84,21 @@ __global__ void __launch_bounds__(kT) agg_fwd(int n, const int* xadj, const int*
     for (long long v = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5); v < n; v += (long long)gridDim.x * kWarps) {
         float a0 = 0.f, a1 = 0.f;
         const int beg = xadj[v], end = xadj[v + 1];
-        for (int e = beg; e < end; ++e) {
-            const int u = adjncy[e];
-            const float w = (float)adjwgt[e];
-            a0 += w * ld(h + (long long)u * rm::H + 2 * lane);
-            a1 += w * ld(h + (long long)u * rm::H + 2 * lane + 1);
+        for (int e = beg; e < end; e += 4) {  // four neighbours' rows in flight
+            float2 x[4];
+            float w[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const bool in = e + q < end;
+                w[q] = in ? (float)adjwgt[e + q] : 0.f;
+                x[q] = in ? ld2(h + (long long)adjncy[e + q] * rm::H + 2 * lane) : make_float2(0.f, 0.f);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (e + q < end) {
+                    a0 += w[q] * x[q].x;
+                    a1 += w[q] * x[q].y;
+                }
         }
         const float d = wdeg[v];
         const float inv = d > 0.f ? 1.0f / d : 0.f;
@@ -94,33 +109,75 @@ __global__ void __launch_bounds__(kT) agg_fwd(int n, const int* xadj, const int*
 
 // out[v] = act(W [in0[v] | in1[v]] + b) with in1 optional (K = 64 or 128),
 // N outputs (64 or 32); W row-major [N][K] in P at woff, bias at boff.
-template <class T, int K, int N, bool RELU>
-__global__ void __launch_bounds__(kT) dense_fwd(int n, const float* P, int woff, int boff, const T* in0,
-                                                const T* in1, T* out) {
-    __shared__ float wt[K * N];  // transposed: wt[k*N + j]
-    __shared__ float bs[N];
-    __shared__ float row[kWarps][K];
+// A block takes kTile nodes at a time: W transposed and the nodes' inputs in
+// shared memory, 4 nodes x N/16 outputs in each thread's registers (a node a
+// warp, each lane its outputs, read shared memory twice per product).  Every
+// output is summed in the order of k from the bias on.  32,771 nodes, K = 128,
+// N = 64: 122 -> 26 us.
+constexpr int kTile = 64;
+
+template <int K, int N>
+constexpr size_t dense_fwd_smem() {
+    return sizeof(float) * ((size_t)K * (N + 4) + N + (size_t)kTile * (K + 4));
+}
+
+template <int K, int N, bool RELU>
+__global__ void __launch_bounds__(kT) dense_fwd(int n, const float* P, int woff, int boff, const float* in0,
+                                                const float* in1, float* out) {
+    extern __shared__ __align__(16) float dsm[];
+    constexpr int XP = K + 4, WP = N + 4, TJ = N / 16;
+    float* wt = dsm;            // transposed: wt[k * WP + j]
+    float* bs = wt + K * WP;
+    float* xs = bs + N;         // [kTile][XP]
     for (int i = threadIdx.x; i < K * N; i += kT) {
         const int j = i / K, k = i % K;
-        wt[k * N + j] = bf16r(P[woff + i]);
+        wt[k * WP + j] = bf16r(P[woff + i]);
     }
     for (int i = threadIdx.x; i < N; i += kT) bs[i] = bf16r(P[boff + i]);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    for (long long v = (long long)blockIdx.x * kWarps + wp; v < n; v += (long long)gridDim.x * kWarps) {
-        for (int k = lane; k < K; k += 32)
-            row[wp][k] = k < rm::H ? ld(in0 + v * rm::H + k) : ld(in1 + v * rm::H + (k - rm::H));
-        __syncwarp();
-#pragma unroll
-        for (int q = 0; q < N / 32; ++q) {
-            const int j = lane + 32 * q;
-            float a = bs[j];
-#pragma unroll 8
-            for (int k = 0; k < K; ++k) a += wt[k * N + j] * row[wp][k];
-            if (RELU) a = fmaxf(a, 0.f);
-            st(out + v * N + j, bf16r(a));
+    const int t0 = 4 * (threadIdx.x / 16), j0 = TJ * (threadIdx.x % 16);
+    for (long long base = (long long)blockIdx.x * kTile; base < n; base += (long long)gridDim.x * kTile) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < kTile * K / 4; i += kT) {
+            const int t = i / (K / 4), k = 4 * (i % (K / 4));
+            const long long v = base + t;
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (v < n) x = *reinterpret_cast<const float4*>(k < rm::H ? in0 + v * rm::H + k : in1 + v * rm::H + (k - rm::H));
+            *reinterpret_cast<float4*>(xs + t * XP + k) = x;
         }
-        __syncwarp();
+        __syncthreads();
+        float acc[4][TJ];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < TJ; ++b) acc[a][b] = bs[j0 + b];
+#pragma unroll 2
+        for (int k = 0; k < K; k += 4) {
+            float4 x[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) x[a] = *reinterpret_cast<const float4*>(xs + (t0 + a) * XP + k);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                float w[TJ];
+#pragma unroll
+                for (int b = 0; b < TJ; ++b) w[b] = wt[(k + q) * WP + j0 + b];
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    const float xq = q == 0 ? x[a].x : q == 1 ? x[a].y : q == 2 ? x[a].z : x[a].w;
+#pragma unroll
+                    for (int b = 0; b < TJ; ++b) acc[a][b] += w[b] * xq;
+                }
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const long long v = base + t0 + a;
+            if (v >= n) break;
+#pragma unroll
+            for (int b = 0; b < TJ; ++b) {
+                const float y = RELU ? fmaxf(acc[a][b], 0.f) : acc[a][b];
+                out[v * N + j0 + b] = bf16r(y);
+            }
+        }
     }
 }
 
@@ -196,73 +253,99 @@ struct LossArgs {
 };
 
 // Head forward + backward.  dz[v] = 2 * sum over row v of dL/dt (the edge's
-// other direction contributes the same to z_v by symmetry).  Parameter
-// gradients (wo, Wf, bo) accumulate in block shared memory, then globally.
+// other direction contributes the same to z_v by symmetry).  A warp a row and
+// a lane per feature: 32 entries' features and labels are prepared a lane
+// each, then each entry is one coalesced row of z, a warp sum for its score,
+// and gradients that stay in the lane's registers until the block adds them
+// up.  (A lane per entry took 97 shared-memory float atomics an entry, all
+// lanes on one address: 1756 us at 320k entries; now 53.)
 __global__ void __launch_bounds__(kT) head_train(int n, const int* xadj, const int* adjncy, const int* adjwgt,
                                                  const int* vwgt, const float* P, const float* z, LossArgs L,
                                                  float* dz, float* G, float* loss) {
-    __shared__ float wf[rm::Z * 2], wo[rm::Z];
-    __shared__ float bo;
-    __shared__ float zv[kWarps][rm::Z];
+    static_assert(rm::Z == 32, "a lane per feature");
     __shared__ float gwf[rm::Z * 2], gwo[rm::Z];
     __shared__ float gbo, sloss;
-    for (int i = threadIdx.x; i < rm::Z * 2; i += kT) { wf[i] = bf16r(P[rm::WF + i]); gwf[i] = 0.f; }
-    for (int i = threadIdx.x; i < rm::Z; i += kT) { wo[i] = bf16r(P[rm::WO + i]); gwo[i] = 0.f; }
-    if (threadIdx.x == 0) { bo = bf16r(P[rm::BO]); gbo = 0.f; sloss = 0.f; }
-    __syncthreads();
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    float my_loss = 0.f;
+    if (wp == 0) {
+        gwf[2 * lane] = gwf[2 * lane + 1] = gwo[lane] = 0.f;
+        if (lane == 0) gbo = sloss = 0.f;
+    }
+    const float wf0 = bf16r(P[rm::WF + 2 * lane]), wf1 = bf16r(P[rm::WF + 2 * lane + 1]);
+    const float wo = bf16r(P[rm::WO + lane]), bo = bf16r(P[rm::BO]);
+    __syncthreads();
+    float my_loss = 0.f, my_bo = 0.f, my_wo = 0.f, my_f0 = 0.f, my_f1 = 0.f;
+    constexpr int Q = 4;  // entries in flight
     for (long long v = (long long)blockIdx.x * kWarps + wp; v < n; v += (long long)gridDim.x * kWarps) {
-        zv[wp][lane] = z[v * rm::Z + lane];
-        __syncwarp();
-        float dzl[rm::Z];
-#pragma unroll
-        for (int j = 0; j < rm::Z; ++j) dzl[j] = 0.f;
+        const float zv = z[v * rm::Z + lane];
+        float dzl = 0.f;
         const int beg = xadj[v], end = xadj[v + 1];
         const uint32_t cv = (uint32_t)vwgt[v];
-        for (int e = beg + lane; e < end; e += 32) {
-            const int u = adjncy[e];
-            float f0, f1;
-            edge_feat(adjwgt[e], (uint32_t)vwgt[u], cv, f0, f1);
-            float t[rm::Z];
-            float s = bo;
-#pragma unroll
-            for (int j = 0; j < rm::Z; ++j) {
-                const float a = z[(long long)u * rm::Z + j] + zv[wp][j];
-                t[j] = a + (wf[2 * j] * f0 + wf[2 * j + 1] * f1);
-                s += wo[j] * fmaxf(t[j], 0.f);
+        for (int e0 = beg; e0 < end; e0 += 32) {
+            int u = 0;
+            float f0 = 0.f, f1 = 0.f, om = 0.f;
+            bool y = false;
+            if (e0 + lane < end) {
+                const int e = e0 + lane;
+                u = adjncy[e];
+                edge_feat(adjwgt[e], (uint32_t)vwgt[u], cv, f0, f1);
+                y = L.label[e] != 0;
+                om = (y ? L.pos_w : 1.f) * L.inv_norm;
             }
-            const float y = L.label[e] ? 1.f : 0.f;
-            const float om = (L.label[e] ? L.pos_w : 1.f) * L.inv_norm;
-            const float p = 1.0f / (1.0f + expf(-s));
+            const unsigned ym = __ballot_sync(0xffffffffu, y);
+            const int cnt = min(32, end - e0);
+            float score = 0.f;  // of this lane's entry
+            for (int i0 = 0; i0 < cnt; i0 += Q) {
+                float t[Q], s[Q], a0[Q], a1[Q];
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    const int src = (i0 + q) & 31;
+                    const int uq = __shfl_sync(0xffffffffu, u, src);
+                    a0[q] = __shfl_sync(0xffffffffu, f0, src);
+                    a1[q] = __shfl_sync(0xffffffffu, f1, src);
+                    // (past the row's end: entry 0 of the chunk's lanes, not used)
+                    t[q] = z[(long long)uq * rm::Z + lane] + zv;
+                }
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    t[q] = t[q] + (wf0 * a0[q] + wf1 * a1[q]);
+                    s[q] = wo * fmaxf(t[q], 0.f);
+                }
+#pragma unroll
+                for (int o = 16; o; o >>= 1)
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    if (i0 + q >= cnt) break;  // uniform
+                    const float w = __shfl_sync(0xffffffffu, om, i0 + q);
+                    const bool cut = (ym >> (i0 + q)) & 1u;
+                    const float sc = s[q] + bo;
+                    const float p = 1.0f / (1.0f + expf(-sc));
+                    if (lane == i0 + q) score = sc;
+                    const float g = w * (p - (cut ? 1.f : 0.f));
+                    my_bo += g;
+                    my_wo += g * fmaxf(t[q], 0.f);
+                    const float dt = t[q] > 0.f ? g * wo : 0.f;
+                    my_f0 += dt * a0[q];
+                    my_f1 += dt * a1[q];
+                    dzl += dt;
+                }
+            }
             // weighted BCE from the logit: softplus(-s) for y = 1, softplus(s) for y = 0
-            const float xs = y > 0.f ? -s : s;
+            const float xs = y ? -score : score;
             my_loss += om * (fmaxf(xs, 0.f) + log1pf(expf(-fabsf(xs))));
-            const float g = om * (p - y);
-            atomicAdd(&gbo, g);
-#pragma unroll
-            for (int j = 0; j < rm::Z; ++j) {
-                const float r = fmaxf(t[j], 0.f);
-                atomicAdd(&gwo[j], g * r);
-                const float dt = t[j] > 0.f ? g * wo[j] : 0.f;
-                atomicAdd(&gwf[2 * j], dt * f0);
-                atomicAdd(&gwf[2 * j + 1], dt * f1);
-                dzl[j] += dt;
-            }
         }
-        // reduce dz over the warp's entries
-#pragma unroll
-        for (int j = 0; j < rm::Z; ++j) {
-            float x = dzl[j];
-#pragma unroll
-            for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-            if (lane == j) dz[v * rm::Z + j] = 2.f * x;
-        }
-        __syncwarp();
+        dz[v * rm::Z + lane] = 2.f * dzl;
     }
+    atomicAdd(&gwo[lane], my_wo);
+    atomicAdd(&gwf[2 * lane], my_f0);
+    atomicAdd(&gwf[2 * lane + 1], my_f1);
 #pragma unroll
     for (int o = 16; o; o >>= 1) my_loss += __shfl_xor_sync(0xffffffffu, my_loss, o);
-    if (lane == 0) atomicAdd(&sloss, my_loss);
+    if (lane == 0) {
+        atomicAdd(&gbo, my_bo);
+        atomicAdd(&sloss, my_loss);
+    }
     __syncthreads();
     for (int i = threadIdx.x; i < rm::Z * 2; i += kT) atomicAdd(G + rm::WF + i, gwf[i]);
     for (int i = threadIdx.x; i < rm::Z; i += kT) atomicAdd(G + rm::WO + i, gwo[i]);
@@ -273,53 +356,114 @@ __global__ void __launch_bounds__(kT) head_train(int n, const int* xadj, const i
 }
 
 // Backward of out = act(W [in0 | in1] + b):  dA = dOut * act'(out);
-// dIn = W^T dA (dIn0, dIn1 optional halves, accumulated with +=);
-// dW += dA in^T; db += dA.  Warp per node, block shared gradient buffers.
+// dIn = W^T dA (both halves, written); dW += dA in^T; db += dA.  A block takes
+// kTile nodes at a time: inputs, dA and its transpose in shared memory; dIn 4
+// nodes x K/16 inputs and dW N/16 x K/16 weights in each thread's registers,
+// the latter over all of the block's nodes.  (A warp a node took a
+// shared-memory float atomic per weight and node: 267 us at 32,771 nodes, K =
+// 128, N = 64; now 48.)
+template <int K, int N>
+constexpr size_t dense_bwd_smem() {
+    return sizeof(float) * ((size_t)N * K + (size_t)kTile * (K + 4) + (size_t)kTile * (N + 4) + (size_t)N * (kTile + 4));
+}
+
 template <int K, int N, bool RELU>
 __global__ void __launch_bounds__(kT) dense_bwd(int n, const float* P, int woff, const float* in0,
                                                 const float* in1, const float* out, const float* dout,
                                                 float* din0, float* din1, float* G, int goff_w, int goff_b) {
-    extern __shared__ float sm[];
-    float* w = sm;             // [N][K] (bf16-rounded)
-    float* gw = w + N * K;     // [N][K]
-    float* gb = gw + N * K;    // [N]
-    float* rows = gb + N;      // [kWarps][K + N]
-    for (int i = threadIdx.x; i < N * K; i += kT) {
-        w[i] = bf16r(P[woff + i]);
-        gw[i] = 0.f;
-    }
-    for (int i = threadIdx.x; i < N; i += kT) gb[i] = 0.f;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    float* xr = rows + wp * (K + N);
-    float* da = xr + K;
-    for (long long v = (long long)blockIdx.x * kWarps + wp; v < n; v += (long long)gridDim.x * kWarps) {
-        for (int k = lane; k < K; k += 32) xr[k] = k < rm::H ? in0[v * rm::H + k] : in1[v * rm::H + (k - rm::H)];
-        for (int j = lane; j < N; j += 32) {
-            float d = dout[v * N + j];
-            if (RELU && !(out[v * N + j] > 0.f)) d = 0.f;
-            da[j] = d;
-            atomicAdd(&gb[j], d);
+    extern __shared__ __align__(16) float sm[];
+    constexpr int XP = K + 4, AP = N + 4, TP = kTile + 4, TJ = N / 16, TK = K / 16;
+    float* w = sm;                // [N][K] (bf16-rounded)
+    float* xs = w + N * K;        // [kTile][XP]
+    float* da = xs + kTile * XP;  // [kTile][AP]
+    float* dt = da + kTile * AP;  // [N][TP], da transposed
+    for (int i = threadIdx.x; i < N * K; i += kT) w[i] = bf16r(P[woff + i]);
+    // a thread's inputs: 4 gk .. 4 gk + 3 of every 64 (16-byte loads of
+    // neighbouring lanes lie side by side)
+    const int gi = threadIdx.x / 16, gk = threadIdx.x % 16;
+    const int j0 = TJ * gi, t0 = 4 * gi, k0 = 4 * gk;
+    static_assert(TK % 4 == 0, "inputs in groups of four");
+    float gw[TJ][TK], gb = 0.f;
+#pragma unroll
+    for (int a = 0; a < TJ; ++a)
+#pragma unroll
+        for (int b = 0; b < TK; ++b) gw[a][b] = 0.f;
+    for (long long base = (long long)blockIdx.x * kTile; base < n; base += (long long)gridDim.x * kTile) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < kTile * K / 4; i += kT) {
+            const int t = i / (K / 4), k = 4 * (i % (K / 4));
+            const long long v = base + t;
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (v < n) x = *reinterpret_cast<const float4*>(k < rm::H ? in0 + v * rm::H + k : in1 + v * rm::H + (k - rm::H));
+            *reinterpret_cast<float4*>(xs + t * XP + k) = x;
         }
-        __syncwarp();
-        for (int k = lane; k < K; k += 32) {
-            float acc = 0.f;
-            const float x = xr[k];
+        for (int i = threadIdx.x; i < kTile * N; i += kT) {
+            const int t = i / N, j = i % N;
+            const long long v = base + t;
+            float d = 0.f;
+            if (v < n) {
+                d = dout[v * N + j];
+                if (RELU && !(out[v * N + j] > 0.f)) d = 0.f;
+            }
+            da[t * AP + j] = d;
+            dt[j * TP + t] = d;
+        }
+        __syncthreads();
+        // dIn, summed in the order of j
+        if (din0) {
+            float acc[4][TK];
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < TK; ++b) acc[a][b] = 0.f;
+#pragma unroll 2
             for (int j = 0; j < N; ++j) {
-                acc += da[j] * w[j * K + k];
-                atomicAdd(&gw[j * K + k], da[j] * x);
+                float d[4], x[TK];
+#pragma unroll
+                for (int a = 0; a < 4; ++a) d[a] = dt[j * TP + t0 + a];
+#pragma unroll
+                for (int b = 0; b < TK; ++b) x[b] = w[j * K + 64 * (b / 4) + k0 + b % 4];
+#pragma unroll
+                for (int a = 0; a < 4; ++a)
+#pragma unroll
+                    for (int b = 0; b < TK; ++b) acc[a][b] += d[a] * x[b];
             }
-            if (k < rm::H) {
-                if (din0) din0[v * rm::H + k] += acc;
-            } else if (din1) {
-                din1[v * rm::H + (k - rm::H)] += acc;
+#pragma unroll
+            for (int c = 0; c < TK / 4; ++c) {
+                float* din = c == 0 ? din0 : din1;
+                if (!din) continue;
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    const long long v = base + t0 + a;
+                    if (v >= n) break;
+                    *reinterpret_cast<float4*>(din + v * rm::H + k0) =
+                        make_float4(acc[a][4 * c], acc[a][4 * c + 1], acc[a][4 * c + 2], acc[a][4 * c + 3]);
+                }
             }
         }
-        __syncwarp();
+        // dW and db over the tile's nodes
+#pragma unroll 2
+        for (int t = 0; t < kTile; ++t) {
+            float d[TJ], x[TK];
+#pragma unroll
+            for (int a = 0; a < TJ; ++a) d[a] = da[t * AP + j0 + a];
+#pragma unroll
+            for (int b = 0; b < TK; ++b) x[b] = xs[t * XP + 64 * (b / 4) + k0 + b % 4];
+#pragma unroll
+            for (int a = 0; a < TJ; ++a)
+#pragma unroll
+                for (int b = 0; b < TK; ++b) gw[a][b] += d[a] * x[b];
+        }
+        if (threadIdx.x < N)
+            for (int t = 0; t < kTile; ++t) gb += dt[threadIdx.x * TP + t];
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < N * K; i += kT) atomicAdd(G + goff_w + i, gw[i]);
-    for (int i = threadIdx.x; i < N; i += kT) atomicAdd(G + goff_b + i, gb[i]);
+#pragma unroll
+    for (int a = 0; a < TJ; ++a)
+#pragma unroll
+        for (int b = 0; b < TK; b += 4)  // 16-byte additions (every offset is a multiple of four floats)
+            atomicAdd(reinterpret_cast<float4*>(G + goff_w + (j0 + a) * K + 64 * (b / 4) + k0),
+                      make_float4(gw[a][b], gw[a][b + 1], gw[a][b + 2], gw[a][b + 3]));
+    if (threadIdx.x < N) atomicAdd(G + goff_b + threadIdx.x, gb);
 }
 
 // dh[u] += sum_{v in N(u)} (w_uv / wdeg[v]) dagg[v]  (gather form; the graph
@@ -329,16 +473,33 @@ __global__ void __launch_bounds__(kT) agg_bwd(int n, const int* xadj, const int*
     const int lane = threadIdx.x & 31;
     for (long long u = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5); u < n; u += (long long)gridDim.x * kWarps) {
         float a0 = 0.f, a1 = 0.f;
-        for (int e = xadj[u]; e < xadj[u + 1]; ++e) {
-            const int v = adjncy[e];
-            const float d = wdeg[v];
-            if (!(d > 0.f)) continue;
-            const float c = (float)adjwgt[e] / d;
-            a0 += c * dagg[(long long)v * rm::H + 2 * lane];
-            a1 += c * dagg[(long long)v * rm::H + 2 * lane + 1];
+        const int beg = xadj[u], end = xadj[u + 1];
+        for (int e = beg; e < end; e += 4) {  // four neighbours' rows in flight
+            float2 x[4];
+            float c[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                c[q] = 0.f;
+                x[q] = make_float2(0.f, 0.f);
+                if (e + q < end) {
+                    const int v = adjncy[e + q];
+                    const float d = wdeg[v];
+                    const float2 g = ld2(dagg + (long long)v * rm::H + 2 * lane);
+                    if (d > 0.f) {  // (else nothing is added)
+                        c[q] = (float)adjwgt[e + q] / d;
+                        x[q] = g;
+                    }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                a0 += c[q] * x[q].x;
+                a1 += c[q] * x[q].y;
+            }
         }
-        dh[u * rm::H + 2 * lane] += a0;
-        dh[u * rm::H + 2 * lane + 1] += a1;
+        float2* o = reinterpret_cast<float2*>(dh + u * rm::H + 2 * lane);
+        const float2 old = *o;
+        *o = make_float2(old.x + a0, old.y + a1);
     }
 }
 
@@ -348,16 +509,24 @@ __global__ void __launch_bounds__(kT) layer0_bwd(int n, const float2* x, const f
     for (int i = threadIdx.x; i < rm::H * 3; i += kT) g[i] = 0.f;
     __syncthreads();
     const int lane = threadIdx.x & 31;
+    float acc[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};  // a lane's two features over the warp's nodes
     for (long long v = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5); v < n; v += (long long)gridDim.x * kWarps) {
         const float2 xv = x[v];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const int j = lane + 32 * q;
             const float d = h0[v * rm::H + j] > 0.f ? dh0[v * rm::H + j] : 0.f;
-            atomicAdd(&g[2 * j], d * xv.x);
-            atomicAdd(&g[2 * j + 1], d * xv.y);
-            atomicAdd(&g[2 * rm::H + j], d);
+            acc[q][0] += d * xv.x;
+            acc[q][1] += d * xv.y;
+            acc[q][2] += d;
         }
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int j = lane + 32 * q;
+        atomicAdd(&g[2 * j], acc[q][0]);
+        atomicAdd(&g[2 * j + 1], acc[q][1]);
+        atomicAdd(&g[2 * rm::H + j], acc[q][2]);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < rm::H * 2; i += kT) atomicAdd(G + rm::W0 + i, g[i]);
@@ -385,12 +554,28 @@ __global__ void count_labels(long long m, const uint8_t* label, unsigned long lo
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(pos, c);
 }
 
+// Blocks of a backward pass: two per SM (every block adds its weight gradients
+// to the sum, so no more than needed).
+int grid_bwd(long long items) {
+    return (int)std::max<long long>(1, std::min<long long>(items, 2 * kNumSMs));
+}
+
+template <int K, int N, bool RELU>
+void launch_dense_fwd(int n, const float* P, int woff, int boff, const float* in0, const float* in1, float* out,
+                      cudaStream_t s) {
+    constexpr size_t smem = dense_fwd_smem<K, N>();
+    KB_CUDA(cudaFuncSetAttribute(dense_fwd<K, N, RELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    dense_fwd<K, N, RELU><<<(int)std::max<long long>(1, std::min<long long>(div_up(n, kTile), 3LL * kNumSMs)), kT, smem,
+                            s>>>(n, P, woff, boff, in0, in1, out);
+    KB_LAUNCH();
+}
+
 template <int K, int N, bool RELU>
 void launch_dense_bwd(int n, const float* P, int woff, const float* in0, const float* in1, const float* out,
                       const float* dout, float* din0, float* din1, float* G, int gw, int gb, cudaStream_t s) {
-    const size_t smem = sizeof(float) * (2 * (size_t)N * K + N + (size_t)kWarps * (K + N));
+    constexpr size_t smem = dense_bwd_smem<K, N>();
     KB_CUDA(cudaFuncSetAttribute(dense_bwd<K, N, RELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dense_bwd<K, N, RELU><<<grid_nodes(n), kT, smem, s>>>(n, P, woff, in0, in1, out, dout, din0, din1, G, gw, gb);
+    dense_bwd<K, N, RELU><<<grid_bwd(div_up(n, kTile)), kT, smem, s>>>(n, P, woff, in0, in1, out, dout, din0, din1, G, gw, gb);
     KB_LAUNCH();
 }
 
@@ -440,12 +625,9 @@ static void forward_cuda_cores(Ctx& ctx, const DevGraph& g, const float* P, cons
     for (int l = 1; l <= 3; ++l) {
         agg_fwd<float><<<gr, kT, 0, s>>>(n, g.xadj, g.adjncy, g.adjwgt, f.wdeg, f.h[l - 1], f.agg[l - 1]);
         KB_LAUNCH();
-        dense_fwd<float, 128, 64, true><<<gr, kT, 0, s>>>(n, P, rm::layer_w(l), rm::layer_b(l), f.h[l - 1],
-                                                           f.agg[l - 1], f.h[l]);
-        KB_LAUNCH();
+        launch_dense_fwd<128, 64, true>(n, P, rm::layer_w(l), rm::layer_b(l), f.h[l - 1], f.agg[l - 1], f.h[l], s);
     }
-    dense_fwd<float, 64, 32, false><<<gr, kT, 0, s>>>(n, P, rm::WZ, rm::BZ, f.h[3], nullptr, f.z);
-    KB_LAUNCH();
+    launch_dense_fwd<64, 32, false>(n, P, rm::WZ, rm::BZ, f.h[3], nullptr, f.z, s);
 }
 
 void rating_infer_tc(Ctx& ctx, const DevGraph& g, const float* params, float* prob, uint32_t* rating);
@@ -509,20 +691,18 @@ void rating_train(Ctx& ctx, const TrainGraph* graphs, int count, int steps, floa
         L.pos_w = P1 > 0 ? (float)std::min(50.0, std::max(1.0, N0 / P1)) : 1.f;
         L.inv_norm = (float)(1.0 / std::max(1.0, L.pos_w * P1 + N0));
         KB_CUDA(cudaMemsetAsync(G, 0, sizeof(float) * rm::kParams, s));
-        for (auto p : dh) KB_CUDA(cudaMemsetAsync(p, 0, sizeof(float) * (size_t)n * rm::H, s));
         forward_cuda_cores(ctx, g, params, f);
         head_train<<<gr, kT, 0, s>>>(n, g.xadj, g.adjncy, g.adjwgt, g.vwgt, params, f.z, L, dz, G, dloss + step);
         KB_LAUNCH();
         launch_dense_bwd<64, 32, false>(n, params, rm::WZ, f.h[3], nullptr, f.z, dz, dh[3], nullptr, G, rm::WZ, rm::BZ,
                                         s);
         for (int l = 3; l >= 1; --l) {
-            KB_CUDA(cudaMemsetAsync(dagg, 0, sizeof(float) * (size_t)n * rm::H, s));
             launch_dense_bwd<128, 64, true>(n, params, rm::layer_w(l), f.h[l - 1], f.agg[l - 1], f.h[l], dh[l],
                                             dh[l - 1], dagg, G, rm::layer_w(l), rm::layer_b(l), s);
             agg_bwd<<<gr, kT, 0, s>>>(n, g.xadj, g.adjncy, g.adjwgt, f.wdeg, dagg, dh[l - 1]);
             KB_LAUNCH();
         }
-        layer0_bwd<<<gr, kT, 0, s>>>(n, f.x, f.h[0], dh[0], G);
+        layer0_bwd<<<grid_bwd(div_up(n, kWarps)), kT, 0, s>>>(n, f.x, f.h[0], dh[0], G);
         KB_LAUNCH();
         b1t *= 0.9f;
         b2t *= 0.999f;
@@ -564,19 +744,17 @@ void rating_grad(Ctx& ctx, const TrainGraph& tg, const float* params, float* G, 
     L.pos_w = P1 > 0 ? (float)std::min(50.0, std::max(1.0, N0 / P1)) : 1.f;
     L.inv_norm = (float)(1.0 / std::max(1.0, L.pos_w * P1 + N0));
     KB_CUDA(cudaMemsetAsync(G, 0, sizeof(float) * rm::kParams, s));
-    for (auto p : dh) KB_CUDA(cudaMemsetAsync(p, 0, sizeof(float) * nn * rm::H, s));
     forward_cuda_cores(ctx, g, params, f);
     head_train<<<gr, kT, 0, s>>>(n, g.xadj, g.adjncy, g.adjwgt, g.vwgt, params, f.z, L, dz, G, dloss);
     KB_LAUNCH();
     launch_dense_bwd<64, 32, false>(n, params, rm::WZ, f.h[3], nullptr, f.z, dz, dh[3], nullptr, G, rm::WZ, rm::BZ, s);
     for (int l = 3; l >= 1; --l) {
-        KB_CUDA(cudaMemsetAsync(dagg, 0, sizeof(float) * nn * rm::H, s));
         launch_dense_bwd<128, 64, true>(n, params, rm::layer_w(l), f.h[l - 1], f.agg[l - 1], f.h[l], dh[l], dh[l - 1],
                                         dagg, G, rm::layer_w(l), rm::layer_b(l), s);
         agg_bwd<<<gr, kT, 0, s>>>(n, g.xadj, g.adjncy, g.adjwgt, f.wdeg, dagg, dh[l - 1]);
         KB_LAUNCH();
     }
-    layer0_bwd<<<gr, kT, 0, s>>>(n, f.x, f.h[0], dh[0], G);
+    layer0_bwd<<<grid_bwd(div_up(n, kWarps)), kT, 0, s>>>(n, f.x, f.h[0], dh[0], G);
     KB_LAUNCH();
     KB_CUDA(cudaMemcpyAsync(loss, dloss, sizeof(float), cudaMemcpyDeviceToHost, s));
     KB_CUDA(cudaStreamSynchronize(s));
