@@ -24,8 +24,10 @@
 //   4. distinct counts -> prefix sum -> xadj; rows copied into place.
 #include "contract.cuh"
 #include "prims.cuh"
+#include "team.cuh"
 
 #include <climits>
+#include <stdexcept>
 
 namespace kb {
 
@@ -130,20 +132,26 @@ __device__ __forceinline__ uint32_t gather_slot(uint32_t key) {
     return (key * 0x9E3779B1u) >> 24;  // kGatherTab == 256
 }
 
+struct GatherSmem {
+    uint32_t tk[kGatherWarps][kGatherTab];
+    uint32_t tv[kGatherWarps][kGatherTab];
+    uint64_t sb[kGatherWarps][kGatherSort];  // used slots, then the sorted entries
+    unsigned tcount[kGatherWarps];
+};
+
+// mcnt / rcap: a node's member count and row capacity where they are not the
+// differences of mbeg / rowoff (those of a team are in no order).
 template <bool UNIT>
-__global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) gather_rows(
-    int nc, const uint32_t* __restrict__ mbeg, const int2* __restrict__ mrow, const int* __restrict__ adjncy,
-    const int* __restrict__ adjwgt, const int* __restrict__ cmap, const uint32_t* __restrict__ rowoff,
-    uint64_t* bucket, uint32_t* ucnt, int* big, unsigned* nbig) {
+__device__ __forceinline__ void gather_all(GatherSmem& sm, int nc, const uint32_t* mbeg, const uint32_t* mcnt,
+                                           const int2* mrow, const int* adjncy, const int* adjwgt, const int* cmap,
+                                           const uint32_t* rowoff, const uint32_t* rcap, uint64_t* bucket,
+                                           uint32_t* ucnt, int* big, unsigned* nbig) {
     static_assert(kGatherTab == 256 && kGatherSort >= kGatherList, "table layout");
-    __shared__ uint32_t tk[kGatherWarps][kGatherTab];
-    __shared__ uint32_t tv[kGatherWarps][kGatherTab];
-    __shared__ uint64_t sb[kGatherWarps][kGatherSort];  // used slots, then the sorted entries
-    __shared__ unsigned tcount[kGatherWarps];
+    unsigned* tcount = sm.tcount;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    volatile uint32_t* K = tk[wp];
-    uint32_t* V = tv[wp];
-    uint64_t* B = sb[wp];
+    volatile uint32_t* K = sm.tk[wp];
+    uint32_t* V = sm.tv[wp];
+    uint64_t* B = sm.sb[wp];
     for (int i = lane; i < kGatherTab; i += 32) {
         K[i] = kEmpty;
         V[i] = 0;
@@ -156,18 +164,18 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) gather_
     uint32_t nm0 = 0, nm1 = 0, nr0 = 0, nr1 = 0;
     if (cc < nc) {
         nm0 = mbeg[cc];
-        nm1 = mbeg[cc + 1];
+        nm1 = mcnt ? nm0 + mcnt[cc] : mbeg[cc + 1];
         nr0 = rowoff[cc];
-        nr1 = rowoff[cc + 1];
+        nr1 = rcap ? nr0 + rcap[cc] : rowoff[cc + 1];
     }
     for (; cc < nc; cc += nwarps) {
         const int c = (int)cc;
         const uint32_t m0 = nm0, m1 = nm1, r0 = nr0, r1 = nr1;
         if (cc + nwarps < nc) {
             nm0 = mbeg[cc + nwarps];
-            nm1 = mbeg[cc + nwarps + 1];
+            nm1 = mcnt ? nm0 + mcnt[cc + nwarps] : mbeg[cc + nwarps + 1];
             nr0 = rowoff[cc + nwarps];
-            nr1 = rowoff[cc + nwarps + 1];
+            nr1 = rcap ? nr0 + rcap[cc + nwarps] : rowoff[cc + nwarps + 1];
         }
         if ((long long)r1 - r0 > kGatherMaxEntries) {
             if (lane == 0) big[atomicAdd(nbig, 1u)] = c;
@@ -317,6 +325,15 @@ __global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) gather_
         }
         __syncwarp();
     }
+}
+
+template <bool UNIT>
+__global__ void __launch_bounds__(kGatherWarps * 32, kGatherBlocksPerSM) gather_rows(
+    int nc, const uint32_t* __restrict__ mbeg, const int2* __restrict__ mrow, const int* __restrict__ adjncy,
+    const int* __restrict__ adjwgt, const int* __restrict__ cmap, const uint32_t* __restrict__ rowoff,
+    uint64_t* bucket, uint32_t* ucnt, int* big, unsigned* nbig) {
+    __shared__ GatherSmem sm;
+    gather_all<UNIT>(sm, nc, mbeg, nullptr, mrow, adjncy, adjwgt, cmap, rowoff, nullptr, bucket, ucnt, big, nbig);
 }
 
 // One thread per fine vertex: merges its neighbours by coarse target in
@@ -589,10 +606,11 @@ constexpr int kBigBlocks = 2 * kNumSMs;
 constexpr int kBigMember = 256;     // longer member rows are walked by the whole block
 
 // bits of one pass in order -> the row's entries from `at` on; returns their number
+template <int BT>
 __device__ __forceinline__ uint32_t big_flush(uint32_t* mask, int words, int base, uint32_t* cnt, uint64_t* out) {
-    __shared__ uint32_t wsum[kBigThreads / 32 + 1];
+    __shared__ uint32_t wsum[BT / 32 + 1];
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    const int per = (words + kBigThreads - 1) / kBigThreads;
+    const int per = (words + BT - 1) / BT;
     const int w0 = min(words, (int)threadIdx.x * per), w1 = min(words, w0 + per);
     uint32_t mine = 0;
     for (int w = w0; w < w1; ++w) mine += __popc(mask[w]);
@@ -605,15 +623,15 @@ __device__ __forceinline__ uint32_t big_flush(uint32_t* mask, int words, int bas
     if (lane == 31) wsum[wp] = incl;
     __syncthreads();
     if (wp == 0) {
-        const uint32_t x = lane < kBigThreads / 32 ? wsum[lane] : 0u;
+        const uint32_t x = lane < BT / 32 ? wsum[lane] : 0u;
         uint32_t t = x;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
             if (lane >= o) t += y;
         }
-        if (lane < kBigThreads / 32) wsum[lane] = t - x;
-        if (lane == 31) wsum[kBigThreads / 32] = t;
+        if (lane < BT / 32) wsum[lane] = t - x;
+        if (lane == 31) wsum[BT / 32] = t;
     }
     __syncthreads();
     uint64_t* o = out + wsum[wp] + (incl - mine);
@@ -628,7 +646,7 @@ __device__ __forceinline__ uint32_t big_flush(uint32_t* mask, int words, int bas
             __stcg(cnt + t, 0u);
         }
     }
-    const uint32_t total = wsum[kBigThreads / 32];
+    const uint32_t total = wsum[BT / 32];
     __syncthreads();
     return total;
 }
@@ -636,21 +654,20 @@ __device__ __forceinline__ uint32_t big_flush(uint32_t* mask, int words, int bas
 // The rows of `list` (count of them).  MEMBERS: from the member rows of the
 // coarse node (member lists as in gather_rows); else from the fill[c] entries
 // that the emission left in the row's bucket, which the result replaces.
-template <bool UNIT, bool MEMBERS>
-__global__ void __launch_bounds__(kBigThreads) big_rows(
-    int nc, const int* __restrict__ list, const unsigned* __restrict__ count, const uint32_t* __restrict__ mbeg,
-    const int2* __restrict__ mrow, const int* __restrict__ adjncy, const int* __restrict__ adjwgt,
-    const int* __restrict__ cmap, const uint32_t* __restrict__ rowoff, const uint32_t* __restrict__ fill,
-    uint64_t* bucket, uint64_t* spare, uint32_t* counters, int range, uint32_t* ucnt) {
-    extern __shared__ uint32_t mask[];
-    const unsigned n = *count;
-    if (blockIdx.x >= n) return;
+// Blocks [0, blocks) take part; mcnt as in gather_all.
+template <bool UNIT, bool MEMBERS, int BT>
+__device__ __forceinline__ void big_all(uint32_t* mask, int nc, const int* list, unsigned n, unsigned blocks,
+                                        const uint32_t* mbeg, const uint32_t* mcnt, const int2* mrow,
+                                        const int* adjncy, const int* adjwgt, const int* cmap, const uint32_t* rowoff,
+                                        const uint32_t* fill, uint64_t* bucket, uint64_t* spare, uint32_t* counters,
+                                        int range, uint32_t* ucnt) {
+    if (blockIdx.x >= n || blockIdx.x >= blocks) return;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     uint32_t* cnt = counters + (size_t)blockIdx.x * range;
-    for (int i = threadIdx.x; i < range; i += kBigThreads) __stcg(cnt + i, 0u);
-    for (int i = threadIdx.x; i < (range + 31) / 32; i += kBigThreads) mask[i] = 0;
+    for (int i = threadIdx.x; i < range; i += BT) __stcg(cnt + i, 0u);
+    for (int i = threadIdx.x; i < (range + 31) / 32; i += BT) mask[i] = 0;
     __syncthreads();
-    for (unsigned i = blockIdx.x; i < n; i += gridDim.x) {
+    for (unsigned i = blockIdx.x; i < n; i += blocks) {
         const int c = list[i];
         uint64_t* row = bucket + rowoff[c];
         uint32_t written = 0;
@@ -682,19 +699,19 @@ __global__ void __launch_bounds__(kBigThreads) big_rows(
                             if (t[q] >= 0 && t[q] != c) add(t[q], w[q]);
                     }
                 };
-                const uint32_t m0 = mbeg[c], m1 = mbeg[c + 1];
-                for (uint32_t m = m0 + wp; m < m1; m += kBigThreads / 32) {
+                const uint32_t m0 = mbeg[c], m1 = mcnt ? m0 + mcnt[c] : mbeg[c + 1];
+                for (uint32_t m = m0 + wp; m < m1; m += BT / 32) {
                     const int2 r = mrow[m];
                     if (r.y <= kBigMember) walk(r.x, r.y, lane, 32);
                 }
                 for (uint32_t m = m0; m < m1; ++m) {
                     const int2 r = mrow[m];
-                    if (r.y > kBigMember) walk(r.x, r.y, (int)threadIdx.x, kBigThreads);
+                    if (r.y > kBigMember) walk(r.x, r.y, (int)threadIdx.x, BT);
                 }
             } else {
                 const uint32_t s = fill[c];
                 const uint64_t* src = base == 0 ? row : spare + rowoff[c];
-                for (uint32_t e = threadIdx.x; e < s; e += kBigThreads) {
+                for (uint32_t e = threadIdx.x; e < s; e += BT) {
                     const uint64_t x = src[e];
                     // (further passes read a copy: the row is overwritten)
                     if (base == 0 && range < nc) spare[rowoff[c] + e] = x;
@@ -702,10 +719,21 @@ __global__ void __launch_bounds__(kBigThreads) big_rows(
                 }
             }
             __syncthreads();
-            written += big_flush(mask, (R + 31) / 32, base, cnt, row + written);
+            written += big_flush<BT>(mask, (R + 31) / 32, base, cnt, row + written);
         }
         if (threadIdx.x == 0) ucnt[c] = written;
     }
+}
+
+template <bool UNIT, bool MEMBERS>
+__global__ void __launch_bounds__(kBigThreads) big_rows(
+    int nc, const int* __restrict__ list, const unsigned* __restrict__ count, const uint32_t* __restrict__ mbeg,
+    const int2* __restrict__ mrow, const int* __restrict__ adjncy, const int* __restrict__ adjwgt,
+    const int* __restrict__ cmap, const uint32_t* __restrict__ rowoff, const uint32_t* __restrict__ fill,
+    uint64_t* bucket, uint64_t* spare, uint32_t* counters, int range, uint32_t* ucnt) {
+    extern __shared__ uint32_t mask[];
+    big_all<UNIT, MEMBERS, kBigThreads>(mask, nc, list, *count, gridDim.x, mbeg, nullptr, mrow, adjncy, adjwgt, cmap,
+                                        rowoff, fill, bucket, spare, counters, range, ucnt);
 }
 
 // Degree statistics of the coarse graph from its row lengths, before the
@@ -752,7 +780,344 @@ __global__ void copy_rows(int nc, const uint32_t* __restrict__ rowoff, const uin
     }
 }
 
+// ---- small levels: the whole contraction by one team (team.cuh).  As
+// launches a level is about 25 kernels, 10 fills and two read-backs, 130-150
+// us of launching however few nodes it has; here it is ten steps a barrier
+// apart and one read-back, 50 us.  Buckets and member lists take their places
+// by atomic cursors (their order does not show: rows come out sorted), only
+// the coarse ids and row starts are prefix sums.  The lines, by coarsening
+// time: a 200k-node level 0.05 ms less than as launches, one of 264k 0.06, of
+// 870k the same; an R-MAT level of 131k nodes with hubs 0.6 ms more (its long
+// rows want the launches' larger blocks), of 62k 0.3 ms less.
+constexpr int kTeamContractNodes = 1 << 18, kTeamContractHubs = 1 << 16, kTeamContractHub = 1024;
+
+struct ContractTeam {
+    int n;
+    const int *label, *xadj, *adjncy, *adjwgt, *vwgt;
+    int* cmap;
+    int* mm;            // n: smallest member
+    uint32_t *pos;      // n: coarse id of a leader
+    uint32_t *cvw, *rowcap, *rowoff, *msize, *mbeg, *mfill, *ucnt;  // n (by coarse id)
+    uint32_t* cxadj;    // n + 1
+    int2* mrow;         // n
+    uint64_t* bucket;   // m
+    int* big;           // n
+    uint32_t* counters; // [cblocks][n]
+    int cblocks;
+    uint32_t* sums;     // [blocks]
+    uint32_t* out;      // [0] bucket cursor, [1] member cursor, [2] long rows, [3] coarse nodes,
+                        // [4] coarse entries, [5..8] degree statistics
+};
+
+// Exclusive prefix sum over the block's 256 threads; *total = the sum.
+__device__ __forceinline__ uint32_t block_scan256(uint32_t x, uint32_t* total, uint32_t* sh) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint32_t incl = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    __syncthreads();
+    if (lane == 31) sh[wid] = incl;
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) {
+        if (w < wid) before += sh[w];
+        all += sh[w];
+    }
+    *total = all;
+    return before + incl - x;
+}
+
+// The sum of sums[0 .. count) and of those before this block.
+__device__ __forceinline__ void sum_before(const uint32_t* sums, int count, uint32_t* before, uint32_t* all,
+                                           uint32_t* sh) {
+    uint32_t b = 0, a = 0;
+    for (int i = threadIdx.x; i < count; i += kThreads) {
+        const uint32_t x = sums[i];
+        a += x;
+        if (i < (int)blockIdx.x) b += x;
+    }
+    a = __reduce_add_sync(0xffffffffu, a);
+    b = __reduce_add_sync(0xffffffffu, b);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+        sh[threadIdx.x >> 5] = a;
+        sh[kThreads / 32 + (threadIdx.x >> 5)] = b;
+    }
+    __syncthreads();
+    a = b = 0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) {
+        a += sh[w];
+        b += sh[kThreads / 32 + w];
+    }
+    *before = b;
+    *all = a;
+}
+
+template <bool UNIT>
+__global__ void __launch_bounds__(kThreads, 4) contract_team(ContractTeam C, TeamArgs T) {
+    static_assert(kThreads == kTeamThreads && kGatherWarps * 32 == kThreads, "one block size");
+    __shared__ GatherSmem sm;
+    __shared__ uint32_t sh[2 * kThreads / 32];
+    extern __shared__ uint32_t mask[];
+    Team team(T);
+    const int n = C.n, lane = threadIdx.x & 31;
+    // contiguous ids of this block (coarse ids: of nc)
+    const int per = (n + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int lo = (int)min((long long)n, (long long)blockIdx.x * per), hi = min(n, lo + per);
+    for (long long i = team.rank(); i < n; i += team.size()) {
+        C.mm[i] = INT_MAX;
+        C.cvw[i] = C.rowcap[i] = C.msize[i] = C.mfill[i] = 0;
+    }
+    if (team.leader())
+        for (int i = 0; i < 9; ++i) C.out[i] = 0;
+    bool alive = team.sync();
+    int nc = 0;
+    do {
+        if (!alive) break;
+        // smallest member of every cluster (lanes with equal labels together)
+        for (long long base = (long long)blockIdx.x * kThreads; base < n; base += team.size()) {
+            const int v = (int)base + threadIdx.x;
+            const int l = v < n ? C.label[v] : -1;
+            const unsigned peers = __match_any_sync(0xffffffffu, l);
+            if (l >= 0 && lane == __ffs(peers) - 1) atomicMin(&C.mm[l], v);
+        }
+        if (!(alive = team.sync())) break;
+        // coarse ids: leaders numbered in id order
+        uint32_t mine = 0;
+        for (int v = lo + threadIdx.x; v < hi; v += kThreads) mine += C.mm[C.label[v]] == v ? 1u : 0u;
+        uint32_t total;
+        block_scan256(mine, &total, sh);
+        if (threadIdx.x == 0) C.sums[blockIdx.x] = total;
+        if (!(alive = team.sync())) break;
+        {
+            uint32_t run, all;
+            sum_before(C.sums, (int)gridDim.x, &run, &all, sh);
+            nc = (int)all;
+            for (int base = lo; base < hi; base += kThreads) {
+                const int v = base + (int)threadIdx.x;
+                const bool leader = v < hi && C.mm[C.label[v]] == v;
+                const uint32_t at = block_scan256(leader ? 1u : 0u, &total, sh);
+                if (leader) C.pos[v] = run + at;
+                run += total;
+            }
+        }
+        if (!(alive = team.sync())) break;
+        // cmap, node weights, row capacities, member counts
+        for (long long base = (long long)blockIdx.x * kThreads; base < n; base += team.size()) {
+            const int v = (int)base + threadIdx.x;
+            int c = -1;
+            uint32_t w = 0, d = 0;
+            if (v < n) {
+                c = (int)C.pos[C.mm[C.label[v]]];
+                C.cmap[v] = c;
+                w = (uint32_t)C.vwgt[v];
+                d = (uint32_t)(C.xadj[v + 1] - C.xadj[v]);
+            }
+            const unsigned peers = __match_any_sync(0xffffffffu, c);
+            const uint32_t sw = __reduce_add_sync(peers, w), sd = __reduce_add_sync(peers, d);
+            if (c >= 0 && lane == __ffs(peers) - 1) {
+                atomicAdd(&C.cvw[c], sw);
+                atomicAdd(&C.rowcap[c], sd);
+                atomicAdd(&C.msize[c], (uint32_t)__popc(peers));
+            }
+        }
+        if (!(alive = team.sync())) break;
+        // places of the buckets and member lists
+        for (long long base = (long long)blockIdx.x * kThreads; base < nc; base += team.size()) {
+            const int c = (int)base + threadIdx.x;
+            const uint32_t d = c < nc ? C.rowcap[c] : 0u, k = c < nc ? C.msize[c] : 0u;
+            uint32_t id = d, ik = k;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, id, o), z = __shfl_up_sync(0xffffffffu, ik, o);
+                if (lane >= o) {
+                    id += y;
+                    ik += z;
+                }
+            }
+            uint32_t bd = 0, bk = 0;
+            if (lane == 31) {
+                bd = atomicAdd(&C.out[0], id);
+                bk = atomicAdd(&C.out[1], ik);
+            }
+            bd = __shfl_sync(0xffffffffu, bd, 31);
+            bk = __shfl_sync(0xffffffffu, bk, 31);
+            if (c < nc) {
+                C.rowoff[c] = bd + id - d;
+                C.mbeg[c] = bk + ik - k;
+            }
+        }
+        if (!(alive = team.sync())) break;
+        for (long long base = (long long)blockIdx.x * kThreads; base < n; base += team.size()) {
+            const int v = (int)base + threadIdx.x;
+            const int c = v < n ? C.cmap[v] : -1;
+            const unsigned peers = __match_any_sync(0xffffffffu, c);
+            const int leader = __ffs(peers) - 1;
+            uint32_t at = 0;
+            if (c >= 0 && lane == leader) at = atomicAdd(&C.mfill[c], (uint32_t)__popc(peers));
+            at = __shfl_sync(0xffffffffu, at, leader);
+            if (c >= 0) {
+                const int b = C.xadj[v];
+                C.mrow[C.mbeg[c] + at + __popc(peers & lanemask_lt())] = make_int2(b, C.xadj[v + 1] - b);
+            }
+        }
+        if (!(alive = team.sync())) break;
+        gather_all<UNIT>(sm, nc, C.mbeg, C.msize, C.mrow, C.adjncy, C.adjwgt, C.cmap, C.rowoff, C.rowcap, C.bucket,
+                         C.ucnt, C.big, C.out + 2);
+        if (!(alive = team.sync())) break;
+        if (const unsigned nbig = C.out[2]) {
+            big_all<UNIT, true, kThreads>(mask, nc, C.big, nbig, C.cblocks, C.mbeg, C.msize, C.mrow, C.adjncy, C.adjwgt,
+                                          C.cmap, C.rowoff, nullptr, C.bucket, nullptr, C.counters, nc, C.ucnt);
+            if (!(alive = team.sync())) break;
+        }
+        // row starts and degree statistics
+        const int cper = (nc + (int)gridDim.x - 1) / (int)gridDim.x;
+        const int clo = (int)min((long long)nc, (long long)blockIdx.x * cper), chi = min(nc, clo + cper);
+        unsigned md = 0, iso = 0, wi = 0, wa = 0;
+        mine = 0;
+        for (int c = clo + threadIdx.x; c < chi; c += kThreads) {
+            const unsigned d = C.ucnt[c], w = C.cvw[c];
+            mine += d;
+            md = max(md, d);
+            wa = max(wa, w);
+            if (d == 0) {
+                ++iso;
+                wi = max(wi, w);
+            }
+        }
+        md = __reduce_max_sync(0xffffffffu, md);
+        iso = __reduce_add_sync(0xffffffffu, iso);
+        wi = __reduce_max_sync(0xffffffffu, wi);
+        wa = __reduce_max_sync(0xffffffffu, wa);
+        if (lane == 0) {
+            if (md) atomicMax(C.out + 5, md);
+            if (iso) atomicAdd(C.out + 6, iso);
+            if (wi) atomicMax(C.out + 7, wi);
+            if (wa) atomicMax(C.out + 8, wa);
+        }
+        block_scan256(mine, &total, sh);
+        if (threadIdx.x == 0) C.sums[blockIdx.x] = total;
+        if (!(alive = team.sync())) break;
+        uint32_t run, all;
+        sum_before(C.sums, (int)gridDim.x, &run, &all, sh);
+        for (int base = clo; base < chi; base += kThreads) {
+            const int c = base + (int)threadIdx.x;
+            const uint32_t at = block_scan256(c < chi ? C.ucnt[c] : 0u, &total, sh);
+            if (c < chi) C.cxadj[c] = run + at;
+            run += total;
+        }
+        if (team.leader()) {
+            C.cxadj[nc] = all;
+            C.out[3] = (uint32_t)nc;
+            C.out[4] = all;
+        }
+    } while (false);
+    team.leave();
+}
+
+// The coarse graph from a team's scratch: rows, row starts, node weights.
+__global__ void copy_level(int nc, const uint32_t* __restrict__ rowoff, const uint32_t* __restrict__ ucnt,
+                           const uint32_t* __restrict__ sxadj, const uint32_t* __restrict__ scvw,
+                           const uint64_t* __restrict__ bucket, int* cxadj, int* cvw, int* cadj, int* cw) {
+    const int lane = threadIdx.x & 31;
+    for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32; r <= nc;
+         r += (long long)gridDim.x * blockDim.x / 32) {
+        const uint32_t dst = sxadj[r];
+        if (lane == 0) {
+            cxadj[r] = (int)dst;
+            if (r < nc) cvw[r] = (int)scvw[r];
+        }
+        if (r == nc) continue;
+        const long long src = rowoff[r];
+        const uint32_t u = ucnt[r];
+        for (uint32_t i = lane; i < u; i += 32) {
+            const uint64_t x = bucket[src + i];
+            cadj[dst + i] = (int)(x >> 32);
+            cw[dst + i] = (int)(uint32_t)x;
+        }
+    }
+}
+
 }  // namespace
+
+// Fills out and the coarse arrays; false when the level is not one for a team.
+static bool contract_by_team(Ctx& ctx, const DevGraph& g, const int* label, int* cmap, DevGraph& out, int** out_xadj,
+                             int** out_adjncy, int** out_adjwgt, int** out_vwgt) {
+    if (g.n > (g.maxdeg > kTeamContractHub ? kTeamContractHubs : kTeamContractNodes)) return false;
+    cudaStream_t st = ctx.stream;
+    const size_t mk = ctx.scratch.mark(), n = (size_t)g.n;
+    auto kernel = g.unit_weights ? contract_team<true> : contract_team<false>;
+    const size_t smem = sizeof(uint32_t) * ((n + 31) / 32);
+    const TeamRoom room = team_room(ctx, (const void*)kernel, smem);
+    const int blocks = team_blocks(room, div_up(g.m > 16LL * g.n ? g.m : g.n, kThreads));
+    ContractTeam C{};
+    C.n = g.n;
+    C.label = label;
+    C.xadj = g.xadj;
+    C.adjncy = g.adjncy;
+    C.adjwgt = g.adjwgt;
+    C.vwgt = g.vwgt;
+    C.cmap = cmap;
+    C.mm = ctx.scratch.alloc<int>(n);
+    uint32_t** arrays[] = {&C.pos, &C.cvw, &C.rowcap, &C.rowoff, &C.msize, &C.mbeg, &C.mfill, &C.ucnt};
+    for (uint32_t** a : arrays) *a = ctx.scratch.alloc<uint32_t>(n);
+    C.cxadj = ctx.scratch.alloc<uint32_t>(n + 1);
+    C.mrow = ctx.scratch.alloc<int2>(n);
+    C.bucket = ctx.scratch.alloc<uint64_t>((size_t)std::max<long long>(g.m, 1));
+    C.big = ctx.scratch.alloc<int>(n);
+    // counters of the long rows: up to 20 B per entry of the level
+    C.cblocks = (int)std::max<long long>(1, std::min<long long>(blocks, 5 * g.m / (long long)n));
+    C.counters = ctx.scratch.alloc<uint32_t>((size_t)C.cblocks * n);
+    C.sums = ctx.scratch.alloc<uint32_t>((size_t)blocks);
+    C.out = ctx.scratch.alloc<uint32_t>(9);
+    bool done;
+    {
+        PhaseScope ps(ctx, "contract_team", 0);
+        done = launch_team(ctx, kernel, room, blocks, smem, C);
+    }
+    if (!done) {
+        ctx.scratch.release(mk);
+        return false;
+    }
+    KB_CUDA(cudaMemcpyAsync(ctx.pinned, C.out + 3, 6 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    KB_CUDA(cudaStreamSynchronize(st));
+    const int nc = (int)ctx.pinned[0];
+    const long long mc = (long long)ctx.pinned[1];
+    if (nc <= 0) throw std::runtime_error("a team of thread blocks gave up (internal)");
+    int* cxadj = ctx.hier.alloc<int>((size_t)nc + 1);
+    int* cvw = ctx.hier.alloc<int>((size_t)nc);
+    int* cadj = ctx.hier.alloc<int>((size_t)std::max<long long>(mc, 1));
+    int* cwgt = ctx.hier.alloc<int>((size_t)std::max<long long>(mc, 1));
+    out = DevGraph{};
+    out.n = nc;
+    out.m = mc;
+    out.maxdeg = (int)ctx.pinned[2];
+    out.iso_count = ctx.pinned[3];
+    out.iso_wmax = ctx.pinned[4];
+    out.maxvw = ctx.pinned[5];
+    out.rows_sorted = 1;
+    out.xadj = cxadj;
+    out.adjncy = cadj;
+    out.adjwgt = cwgt;
+    out.vwgt = cvw;
+    *out_xadj = cxadj;
+    *out_adjncy = cadj;
+    *out_adjwgt = cwgt;
+    *out_vwgt = cvw;
+    {
+        PhaseScope ps(ctx, "contract_rows", 16.0 * mc + 12.0 * nc);
+        copy_level<<<grid_for(32LL * (nc + 1), 256), 256, 0, st>>>(nc, C.rowoff, C.ucnt, C.cxadj, C.cvw, C.bucket, cxadj,
+                                                                  cvw, cadj, cwgt);
+        KB_LAUNCH();
+    }
+    ctx.scratch.release(mk);
+    return true;
+}
 
 void contract(Ctx& ctx, const DevGraph& g, const int* label, int* cmap, DevGraph& out,
               int** out_xadj, int** out_adjncy, int** out_adjwgt, int** out_vwgt) {
@@ -769,6 +1134,7 @@ void contract(Ctx& ctx, const DevGraph& g, const int* label, int* cmap, DevGraph
         *out_adjncy = *out_adjwgt = *out_vwgt = nullptr;
         return;
     }
+    if (contract_by_team(ctx, g, label, cmap, out, out_xadj, out_adjncy, out_adjwgt, out_vwgt)) return;
     // device scalars: [0] coarse nodes, [38] long rows, [39] coarse entries,
     // [40..43] the coarse graph's degree statistics
     uint32_t* tot = reinterpret_cast<uint32_t*>(ctx.dscalars);

@@ -65,13 +65,14 @@ TeamRoom team_room(Ctx& ctx, const void* kernel, size_t smem) {
     };
     static std::mutex mu;
     static std::vector<Known> known;
+    smem = (smem + 4095) / 4096 * 4096;  // (few distinct sizes are kept)
     std::lock_guard<std::mutex> lk(mu);
     for (const Known& k : known)
         if (k.kernel == kernel && k.device == ctx.device && k.smem == smem)
             return TeamRoom{k.room.most / std::max(ctx.team_share, 1), k.room.wide_cluster};
     TeamRoom r{0, false};
     int per = 0, sms = 0, clusters = 0;
-    if (smem > 40 * 1024)  // with the kernel's own shared memory above the default limit
+    if (smem > 8 * 1024)  // (with the kernel's own shared memory it may exceed the default limit)
         KB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
     KB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kTeamThreads, smem));
     KB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
