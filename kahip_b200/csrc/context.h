@@ -52,6 +52,7 @@ public:
         return p;
     }
     size_t mark() const { return top_; }
+    char* top() const { return base_ + top_; }
     void release(size_t m) { top_ = m; }
     size_t capacity() const { return cap_; }
     size_t peak() const { return peak_; }
@@ -83,6 +84,12 @@ struct Ctx {
     unsigned* team_bar = nullptr;          // barrier counters of a team of blocks (team.cuh)
     int team_share = 1;                    // calls that share the device with this one (team.cuh)
     uint32_t* pinned = nullptr;            // 64 words, page-locked
+    // page-locked staging for small transfers of pageable host memory, kept
+    // with the context (at most kStageMax bytes)
+    static constexpr size_t kStageMax = (size_t)32 << 20;
+    char* stage = nullptr;
+    size_t stage_cap = 0;
+    char* staging(size_t bytes);           // at least that many, null above kStageMax
     // timing: 0 off, 1 every kernel family, 2 only the LP clustering sweep
     int timing = 0;
     std::vector<PhaseTimer> phases;

@@ -372,8 +372,7 @@ int max_degree(Ctx& ctx, const DevGraph& g) {
 }
 
 void check_graph_begin(Ctx& ctx) {
-    KB_CUDA(cudaMemsetAsync(ctx.dscalars + 2, 0, 2 * sizeof(int), ctx.stream));  // [2] flags, [3] weight sum
-    KB_CUDA(cudaMemsetAsync(ctx.dscalars + 8, 0, 4 * sizeof(int), ctx.stream));  // [8..11] degree statistics
+    KB_CUDA(cudaMemsetAsync(ctx.dscalars + 2, 0, 10 * sizeof(int), ctx.stream));
 }
 
 void check_graph_range(Ctx& ctx, const DevGraph& g, int v_lo, int v_hi, bool unit_known) {
@@ -386,8 +385,8 @@ void check_graph_range(Ctx& ctx, const DevGraph& g, int v_lo, int v_hi, bool uni
 }
 
 int check_graph_end(Ctx& ctx, uint32_t* total_weight, DevGraph* stats) {
-    KB_CUDA(cudaMemcpyAsync(ctx.pinned + 2, ctx.dscalars + 2, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
-    KB_CUDA(cudaMemcpyAsync(ctx.pinned + 8, ctx.dscalars + 8, 4 * sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
+    // [2] flags, [3] weight sum, [8..11] degree statistics
+    KB_CUDA(cudaMemcpyAsync(ctx.pinned + 2, ctx.dscalars + 2, 10 * sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
     KB_CUDA(cudaStreamSynchronize(ctx.stream));
     if (total_weight) *total_weight = ctx.pinned[3];
     if (stats) {

@@ -32,6 +32,7 @@ Ctx::~Ctx() {
     if (origin) cudaEventDestroy(origin);
     if (copy_stream) cudaStreamDestroy(copy_stream);
     if (pinned) cudaFreeHost(pinned);
+    if (stage) cudaFreeHost(stage);
     if (dscalars) cudaFree(dscalars);
     hier.free_all();
     scratch.free_all();
@@ -93,6 +94,20 @@ TeamRoom team_room(Ctx& ctx, const void* kernel, size_t smem) {
     if (!r.wide_cluster) (void)cudaGetLastError();
     known.push_back(Known{kernel, ctx.device, smem, r});
     return TeamRoom{r.most / std::max(ctx.team_share, 1), r.wide_cluster};
+}
+
+char* Ctx::staging(size_t bytes) {
+    if (bytes > kStageMax) return nullptr;
+    if (bytes > stage_cap) {
+        size_t cap = (size_t)1 << 20;
+        while (cap < bytes) cap <<= 1;
+        if (stage) cudaFreeHost(stage);
+        stage = nullptr;
+        stage_cap = 0;
+        KB_CUDA(cudaMallocHost(&stage, cap));
+        stage_cap = cap;
+    }
+    return stage;
 }
 
 int Ctx::phase_id(const char* name) {
@@ -187,21 +202,36 @@ struct Level {
     int* part = nullptr;
 };
 
-uint32_t read_max_bw(Ctx& ctx, const uint32_t* bw, int k, std::vector<uint32_t>& host) {
-    host.resize((size_t)k);
-    KB_CUDA(cudaMemcpyAsync(host.data(), bw, sizeof(uint32_t) * (size_t)k, cudaMemcpyDeviceToHost, ctx.stream));
+// Cut and block weights (left in bw, their maximum returned) with one
+// synchronisation.
+long long read_cut_and_max(Ctx& ctx, const DevGraph& g, const int* part, int k, uint32_t* bw, uint32_t* max_bw) {
+    unsigned long long* c = reinterpret_cast<unsigned long long*>(ctx.dscalars + 32);
+    block_weights_and_cut(ctx, g, part, k, bw, c);
+    const size_t bytes = sizeof(uint32_t) * (size_t)k;
+    std::vector<uint32_t> big;
+    uint32_t* host = reinterpret_cast<uint32_t*>(ctx.staging(bytes));
+    if (!host) {
+        big.resize((size_t)k);
+        host = big.data();
+    }
+    KB_CUDA(cudaMemcpyAsync(host, bw, bytes, cudaMemcpyDeviceToHost, ctx.stream));
+    KB_CUDA(cudaMemcpyAsync(ctx.pinned + 32, c, sizeof(*c), cudaMemcpyDeviceToHost, ctx.stream));
     KB_CUDA(cudaStreamSynchronize(ctx.stream));
     uint32_t mx = 0;
-    for (uint32_t x : host) mx = std::max(mx, x);
-    return mx;
+    for (int b = 0; b < k; ++b) mx = std::max(mx, host[b]);
+    *max_bw = mx;
+    unsigned long long h;
+    std::memcpy(&h, ctx.pinned + 32, sizeof(h));
+    return (long long)h / 2;
 }
 
 long long read_cut(Ctx& ctx, const DevGraph& g, const int* part, int k, uint32_t* bw) {
     unsigned long long* c = reinterpret_cast<unsigned long long*>(ctx.dscalars + 32);
     block_weights_and_cut(ctx, g, part, k, bw, c);
-    unsigned long long h = 0;
-    KB_CUDA(cudaMemcpyAsync(&h, c, sizeof(h), cudaMemcpyDeviceToHost, ctx.stream));
+    KB_CUDA(cudaMemcpyAsync(ctx.pinned + 32, c, sizeof(*c), cudaMemcpyDeviceToHost, ctx.stream));
     KB_CUDA(cudaStreamSynchronize(ctx.stream));
+    unsigned long long h;
+    std::memcpy(&h, ctx.pinned + 32, sizeof(h));
     return (long long)h / 2;
 }
 
@@ -337,7 +367,6 @@ static int partition_once(Ctx& ctx, const DevGraph& g0, const Knobs& kn, int* d_
     // -------------------------------------------------------- uncoarsening
     auto t2 = clk::now();
     uint32_t* bw = ctx.hier.alloc<uint32_t>((size_t)k);
-    std::vector<uint32_t> hbw;
     bool balanced = true;
     long long final_cut = 0;
     // LP refinement: a vertex can only move if it has a neighbour in another
@@ -388,22 +417,20 @@ static int partition_once(Ctx& ctx, const DevGraph& g0, const Knobs& kn, int* d_
         }
         if (l == 0) balanced = ok;
         if (collect || l == 0) {
-            long long c = read_cut(ctx, g, lv[l].part, k, bw);
-            uint32_t mx = read_max_bw(ctx, bw, k, hbw);
+            uint32_t mx = 0;
+            const long long c = read_cut_and_max(ctx, g, lv[l].part, k, bw, &mx);
             if (l == 0) { final_cut = c; balanced = mx <= bound; }
             if (st && l < 64) { st->level_cut[l] = c; st->level_maxbw[l] = mx; }
         }
     }
     ctx.scratch.release(mkb);
+    KB_CUDA(cudaMemcpyAsync(ctx.pinned + 36, ctx.dscalars + 60, sizeof(int), cudaMemcpyDeviceToHost, s));
     KB_CUDA(cudaStreamSynchronize(s));
     if (host_part) KB_CUDA(cudaStreamSynchronize(ctx.copies()));
     double ms_uncoarsen = ms_since(t2);
 
-    {
-        int err = 0;
-        KB_CUDA(cudaMemcpy(&err, ctx.dscalars + 60, sizeof(int), cudaMemcpyDeviceToHost));
-        if (err) throw std::runtime_error("device hash table overflow (internal invariant broken)");
-    }
+    if (ctx.pinned[36])
+        throw std::runtime_error("device hash table overflow or a team of thread blocks gave up (internal)");
     *edgecut = final_cut;
     if (st) {
         st->levels = L + 1;
