@@ -73,22 +73,34 @@ __global__ void cluster_decide(SList pl, const int* hpl, const unsigned* hpc, in
     }
 }
 
-// reset = 0: no admission data was gathered (every proposal is admitted)
+// reset = 0: no admission data was gathered (every proposal is admitted).
+// The blocks take stripes as in FOR_EACH_PROPOSAL, their warps 32 proposals at
+// a time; track (optional): the moved vertices' neighbours are flagged.
 __global__ void cluster_apply(SList pl, const int* hpl, const unsigned* hpc, const int* pt, const int* vwgt,
-                              int* label, uint32_t* cw, uint32_t* inc, int* minv, int reset) {
-    FOR_EACH_PROPOSAL(pl, hpl, hpc, v) {
-        int t = pt[v];
-        if (t == -1) continue;
-        int b = t >= 0 ? t : -2 - t;
-        if (reset) {
-            inc[b] = 0;
-            minv[b] = INT_MAX;
+                              int* label, uint32_t* cw, uint32_t* inc, int* minv, int reset,
+                              const int* __restrict__ xadj, const int* __restrict__ adjncy, uint8_t* track) {
+    const unsigned s = blockIdx.x % (kStripes + 1), G = gridDim.x / (kStripes + 1);
+    const unsigned n = s < kStripes ? pl.counts[s] : *hpc;
+    const int* list = s < kStripes ? pl.data + (long long)s * pl.cap : hpl;
+    const unsigned lane = threadIdx.x & 31;
+    for (unsigned i = (blockIdx.x / (kStripes + 1)) * blockDim.x + (threadIdx.x & ~31u); i < n; i += G * blockDim.x) {
+        const int v = i + lane < n ? list[i + lane] : -1;
+        bool moved = false;
+        if (v >= 0) {
+            const int t = pt[v], b = t >= 0 ? t : -2 - t;
+            if (reset) {
+                inc[b] = 0;
+                minv[b] = INT_MAX;
+            }
+            if (t >= 0) {
+                const uint32_t cv = (uint32_t)vwgt[v];
+                atomicSub(&cw[label[v]], cv);
+                atomicAdd(&cw[t], cv);
+                label[v] = t;
+                moved = true;
+            }
         }
-        if (t < 0) continue;
-        uint32_t cv = (uint32_t)vwgt[v];
-        atomicSub(&cw[label[v]], cv);
-        atomicAdd(&cw[t], cv);
-        label[v] = t;
+        if (track) flag_neighbours(track, xadj, adjncy, moved, v);
     }
 }
 
@@ -397,6 +409,8 @@ struct ClusterArgs {
     int singletons, all_fit, admit_all, fuse;  // round 0 (SweepArgs)
     int* label;
     uint32_t* cw;
+    uint8_t* hot;        // n (SweepArgs::hot), null: not tracked
+    int track_from;      // round
     uint32_t* tie;       // singletons: n
     unsigned* counters;  // 2 kTeamSet
 };
@@ -419,6 +433,7 @@ __global__ void __launch_bounds__(kThreads, 4) cluster_team(SweepArgs a, Cluster
         a.inc[v] = 0;
         a.minv[v] = INT_MAX;
         if (C.singletons) C.tie[v] = hash32(ks_tie0, (uint32_t)v);
+        if (C.hot) C.hot[v] = 1;
     }
     if (blockIdx.x == 0)
         for (int i = threadIdx.x; i < 2 * kTeamSet; i += kThreads) C.counters[i] = 0;
@@ -432,8 +447,10 @@ __global__ void __launch_bounds__(kThreads, 4) cluster_team(SweepArgs a, Cluster
         a.all_fit = r == 0 ? C.all_fit : 0;
         a.admit_all = r == 0 ? C.admit_all : 0;
         a.fuse_apply = r == 0 ? C.fuse : 0;
+        a.hot = r > C.track_from ? C.hot : nullptr;
         for (uint32_t s = 0; alive && s < a.S; ++s, p ^= 1) {
             a.s = s;
+            a.track = r >= C.track_from && (r + 1 < C.rounds || s + 1 < a.S) ? C.hot : nullptr;
             use_set(a, C.counters, p);
             if (!(alive = team_sweep<CLUSTER, UNIT, false>(team, a, queue, S, red))) break;
             if (a.fuse_apply) continue;
@@ -447,17 +464,21 @@ __global__ void __launch_bounds__(kThreads, 4) cluster_team(SweepArgs a, Cluster
                 if (!(alive = team.sync())) break;
             }
             each_proposal(a, [&](int2&, int v, int t) {
-                if (v < 0) return;
-                const int b = t >= 0 ? t : -2 - t;
-                if (!a.admit_all) {
-                    a.inc[b] = 0;
-                    a.minv[b] = INT_MAX;
+                if (v >= 0) {
+                    const int b = t >= 0 ? t : -2 - t;
+                    if (!a.admit_all) {
+                        a.inc[b] = 0;
+                        a.minv[b] = INT_MAX;
+                    }
+                    if (t >= 0) {
+                        const uint32_t cv = (uint32_t)a.vwgt[v];
+                        atomicSub(&C.cw[C.label[v]], cv);
+                        atomicAdd(&C.cw[t], cv);
+                        C.label[v] = t;
+                    }
                 }
-                if (t < 0) return;
-                const uint32_t cv = (uint32_t)a.vwgt[v];
-                atomicSub(&C.cw[C.label[v]], cv);
-                atomicAdd(&C.cw[t], cv);
-                C.label[v] = t;
+                __syncwarp();
+                if (a.track) flag_neighbours(a.track, a.xadj, a.adjncy, v >= 0 && t >= 0, v);
             });
             alive = team.sync();
         }
@@ -616,6 +637,8 @@ bool lp_cluster_team(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, in
     C.level = level;
     C.label = label;
     C.cw = ctx.scratch.alloc<uint32_t>(n);
+    C.track_from = track_round(g, C.rounds);
+    C.hot = C.rounds > C.track_from ? ctx.scratch.alloc<uint8_t>(n) : nullptr;
     C.tie = ctx.scratch.alloc<uint32_t>(n);
     a.lab = label;
     a.lw = C.cw;
@@ -711,7 +734,11 @@ void lp_cluster(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, int* la
     a.S = (uint32_t)kn.lpc_subrounds;
     a.inc = inc;
     a.minv = minv;
+    const int first = track_round(g, kn.lpc_rounds);
+    uint8_t* hot = kn.lpc_rounds > first ? ctx.scratch.alloc<uint8_t>(n) : nullptr;
+    if (hot) fill_u8(hot, g.n, 1, st);
     for (int r = 0; r < kn.lpc_rounds; ++r) {
+        a.hot = r > first ? hot : nullptr;
         a.ks_sub = stream_key(kn.seed, TAG_CSUB, level, r);
         a.ks_tie = stream_key(kn.seed, TAG_CTIE, level, r);
         // round 0 is one fully synchronous sub-round (every cluster is still a
@@ -744,7 +771,10 @@ void lp_cluster(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, int* la
         a.cw_w = cw;
         for (uint32_t s = 0; s < a.S; ++s) {
             a.s = s;
-            launch_sweep<CLUSTER>(ctx, g, a, b, sweep_bytes(g, 1.0 / a.S));
+            // (nothing looks at the flags after the last sub-round)
+            a.track = r >= first && (r + 1 < kn.lpc_rounds || s + 1 < a.S) ? hot : nullptr;
+            // (a sweep of the flagged vertices: the flags are all it surely reads)
+            launch_sweep<CLUSTER>(ctx, g, a, b, a.hot ? 1.0 * g.n / a.S : sweep_bytes(g, 1.0 / a.S));
             if (a.fuse_apply) continue;
             PhaseScope ps(ctx, "lp_cluster_admit", 0);
             if (!a.admit_all) {
@@ -753,7 +783,8 @@ void lp_cluster(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, int* la
                 KB_LAUNCH();
             }
             cluster_apply<<<admit_blocks(), kThreads, 0, st>>>(b.plist, b.hplist, a.hpcount, b.pt, g.vwgt, label, cw,
-                                                               inc, minv, a.admit_all ? 0 : 1);
+                                                               inc, minv, a.admit_all ? 0 : 1, g.xadj, g.adjncy,
+                                                               a.track);
             KB_LAUNCH();
         }
     }

@@ -84,6 +84,14 @@ struct SweepArgs {
     int fuse_apply;                     // singletons + all_fit + admit_all, no row above kWin:
                                         // moves are applied in the sweep (nothing reads labels
                                         // or cluster weights of others in that round)
+    // CLUSTER: vertices that must be looked at again.  A vertex is quiet when
+    // no other cluster has more of its weight than its own, whatever their
+    // sizes; it then stays until a neighbour moves (ties, cluster weights and
+    // bounds cannot change that), so a sweep may pass it over with the same
+    // result.  hot: sweep the flagged only (null: all); track: clear the flag
+    // of the quiet, set those of a moved vertex's neighbours
+    const uint8_t* hot;
+    uint8_t* track;
     int* label_w;                       // fuse_apply: labels, written by their own vertex
     uint32_t* cw_w;                     // fuse_apply: cluster weights
     int stash;                          // host: sweep with lane_vertex's label stash
@@ -228,6 +236,8 @@ template <int MODE>
 __device__ __forceinline__ bool member(const SweepArgs& a, int v) {
     if (MODE == BALANCE) return a.lw[a.lab[v]] > a.bound;
     if (MODE == REFINE && a.active && !a.active[v]) return false;
+    if (MODE == CLUSTER && a.hot)
+        return hash_range(hash32(a.ks_sub, (uint32_t)v), a.S) == a.s && a.hot[v];
     return hash_range(hash32(a.ks_sub, (uint32_t)v), a.S) == a.s;
 }
 
@@ -611,6 +621,12 @@ __device__ __forceinline__ int lane_vertex(const SweepArgs& a, int v, uint32_t* 
     if (overflow) return 1;
     wv += 1;
     we += (unsigned)(end - beg);
+    if (MODE == CLUSTER && a.track) {
+        uint32_t most = 0;
+#pragma unroll
+        for (int i = 0; i < NS; ++i) most = max(most, sc[i]);
+        if (most <= cown) a.track[v] = 0;
+    }
     // best candidate: largest connection, ties by smaller tie hash, then
     // smaller label; hashes are computed only for ties
     uint32_t ok[NS];
@@ -921,17 +937,22 @@ __device__ __forceinline__ void hash_vertex(const SweepArgs& a, int v, uint32_t*
     }
     __syncwarp();
     uint64_t key = 0;
-    uint32_t id = kEmpty;
+    uint32_t id = kEmpty, most = 0;
     for (int s = lane; s < cap; s += 32) {
         const uint32_t l = tk[s];
         if (l == kEmpty) continue;
         const uint32_t c = tv[s];
         tk[s] = kEmpty;
         tv[s] = 0;
+        most = max(most, c);
         if (cand_ok<MODE>(a, l, c, cv)) better(key, id, cand_key(c, a.ks_tie, l), l);
     }
     group_argmax<32>(key, id, 0xffffffffu);
     co = __reduce_add_sync(0xffffffffu, co);
+    if (MODE == CLUSTER) {
+        most = __reduce_max_sync(0xffffffffu, most);
+        if (lane == 0 && a.track && most <= co) a.track[v] = 0;
+    }
     if (lane == 0) {
         wv += 1;
         we += (unsigned)(end - beg);
@@ -1005,6 +1026,59 @@ __device__ __forceinline__ void mark_row(const NextActive& na, const int* adjncy
             }
         }
     }
+}
+
+// flags[target] = 1 for the entries [beg, end) by the threads t of nt.
+__device__ __forceinline__ void flag_row(uint8_t* flags, const int* adjncy, int beg, int end, int t, int nt) {
+    int e = beg + t;
+    for (; e + 3 * nt < end; e += 4 * nt) {
+        const int u0 = adjncy[e], u1 = adjncy[e + nt], u2 = adjncy[e + 2 * nt], u3 = adjncy[e + 3 * nt];
+        flags[u0] = 1;
+        flags[u1] = 1;
+        flags[u2] = 1;
+        flags[u3] = 1;
+    }
+    for (; e < end; e += nt) flags[adjncy[e]] = 1;
+}
+
+// Flags the neighbours of the lanes' moved vertices: a lane its own short row,
+// the warp the long ones.  All lanes call it (moved: the lane's vertex v).
+__device__ __forceinline__ void flag_neighbours(uint8_t* flags, const int* xadj, const int* adjncy, bool moved,
+                                                int v) {
+    const int lane = threadIdx.x & 31;
+    int e0 = 0, e1 = 0;
+    if (moved) {
+        e0 = xadj[v];
+        e1 = xadj[v + 1];
+        if (e1 - e0 <= kHubMark) flag_row(flags, adjncy, e0, e1, 0, 1);
+    }
+    unsigned wm = __ballot_sync(0xffffffffu, e1 - e0 > kHubMark);
+    while (wm) {
+        const int src = __ffs(wm) - 1;
+        wm &= wm - 1;
+        const int b = __shfl_sync(0xffffffffu, e0, src), d = __shfl_sync(0xffffffffu, e1, src);
+        flag_row(flags, adjncy, b, d, lane, 32);
+    }
+}
+
+// The first clustering round (of those after round 0) that tracks the quiet,
+// the number of rounds if none is to.  What tracking costs is the marking of
+// the moved vertices' neighbours, and the more rounds follow, the more sweeps
+// it shortens.  Unit-weight meshes (mean degree above 8, the input level of
+// most runs): in round 1 so many vertices move that hardly one has no moved
+// neighbour, so from round 2 on.  2^24-node geometric graph, 5 rounds: sweeps
+// of rounds 3 and 4 0.60 and 0.57 -> 0.44 and 0.30 ms a sub-round, admission
+// 0.05 more, coarsening 10.8 -> 10.4 ms.  Coarser levels and thin graphs: from
+// round 1 on if there are many rounds (4M nodes, 10 rounds: coarsening 5.24 ->
+// 4.29 ms), else not at all (5 rounds on the levels of a 3M-node 3D mesh: 3.18
+// -> 3.23 ms).  Rows of many entries: not at all, a moved hub marks them all
+// (R-MAT 2^20 from round 1 on: 33 -> 47 ms).
+constexpr int kTrackDegree = 256, kTrackRounds = 8;
+inline int track_round(const DevGraph& g, int rounds) {
+    if (g.maxdeg > kTrackDegree) return rounds;
+    const bool mesh = g.unit_weights && g.m > 8LL * g.n;
+    const int first = mesh ? 2 : 1;
+    return first + 1 < rounds && (mesh || rounds >= kTrackRounds) ? first : rounds;
 }
 
 // -------------------------------------------------------------- team forms

@@ -144,6 +144,22 @@ def test_cluster_hubs(N, O, hub):
         assert np.array_equal(O.lp_cluster(g, kn_o, 0), N.lp_cluster(g, kn_p, 0))
 
 
+@pytest.mark.parametrize("n,hub", [(3000, 0), (3000, 256), (3000, 257), (140000, 0), (140000, 256)])
+@pytest.mark.parametrize("rounds", [1, 2, 3, 4, 5, 7, 8, 12])
+def test_cluster_quiet_rounds(N, O, graphs, n, hub, rounds):
+    """Around the first round that passes over vertices that cannot move, with
+    and without a row too long for it, as a team and as launches."""
+    g = hub_graph(n, hub, hub) if hub else graphs.rgg2d(n, seed=n)
+    for unit in (True, False):
+        if not unit:
+            weighted(g, hub + 1)
+        kn_o, kn_p = O.knobs(g, 4, 0.03, 3, 1), N.derive_knobs(g["n"], g["vwgt"], 4, 0.03, 3, 1)
+        kn_o.lpc_rounds = kn_p.lpc_rounds = rounds
+        for bound in (kn_p.cluster_bound, 9):  # 9: weights near the bound decide
+            kn_o.cluster_bound = kn_p.cluster_bound = bound
+            assert np.array_equal(O.lp_cluster(g, kn_o, 1), N.lp_cluster(g, kn_p, 1))
+
+
 def test_cluster_unsorted_rows(N, O, graphs):
     """Rows in no order and a target listed twice: no singleton shortcut."""
     g = graphs.rgg2d(3000, seed=4)
