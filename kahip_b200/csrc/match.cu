@@ -15,23 +15,27 @@
 // eligible edge left adds a pair; the result depends only on the graph, the
 // ratings and the stream key.
 //
+// A proposal stands while its target is unmatched: the eligible set only
+// shrinks, so its largest key stays the largest.  A later round reads the rows
+// of those vertices only whose target was taken.
+//
 // Layout: state[v] >= 0 is v's weight while unmatched, -1 matched, -2
-// retired; best[v] the proposal of this round; mate[v] the partner or -1;
-// cnt[r] the pairs formed in round r (a round after one with no new pair
-// exits at once, so the host never waits between rounds).
+// retired; best[v] the proposal; mate[v] the partner or -1; cnt[r] the pairs
+// formed in round r (a round with no new pair is the last).
 #include "match.cuh"
 
 #include "common.cuh"
+#include "team.cuh"
 
 namespace kb {
 
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = kTeamThreads, kWarps = kThreads / 32;
 constexpr int kLaneDeg = 32;  // rows longer than this are scanned by the whole warp
 
 struct MatchArgs {
-    int n;
+    int n, rounds;
     const int* xadj;
     const int* adjncy;
     const int* adjwgt;
@@ -39,6 +43,10 @@ struct MatchArgs {
     int* state;
     int* best;
     int* mate;
+    int* list;  // the warps' unmatched vertices, each warp's where its own begin
+    int* todo;  // those of them that look for a new target
+    int* label;
+    const int* vwgt;
     unsigned* cnt;
     uint64_t ks;
     uint32_t maxvw;
@@ -46,10 +54,11 @@ struct MatchArgs {
 
 // Primary key: IEEE bits of 1.0*w*w / (uint32)(c(u)*c(v)) (order-preserving
 // for non-negative doubles; 0/0 counts as 0), or the supplied rating.
+// x is the entry's weight (unused where all are 1) or its rating.
 template <bool UNIT, bool ARRAY>
-__device__ __forceinline__ uint64_t primary(const MatchArgs& A, int e, uint32_t cv, uint32_t cu) {
-    if (ARRAY) return (uint64_t)__ldg(A.rq + e);
-    const int w = UNIT ? 1 : __ldg(A.adjwgt + e);
+__device__ __forceinline__ uint64_t primary(uint32_t x, uint32_t cv, uint32_t cu) {
+    if (ARRAY) return (uint64_t)x;
+    const int w = UNIT ? 1 : (int)x;
     double r = 1.0 * w * w / (double)(uint32_t)(cu * cv);
     if (r != r) r = 0.0;
     return (uint64_t)__double_as_longlong(r);
@@ -61,129 +70,198 @@ __device__ __forceinline__ uint64_t secondary(uint64_t ks, uint32_t a, uint32_t 
     return ((uint64_t)h << 32) | (uint32_t)~(lo + hi);
 }
 
+// The entry with the largest key so far; the secondary keys are computed for
+// equal primaries only.
 struct Best {
     int u = -1;
     uint64_t k1 = 0, k2 = 0;
-    __device__ __forceinline__ void offer(int cu, uint64_t a, uint64_t b) {
-        if (u < 0 || a > k1 || (a == k1 && b > k2)) {
+    bool has2 = false;
+    __device__ __forceinline__ void offer(uint64_t ks, int v, int cu, uint64_t a) {
+        if (u < 0 || a > k1) {
             u = cu;
             k1 = a;
-            k2 = b;
+            has2 = false;
+        } else if (a == k1) {
+            settle(ks, v);
+            const uint64_t b = secondary(ks, (uint32_t)v, (uint32_t)cu);
+            if (b > k2) {
+                u = cu;
+                k2 = b;
+            }
         }
+    }
+    __device__ __forceinline__ void settle(uint64_t ks, int v) {
+        if (!has2 && u >= 0) k2 = secondary(ks, (uint32_t)v, (uint32_t)u);
+        has2 = true;
     }
 };
 
+// The entries e, e + step, .. (entries() of them) below end of v's row, their
+// reads issued together.  Eight where the keys are the supplied ratings (1M
+// nodes, 16 rounds: 728 -> 531 us against four with a scalar tail); computing
+// them from the weights leaves registers for four.
+template <bool ARRAY>
+__host__ __device__ constexpr int entries() {
+    return ARRAY ? 8 : 4;
+}
 template <bool UNIT, bool ARRAY>
-__device__ __forceinline__ void consider(const MatchArgs& A, int v, uint32_t cv, int e, int u, int su, Best& b) {
-    if (u == v || su < 0) return;
-    if ((uint64_t)cv + (uint32_t)su > A.maxvw) return;
-    b.offer(u, primary<UNIT, ARRAY>(A, e, cv, (uint32_t)su), secondary(A.ks, (uint32_t)v, (uint32_t)u));
+__device__ __forceinline__ void consider(const MatchArgs& A, int v, uint32_t cv, int e, int step, int end, Best& b) {
+    constexpr int kEntries = entries<ARRAY>();
+    int u[kEntries], su[kEntries];
+    uint32_t x[kEntries];
+#pragma unroll
+    for (int j = 0; j < kEntries; ++j) {
+        const int at = e + j * step;
+        u[j] = at < end ? __ldg(A.adjncy + at) : v;
+        x[j] = UNIT || at >= end ? 0u : ARRAY ? __ldg(A.rq + at) : (uint32_t)__ldg(A.adjwgt + at);
+    }
+#pragma unroll
+    for (int j = 0; j < kEntries; ++j) su[j] = A.state[u[j]];
+#pragma unroll
+    for (int j = 0; j < kEntries; ++j) {
+        if (u[j] == v || su[j] < 0 || (uint64_t)cv + (uint32_t)su[j] > A.maxvw) continue;
+        b.offer(A.ks, v, u[j], primary<UNIT, ARRAY>(x[j], cv, (uint32_t)su[j]));
+    }
 }
 
+// The proposal of the lane's vertex v (weight sv) where scan is set: a lane
+// per row, the warp for rows above kLaneDeg.  All lanes call it.
 template <bool UNIT, bool ARRAY>
-__global__ void __launch_bounds__(kThreads) match_propose(MatchArgs A, int r) {
-    if (r > 0 && A.cnt[r - 1] == 0) return;
+__device__ __forceinline__ int propose(const MatchArgs& A, bool scan, int v, int sv) {
     const int lane = threadIdx.x & 31;
-    const long long nwarps = (long long)gridDim.x * (kThreads / 32);
-    for (long long base = ((long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * 32; base < A.n;
-         base += nwarps * 32) {
-        const int v = (int)base + lane;
-        int sv = -1, beg = 0, end = 0;
-        if (v < A.n) {
-            sv = A.state[v];
-            if (sv >= 0) {
-                beg = __ldg(A.xadj + v);
-                end = __ldg(A.xadj + v + 1);
+    const int beg = scan ? __ldg(A.xadj + v) : 0, end = scan ? __ldg(A.xadj + v + 1) : 0;
+    const bool heavy = end - beg > kLaneDeg;
+    Best b;
+    if (!heavy)
+        for (int e = beg; e < end; e += entries<ARRAY>()) consider<UNIT, ARRAY>(A, v, (uint32_t)sv, e, 1, end, b);
+    unsigned hm = __ballot_sync(0xffffffffu, heavy);
+    while (hm) {
+        const int src = __ffs(hm) - 1;
+        hm &= hm - 1;
+        const int hv = __shfl_sync(0xffffffffu, v, src);
+        const int hb = __shfl_sync(0xffffffffu, beg, src);
+        const int he = __shfl_sync(0xffffffffu, end, src);
+        const uint32_t hs = (uint32_t)__shfl_sync(0xffffffffu, sv, src);
+        Best c;
+        for (int e = hb + lane; e < he; e += 32 * entries<ARRAY>()) consider<UNIT, ARRAY>(A, hv, hs, e, 32, he, c);
+        // warp arg-max; keys of distinct neighbours differ, so the
+        // winner does not depend on the reduction order
+        c.settle(A.ks, hv);
+#pragma unroll
+        for (int off = 16; off; off >>= 1) {
+            const int ou = __shfl_xor_sync(0xffffffffu, c.u, off);
+            const uint64_t o1 = __shfl_xor_sync(0xffffffffu, c.k1, off);
+            const uint64_t o2 = __shfl_xor_sync(0xffffffffu, c.k2, off);
+            if (ou >= 0 && (c.u < 0 || o1 > c.k1 || (o1 == c.k1 && o2 > c.k2))) {
+                c.u = ou;
+                c.k1 = o1;
+                c.k2 = o2;
             }
         }
-        const bool heavy = sv >= 0 && end - beg > kLaneDeg;
-        Best b;
-        if (sv >= 0 && !heavy) {
-            // four entries per step, their loads issued together
-            int e = beg;
-            for (; e + 4 <= end; e += 4) {
-                int u[4], su[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) u[j] = __ldg(A.adjncy + e + j);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) su[j] = A.state[u[j]];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) consider<UNIT, ARRAY>(A, v, (uint32_t)sv, e + j, u[j], su[j], b);
-            }
-            for (; e < end; ++e) {
-                const int u = __ldg(A.adjncy + e);
-                consider<UNIT, ARRAY>(A, v, (uint32_t)sv, e, u, A.state[u], b);
-            }
-        }
-        unsigned hm = __ballot_sync(0xffffffffu, heavy);
-        while (hm) {
-            const int src = __ffs(hm) - 1;
-            hm &= hm - 1;
-            const int hv = __shfl_sync(0xffffffffu, v, src);
-            const int hb = __shfl_sync(0xffffffffu, beg, src);
-            const int he = __shfl_sync(0xffffffffu, end, src);
-            const uint32_t hs = (uint32_t)__shfl_sync(0xffffffffu, sv, src);
-            Best c;
-            for (int e = hb + lane; e < he; e += 32) {
-                const int u = __ldg(A.adjncy + e);
-                consider<UNIT, ARRAY>(A, hv, hs, e, u, A.state[u], c);
-            }
-            // warp arg-max; keys of distinct neighbours differ, so the
-            // winner does not depend on the reduction order
-#pragma unroll
-            for (int off = 16; off; off >>= 1) {
-                const int ou = __shfl_xor_sync(0xffffffffu, c.u, off);
-                const uint64_t o1 = __shfl_xor_sync(0xffffffffu, c.k1, off);
-                const uint64_t o2 = __shfl_xor_sync(0xffffffffu, c.k2, off);
-                if (ou >= 0) c.offer(ou, o1, o2);
-            }
-            if (lane == src) b = c;
-        }
-        if (sv >= 0) A.best[v] = b.u;
+        if (lane == src) b = c;
     }
+    return b.u;
 }
 
-__global__ void __launch_bounds__(kThreads) match_commit(MatchArgs A, int r) {
-    if (r > 0 && A.cnt[r - 1] == 0) return;
-    unsigned pairs = 0;
-    for (long long v = (long long)blockIdx.x * kThreads + threadIdx.x; v < A.n; v += (long long)gridDim.x * kThreads) {
-        if (A.state[v] < 0) continue;
-        const int b = A.best[v];
-        if (b >= 0 && A.best[b] == (int)v) {
-            A.mate[v] = b;
-            A.state[v] = -1;
-            pairs += (int)v < b;
-        } else if (b < 0) {
-            A.state[v] = -2;
-        }
-    }
-    // warp-aggregated count of the pairs formed
-#pragma unroll
-    for (int off = 16; off; off >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, off);
-    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(A.cnt + r, pairs);
+// Adds the lanes' v where take is set to the warp's list of n.
+__device__ __forceinline__ void append(int* list, int& n, bool take, int v) {
+    const unsigned m = __ballot_sync(0xffffffffu, take);
+    if (take) list[n + __popc(m & ((1u << (threadIdx.x & 31)) - 1))] = v;
+    n += __popc(m);
 }
 
-__global__ void match_init(int n, const int* vwgt, int* state, int* mate) {
-    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
-        state[v] = vwgt[v];
-        mate[v] = -1;
-    }
-}
+constexpr int kBatch = 4;  // vertices a lane has reads in flight for
 
-__global__ void match_label(int n, const int* mate, int* label) {
-    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
-        const int m = mate[v];
-        label[v] = (m >= 0 && m < (int)v) ? m : (int)v;
-    }
-}
-
-int grid_for(long long items) {
-    return (int)std::max<long long>(1, std::min<long long>(div_up(items, kThreads), (long long)kNumSMs * 8));
-}
-
+// All rounds and the labels in one kernel, two barriers a round.  Bound by the
+// first round's gathers of the neighbours' states; later rounds by the chain
+// of reads per vertex.  Every warp keeps a run of consecutive vertices (their
+// rows share lines) and lists those still unmatched.  As two launches a round
+// over all vertices with every unmatched row read again, 16 rounds on a 2D
+// geometric graph of 1M nodes took 1.09 ms, the 11 levels of its hierarchy
+// 2.68 ms of GPU time and 387 launches; now 0.53 and 1.31 ms and 11.
 template <bool UNIT, bool ARRAY>
-void launch_propose(const MatchArgs& A, int r, int grid, cudaStream_t s) {
-    match_propose<UNIT, ARRAY><<<grid, kThreads, 0, s>>>(A, r);
+__global__ void __launch_bounds__(kThreads, 4) match_team(MatchArgs A, TeamArgs T) {
+    __shared__ unsigned pairs;
+    Team team(T);
+    const int lane = threadIdx.x & 31;
+    const long long warps = (long long)gridDim.x * kWarps, w = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
+    const long long share = ((A.n + warps - 1) / warps + 31) & ~31ll;
+    const int first = (int)min((long long)A.n, w * share), own = (int)min((long long)A.n - first, share);
+    for (int i = lane; i < own; i += 32) {
+        A.state[first + i] = A.vwgt[first + i];
+        A.mate[first + i] = -1;
+    }
+    if (team.leader())
+        for (int r = 0; r < A.rounds; ++r) A.cnt[r] = 0;
+    if (threadIdx.x == 0) pairs = 0;
+    bool alive = team.sync();
+    int *list = A.list + first, *todo = A.todo + first;
+    int left = own;
+    for (int r = 0; alive && r < A.rounds; ++r) {
+        int looking = left;
+        if (r > 0) {
+            looking = 0;
+            for (int i = lane; i - lane < left; i += 32 * kBatch) {
+                int v[kBatch], b[kBatch];
+#pragma unroll
+                for (int q = 0; q < kBatch; ++q) v[q] = i + 32 * q < left ? list[i + 32 * q] : -1;
+#pragma unroll
+                for (int q = 0; q < kBatch; ++q) b[q] = v[q] >= 0 ? A.best[v[q]] : 0;
+#pragma unroll
+                for (int q = 0; q < kBatch; ++q) b[q] = A.state[b[q]];
+#pragma unroll
+                for (int q = 0; q < kBatch; ++q) append(todo, looking, v[q] >= 0 && b[q] < 0, v[q]);
+            }
+            __syncwarp();
+        }
+        for (int i = lane; i - lane < looking; i += 32) {
+            const bool in = i < looking;
+            const int v = !in ? -1 : r == 0 ? first + i : todo[i];
+            const int b = propose<UNIT, ARRAY>(A, in, v, in ? A.state[v] : 0);
+            if (in) A.best[v] = b;
+        }
+        if (!(alive = team.sync())) break;
+        unsigned formed = 0;
+        int kept = 0;
+        for (int i = lane; i - lane < left; i += 32 * kBatch) {
+            int v[kBatch], b[kBatch], o[kBatch];
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) v[q] = i + 32 * q >= left ? -1 : r == 0 ? first + i + 32 * q : list[i + 32 * q];
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) b[q] = v[q] >= 0 ? A.best[v[q]] : -1;
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) o[q] = b[q] >= 0 ? A.best[b[q]] : -1;
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) {
+                const bool mutual = b[q] >= 0 && o[q] == v[q];
+                if (mutual) {
+                    A.mate[v[q]] = b[q];
+                    A.state[v[q]] = -1;
+                    formed += v[q] < b[q];
+                } else if (v[q] >= 0 && b[q] < 0) {
+                    A.state[v[q]] = -2;
+                }
+                append(list, kept, b[q] >= 0 && !mutual, v[q]);
+            }
+        }
+        left = kept;
+        __syncwarp();
+        formed = __reduce_add_sync(0xffffffffu, formed);
+        if (lane == 0 && formed) atomicAdd(&pairs, formed);
+        __syncthreads();
+        if (threadIdx.x == 0 && pairs) {
+            atomicAdd(A.cnt + r, pairs);
+            pairs = 0;
+        }
+        if (!(alive = team.sync())) break;
+        if (*(volatile unsigned*)(A.cnt + r) == 0) break;
+    }
+    if (alive)
+        for (int i = lane; i < own; i += 32) {
+            const int v = first + i, m = A.mate[v];
+            A.label[v] = (m >= 0 && m < v) ? m : v;
+        }
+    team.leave();
 }
 
 }  // namespace
@@ -199,35 +277,30 @@ void hem_match(Ctx& ctx, const DevGraph& g, const Knobs& kn, int level, const ui
     A.adjncy = g.adjncy;
     A.adjwgt = g.adjwgt;
     A.rq = rating_q;
+    A.rounds = R;
+    A.vwgt = g.vwgt;
+    A.label = label;
     A.state = ctx.scratch.alloc<int>((size_t)g.n);
     A.best = ctx.scratch.alloc<int>((size_t)g.n);
     A.mate = ctx.scratch.alloc<int>((size_t)g.n);
+    A.list = ctx.scratch.alloc<int>((size_t)g.n);
+    A.todo = ctx.scratch.alloc<int>((size_t)g.n);
     A.cnt = ctx.scratch.alloc<unsigned>((size_t)std::max(R, 1));
     A.ks = stream_key(kn.seed, TAG_MATCH, level, 0);
     A.maxvw = kn.max_vertex_weight;
-    const int grid = grid_for(g.n);
-    KB_CUDA(cudaMemsetAsync(A.cnt, 0, sizeof(unsigned) * (size_t)std::max(R, 1), s));
-    match_init<<<grid, kThreads, 0, s>>>(g.n, g.vwgt, A.state, A.mate);
-    KB_LAUNCH();
-    // round 0 scans every row: its algorithmic bytes are exact (per vertex
+    auto kernel = rating_q ? match_team<false, true> : g.unit_weights ? match_team<true, false> : match_team<false, false>;
+    const TeamRoom room = team_room(ctx, (const void*)kernel, 0);
+    // a vertex a thread, and with long rows one warp to 1024 entries
+    const int blocks = team_blocks(room, std::max<long long>(div_up(g.n, kThreads), g.m / (1024 * kWarps)));
+    // round 0 reads every row: its algorithmic bytes are exact (per vertex
     // state, xadj, proposal write; per entry adjncy, state gather, plus the
-    // weight or supplied rating); later rounds scan only unmatched rows
+    // weight or supplied rating); what later rounds read depends on the graph
     const double row_bytes = 4.0 * ((g.unit_weights && !rating_q) ? 2 : 3) * (double)g.m;
-    const double round0_bytes = row_bytes + 12.0 * (double)g.n;
-    for (int r = 0; r < R; ++r) {
-        {
-            PhaseScope ps(ctx, r == 0 ? "match_sweep0" : "match_sweep", r == 0 ? round0_bytes : 0.0);
-            if (rating_q) launch_propose<false, true>(A, r, grid, s);
-            else if (g.unit_weights) launch_propose<true, false>(A, r, grid, s);
-            else launch_propose<false, false>(A, r, grid, s);
-            KB_LAUNCH();
-        }
-        PhaseScope ps(ctx, "match_commit", 0);
-        match_commit<<<grid, kThreads, 0, s>>>(A, r);
-        KB_LAUNCH();
+    {
+        PhaseScope ps(ctx, "match_team", row_bytes + 12.0 * (double)g.n);
+        // (a device that cannot hold the grid now can hold one cluster later)
+        if (!launch_team(ctx, kernel, room, blocks, 0, A)) launch_team(ctx, kernel, room, team_blocks(room, 8), 0, A);
     }
-    match_label<<<grid, kThreads, 0, s>>>(g.n, A.mate, label);
-    KB_LAUNCH();
     ctx.scratch.release(mk);
 }
 

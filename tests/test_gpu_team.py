@@ -201,3 +201,22 @@ def test_initial_partition_gangs(N, O, graphs, n, k):
         for mode in (0, 1):
             kn_o, kn_p = O.knobs(g, k, 0.03, 5, mode), N.derive_knobs(g["n"], g["vwgt"], k, 0.03, 5, mode)
             assert np.array_equal(O.initial_partition_batched(g, kn_o), N.initial_partition_device(g, kn_p))
+
+
+@pytest.mark.parametrize("n,hub", [(1, 0), (33, 0), (256, 0), (257, 0), (2049, 0), (4097, 0), (40001, 0), (160000, 0),
+                                   (5000, 32), (5000, 33), (5000, 128), (5000, 1025)])
+def test_match_sizes(N, O, graphs, n, hub):
+    """Teams of every form, rows of every batch remainder, and the reuse of
+    proposals over the rounds, for unit weights, weights and ratings with ties."""
+    g = hub_graph(n, hub, hub) if hub else graphs.rgg2d(n, seed=n) if n > 33 else \
+        csr_from_edges(n, [(i, i + 1) for i in range(n - 1)])
+    for unit in (True, False):
+        if not unit:
+            weighted(g, n + hub)
+        src = np.repeat(np.arange(n), np.diff(g["xadj"])).astype(np.int64)
+        rating = ((src + g["adjncy"]) * 7919 % 13).astype(np.uint32)  # symmetric, many equal
+        for rounds in (1, 2, 16):
+            kn_o, kn_p = O.knobs(g, 2, 0.03, 9, 0), N.derive_knobs(n, g["vwgt"], 2, 0.03, 9, 0)
+            kn_o.match_rounds = kn_p.match_rounds = rounds
+            for rq in (None, rating):
+                assert np.array_equal(O.hem_match(g, kn_o, 1, rq), N.hem_match(g, kn_p, 1, rq))
