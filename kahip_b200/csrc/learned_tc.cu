@@ -2,24 +2,32 @@
 // on the 5th-generation tensor cores (tcgen05), fused with the neighbour
 // gather that feeds them.
 //
-// One CTA = two warpgroups (8 warps) holding NOUT columns of TMEM (the
-// 128 x NOUT FP32 accumulator of one tile).  Per tile of 128 nodes:
-//   1. the warps gather the tile's A operand into shared memory: row r =
-//      [h(v) | weighted mean of h over N(v)] (BF16; sums in FP32), written
-//      in the no-swizzle K-major core-matrix layout (8 rows x 16 bytes per
-//      core matrix, contiguous);
-//   2. one thread issues K/16 tcgen05.mma (M=128, N=NOUT, K=16, BF16 in,
+// One CTA an SM: 28 warps gather, four issue the MMAs and read the results
+// from 64 columns of TMEM (the 128 x 64 FP32 accumulator of one tile).  Per
+// tile of 128 nodes:
+//   1. the gathering warps put the tile's A operand into one of three stages
+//      in shared memory: row r = [h(v) | weighted mean of h over N(v)] (BF16;
+//      sums in FP32), in the no-swizzle K-major core-matrix layout (8 rows x
+//      16 bytes per core matrix, contiguous), four rows a warp at a time, and
+//      arrive at the stage's mbarrier;
+//   2. one thread issues K/16 tcgen05.mma (M=128, N=64, K=16, BF16 in,
 //      FP32 accumulate in TMEM) reading A and the layer's weights (B, loaded
 //      once per CTA in the same layout) from shared memory, then
 //      tcgen05.commit to an mbarrier;
-//   3. every warp waits on the mbarrier (bounded), reads 32 TMEM lanes
-//      (= 32 rows; warp w accesses lanes 32 (w % 4) ..) and half of the
-//      columns with tcgen05.ld, adds the bias, applies ReLU, rounds to BF16
-//      and stores its part of the rows.
-// The gather (HBM/L2-bound) dominates; the MMAs take a few hundred cycles
-// per tile.  Descriptor bit layouts follow the PTX ISA's tcgen05 matrix and
-// instruction descriptors (as spelled out in CUTLASS's
-// cute/arch/mma_sm100_desc.hpp).
+//   3. the reading warps wait on it (every wait is bounded), read their 32
+//      TMEM lanes (= 32 rows) with tcgen05.ld, add the bias, apply ReLU, round
+//      to BF16 and store the rows.
+// In the last layer step 3 writes the rows back as an A operand, and a second
+// MMA with Wz gives the 32 outputs z of the tile: h3 never leaves the SM.
+//
+// The gather dominates (the MMAs take a few hundred cycles per tile), by the
+// latency of its chain of reads and about as many issue slots; neither the
+// hit rate of L1 (16 to 32 warps a CTA, 1 to 4 CTAs an SM: 340-360 us) nor
+// prefetches into L2 nor the stores' bank conflicts move it by more than 3 %.
+// Gathering ahead of the MMAs does: 1M nodes, 13.1M entries, a layer 340 ->
+// 319 us, the last one with z 407 -> 290 us.
+// Descriptor bit layouts follow the PTX ISA's tcgen05 matrix and instruction
+// descriptors (as spelled out in CUTLASS's cute/arch/mma_sm100_desc.hpp).
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -36,17 +44,20 @@ void launch_head_bf16(Ctx& ctx, const DevGraph& g, const float* P, const __nv_bf
 namespace {
 
 constexpr int kTile = 128;               // nodes per tile = MMA M
-constexpr int kTcThreads = 256;          // two warpgroups: all gather, both read TMEM
-constexpr int kGatherRows = kTile / (kTcThreads / 32);  // rows gathered per warp
-constexpr long long kWaitLimit = 1 << 24;  // mbarrier polls before giving up
+constexpr int kTcThreads = 1024;         // a CTA an SM
+constexpr int kReadWarps = 4;            // issue the MMAs and read TMEM; the others gather
+constexpr int kStages = 3;               // A operands
+constexpr int kWaitLimit = 1 << 24;  // mbarrier polls before giving up
 
-// byte offset of element (r, c) of a K-major operand with `rows` rows in the
-// no-swizzle core-matrix layout: core matrices of 8 rows x 8 BF16 (128 B,
-// row-major inside); consecutive row groups 128 B apart (SBO), consecutive
-// K groups rows*16 B apart (LBO)
-__host__ __device__ constexpr uint32_t core_off(int r, int c, int rows) {
-    return (uint32_t)((c >> 3) * (rows * 16) + (r >> 3) * 128 + (r & 7) * 16 + (c & 7) * 2);
+// byte offset of element (r, c) of a K-major operand in the no-swizzle
+// core-matrix layout: core matrices of 8 rows x 8 BF16 (128 B, row-major
+// inside); consecutive row groups 128 B apart (SBO), consecutive K groups lbo
+// bytes (LBO): rows * 16 in B, 16 more in A, whose rows are written eight
+// K groups at a time, which would all fall on the same banks
+__host__ __device__ constexpr uint32_t core_off(int r, int c, int lbo) {
+    return (uint32_t)((c >> 3) * lbo + (r >> 3) * 128 + (r & 7) * 16 + (c & 7) * 2);
 }
+constexpr int kLboA = kTile * 16 + 16;
 
 // shared-memory matrix descriptor: start >> 4 [0,14), LBO >> 4 [16,30),
 // SBO >> 4 [32,46), version 1 [46,48), base offset 0, no swizzle [61,64) = 0
@@ -66,12 +77,14 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-// Weights of one layer, BF16, in the B-operand layout (NOUT rows x K).
-template <int K, int NOUT>
-__global__ void pack_weights(const float* P, int woff, __nv_bfloat16* out) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NOUT * K; i += gridDim.x * blockDim.x) {
-        const int j = i / K, c = i % K;
-        out[core_off(j, c, NOUT) / 2] = __float2bfloat16(P[woff + i]);
+// The layers' weights, BF16, in the B-operand layout (rows x K): three of 64
+// rows x 128, then Wz, 32 x 64.
+constexpr int kPackLayer = rm::H * 2 * rm::H, kPackAll = 3 * kPackLayer + rm::Z * rm::H;
+__global__ void pack_weights(const float* P, __nv_bfloat16* out) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kPackAll; i += gridDim.x * blockDim.x) {
+        const int l = i / kPackLayer, r = i % kPackLayer;
+        if (l < 3) out[l * kPackLayer + core_off(r / 128, r % 128, 64 * 16) / 2] = __float2bfloat16(P[rm::layer_w(l + 1) + r]);
+        else out[l * kPackLayer + core_off(r / 64, r % 64, 32 * 16) / 2] = __float2bfloat16(P[rm::WZ + r]);
     }
 }
 
@@ -127,234 +140,330 @@ __global__ void __launch_bounds__(kLongThreads) long_row_sums(const int* xadj, c
     }
 }
 
-template <bool AGG, int NOUT, bool RELU>
-__global__ void __launch_bounds__(kTcThreads) fused_layer_tc(int n, const int* xadj, const int* adjncy,
-                                                             const int* adjwgt, const float* wdeg,
-                                                             const __nv_bfloat16* h, const __nv_bfloat16* wpk,
-                                                             const float* P, int boff, __nv_bfloat16* out,
-                                                             const int* hrank, const float* hagg, int* err) {
-    constexpr int K = AGG ? 128 : 64;
-    constexpr uint32_t A_BYTES = kTile * K * 2, B_BYTES = NOUT * K * 2;
-    constexpr uint32_t LBO_A = kTile * 16, LBO_B = NOUT * 16, SBO = 128;
+// One layer's tile product: D (kTile x NOUT, TMEM) = A B^T, K columns of A,
+// committed to the mbarrier.  By one thread.
+template <int K, int NOUT>
+__device__ __forceinline__ void issue_mma(uint32_t tmem, uint32_t sa_addr, uint32_t sb_addr, uint32_t mbar_addr) {
+    constexpr uint32_t LBO_A = kLboA, LBO_B = NOUT * 16, SBO = 128;
+    constexpr uint32_t idesc = instr_desc<NOUT>();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+    for (int kk = 0; kk < K / 16; ++kk) {
+        const uint64_t da = smem_desc(sa_addr + (uint32_t)kk * 2u * LBO_A, LBO_A, SBO);
+        const uint64_t db = smem_desc(sb_addr + (uint32_t)kk * 2u * LBO_B, LBO_B, SBO);
+        const uint32_t acc = kk > 0 ? 1u : 0u;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem),
+            "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+    }
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar_addr)
+                 : "memory");
+}
+
+__device__ __forceinline__ bool try_bar(uint32_t bar, uint32_t phase) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, P;\n\t}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(phase)
+        : "memory");
+    return done != 0;
+}
+__device__ __forceinline__ bool poll_bar(uint32_t bar, uint32_t phase) {
+    for (int it = 0; it < kWaitLimit; ++it)
+        if (try_bar(bar, phase)) return true;
+    return false;
+}
+
+// Bounded wait of a whole warp for the phase; false: it did not complete, here
+// or in another warp of the CTA (dead), and the CTA is to leave.
+__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t phase, volatile int* dead, int* err) {
+    bool ok = false;
+    for (int it = 0; it < kWaitLimit; ++it) {
+        ok = try_bar(bar, phase);
+        if (ok || ((it & 255) == 255 && *dead)) break;
+    }
+    if (!ok) {
+        *dead = 1;
+        atomicExch(err, 1);
+    }
+    return __all_sync(0xffffffffu, ok);
+}
+
+__device__ __forceinline__ void arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// Barrier of the reading warps; true if ok is in all of them.
+__device__ __forceinline__ bool read_sync(bool ok) {
+    int all;
+    asm volatile(
+        "{\n\t.reg .pred P, Q;\n\t"
+        "setp.ne.s32 P, %1, 0;\n\t"
+        "barrier.cta.red.and.pred Q, 1, %2, P;\n\t"
+        "selp.s32 %0, 1, 0, Q;\n\t}\n"
+        : "=r"(all)
+        : "r"((int)ok), "n"(kReadWarps * 32)
+        : "memory");
+    return all != 0;
+}
+
+// 16 accumulator columns of the warp's 32 TMEM lanes plus bias, rounded.
+template <bool RELU>
+__device__ __forceinline__ void read_columns(uint32_t taddr, const float* bias, uint4 (&out)[2]) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+        "%12, %13, %14, %15}, [%16];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(out);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        float y0 = __uint_as_float(r[2 * q]) + bias[2 * q];
+        float y1 = __uint_as_float(r[2 * q + 1]) + bias[2 * q + 1];
+        if (RELU) {
+            y0 = fmaxf(y0, 0.f);
+            y1 = fmaxf(y1, 0.f);
+        }
+        o[q] = __floats2bfloat162_rn(y0, y1);
+    }
+}
+
+// The gathering warps' part of a layer: rows of the CTA's tiles, four of a
+// warp at a time (one per group of 8 lanes), dealt to the warps in turn.  Lane
+// j of a group owns features 8j .. 8j+7 (16 bytes of a row) and keeps four
+// neighbour rows in flight; the next four entries' targets and weights, or
+// the next row's first, are loaded behind them.
+__device__ __forceinline__ void gather_rows(int n, const int* __restrict__ xadj, const int* __restrict__ adjncy,
+                                            const int* __restrict__ adjwgt, const float* __restrict__ wdeg,
+                                            const __nv_bfloat16* __restrict__ h, const int* hrank, const float* hagg,
+                                            int t0, int mine, unsigned char* smem, uint32_t full, uint32_t free_,
+                                            volatile int* dead, int* err) {
+    constexpr int kQuads = kTile / 4, kWarps = kTcThreads / 32 - kReadWarps;
+    const int lane = threadIdx.x & 31, grp = lane >> 3, j = lane & 7;
+    const uint4* hj = reinterpret_cast<const uint4*>(h) + j;
+    const long long v0 = (long long)t0 * kTile + grp;
+    const int quads = mine * kQuads;
+    int q = (threadIdx.x >> 5) - kReadWarps;
+    auto row = [&](int quad, int& beg, int& end) {
+        const long long v = v0 + 4ll * quad;
+        beg = end = 0;
+        if (quad < quads && v < n) {
+            beg = xadj[v];
+            end = xadj[v + 1];
+        }
+    };
+    int beg, end, u[4], w[4];
+    row(q, beg, end);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (beg + k < end) { u[k] = adjncy[beg + k]; w[k] = adjwgt[beg + k]; }
+    for (; q < quads; q += kWarps) {
+        const long long v = v0 + 4ll * q;
+        const bool in = v < n;
+        int nbeg, nend;
+        row(q + kWarps, nbeg, nend);
+        const uint4 x = in ? hj[v * 8] : make_uint4(0u, 0u, 0u, 0u);
+        const float d = in ? wdeg[v] : 0.f;
+        // packed FP32 pairs: features 2i, 2i + 1
+        f32x2 a2[4] = {0ull, 0ull, 0ull, 0ull};
+        auto add = [&](const uint4& hu, float wk) {
+            const f32x2 w2 = pack2(wk, wk);
+            const uint32_t b[4] = {hu.x, hu.y, hu.z, hu.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                a2[i] = fma2(w2, pack2(__uint_as_float(b[i] << 16), __uint_as_float(b[i] & 0xffff0000u)), a2[i]);
+        };
+        const bool long_row = end - beg > kLongRow;
+        if (long_row) {
+            // its weighted sum was formed by long_row_sums
+            const float* src = hagg + (size_t)hrank[v] * rm::H + 8 * j;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a2[i] = pack2(src[2 * i], src[2 * i + 1]);
+        }
+        int e = long_row ? end : beg;
+        for (; e + 4 <= end; e += 4) {
+            uint4 hu[4];
+            float wk[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) { hu[k] = hj[(long long)u[k] * 8]; wk[k] = (float)w[k]; }
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (e + 4 + k < end) { u[k] = adjncy[e + 4 + k]; w[k] = adjwgt[e + 4 + k]; }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) add(hu[k], wk[k]);
+        }
+        uint4 hu[3];
+        float wk[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (e + k < end) { hu[k] = hj[(long long)u[k] * 8]; wk[k] = (float)w[k]; }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (nbeg + k < nend) { u[k] = adjncy[nbeg + k]; w[k] = adjwgt[nbeg + k]; }
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (e + k < end) add(hu[k], wk[k]);
+        const float inv = d > 0.f ? 1.0f / d : 0.f;
+        uint4 a;
+        __nv_bfloat162* pa = reinterpret_cast<__nv_bfloat162*>(&a);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float lo, hi;
+            unpack2(a2[i], lo, hi);
+            pa[i] = __floats2bfloat162_rn(lo * inv, hi * inv);
+        }
+        __syncwarp();
+        const int i = q / kQuads, s = i % kStages;
+        if (i >= kStages && !wait_bar(free_ + 8 * s, (i / kStages - 1) & 1, dead, err)) break;
+        unsigned char* sa = smem + (size_t)s * 16 * kLboA;
+        const int r = (q % kQuads) * 4 + grp;
+        *reinterpret_cast<uint4*>(sa + core_off(r, 8 * j, kLboA)) = x;
+        *reinterpret_cast<uint4*>(sa + core_off(r, 64 + 8 * j, kLboA)) = a;
+        // generic-proxy writes -> visible to the tensor core (async proxy)
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) arrive(full + 8 * s);
+        beg = nbeg;
+        end = nend;
+    }
+}
+
+// Layer l of the network; LAST: layer 3 and z.  wpk: the layer's weights,
+// with those of Wz behind them in the last.
+template <bool LAST>
+__global__ void __launch_bounds__(kTcThreads, 1)
+    fused_layer_tc(int n, const int* xadj, const int* adjncy, const int* adjwgt, const float* wdeg,
+                   const __nv_bfloat16* h, const __nv_bfloat16* wpk, const float* P, int boff, __nv_bfloat16* out,
+                   const int* hrank, const float* hagg, int* err) {
+    constexpr uint32_t A_BYTES = 16 * kLboA, B_BYTES = (kPackLayer + (LAST ? rm::Z * rm::H : 0)) * 2;
     extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char* sa = smem;
-    unsigned char* sb = smem + A_BYTES;
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + A_BYTES + B_BYTES);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 1);
-    float* bias = reinterpret_cast<float*>(tslot + 4);
+    unsigned char* sb = smem + kStages * A_BYTES;
+    uint64_t* mbar = reinterpret_cast<uint64_t*>(sb + B_BYTES);  // full[kStages], free[kStages], done
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 2 * kStages + 1);
+    volatile int* dead = reinterpret_cast<volatile int*>(tslot + 1);
+    float* bias = reinterpret_cast<float*>(tslot + 2);  // 64, LAST: and 32 of z
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
     // B operand and bias, once per CTA
     for (uint32_t i = tid * 16; i < B_BYTES; i += kTcThreads * 16)
         *reinterpret_cast<uint4*>(sb + i) = *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(wpk) + i);
-    for (int j = tid; j < NOUT; j += kTcThreads) bias[j] = __bfloat162float(__float2bfloat16(P[boff + j]));
+    for (int j = tid; j < rm::H + (LAST ? rm::Z : 0); j += kTcThreads)
+        bias[j] = __bfloat162float(__float2bfloat16(P[j < rm::H ? boff + j : rm::BZ + j - rm::H]));
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar)));
+        *dead = 0;
+        for (int i = 0; i < kStages; ++i) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(mbar + i)), "r"(kTile / 4));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar + kStages + i)));
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar + 2 * kStages)));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
-                     "r"((uint32_t)NOUT));
+                     "r"((uint32_t)rm::H));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // B
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tslot;
-    const uint32_t sa_addr = smem_u32(sa), sb_addr = smem_u32(sb), mbar_addr = smem_u32(mbar);
+    const uint32_t full = smem_u32(mbar), free_ = smem_u32(mbar + kStages), done = smem_u32(mbar + 2 * kStages);
 
-    uint32_t phase = 0;
-    bool ok = true;
-    const long long tiles = ((long long)n + kTile - 1) / kTile;
-    for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-        // 1. gather the A tile: warp w fills kGatherRows rows, four rows at
-        // a time (one per group of 8 lanes); lane j of a group owns features
-        // 8j .. 8j+7 (16 bytes of a row) and keeps four neighbour rows in
-        // flight
-        {
-            const int grp = lane >> 3, j = lane & 7;
-            for (int r = warp * kGatherRows + grp; r < (warp + 1) * kGatherRows; r += 4) {
-                const long long v = t * kTile + r;
-                float x[8], acc[8];
+    // the CTA's tiles are consecutive; what was gathered for one serves the next
+    const int tiles = (n + kTile - 1) / kTile, share = (tiles + gridDim.x - 1) / gridDim.x;
+    const int t0 = min(tiles, (int)blockIdx.x * share), mine = min(tiles, t0 + share) - t0;
+    if (warp >= kReadWarps) {
+        gather_rows(n, xadj, adjncy, adjwgt, wdeg, h, hrank, hagg, t0, mine, smem, full, free_, dead, err);
+    } else {
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int i = 0; i < mine && ok; ++i) {
+            const int s = i % kStages;
+            unsigned char* sa = smem + (size_t)s * A_BYTES;
+            if (warp == 0) {
+                // all lanes wait, one issues
+                ok = wait_bar(full + 8 * s, (i / kStages) & 1, dead, err);
+                if (ok && lane == 0) issue_mma<128, rm::H>(tmem, smem_u32(sa), smem_u32(sb), done);
+                __syncwarp();
+            }
+            ok = ok && wait_bar(done, phase, dead, err);
+            phase ^= 1u;
+            if (!LAST && tid == 0) arrive(free_ + 8 * s);  // the operand has been used
+            // warp w reads TMEM lanes 32 w .. +31, its rows
+            const long long v = (long long)(t0 + i) * kTile + tid;
+            if (ok) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-                for (int q = 0; q < 8; ++q) { x[q] = 0.f; acc[q] = 0.f; }
-                if (v < n) {
-                    const uint4 hv = reinterpret_cast<const uint4*>(h + v * rm::H)[j];
-                    const __nv_bfloat162* hp = reinterpret_cast<const __nv_bfloat162*>(&hv);
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) { x[2 * q] = __low2float(hp[q]); x[2 * q + 1] = __high2float(hp[q]); }
-                    if (AGG && end_of(xadj, v) - xadj[v] > kLongRow) {
-                        // long row: its weighted sum was formed by long_row_sums
-                        const float* src = hagg + (size_t)hrank[v] * rm::H + 8 * j;
-                        const float d = wdeg[v];
-                        const float inv = d > 0.f ? 1.0f / d : 0.f;
-#pragma unroll
-                        for (int q = 0; q < 8; ++q) acc[q] = src[q] * inv;
-                    } else if (AGG) {
-                        const int beg = xadj[v], end = xadj[v + 1];
-                        int e = beg;
-                        for (; e + 4 <= end; e += 4) {
-                            int u[4];
-                            float w[4];
-                            uint4 hu[4];
-#pragma unroll
-                            for (int k = 0; k < 4; ++k) { u[k] = adjncy[e + k]; w[k] = (float)adjwgt[e + k]; }
-#pragma unroll
-                            for (int k = 0; k < 4; ++k) hu[k] = reinterpret_cast<const uint4*>(h + (long long)u[k] * rm::H)[j];
-#pragma unroll
-                            for (int k = 0; k < 4; ++k) {
-                                const __nv_bfloat162* p2 = reinterpret_cast<const __nv_bfloat162*>(&hu[k]);
-#pragma unroll
-                                for (int q = 0; q < 4; ++q) {
-                                    acc[2 * q] += w[k] * __low2float(p2[q]);
-                                    acc[2 * q + 1] += w[k] * __high2float(p2[q]);
-                                }
-                            }
-                        }
-                        for (; e < end; ++e) {
-                            const float w = (float)adjwgt[e];
-                            const uint4 hu = reinterpret_cast<const uint4*>(h + (long long)adjncy[e] * rm::H)[j];
-                            const __nv_bfloat162* p2 = reinterpret_cast<const __nv_bfloat162*>(&hu);
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                acc[2 * q] += w * __low2float(p2[q]);
-                                acc[2 * q + 1] += w * __high2float(p2[q]);
-                            }
-                        }
-                        const float d = wdeg[v];
-                        const float inv = d > 0.f ? 1.0f / d : 0.f;
-#pragma unroll
-                        for (int q = 0; q < 8; ++q) acc[q] *= inv;
+                for (int c0 = 0; c0 < rm::H; c0 += 16) {
+                    uint4 y[2];
+                    read_columns<true>(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, bias + c0, y);
+                    if (LAST) {
+                        *reinterpret_cast<uint4*>(sa + core_off(tid, c0, kLboA)) = y[0];
+                        *reinterpret_cast<uint4*>(sa + core_off(tid, c0 + 8, kLboA)) = y[1];
+                    } else if (v < n) {
+                        uint4* dst = reinterpret_cast<uint4*>(out + v * rm::H + c0);
+                        dst[0] = y[0];
+                        dst[1] = y[1];
                     }
                 }
-                uint4 ox, oa;
-                __nv_bfloat162* px = reinterpret_cast<__nv_bfloat162*>(&ox);
-                __nv_bfloat162* pa = reinterpret_cast<__nv_bfloat162*>(&oa);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    px[q] = __floats2bfloat162_rn(x[2 * q], x[2 * q + 1]);
-                    pa[q] = __floats2bfloat162_rn(acc[2 * q], acc[2 * q + 1]);
-                }
-                *reinterpret_cast<uint4*>(sa + core_off(r, 8 * j, kTile)) = ox;
-                if (AGG) *reinterpret_cast<uint4*>(sa + core_off(r, 64 + 8 * j, kTile)) = oa;
             }
-        }
-        // generic-proxy smem writes -> visible to the tensor core (async proxy)
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        // 2. one thread issues the MMAs and commits them to the mbarrier
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            constexpr uint32_t idesc = instr_desc<NOUT>();
+            if (LAST) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                ok = read_sync(ok);
+                if (ok && tid == 0) issue_mma<64, rm::Z>(tmem, smem_u32(sa), smem_u32(sb) + kPackLayer * 2, done);
+                ok = ok && wait_bar(done, phase, dead, err);
+                phase ^= 1u;
+                if (tid == 0) arrive(free_ + 8 * s);
+                if (ok) {
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-            for (int kk = 0; kk < K / 16; ++kk) {
-                const uint64_t da = smem_desc(sa_addr + (uint32_t)kk * 2u * LBO_A, LBO_A, SBO);
-                const uint64_t db = smem_desc(sb_addr + (uint32_t)kk * 2u * LBO_B, LBO_B, SBO);
-                const uint32_t acc = kk > 0 ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "setp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem),
-                    "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                mbar_addr)
-                         : "memory");
-        }
-        // 3. wait for the accumulator (bounded)
-        {
-            uint32_t done = 0;
-            for (long long it = 0; it < kWaitLimit && !done; ++it) {
-                asm volatile(
-                    "{\n\t.reg .pred P;\n\t"
-                    "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
-                    "selp.u32 %0, 1, 0, P;\n\t}\n"
-                    : "=r"(done)
-                    : "r"(mbar_addr), "r"(phase)
-                    : "memory");
-            }
-            if (!done) {
-                ok = false;
-                if (lane == 0) atomicExch(err, 1);
-            }
-        }
-        phase ^= 1u;
-        if (!__all_sync(0xffffffffu, ok)) ok = false;
-        if (ok) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // warp w reads TMEM lanes 32 (w % 4) .. +31 (its rows) and the
-            // (w / 4)-th half of the columns
-            const int lanes = (warp & 3) * 32;
-            const long long v = t * kTile + lanes + lane;
-#pragma unroll
-            for (int c0 = (warp >> 2) * (NOUT / 2); c0 < (warp >> 2) * (NOUT / 2) + NOUT / 2; c0 += 16) {
-                uint32_t r[16];
-                const uint32_t taddr = tmem + ((uint32_t)lanes << 16) + (uint32_t)c0;
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
-                    "%12, %13, %14, %15}, [%16];\n"
-                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                      "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-                      "=r"(r[14]), "=r"(r[15])
-                    : "r"(taddr));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (v < n) {
-                    __nv_bfloat162 o[8];
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        float y0 = __uint_as_float(r[2 * q]) + bias[c0 + 2 * q];
-                        float y1 = __uint_as_float(r[2 * q + 1]) + bias[c0 + 2 * q + 1];
-                        if (RELU) {
-                            y0 = fmaxf(y0, 0.f);
-                            y1 = fmaxf(y1, 0.f);
+                    for (int c0 = 0; c0 < rm::Z; c0 += 16) {
+                        uint4 y[2];
+                        read_columns<false>(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, bias + rm::H + c0, y);
+                        if (v < n) {
+                            uint4* dst = reinterpret_cast<uint4*>(out + v * rm::Z + c0);
+                            dst[0] = y[0];
+                            dst[1] = y[1];
                         }
-                        o[q] = __floats2bfloat162_rn(y0, y1);
                     }
-                    uint4* dst = reinterpret_cast<uint4*>(out + v * NOUT + c0);
-                    dst[0] = *reinterpret_cast<uint4*>(&o[0]);
-                    dst[1] = *reinterpret_cast<uint4*>(&o[4]);
                 }
             }
+            // the accumulator has been read
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            ok = read_sync(ok);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        ok = ok && !(*reinterpret_cast<volatile int*>(err));
+        // a timed-out MMA may still be in flight: one more bounded wait
+        if (!ok) poll_bar(done, phase ^ 1u);
     }
-    // a timed-out MMA may still be in flight: give it one more bounded wait
-    if (!ok) {
-        uint32_t done = 0;
-        for (long long it = 0; it < kWaitLimit && !done; ++it) {
-            asm volatile(
-                "{\n\t.reg .pred P;\n\t"
-                "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
-                "selp.u32 %0, 1, 0, P;\n\t}\n"
-                : "=r"(done)
-                : "r"(mbar_addr), "r"(phase ^ 1u)
-                : "memory");
-        }
-    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)NOUT));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)rm::H));
 }
 
-template <bool AGG, int NOUT, bool RELU>
-void launch_fused(Ctx& ctx, const DevGraph& g, const float* wdeg, const __nv_bfloat16* h,
-                  const __nv_bfloat16* wpk, const float* P, int boff, __nv_bfloat16* out, const int* hrank,
-                  const float* hagg, int* err) {
-    constexpr int K = AGG ? 128 : 64;
-    const size_t smem = (size_t)kTile * K * 2 + (size_t)NOUT * K * 2 + 64 + NOUT * sizeof(float);
-    KB_CUDA(cudaFuncSetAttribute(fused_layer_tc<AGG, NOUT, RELU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
+template <bool LAST>
+void launch_fused(Ctx& ctx, const DevGraph& g, const float* wdeg, const __nv_bfloat16* h, const __nv_bfloat16* wpk,
+                  const float* P, int layer, __nv_bfloat16* out, const int* hrank, const float* hagg, int* err) {
+    const size_t smem = (size_t)kStages * 16 * kLboA + (size_t)(kPackLayer + rm::Z * rm::H) * 2 +
+                        (2 * kStages + 1) * 8 + 8 + (rm::H + rm::Z) * sizeof(float);
+    KB_CUDA(cudaFuncSetAttribute(fused_layer_tc<LAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const long long tiles = ((long long)g.n + kTile - 1) / kTile;
-    // ~48 KB of shared memory per CTA: four CTAs per SM
-    const int grid = (int)std::max<long long>(1, std::min<long long>(tiles, 4LL * kNumSMs));
-    fused_layer_tc<AGG, NOUT, RELU><<<grid, kTcThreads, smem, ctx.stream>>>(g.n, g.xadj, g.adjncy, g.adjwgt, wdeg,
-                                                                             h, wpk, P, boff, out, hrank, hagg,
-                                                                             err);
+    const int grid = (int)std::max<long long>(1, std::min<long long>(tiles, (long long)kNumSMs));
+    fused_layer_tc<LAST><<<grid, kTcThreads, smem, ctx.stream>>>(g.n, g.xadj, g.adjncy, g.adjwgt, wdeg, h, wpk, P,
+                                                                 rm::layer_b(layer), out, hrank, hagg, err);
     KB_LAUNCH();
 }
 
@@ -368,9 +477,7 @@ void rating_infer_tc(Ctx& ctx, const DevGraph& g, const float* P, float* prob, u
     __nv_bfloat16* ha = ctx.scratch.alloc<__nv_bfloat16>(nn * rm::H);
     __nv_bfloat16* hb = ctx.scratch.alloc<__nv_bfloat16>(nn * rm::H);
     __nv_bfloat16* z = ctx.scratch.alloc<__nv_bfloat16>(nn * rm::Z);
-    __nv_bfloat16* wl[3];
-    for (auto& p : wl) p = ctx.scratch.alloc<__nv_bfloat16>((size_t)rm::H * 2 * rm::H);
-    __nv_bfloat16* wz = ctx.scratch.alloc<__nv_bfloat16>((size_t)rm::Z * rm::H);
+    __nv_bfloat16* wpk = ctx.scratch.alloc<__nv_bfloat16>((size_t)kPackAll);
     int* err = ctx.dscalars + 60;
     // long rows (more than kLongRow entries): at most m / (kLongRow + 1) of them
     const long long lmax = g.m / (kLongRow + 1) + 1;
@@ -387,11 +494,7 @@ void rating_infer_tc(Ctx& ctx, const DevGraph& g, const float* P, float* prob, u
                                                                                              hlist, hcount);
             KB_LAUNCH();
         }
-        for (int l = 1; l <= 3; ++l) {
-            pack_weights<128, 64><<<32, 256, 0, s>>>(P, rm::layer_w(l), wl[l - 1]);
-            KB_LAUNCH();
-        }
-        pack_weights<64, 32><<<8, 256, 0, s>>>(P, rm::WZ, wz);
+        pack_weights<<<div_up(kPackAll, 256), 256, 0, s>>>(P, wpk);
         KB_LAUNCH();
         launch_layer0_bf16(ctx, g, P, wdeg, ha);
         __nv_bfloat16* cur = ha;
@@ -402,10 +505,11 @@ void rating_infer_tc(Ctx& ctx, const DevGraph& g, const float* P, float* prob, u
                     g.xadj, g.adjncy, g.adjwgt, cur, hlist, hcount, hagg);
                 KB_LAUNCH();
             }
-            launch_fused<true, 64, true>(ctx, g, wdeg, cur, wl[l - 1], P, rm::layer_b(l), nxt, hrank, hagg, err);
+            const __nv_bfloat16* w = wpk + (l - 1) * kPackLayer;
+            if (l < 3) launch_fused<false>(ctx, g, wdeg, cur, w, P, l, nxt, hrank, hagg, err);
+            else launch_fused<true>(ctx, g, wdeg, cur, w, P, l, z, hrank, hagg, err);
             std::swap(cur, nxt);
         }
-        launch_fused<false, 32, false>(ctx, g, wdeg, cur, wz, P, rm::BZ, z, hrank, hagg, err);
     }
     PhaseScope ps(ctx, "rating_head", 0);
     launch_head_bf16(ctx, g, P, z, prob, rating);

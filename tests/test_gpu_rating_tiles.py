@@ -65,3 +65,25 @@ def test_no_edges(N):
     g = csr_from_edges(70, [])
     grad, loss = N.rating_grad(g, np.zeros(0, np.uint8), random_params(1))
     assert loss == 0.0 and not grad.any()
+
+
+@pytest.mark.parametrize("n,hub", [(1, 0), (2, 1), (127, 3), (128, 126), (129, 128), (1100, 1024), (1100, 1025),
+                                   (128 * 148 + 1, 40), (128 * 148 * 4 + 5, 1500)])
+def test_tensor_core_forward(N, n, hub):
+    """Part tiles, one to five tiles a CTA (three are gathered ahead), nodes
+    without edges, rows at the limit of the separate sums."""
+    import torch
+    g = graph(n, hub, n + 1)
+    pad = 5  # isolated nodes at the end
+    g = dict(g, n=n + pad, xadj=np.concatenate([g["xadj"], np.full(pad, g["xadj"][-1], g["xadj"].dtype)]),
+             vwgt=np.concatenate([g["vwgt"], np.arange(pad, dtype=np.int32)]))
+    P = random_params(n + 7)
+    prob, rating = N.rating_infer(g, P, use_tc=True)
+    if g["m"] == 0:
+        assert prob.size == 0
+        return
+    s, _ = torch_forward(g, P)
+    ref = torch.sigmoid(s).detach().numpy()
+    assert np.abs(prob - ref).max() < 5e-2 and np.abs(prob - ref).mean() < 2e-3
+    q = np.clip(np.floor((1.0 - prob) * np.float32(16777216.0)), 0, 16777215)
+    assert np.array_equal(rating, q.astype(np.uint32))
