@@ -37,10 +37,10 @@ __global__ void __launch_bounds__(kThreads, 4) lane_kernel(SweepArgs a) {
 }
 
 template <int MODE, int BT>
-__global__ void __launch_bounds__(BT) heavy_kernel(SweepArgs a, uint32_t* gtk, uint32_t* gtv, int gcap, int which,
+__global__ void __launch_bounds__(BT) heavy_kernel(SweepArgs a, uint32_t* gtk, uint32_t* gtv, int gcap, int long_rows,
                                                    int stab) {
     extern __shared__ uint32_t htab[];
-    heavy_sweep<MODE, BT>(a, gtk, gtv, gcap, which, stab, htab);
+    heavy_sweep<MODE, BT>(a, gtk, gtv, gcap, long_rows != 0, stab, htab);
 }
 
 // ---------------------------------------------------------------- admission
@@ -226,7 +226,8 @@ __global__ void block_scan_kernel(const uint32_t* bw, int k, uint32_t bound, int
 
 // ------------------------------------------------------------- host helpers
 
-constexpr int kCntHeavy = 2 * kStripes, kCntHeavyProp = 2 * kStripes + 1, kCntMoved = 2 * kStripes + 2;
+constexpr int kCntHeavy = 2 * kStripes, kCntHeavyProp = 2 * kStripes + 1, kCntHuge = 2 * kStripes + 2,
+              kCntMoved = 2 * kStripes + 3;
 
 int admit_blocks() { return (kStripes + 1) * 4; }
 
@@ -359,10 +360,10 @@ void launch_sweep(Ctx& ctx, const DevGraph& g, SweepArgs a, const SweepBuffers& 
             // rows that fit the shared tables on many blocks, the longest
             // rows on the blocks that own a global table
             heavy_kernel<MODE, kThreads><<<8 * kNumSMs, kThreads, 8 * kSmemTab, ctx.stream>>>(a, nullptr, nullptr,
-                                                                                              b.gcap, 1, kSmemTab);
+                                                                                              b.gcap, 0, kSmemTab);
             KB_LAUNCH();
             const int tab = big_tab_ok<MODE>() ? kBigTab : kSmemTab;
-            heavy_kernel<MODE, 1024><<<b.hblocks, 1024, 8 * tab, ctx.stream>>>(a, b.gtk, b.gtv, b.gcap, 2, tab);
+            heavy_kernel<MODE, 1024><<<b.hblocks, 1024, 8 * tab, ctx.stream>>>(a, b.gtk, b.gtv, b.gcap, 1, tab);
             KB_LAUNCH();
         }
     }
@@ -380,6 +381,7 @@ SweepArgs sweep::base_args(const DevGraph& g, const SweepBuffers& b) {
     a.pt = b.pt;
     a.pc = b.pc;
     a.hcount = b.counters + kCntHeavy;
+    a.hugecount = b.counters + kCntHuge;
     a.heavy = b.heavy;
     a.plist = b.plist;
     a.hplist = b.hplist;

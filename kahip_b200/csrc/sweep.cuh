@@ -65,7 +65,7 @@ struct SweepArgs {
     uint32_t* H;                        // REFINE/BALANCE: weight per (target, class)
     int* minvP;                         // smallest proposer per (target, class)
     int* heavy; unsigned* hcount;       // deferred high-degree vertices
-    unsigned* hugecount;                // a team: those listed from heavy's end
+    unsigned* hugecount;                // those of them listed from heavy's end
     // a team: the level's long rows, when they are listed; the proposals, a
     // list of (vertex, target) of capacity tcap per warp with its length in
     // shared memory
@@ -131,6 +131,12 @@ template <int MODE>
 __device__ __forceinline__ bool cand_ok(const SweepArgs& a, uint32_t b, uint32_t c, uint32_t cv) {
     if (MODE == BALANCE) return (uint64_t)a.lw[b] + cv <= a.bound;
     return c > 0 && (uint64_t)a.lw[b] + cv < a.bound;
+}
+// As cand_ok, with the label's weight w at hand.
+template <int MODE>
+__device__ __forceinline__ bool fits(const SweepArgs& a, uint32_t w, uint32_t c, uint32_t cv) {
+    if (MODE == BALANCE) return (uint64_t)w + cv <= a.bound;
+    return c > 0 && (uint64_t)w + cv < a.bound;
 }
 
 __device__ __forceinline__ int loss_bucket(long long loss) {
@@ -243,6 +249,7 @@ __device__ __forceinline__ bool member(const SweepArgs& a, int v) {
 
 // ------------------------------------------------ chunk-cooperative path
 
+constexpr int kSmemTab = 4096;            // table slots of a block with a row above kWin
 constexpr int kWin = 128;                 // edges per window (<= 4 batches)
 constexpr int kBatches = kWin / 32;
 constexpr int kTab = 2 * kWin;            // table slots per warp (load <= 1/2)
@@ -294,7 +301,8 @@ __device__ __forceinline__ void chunk_process(const SweepArgs& a, WarpTable& T, 
         beg = a.xadj[v];
         deg = a.xadj[v + 1] - beg;
         if (deg > kWin) {  // high degree: block-per-vertex kernel decides it
-            a.heavy[atomicAdd(a.hcount, 1u)] = v;
+            if (deg > kSmemTab / 2) a.heavy[a.n - 1 - (int)atomicAdd(a.hugecount, 1u)] = v;
+            else a.heavy[atomicAdd(a.hcount, 1u)] = v;
             deg = 0;
             heavy = true;
         } else {
@@ -722,7 +730,7 @@ __device__ __forceinline__ void lane_sweep(const SweepArgs& a, SweepQueue& queue
         if (status == 1) oq[oqn + __popc(om & lanemask_lt())] = v;
         oqn += __popc(om);
         __syncwarp();
-        append_aggregated(status == 2, v, a.heavy, a.hcount);
+        defer_row<kSmemTab / 2>(a, status == 2, v);
         append_striped(status == 3, v, a.plist);
         if (oqn >= 32) overflow_pass();
     };
@@ -769,7 +777,6 @@ __device__ __forceinline__ void lane_sweep(const SweepArgs& a, SweepQueue& queue
 // longer rows, in the block's global-memory table of `gcap` slots
 // (gcap >= 2 * maxdeg, power of two; gtk may be null when every row fits
 // the shared table).
-constexpr int kSmemTab = 4096;
 
 // Linear probing that looks before it swaps (most entries find their label
 // there).  The caller guarantees at most cap / 2 distinct keys, so the probe
@@ -790,6 +797,39 @@ __device__ __forceinline__ void table_add(uint32_t* tk, uint32_t* tv, int cap, u
         s = (s + 1) & (uint32_t)(cap - 1);
     }
     atomicOr(err, 1);
+}
+
+// The best candidate among the first cap slots of a table by the threads t of
+// NT, which leave it empty; most: the largest connection.  U slots a thread are
+// in flight, and a target's weight is read only for a connection that is not
+// below the best so far: one slot at a time, the chain of reads (label,
+// connection, target weight) was a fifth of the longest rows' time (R-MAT 2^20:
+// 0.52 -> 0.41 ms a sub-round).
+template <int MODE, int U>
+__device__ __forceinline__ void scan_table(const SweepArgs& a, uint32_t* tk, uint32_t* tv, int cap, int t, int NT,
+                                           uint32_t cv, uint64_t& key, uint32_t& id, uint32_t& most) {
+    for (int s = t; s < cap; s += U * NT) {
+        uint32_t l[U], c[U], w[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) l[q] = s + q * NT < cap ? tk[s + q * NT] : kEmpty;
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            c[q] = 0;
+            if (l[q] == kEmpty) continue;
+            c[q] = tv[s + q * NT];
+            tk[s + q * NT] = kEmpty;
+            tv[s + q * NT] = 0;
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            if (l[q] != kEmpty && c[q] < (uint32_t)(key >> 32)) l[q] = kEmpty;
+            most = max(most, c[q]);
+            w[q] = l[q] != kEmpty ? a.lw[l[q]] : 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            if (l[q] != kEmpty && fits<MODE>(a, w[q], c[q], cv)) better(key, id, cand_key(c[q], a.ks_tie, l[q]), l[q]);
+    }
 }
 
 template <int BT>
@@ -828,15 +868,8 @@ __device__ __forceinline__ void heavy_vertex(const SweepArgs& a, int v, uint32_t
     }
     __syncthreads();
     uint64_t key = 0;
-    uint32_t id = kEmpty;
-    for (int s = threadIdx.x; s < cap; s += BT) {
-        const uint32_t l = tk[s];
-        if (l == kEmpty) continue;
-        const uint32_t c = tv[s];
-        tk[s] = kEmpty;
-        tv[s] = 0;
-        if (cand_ok<MODE>(a, l, c, cv)) better(key, id, cand_key(c, a.ks_tie, l), l);
-    }
+    uint32_t id = kEmpty, most = 0;
+    scan_table<MODE, 4>(a, tk, tv, cap, (int)threadIdx.x, BT, cv, key, id, most);
     group_argmax<32>(key, id, 0xffffffffu);
     co = __reduce_add_sync(0xffffffffu, co);
     if (lane == 0) {
@@ -871,16 +904,18 @@ __device__ __forceinline__ int heavy_cap(int deg, int most) {
     return cap;
 }
 
-// The listed vertices, a block each.  `which`: 0 = every one, 1 = only those
-// whose table fits in shared memory, 2 = only the others (the two kinds can
-// run as separate launches with different grids; the decisions do not depend
-// on the order).  The shared-memory table htab (stab slots, a power of two,
-// keys then values) has kSmemTab slots in the many-block launches, more in
-// the launch of the longest rows, whose rows up to stab / 2 entries then
-// stay out of the global table.
+// The listed vertices, a block each: those from the list's front, whose tables
+// have at most kSmemTab slots, or (long_rows) those from its end, whose tables
+// lie in shared memory up to stab slots and in the block's global table (gcap
+// slots) above.  The two kinds are separate launches with different grids; the
+// decisions do not depend on the order.  htab: stab keys, then stab values.
+// Two lists: with one, a block of the long rows' launch looked at hundreds of
+// shorter rows for each of its own, two dependent reads each (R-MAT 2^20: with
+// 0.41 ms a sub-round
+// instead of 0.31).
 template <int MODE, int BT>
-__device__ __forceinline__ void heavy_sweep(const SweepArgs& a, uint32_t* gtk, uint32_t* gtv, int gcap, int which,
-                                            int stab, uint32_t* htab) {
+__device__ __forceinline__ void heavy_sweep(const SweepArgs& a, uint32_t* gtk, uint32_t* gtv, int gcap,
+                                            bool long_rows, int stab, uint32_t* htab) {
     __shared__ HeavyRed<BT> red;
     for (int s = threadIdx.x; s < stab; s += BT) {
         htab[s] = kEmpty;
@@ -889,12 +924,11 @@ __device__ __forceinline__ void heavy_sweep(const SweepArgs& a, uint32_t* gtk, u
     __syncthreads();
     uint32_t* gk = gtk ? gtk + (size_t)blockIdx.x * gcap : nullptr;
     uint32_t* gv = gtv ? gtv + (size_t)blockIdx.x * gcap : nullptr;
-    const unsigned count = *a.hcount;
+    const unsigned count = long_rows ? *a.hugecount : *a.hcount;
     unsigned wv = 0, we = 0;  // thread 0's
     for (unsigned i = blockIdx.x; i < count; i += gridDim.x) {
-        const int v = a.heavy[i];
+        const int v = a.heavy[long_rows ? a.n - 1 - (int)i : (int)i];
         const int cap = heavy_cap(a.xadj[v + 1] - a.xadj[v], gcap);
-        if ((which == 1 && cap > kSmemTab) || (which == 2 && cap <= kSmemTab)) continue;
         heavy_vertex<MODE, BT, false>(a, v, cap <= stab ? htab : gk, cap <= stab ? htab + stab : gv, cap, red, wv, we);
     }
     if (wv) {
@@ -938,15 +972,7 @@ __device__ __forceinline__ void hash_vertex(const SweepArgs& a, int v, uint32_t*
     __syncwarp();
     uint64_t key = 0;
     uint32_t id = kEmpty, most = 0;
-    for (int s = lane; s < cap; s += 32) {
-        const uint32_t l = tk[s];
-        if (l == kEmpty) continue;
-        const uint32_t c = tv[s];
-        tk[s] = kEmpty;
-        tv[s] = 0;
-        most = max(most, c);
-        if (cand_ok<MODE>(a, l, c, cv)) better(key, id, cand_key(c, a.ks_tie, l), l);
-    }
+    scan_table<MODE, 4>(a, tk, tv, cap, lane, 32, cv, key, id, most);
     group_argmax<32>(key, id, 0xffffffffu);
     co = __reduce_add_sync(0xffffffffu, co);
     if (MODE == CLUSTER) {
@@ -1486,7 +1512,7 @@ __device__ __forceinline__ bool balance_steps(Team& team, SweepArgs a, const Bal
 struct SweepBuffers {
     int *pt, *pc;
     unsigned* counters;  // [0, kStripes) unused, [kStripes, 2 kStripes) proposals,
-                         // [2 kStripes] heavy, [+1] heavy proposals, [+2] moved
+                         // [2 kStripes] heavy, [+1] heavy proposals, [+2] longest, [+3] moved
     int* heavy;
     int* hplist;
     SList plist;

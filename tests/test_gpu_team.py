@@ -160,6 +160,28 @@ def test_cluster_quiet_rounds(N, O, graphs, n, hub, rounds):
             assert np.array_equal(O.lp_cluster(g, kn_o, 1), N.lp_cluster(g, kn_p, 1))
 
 
+@pytest.mark.parametrize("hubs", [(2048, 2049), (2049,) * 5, (8192, 8193, 129, 2048), (30000, 9000, 2500)])
+def test_cluster_giant_rows(N, O, hubs):
+    """Rows listed from both ends: a block's smaller table, its larger one and
+    the one in global memory."""
+    n = 40000
+    rng = np.random.default_rng(len(hubs))
+    lo = [np.arange(n - 1)] + [np.full(h, c) for c, h in enumerate(hubs)]
+    hi = [np.arange(1, n)] + [rng.choice(np.arange(len(hubs) + 1, n), h, False) for h in hubs]
+    edges = np.unique(np.stack([np.concatenate(lo), np.concatenate(hi)], 1), axis=0)
+    g = csr_from_edges(n, [tuple(map(int, e)) for e in edges])
+    for unit in (True, False):
+        if not unit:
+            weighted(g, 7)
+        kn_o, kn_p = O.knobs(g, 2, 0.03, 1, 1), N.derive_knobs(n, g["vwgt"], 2, 0.03, 1, 1)
+        for level in (0, 2):
+            assert np.array_equal(O.lp_cluster(g, kn_o, level), N.lp_cluster(g, kn_p, level))
+        part = skewed(n, 1100, 5)  # no dense counters: the refinement's tables
+        kn_o, kn_p = O.knobs(g, 1100, 0.03, 1, 0), N.derive_knobs(n, g["vwgt"], 1100, 0.03, 1, 0)
+        assert np.array_equal(O.lp_refine(g, kn_o, part, kn_o.upper_bound, 0),
+                              N.lp_refine(g, kn_p, part, kn_p.upper_bound, 0))
+
+
 def test_cluster_unsorted_rows(N, O, graphs):
     """Rows in no order and a target listed twice: no singleton shortcut."""
     g = graphs.rgg2d(3000, seed=4)
