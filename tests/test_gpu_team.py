@@ -194,6 +194,27 @@ def test_cluster_unsorted_rows(N, O, graphs):
     assert np.array_equal(O.lp_cluster(h, kn_o, 0), N.lp_cluster(h, kn_p, 0))
 
 
+@pytest.mark.parametrize("where", ["first", "last", "middle", "hub", "end"])
+@pytest.mark.parametrize("n", [40, 3000, 40000])
+def test_one_unsorted_row(N, O, where, n):
+    """The check of the rows' order finds a single exchanged pair in any place
+    (a row's target listed twice would otherwise take the singleton shortcut)."""
+    rng = np.random.default_rng(n)
+    edges = {(v, v + 1) for v in range(n - 1)} | {(n // 2, int(u)) for u in rng.integers(0, n, n // 3) if u != n // 2}
+    g = csr_from_edges(n, sorted({(min(e), max(e)) for e in edges}))
+    x, adj, wgt = g["xadj"], g["adjncy"].copy(), g["adjwgt"].copy()
+    v = {"first": 1, "last": n - 2, "middle": n // 3, "hub": n // 2, "end": n // 2}[where]
+    e = x[v + 1] - 2 if where == "end" else x[v] + (x[v + 1] - x[v]) // 2 - 1
+    adj[e + 1], wgt[e + 1] = adj[e], wgt[e] + 2  # the same target twice
+    h = dict(g, adjncy=adj, adjwgt=wgt)
+    kn_o, kn_p = O.knobs(h, 2, 0.03, 1, 0), N.derive_knobs(n, h["vwgt"], 2, 0.03, 1, 0)
+    assert np.array_equal(O.lp_cluster(h, kn_o, 0), N.lp_cluster(h, kn_p, 0))
+    bad = dict(g, adjncy=g["adjncy"].copy())
+    bad["adjncy"][e] = n
+    with pytest.raises(Exception):
+        N.kaffpa_ex(bad["xadj"], bad["adjncy"], 2)
+
+
 def test_teams_side_by_side(N, graphs):
     """Workers share the device: every result is the single call's."""
     gs = [graphs.rgg2d(20000 + 977 * i, seed=i) for i in range(6)] + [graphs.rmat(13, samples=4 << 13, seed=1)]
