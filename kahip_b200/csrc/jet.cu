@@ -14,7 +14,9 @@
 //                neighbours (larger gain, then smaller id) already moved;
 //                kept when >= 0;
 //   jet_apply    moves, block weights (integer atomics: order-free).
-// Then the host repairs the balance if needed (balance()).  The partition
+// Then the balance is repaired if needed.  jet_loop runs the iterations of a
+// level in one kernel; the steps as launches, with the repair called by the
+// host, serve what its tables cannot hold.  The partition
 // an iteration leaves is judged at the start of the next one: jet_choose
 // scans every row anyway, so it also sums the cut of the partition it reads
 // (locked rows included), and the block weights are kept current by

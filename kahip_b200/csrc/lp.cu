@@ -10,12 +10,12 @@
 // ties broken by hash(tie stream, label) then label id; moves are admitted
 // into capacity-limited targets without sorting (see decide kernels).
 //
-// Work distribution: a warp takes 32 consecutive vertex ids, ballots which of
-// them take part in this sub-round, and hands them to groups of G lanes
-// (G = 8/16/32 by average degree).  A group aggregates one vertex's
-// neighbourhood: degree <= G in registers (match_any + redux), degree <=
-// kTable/2 in a per-group shared-memory hash table, larger degrees are
-// deferred to a block-per-vertex kernel with a global-memory table.
+// Work distribution (sweep.cuh): a lane per vertex with its connections in
+// register slots; vertices of more labels by their warp, rows above 128 entries
+// by a block with a hash table.  Where a level and k allow, all steps of a
+// phase are one kernel (cluster_team, refine_team, balance_team); the launches
+// per step serve what is beyond those: clustering of large levels or of rows
+// too long for a block's table, and refinement with k above 1024 and such rows.
 #include "lp.cuh"
 #include "prims.cuh"
 #include "sweep.cuh"
